@@ -22,6 +22,10 @@ TEST_ALL_PATH = os.path.join(LIB_DIR, "test_all")
 SOURCES = [
     "capi_runtime.cu",
     "spmm_kernels.cu",
+    "spmm_shapes_v4.cu",
+    "spmm_shapes_v2.cu",
+    "spmm_shapes_v1.cu",
+    "coo_kernels.cu",
     "sddmm_kernels.cu",
     "structure_kernels.cu",
     "graph_layer.cu",

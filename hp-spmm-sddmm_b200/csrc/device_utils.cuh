@@ -12,9 +12,13 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
   return p;
 }
 
-__device__ __forceinline__ uint64_t policy_evict_first() {
+// The policy of a kernel whose gathers always carry one: evict-last, or the cache's normal treatment.
+__device__ __forceinline__ uint64_t policy_for_gathers(int keep) {
   uint64_t p;
-  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  if (keep)
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  else
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 
@@ -72,6 +76,15 @@ __device__ __forceinline__ void red_add_v4(float* p, float4 v) {
   asm volatile("red.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(v.x), "f"(v.y),
                "f"(v.z), "f"(v.w)
                : "memory");
+}
+
+// Adds to a device-wide counter after everything this thread has written or seen written (by the lanes it has
+// synchronised with) is visible.  A release only: __threadfence, which acquires as well, also drops the SM's L1
+// lines, and with one such fence per piece of a split row the gathers of the whole SM started over cold.
+__device__ __forceinline__ int atomic_add_release(int* p, int v) {
+  int old;
+  asm volatile("atom.release.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
 }
 
 __device__ __forceinline__ void fma4(float4& acc, float a, const float4& b) {

@@ -36,8 +36,8 @@ struct hpspmm_ctx {
 // Chunk table of one sparsity structure.
 //   chunk_start[c]  first nnz of chunk c (n_chunks + 1 entries)
 //   chunk_row[c]    row holding nnz chunk_start[c]
-//   carry_row[c]    row whose partial sum chunk c hands on, or -1
-//   carry_val[c*K..] that partial sum
+//   carry_val[c*K..] partial sum of a row that chunk c hands on
+//   rec             the same per chunk in the order in which warps take them, see hpspmm_spmm_args
 struct hpspmm_plan {
   int device;
   int64_t M, nnz;
@@ -48,16 +48,67 @@ struct hpspmm_plan {
   int32_t* chunk_start;
   int32_t* chunk_row;
   int32_t* chunk_order;  // chunk ids, most rows first: the order in which warps take chunks
-  int32_t* carry_row;
   float* carry_val;
-  int32_t* run_counter;  // one per chunk, zero between launches: pieces of a split row that have finished
+  int32_t* run_counter;  // hpspmm_counter_slabs(max_K) per chunk, zero between launches: pieces of a split row that have finished
   // rows that hold entries: ids (ascending, then the sentinel M), their ends in the entry array, and
   // for every chunk the position in this list of the row holding its first entry
   int32_t* nz_id;
   int32_t* nz_end;
   int32_t* chunk_ri;
+  int2* nz;        // (nz_id, nz_end) as one word per row: what the product kernels step through
+  int4* rec;
   size_t bytes;
 };
+
+// What the CSR product kernels are launched with.
+//   rec, 32 bytes per slot of the schedule: {n0, ri, row, row_end} {chunk, row_start, n1, -}: entries [n0, n1) of the
+//   chunk, the row holding entry n0 with its bounds and its position in the list of rows.  One aligned load gives a
+//   warp all it needs, where chunk_order -> chunk_start / chunk_ri -> nz_id are three dependent ones.
+//   Null for calls whose scratch has no room: the kernel then reads chunk_start / chunk_row in matrix order, and
+//   with nz null it steps from row to row along row_ptr.
+struct hpspmm_spmm_args {
+  int M, K, n_chunks, S;
+  int off, cols;               // columns of this launch: [off, off + cols), in slabs of the shape's width
+  int n_chunk_blocks, slab0;   // filled in by the launcher
+  int keep_b;                  // L2 evict-last on the gathers of B
+  const int32_t* row_ptr;
+  const int32_t* col_idx;
+  const float* vals;
+  const float* B;
+  float* C;
+  const int4* rec;
+  const int2* nz;
+  const int32_t* chunk_start;
+  const int32_t* chunk_row;
+  float* carry;
+  int32_t* counter;
+};
+// Shape of the kernel for `cols` columns: VEC-wide vectors, W lanes and R vectors per lane to a group (warp_frag.cuh).
+struct hpspmm_spmm_shape {
+  int VEC, W, R;
+  bool lat;    // few chunks: columns split over more warps, more gathers in flight per warp
+  bool hint;
+};
+// widest vector the rows of the dense operands keep aligned; addresses: bitwise or of the operands' addresses
+int hpspmm_vector_width(int64_t K, uintptr_t addresses);
+hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, bool hint);
+// Widest slab one shape covers (four vectors per lane, eight of 4 bytes).  A wider product runs as that many full
+// slabs and one launch for the rest, so that only the last vector of a lane can ever lie outside a slab.
+static inline int hpspmm_widest_slab(int VEC) { return VEC == 1 ? 256 : 128 * VEC; }
+static inline int hpspmm_launch_cols(int VEC, int K, int off) {
+  const int widest = hpspmm_widest_slab(VEC), left = K - off;
+  return left < widest ? left : left / widest * widest;
+}
+// triples per warp of the COO product
+int32_t hpspmm_coo_chunk_nnz(int64_t K, int64_t nnz);
+int hpspmm_spmm_launch_v4(hpspmm_ctx* ctx, const hpspmm_spmm_args& a, const hpspmm_spmm_shape& sh, bool shared_counters,
+                          cudaStream_t s);
+int hpspmm_spmm_launch_v2(hpspmm_ctx* ctx, const hpspmm_spmm_args& a, const hpspmm_spmm_shape& sh, bool shared_counters,
+                          cudaStream_t s);
+int hpspmm_spmm_launch_v1(hpspmm_ctx* ctx, const hpspmm_spmm_args& a, const hpspmm_spmm_shape& sh, bool shared_counters,
+                          cudaStream_t s);
+// sets of per-chunk counters a product of up to K columns may need: one per slab, no slab narrower than 32 columns
+static inline int64_t hpspmm_counter_slabs(int64_t K) { return (K + 31) / 32; }
 
 static inline int hpspmm_set_err(hpspmm_ctx* ctx, int status, const char* what, cudaError_t e) {
   if (ctx) snprintf(ctx->err, sizeof(ctx->err), "%s: %s", what, cudaGetErrorString(e));
@@ -123,14 +174,6 @@ int hpspmm_ensure_stage(hpspmm_ctx* ctx, size_t bytes);
 // nominal chunk size for a dense width and a matrix of nnz entries
 int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz);
 
-// Builds chunk_start / chunk_row for (M, nnz, row_ptr) into the given arrays (device).
-// split_count (device int, may be null) receives the number of chunks ending mid-row.
-// run_counter (n_chunks + 1 ints, may be null) is zeroed.
-int hpspmm_launch_chunk_table(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr,
-                              int32_t chunk_nnz, int64_t n_chunks, int32_t* chunk_start,
-                              int32_t* chunk_row, int* split_count, cudaStream_t stream,
-                              int32_t* run_counter);
-
 // Processing order of the chunks: chunk ids sorted by estimated cost (entries / 8 + rows / 2),
 // most expensive first (stable 8-bit counting-sort passes on the device).  Chunks full of short
 // rows started last leave the GPU draining; started first they overlap with the others.
@@ -143,12 +186,27 @@ int hpspmm_order_chunks_by_cost(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t n
                                 const int32_t* chunk_row, int32_t* order_out, void* scratch,
                                 cudaStream_t stream);
 
-// The rows that hold entries, as the product kernels of a plan walk them: nz_id / nz_end need M + 1
-// ints each, chunk_ri n_chunks; scratch needs hpspmm_row_list_scratch_bytes(M) bytes.
-size_t hpspmm_row_list_scratch_bytes(int64_t M);
-int hpspmm_build_row_list(hpspmm_ctx* ctx, int64_t M, int64_t n_chunks, const int32_t* row_ptr,
-                          const int32_t* chunk_row, int32_t* nz_id, int32_t* nz_end, int32_t* chunk_ri,
-                          void* scratch, cudaStream_t stream);
+// Builds the structure a product walks, in two launches: the list of rows that hold entries (nz, hpspmm_nz_bytes(M)
+// bytes, with sentinels (M, INT_MAX) at its end) and one record per chunk in matrix order (rec_out, 2 * n_chunks int4).
+// counts: hpspmm_row_tiles(M) ints of scratch.  counter (n_counter ints) is zeroed.  The arrays of `tables` are
+// filled as well where they are given (a plan exposes them), and split_count receives the number of chunks that
+// begin inside a row.
+struct hpspmm_structure_tables {
+  int32_t* chunk_start;
+  int32_t* chunk_row;
+  int32_t* chunk_ri;
+  int32_t* nz_id;
+  int32_t* nz_end;
+  int* split_count;
+};
+int64_t hpspmm_row_tiles(int64_t M);
+size_t hpspmm_nz_bytes(int64_t M);
+int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr, int32_t S, int64_t n_chunks,
+                           int2* nz, int4* rec_out, int32_t* counts, int32_t* counter, int64_t n_counter,
+                           const hpspmm_structure_tables& tables, cudaStream_t stream);
+// rec[slot] = rec_in[order[slot]]
+int hpspmm_order_records(hpspmm_ctx* ctx, int64_t n_chunks, const int32_t* order, const int4* rec_in, int4* rec,
+                         cudaStream_t stream);
 
 // ---- counter-based PRNG shared by host and device --------------------------------------
 // splitmix64 finaliser over (seed, stream, index); 24 high bits -> [0, 1).

@@ -5,114 +5,90 @@
 // table of the SpMM (one warp per chunk); A's values are not multiplied in.
 #include "device_utils.cuh"
 #include "hpspmm_internal.h"
+#include "warp_frag.cuh"
 
 namespace {
 
 using namespace hpspmm;
 
-constexpr int kBlockThreads = 256;
-
-__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
-  acc = fmaf(a.x, b.x, acc);
-  acc = fmaf(a.y, b.y, acc);
-  acc = fmaf(a.z, b.z, acc);
-  acc = fmaf(a.w, b.w, acc);
-  return acc;
-}
-
-// Row holding entry j, searching upward from `row` (entry j lies beyond the end of `row`).
-__device__ __forceinline__ void next_row(const int* __restrict__ row_ptr, int M, int j, int& row,
-                                         int& row_end) {
-  ++row;
-  int e = __ldg(row_ptr + row + 1);
-  int probes = 0;
-  while (e <= j) {
-    if (++probes == 8) {
-      int lo = row + 1, hi = M + 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(row_ptr + mid) <= j)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      row = lo - 1;
-      e = __ldg(row_ptr + row + 1);
-      break;
-    }
-    ++row;
-    e = __ldg(row_ptr + row + 1);
-  }
-  row_end = e;
-}
-
-// ---- warp kernel: one warp per chunk, G = 32/W interleaved lane groups, K = 4 * W --------
+// ---- warp kernel: one warp per chunk, G = 32/W interleaved lane groups (warp_frag.cuh) -----------
 // Same shape as the SpMM warp kernel: (col) tiles of 32 entries staged in shared memory with
-// asynchronous copies; in every step group g takes entry G*s+g and gathers its float4 of that
-// row of Y, U = 4 steps at a time.  The fragment of the current row of X stays in registers;
-// row changes are warp-uniform.  The four partial dot products of a batch are reduced across
-// the W lanes of each group with a transposing butterfly (4 shuffles for 4 results at W = 8).
+// asynchronous copies; in every step group g takes entry G*s+g and gathers its fragment of that
+// row of Y, U steps at a time.  The fragment of the current row of X stays in registers; row
+// changes are warp-uniform.  The U partial dot products of a batch are reduced across the W lanes
+// of each group with a transposing butterfly (4 shuffles for 4 results at W = 8).
 
-// Sums p[0..3] over each group of 4 adjacent lanes; afterwards p[0] of lane l holds the total
-// of the value whose index is the 2-bit reversal of (l & 3).
-__device__ __forceinline__ void reduce4_transposed(float (&p)[4], int lane) {
-  {
-    const bool up = lane & 1;
+// log2 of a power of two
+__host__ __device__ constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
+
+// Sums p[0..U-1] over the W lanes of a group.  While values remain to be split, each exchange hands the partner
+// half of them; afterwards lane l holds in the return value the total of entry `which(l)`.
+template <int U, int W>
+__device__ __forceinline__ float reduce_transposed(float (&p)[U], int lane) {
+  int n = U, d = 1;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float send = up ? p[i] : p[i + 2];
-      const float keep = up ? p[i + 2] : p[i];
-      p[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-    }
+  for (int s = 0; s < ilog2(U); ++s) {
+    const bool up = (lane & d) != 0;
+    n >>= 1;
+#pragma unroll
+    for (int i = 0; i < U / 2; ++i)
+      if (i < n) {
+        const float send = up ? p[i] : p[i + n];
+        const float keep = up ? p[i + n] : p[i];
+        p[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+      }
+    d <<= 1;
   }
-  {
-    const bool up = lane & 2;
-    const float send = up ? p[0] : p[1];
-    const float keep = up ? p[1] : p[0];
-    p[0] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+  float total = p[0];
+#pragma unroll
+  for (int s = ilog2(U); s < ilog2(W); ++s) {
+    total += __shfl_xor_sync(0xffffffffu, total, d);
+    d <<= 1;
   }
+  return total;
 }
 
-// SLAB = 0: X and Y are 4 * W columns wide.  SLAB = 1 / 2: the kernel covers a slab of 4 * W columns of wider
-// X and Y (row stride ld); 1 writes the partial dot products, 2 adds them to what earlier slabs wrote.
-// When a row ends the kernel steps to the next row that holds entries through the list nz_id / nz_end (chunk_ri:
-// position in that list of the row holding a chunk's first entry), so it never looks at an empty row.
-// resident 64-thread blocks per SM the kernel is compiled for: 20 (48 registers) measured 0.193 / 0.318 /
-// 0.542 ms at K = 32 / 64 / 128 on the R-MAT scale-20 graph against 0.204 / 0.318 / 0.555 ms at 18 (56 registers)
-#ifndef HPSPMM_SDDMM_MINB
-#define HPSPMM_SDDMM_MINB 20
-#endif
-template <int W, bool HINT, int BT, int SLAB>
-__global__ void __launch_bounds__(BT, HPSPMM_SDDMM_MINB)
-sddmm_warp_kernel(int M, int n_chunks, const int* __restrict__ row_ptr,
-                  const int* __restrict__ col_idx, const float* __restrict__ X,
-                  const float* __restrict__ Y, float* __restrict__ out,
-                  const int* __restrict__ chunk_start, const int* __restrict__ chunk_row,
-                  const int* __restrict__ chunk_order, int ld, const int* __restrict__ nz_id,
-                  const int* __restrict__ nz_end, const int* __restrict__ chunk_ri) {
-  const int64_t K = SLAB ? (int64_t)ld : (int64_t)(4 * W);
+template <int U>
+__device__ __forceinline__ int reduced_entry(int l) {   // the entry whose total lane l < U holds: l with its bits reversed
+  int w = 0;
+#pragma unroll
+  for (int s = 0; s < ilog2(U); ++s) w |= ((l >> s) & 1) << (ilog2(U) - 1 - s);
+  return w;
+}
+
+// KS: row stride of X and Y when it is a compile-time constant, else 0.  The slab is columns [off0, off0 + cols) of
+// X and Y; add: add to what an earlier slab wrote.
+// The kernel walks the list nz of the rows that hold entries and never looks at an empty row.
+// SERIAL: a row end waits for the next row's fragment of X.  With many chunks per SM other warps cover that, and the
+// path needs no registers beyond the gathers' (16 M entries, 64 columns: 0.327 ms against 0.366).  With few chunks the
+// waits add up instead -- a chunk of very short rows waits once per row -- so there all row bounds of a tile come from
+// one load and the entries of a batch gather their own rows of X (70 K entries of a power-law graph in chunks of 64,
+// 64 columns: 8.6 us against 12.6).
+template <int VEC, int W, int R, int U, int KS, bool HINT, int BT, int MINB, bool SERIAL>
+__global__ void __launch_bounds__(BT, MINB)
+sddmm_warp_kernel(int n_chunks, int ld, int off0, int cols, int add, int keep_y, const int* __restrict__ col_idx,
+                  const float* __restrict__ X, const float* __restrict__ Y, float* __restrict__ out,
+                  const int4* __restrict__ rec, const int2* __restrict__ nz) {
+  constexpr int CW = VEC * W * R;
   constexpr int G = 32 / W;
   constexpr int T = 32;
-  constexpr int U = 4;
   constexpr int BATCH = U * G;
   constexpr int STAGES = 2;
-  static_assert(T % BATCH == 0, "batch must tile the staged tile");
+  static_assert(T % BATCH == 0 && (U <= W || W == 1), "batch must tile the staged tile; a lane holds one total");
   __shared__ int tiles[BT / 32][STAGES][T];
 
   const int lane = threadIdx.x & 31;
   const int g = lane / W;
   const int l = lane % W;
-  const int slot = (int)(((int64_t)blockIdx.x * BT + threadIdx.x) >> 5);
+  const int slot = (int)((blockIdx.x * (unsigned)BT + threadIdx.x) >> 5);
   if (slot >= n_chunks) return;
-  const int chunk = chunk_order != nullptr ? __ldg(chunk_order + slot) : slot;
-  const uint64_t policy = HINT ? policy_evict_last() : 0ull;
+  const uint64_t policy = HINT ? policy_for_gathers(keep_y) : 0ull;
   int(*my)[T] = tiles[threadIdx.x >> 5];
 
-  const int n0 = __ldg(chunk_start + chunk);
-  const int n1 = __ldg(chunk_start + chunk + 1);
-  int ri = __ldg(chunk_ri + chunk);
-  int row = __ldg(nz_id + ri);
-  int row_end = __ldg(nz_end + ri);
+  const int4 p = __ldg(rec + 2 * (int64_t)slot);
+  const int n0 = p.x;
+  int ri = p.y, row = p.z, row_end = p.w;
+  const int n1 = __ldg(&rec[2 * (int64_t)slot + 1].z);
 
   auto stage_tile = [&](int stage, int base) {
     const int j = base + lane;
@@ -125,27 +101,52 @@ sddmm_warp_kernel(int M, int n_chunks, const int* __restrict__ row_ptr,
   stage_tile(0, n0);
   stage_tile(1, n0 + T);
 
-  float4 x = __ldg(reinterpret_cast<const float4*>(X + (int64_t)row * K + l * 4));
-  const float* Yl = Y + l * 4;
-  // entry `next_entry` starts a later row: find it and fetch its fragment of X
-  auto next_x = [&](int next_entry) {
-    (void)next_entry;   // the list of rows that hold entries names the row directly
-    ++ri;
-    row = __ldg(nz_id + ri);
-    row_end = __ldg(nz_end + ri);
-    x = __ldg(reinterpret_cast<const float4*>(X + (int64_t)row * K + l * 4));
+  // a lane beyond the slab's width works on column 0 of the slab with an x of zero
+  const int kw = KS ? CW : cols;
+  const bool live_last = KS || ((R - 1) * W + l) * VEC < kw;
+  const unsigned stride = (KS ? KS : ld) * 4u;
+  const int o_first = off0 + ((R > 1 || live_last) ? l * VEC : 0);
+  const int o_last = off0 + (live_last ? ((R - 1) * W + l) * VEC : 0);
+  const char* Yl = reinterpret_cast<const char*>(Y + o_first);
+  const char* Yl_last = reinterpret_cast<const char*>(Y + o_last);
+  float x[R][VEC];
+  auto load_x = [&](float (&x)[R][VEC], int row) {
+    const float* xr = X + (int64_t)row * (KS ? KS : ld);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      gather_vec<VEC, false>(x[r], xr + (R > 1 && r == R - 1 ? o_last : o_first + r * W * VEC), 0ull);
+      if (r == R - 1 && !live_last)
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) x[r][k] = 0.f;
+    }
   };
-
+  bool have_x = SERIAL;   // x holds the fragment of the current row
+  if (SERIAL) load_x(x, row);
+  auto gather = [&](float (&y)[R][VEC], int col) {
+    const char* q = Yl + (uint64_t)(unsigned)col * stride;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (R > 1 && r == R - 1)
+        gather_vec<VEC, HINT>(y[r], reinterpret_cast<const float*>(Yl_last + (uint64_t)(unsigned)col * stride), policy);
+      else
+        gather_vec<VEC, HINT>(y[r], reinterpret_cast<const float*>(q) + r * W * VEC, policy);
+    }
+  };
+  auto dot = [&](const float (&x)[R][VEC], const float (&y)[R][VEC]) {
+    float s = 0.f;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int k = 0; k < VEC; ++k)
+        // (0 * inf of a lane outside the slab must not reach the sum)
+        s = (KS || r < R - 1 || live_last) ? fmaf(x[r][k], y[r][k], s) : s;
+    return s;
+  };
   // reduce the U partial dot products of a batch over the W lanes of each group and store the U * G results
   auto finish_batch = [&](float (&part)[U], int j0) {
-    reduce4_transposed(part, lane);
-    float total = part[0];
-    total += __shfl_xor_sync(0xffffffffu, total, 4);
-    if (W >= 16) total += __shfl_xor_sync(0xffffffffu, total, 8);
-    if (W >= 32) total += __shfl_xor_sync(0xffffffffu, total, 16);
-    const int which = ((l & 1) << 1) | ((l >> 1) & 1);   // which of the U entries lane l holds
-    const int j = j0 + which * G + g;
-    if (l < 4 && j < n1) out[j] = SLAB == 2 ? out[j] + total : total;
+    const float total = reduce_transposed<U, W>(part, lane);
+    const int j = j0 + reduced_entry<U>(l) * G + g;
+    if (l < U && j < n1) out[j] = add ? out[j] + total : total;
   };
 
   int stage = 0;
@@ -156,28 +157,30 @@ sddmm_warp_kernel(int M, int n_chunks, const int* __restrict__ row_ptr,
     if (base + T <= n1 && row_end >= base + T) {
       // Fast tile: all 32 entries belong to the current row.  Fully unrolled, every shared-memory offset a
       // compile-time constant, no tests between gathers (two thirds of the tiles of a power-law graph).
+      if (!SERIAL && !have_x) load_x(x, row);
+      have_x = true;
 #pragma unroll
       for (int u0 = 0; u0 < T; u0 += BATCH) {
-        float4 y[U];
+        float y[U][R][VEC];
 #pragma unroll
-        for (int i = 0; i < U; ++i) y[i] = ld_gather<HINT>(Yl + (int64_t)tile[u0 + i * G] * K, policy);
+        for (int i = 0; i < U; ++i) gather(y[i], tile[u0 + i * G]);
         float part[U];
 #pragma unroll
-        for (int i = 0; i < U; ++i) part[i] = dot4(x, y[i], 0.f);
+        for (int i = 0; i < U; ++i) part[i] = dot(x, y[i]);
         finish_batch(part, base + u0);
       }
-    } else {
+    } else if (SERIAL) {
 #pragma unroll 1
       for (int u0 = 0; u0 < T; u0 += BATCH) {
         const int j0 = base + u0;
         if (j0 >= n1) break;
-        float4 y[U];
+        float y[U][R][VEC];
 #pragma unroll
-        for (int i = 0; i < U; ++i) y[i] = ld_gather<HINT>(Yl + (int64_t)tile[u0 + i * G] * K, policy);
+        for (int i = 0; i < U; ++i) gather(y[i], tile[u0 + i * G]);
         float part[U];
         if (row_end >= j0 + BATCH) {
 #pragma unroll
-          for (int i = 0; i < U; ++i) part[i] = dot4(x, y[i], 0.f);
+          for (int i = 0; i < U; ++i) part[i] = dot(x, y[i]);
         } else {
 #pragma unroll
           for (int i = 0; i < U; ++i) {
@@ -187,15 +190,87 @@ sddmm_warp_kernel(int M, int n_chunks, const int* __restrict__ row_ptr,
             int cur = lo;
             part[i] = 0.f;
             while (row_end < hi) {   // warp-uniform: the current row ends inside this step
-              if (mine >= cur && mine < row_end) part[i] = dot4(x, y[i], 0.f);
+              if (mine >= cur && mine < row_end) part[i] = dot(x, y[i]);
               cur = row_end;
-              next_x(cur);
+              ++ri;
+              const int2 nx = __ldg(nz + ri);
+              row = nx.x;
+              row_end = nx.y;
+              load_x(x, row);
             }
-            if (mine >= cur) part[i] = dot4(x, y[i], 0.f);
+            if (mine >= cur) part[i] = dot(x, y[i]);
           }
         }
         finish_batch(part, j0);
       }
+    } else {
+      // Rows end inside this tile (or just before it).  Lane i holds the i-th row from the tile's first one on; bit p
+      // of `starts` (p > 0) says that entry p of the tile opens a new row.  In a batch that holds several row starts every
+      // entry gathers the fragment of its own row of X beside that of Y (neighbours share rows and hit the same lines):
+      // waiting for the next row's fragment at each row end cost a memory latency per row.
+      if (row_end == base) {                 // the current row ended with the previous tile
+        ++ri;
+        have_x = false;
+      }
+      const int2 mine_nz = __ldg(nz + ri + lane);
+      const int limit = min(T, n1 - base);   // entries of this tile inside the chunk
+      const unsigned p = (unsigned)(mine_nz.y - base);
+      const unsigned starts = __reduce_or_sync(0xffffffffu, p < (unsigned)limit ? 1u << p : 0u);
+      int passed = 0;                        // row starts before the batch
+#pragma unroll 1
+      for (int u0 = 0; u0 < limit; u0 += BATCH) {
+        float y[U][R][VEC];
+        float part[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) gather(y[i], tile[u0 + i * G]);
+        const unsigned here = BATCH == 32 ? starts : (starts >> u0) & ((1u << (BATCH & 31)) - 1u);
+        const int n_here = __popc(here);     // all of this is warp-uniform
+        if (n_here <= 1) {
+          // one row, or the end of one and the start of the next: the fragments of both travel with the gathers
+          if (!have_x) load_x(x, __shfl_sync(0xffffffffu, mine_nz.x, passed));
+          have_x = true;
+          if (n_here == 0) {
+#pragma unroll
+            for (int i = 0; i < U; ++i) part[i] = dot(x, y[i]);
+          } else {
+            float x2[R][VEC];
+            load_x(x2, __shfl_sync(0xffffffffu, mine_nz.x, passed + 1));
+            const int first = __ffs(here) - 1 - g;   // entry i * G of this group lies in the next row from here on
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+              float xi[R][VEC];
+#pragma unroll
+              for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) xi[r][k] = i * G >= first ? x2[r][k] : x[r][k];
+              part[i] = dot(xi, y[i]);
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+              for (int k = 0; k < VEC; ++k) x[r][k] = x2[r][k];
+          }
+        } else {
+          constexpr int H = U >= 2 ? U / 2 : 1;
+#pragma unroll
+          for (int i0 = 0; i0 < U; i0 += H) {
+            float xs[H][R][VEC];
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+              const int q = (i0 + i) * G + g;   // entry u0 + q of the tile
+              load_x(xs[i], __shfl_sync(0xffffffffu, mine_nz.x, passed + __popc(here & (0xffffffffu >> (31 - q)))));
+            }
+#pragma unroll
+            for (int i = 0; i < H; ++i) part[i0 + i] = dot(xs[i], y[i0 + i]);
+          }
+          have_x = false;
+        }
+        passed += n_here;
+        finish_batch(part, base + u0);
+      }
+      ri += passed;
+      row = __shfl_sync(0xffffffffu, mine_nz.x, passed);
+      row_end = __shfl_sync(0xffffffffu, mine_nz.y, passed);
     }
     __syncwarp();
     stage_tile(stage, base + STAGES * T);
@@ -204,62 +279,69 @@ sddmm_warp_kernel(int M, int n_chunks, const int* __restrict__ row_ptr,
   cp_async_wait<0>();
 }
 
-// Any K: one warp per chunk, one entry at a time, lanes stride over the columns.
-template <int VEC>
-__global__ void __launch_bounds__(kBlockThreads)
-sddmm_generic_kernel(int M, int K, int n_chunks, const int* __restrict__ row_ptr,
-                     const int* __restrict__ col_idx, const float* __restrict__ X,
-                     const float* __restrict__ Y, float* __restrict__ out,
-                     const int* __restrict__ chunk_start, const int* __restrict__ chunk_row) {
-  const int lane = threadIdx.x & 31;
-  const int worker = (int)(((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) >> 5);
-  if (worker >= n_chunks) return;
-  const int n0 = __ldg(chunk_start + worker);
-  const int n1 = __ldg(chunk_start + worker + 1);
-  int row = __ldg(chunk_row + worker);
-  int row_end = __ldg(row_ptr + row + 1);
-  for (int j = n0; j < n1; ++j) {
-    if (j >= row_end) next_row(row_ptr, M, j, row, row_end);
-    const float* xr = X + (int64_t)row * K;
-    const float* yr = Y + (int64_t)__ldg(col_idx + j) * K;
-    float s = 0.f;
-    if (VEC == 4) {
-      for (int c = lane * 4; c < K; c += 128) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(xr + c));
-        const float4 b = __ldg(reinterpret_cast<const float4*>(yr + c));
-        s = dot4(a, b, s);
-      }
-    } else {
-      for (int c = lane; c < K; c += 32) s = fmaf(__ldg(xr + c), __ldg(yr + c), s);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[j] = s;
-  }
-}
-
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-struct sddmm_row_list {
-  const int32_t* nz_id;
-  const int32_t* nz_end;
-  const int32_t* chunk_ri;
+struct sddmm_args {
+  int n_chunks, K, off, cols, keep_y;
+  const int32_t* col_idx;
+  const float *X, *Y;
+  float* out;
+  const int4* rec;
+  const int2* nz;
 };
 
-template <int W, int SLAB>
-void launch_sddmm(bool hint, int M, int n_chunks, const int32_t* row_ptr, const int32_t* col_idx,
-                  const float* X, const float* Y, float* out, const int32_t* chunk_start,
-                  const int32_t* chunk_row, const int32_t* chunk_order, cudaStream_t s, sddmm_row_list rows,
-                  int ld = 4 * W) {
-  constexpr int BT = 64;
-  const int cpb = BT / 32;
-  const unsigned grid = (unsigned)((n_chunks + cpb - 1) / cpb);
-#define HPSPMM_SDDMM_LAUNCH(H)                                                                            \
-  sddmm_warp_kernel<W, H, BT, SLAB><<<grid, BT, 0, s>>>(M, n_chunks, row_ptr, col_idx, X, Y, out,          \
-                                                        chunk_start, chunk_row, chunk_order, ld,          \
-                                                        rows.nz_id, rows.nz_end, rows.chunk_ri)
-  if (hint) HPSPMM_SDDMM_LAUNCH(true); else HPSPMM_SDDMM_LAUNCH(false);
-#undef HPSPMM_SDDMM_LAUNCH
+// one launch per slab of the width: the first writes the partial dot products, the others add theirs
+template <int VEC, int W, int R, int U, int KS, bool HINT, int MINB>
+int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
+  constexpr int BT = 64, CW = VEC * W * R;
+  const unsigned grid = (unsigned)((a.n_chunks + BT / 32 - 1) / (BT / 32));
+  for (int off = a.off; off < a.off + a.cols; off += CW) {
+    const int left = a.off + a.cols - off;
+    sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, (KS > 0)><<<grid, BT, 0, s>>>(
+        a.n_chunks, a.K, off, left < CW ? left : CW, off > 0 ? 1 : 0, a.keep_y, a.col_idx, a.X, a.Y, a.out, a.rec, a.nz);
+    ctx->launches++;
+  }
+  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
+  return HPSPMM_OK;
+}
+
+// 20 resident blocks per SM (48 registers) measured 0.193 / 0.318 / 0.542 ms at K = 32 / 64 / 128 on the R-MAT
+// scale-20 graph against 0.204 / 0.318 / 0.555 ms at 18 (56 registers)
+int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_shape& sh, cudaStream_t s) {
+#define GO(V, W, R, U, KS, H, MINB) return launch_sddmm<V, W, R, U, KS, H, MINB>(ctx, a, s)
+  if (sh.VEC == 4) {
+    // (the fixed strides are the SERIAL form)
+    if (sh.lat) {
+    } else if (a.K == 32) { if (sh.hint) GO(4, 8, 1, 4, 32, true, 20); else GO(4, 8, 1, 4, 32, false, 20); }
+    else if (a.K == 64) { if (sh.hint) GO(4, 16, 1, 4, 64, true, 20); else GO(4, 16, 1, 4, 64, false, 20); }
+    else if (a.K == 128) { if (sh.hint) GO(4, 32, 1, 4, 128, true, 20); else GO(4, 32, 1, 4, 128, false, 20); }
+    if (sh.W == 2) GO(4, 2, 1, 2, 0, true, 16);
+    if (sh.W == 4) GO(4, 4, 1, 4, 0, true, 16);
+    if (sh.W == 8) GO(4, 8, 1, 4, 0, true, 16);
+    if (sh.W == 16) GO(4, 16, 1, 4, 0, true, 16);
+    if (sh.R == 1) GO(4, 32, 1, 4, 0, true, 16);
+    if (sh.R == 2) GO(4, 32, 2, 2, 0, true, 16);
+    if (sh.R == 3) GO(4, 32, 3, 2, 0, true, 12);
+    GO(4, 32, 4, 2, 0, true, 10);
+  }
+  if (sh.VEC == 2) {
+    if (sh.W == 2) GO(2, 2, 1, 2, 0, true, 16);
+    if (sh.W == 4) GO(2, 4, 1, 4, 0, true, 16);
+    if (sh.W == 8) GO(2, 8, 1, 8, 0, true, 16);
+    if (sh.W == 16) GO(2, 16, 1, 8, 0, true, 16);
+    if (sh.R == 1) GO(2, 32, 1, 8, 0, true, 16);
+    if (sh.R == 2) GO(2, 32, 2, 4, 0, true, 16);
+    GO(2, 32, 4, 4, 0, true, 12);
+  }
+  if (sh.W == 1) GO(1, 1, 1, 1, 0, true, 16);
+  if (sh.W == 4) GO(1, 4, 1, 4, 0, true, 16);
+  if (sh.W == 8) GO(1, 8, 1, 8, 0, true, 16);
+  if (sh.W == 16) GO(1, 16, 1, 8, 0, true, 16);
+  if (sh.R == 1) GO(1, 32, 1, 8, 0, true, 16);
+  if (sh.R == 2) GO(1, 32, 2, 8, 0, true, 16);
+  if (sh.R <= 4) GO(1, 32, 4, 4, 0, true, 16);
+  GO(1, 32, 8, 4, 0, true, 12);
+#undef GO
 }
 
 }  // namespace
@@ -287,83 +369,38 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   cudaStream_t s = (cudaStream_t)stream;
   const int hint_mode = opts ? opts->b_l2_hint : 0;
   const bool hint = hint_mode == 2 || (hint_mode == 0 && K >= 64);
-  const int32_t* chunk_start;
-  const int32_t* chunk_row;
-  const int32_t* chunk_order = nullptr;
-  sddmm_row_list rows = {nullptr, nullptr, nullptr};
-  int64_t n_chunks;
+  sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, col_idx, X, Y, out_vals, nullptr, nullptr};
   if (plan) {
     HPSPMM_REQUIRE(ctx, plan->M == M && plan->nnz == nnz, "plan built for another matrix");
     HPSPMM_REQUIRE(ctx, plan->device == ctx->device, "plan built on another device");
-    chunk_start = plan->chunk_start;
-    chunk_row = plan->chunk_row;
-    chunk_order = plan->chunk_order;
-    n_chunks = plan->n_chunks;
-    rows = sddmm_row_list{plan->nz_id, plan->nz_end, plan->chunk_ri};
+    a.n_chunks = (int)plan->n_chunks;
+    a.rec = plan->rec;
+    a.nz = plan->nz;
   } else {
     int32_t S = (opts && opts->chunk_nnz > 0) ? opts->chunk_nnz : hpspmm_default_chunk_nnz(K, nnz);
     S = (S + 31) / 32 * 32;
-    n_chunks = (nnz + S - 1) / S;
-    const size_t b_int = align_up((size_t)(n_chunks + 1) * 4, 256);
-    const size_t b_nz = align_up((size_t)(M + 2) * 4, 256);
-    const size_t b_sort = hpspmm_order_scratch_bytes(n_chunks), b_list = hpspmm_row_list_scratch_bytes(M);
-    int st = hpspmm_ensure_scratch(ctx, 4 * b_int + 2 * b_nz + (b_sort > b_list ? b_sort : b_list));
+    const int64_t n_chunks = (nnz + S - 1) / S;
+    const size_t b_tiles = align_up((size_t)hpspmm_row_tiles(M) * 4, 256);
+    const size_t b_rec = align_up((size_t)n_chunks * 32, 256);
+    int st = hpspmm_ensure_scratch(ctx, b_tiles + b_rec + hpspmm_nz_bytes(M));
     if (st != HPSPMM_OK) return st;
-    char* sb = (char*)ctx->scratch;
-    int32_t* cs = (int32_t*)sb;
-    int32_t* cr = (int32_t*)(sb + b_int);
-    int32_t* co = (int32_t*)(sb + 2 * b_int);
-    int32_t* cri = (int32_t*)(sb + 3 * b_int);
-    int32_t* nzi = (int32_t*)(sb + 4 * b_int);
-    int32_t* nze = (int32_t*)(sb + 4 * b_int + b_nz);
-    void* tmp = sb + 4 * b_int + 2 * b_nz;
-    st = hpspmm_launch_chunk_table(ctx, M, nnz, row_ptr, S, n_chunks, cs, cr, nullptr, s, nullptr);
+    char* base = (char*)ctx->scratch;
+    int4* rec = (int4*)(base + b_tiles);
+    int2* nz = (int2*)(base + b_tiles + b_rec);
+    st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, n_chunks, nz, rec, (int32_t*)base, nullptr, 0,
+                                hpspmm_structure_tables{}, s);
     if (st != HPSPMM_OK) return st;
-    st = hpspmm_order_chunks_by_cost(ctx, M, N, n_chunks, row_ptr, nullptr, cs, cr, co, tmp, s);
-    if (st != HPSPMM_OK) return st;
-    st = hpspmm_build_row_list(ctx, M, n_chunks, row_ptr, cr, nzi, nze, cri, tmp, s);
-    if (st != HPSPMM_OK) return st;
-    rows = sddmm_row_list{nzi, nze, cri};
-    chunk_start = cs;
-    chunk_row = cr;
-    chunk_order = co;
+    a.n_chunks = (int)n_chunks;
+    a.rec = rec;
+    a.nz = nz;
   }
-  const int m = (int)M, nc = (int)n_chunks;
-  if (K == 32) {
-    launch_sddmm<8, 0>(hint, m, nc, row_ptr, col_idx, X, Y, out_vals, chunk_start, chunk_row, chunk_order, s, rows);
-  } else if (K == 64) {
-    launch_sddmm<16, 0>(hint, m, nc, row_ptr, col_idx, X, Y, out_vals, chunk_start, chunk_row, chunk_order, s, rows);
-  } else if (K == 128) {
-    launch_sddmm<32, 0>(hint, m, nc, row_ptr, col_idx, X, Y, out_vals, chunk_start, chunk_row, chunk_order, s, rows);
-  } else if (K % 32 == 0 && K <= 512) {
-    // other multiples of 32: column slabs of 128, 64 and 32; the first writes, the others add their share
-    int64_t off = 0;
-    while (off < K) {
-      const int64_t w = K - off >= 128 ? 128 : (K - off >= 64 ? 64 : 32);
-#define HPSPMM_SDDMM(WW)                                                                                  \
-  if (off == 0)                                                                                           \
-    launch_sddmm<WW, 1>(hint, m, nc, row_ptr, col_idx, X + off, Y + off, out_vals, chunk_start, chunk_row, \
-                        chunk_order, s, rows, (int)K);                                                    \
-  else                                                                                                    \
-    launch_sddmm<WW, 2>(hint, m, nc, row_ptr, col_idx, X + off, Y + off, out_vals, chunk_start, chunk_row, \
-                        chunk_order, s, rows, (int)K)
-      if (w == 128) { HPSPMM_SDDMM(32); }
-      else if (w == 64) { HPSPMM_SDDMM(16); }
-      else { HPSPMM_SDDMM(8); }
-#undef HPSPMM_SDDMM
-      off += w;
-      if (off < K) ctx->launches++;
-    }
-  } else {
-    const unsigned grid = (unsigned)((n_chunks + kBlockThreads / 32 - 1) / (kBlockThreads / 32));
-    if ((K & 3) == 0)
-      sddmm_generic_kernel<4><<<grid, kBlockThreads, 0, s>>>(m, (int)K, nc, row_ptr, col_idx, X, Y,
-                                                             out_vals, chunk_start, chunk_row);
-    else
-      sddmm_generic_kernel<1><<<grid, kBlockThreads, 0, s>>>(m, (int)K, nc, row_ptr, col_idx, X, Y,
-                                                             out_vals, chunk_start, chunk_row);
+  const int VEC = hpspmm_vector_width(K, (uintptr_t)X | (uintptr_t)Y);
+  for (a.off = 0; a.off < a.K; a.off += a.cols) {
+    a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
+    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hint);
+    sh.lat = a.n_chunks <= ctx->sm_count * 80;   // up to about two waves of resident warps
+    const int st = launch_sddmm_shape(ctx, a, sh, s);
+    if (st != HPSPMM_OK) return st;
   }
-  ctx->launches++;
-  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;
 }

@@ -5,20 +5,9 @@
 // inside a row no longer than S is moved back to the start of that row, so short rows
 // stay whole; a cut inside a longer ("heavy") row stays where it is, so heavy rows are
 // split across chunks (a merge-path split restricted to heavy rows).  One warp owns one
-// chunk.  The warp stages (col, val) tiles of 32 entries in shared memory with
-// asynchronous copies, two tiles ahead of their use.  For K = 4*W the warp is G = 32/W
-// lane groups; in every step group g takes entry G*s+g of the tile, reads its (col, val)
-// pair as one shared-memory broadcast, and gathers its float4 of that row of B, so one
-// warp instruction gathers G rows and no two groups ever diverge (row ends are warp-
-// uniform).  Gathers are issued U steps at a time before the first FMA.  When a row
-// ends, the groups' partial sums are combined with shuffles and the row is stored once,
-// by plain stores.  A chunk that ends inside a heavy row hands its partial sum on through
-// a carry slot, and the carries of a split row are added, in chunk order, to the row its last
-// piece stored.  Who adds them depends on the width: at 32 columns a second, small kernel; at 64
-// and 128 columns the pieces themselves -- each bumps a per-row counter (one atomicAdd) when its
-// part is visible, and the piece that finds the counter complete sums the carries.  Either way
-// the order of the additions is fixed by the chunking, so results are bit-reproducible from run
-// to run.  Empty rows are zeroed by extra blocks at the end of the same grid.
+// chunk; the kernel is in spmm_warp.cuh, its instances per vector width in spmm_shapes_v*.cu,
+// the tables it walks are built in structure_kernels.cu.  This file holds the entry points, the
+// choice of chunk size and shape, the row-split kernels and the TMA-fed kernel.
 // HPSPMM_ALGO_ROW_SPLIT keeps the reference's GESpMM shape (one sub-warp per row, every row
 // summed in storage order), which reproduces the CPU oracle bit for bit.
 #include <algorithm>
@@ -29,6 +18,7 @@
 
 #include "device_utils.cuh"
 #include "hpspmm_internal.h"
+#include "spmm_warp.cuh"
 
 namespace {
 
@@ -36,20 +26,16 @@ using namespace hpspmm;
 
 constexpr int kBlockThreads = 256;
 
-// resident 64-thread blocks per SM the contiguous warp kernels are compiled for (20 -> 48 registers)
-#ifndef HPSPMM_WARP_MINB
-#define HPSPMM_WARP_MINB 20
-#endif
-
 // ---- chunk table -----------------------------------------------------------------------
 
+// Used where there is no room for the records of hpspmm_build_structure: first entry of every chunk and the row
+// that holds it, by binary search per cut.
 __global__ void chunk_table_kernel(int M, int nnz, const int* __restrict__ row_ptr, int S,
                                    int n_chunks, int* __restrict__ chunk_start,
-                                   int* __restrict__ chunk_row, int* __restrict__ split_count,
-                                   int* __restrict__ run_counter) {
+                                   int* __restrict__ chunk_row, int* __restrict__ run_counter) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c > n_chunks) return;
-  if (run_counter != nullptr) run_counter[c] = 0;   // per-row counters of the in-kernel carry settlement
+  run_counter[c] = 0;   // per-row counters of the in-kernel carry settlement
   if (c == n_chunks) {
     chunk_start[c] = nnz;
     return;
@@ -67,129 +53,33 @@ __global__ void chunk_table_kernel(int M, int nnz, const int* __restrict__ row_p
   int r = lo - 1;
   r = r < 0 ? 0 : (r > M - 1 ? M - 1 : r);  // only a malformed row_ptr can need this
   const int rs = __ldg(row_ptr + r), re = __ldg(row_ptr + r + 1);
-  const int start = (re - rs <= S) ? rs : t;
-  chunk_start[c] = c == 0 ? 0 : start;
+  chunk_start[c] = c == 0 ? 0 : ((re - rs <= S) ? rs : t);
   chunk_row[c] = r;
-  if (split_count != nullptr && c > 0 && start != rs) atomicAdd(split_count, 1);
 }
 
-// ---- empty rows ------------------------------------------------------------------------
-
-// Blocks past the chunk blocks walk all rows and write zeros into the empty ones.
-__device__ __forceinline__ void zero_empty_rows(int M, int K, const int* __restrict__ row_ptr,
-                                                float* __restrict__ C, int zero_block,
-                                                int n_zero_blocks, int block_threads = kBlockThreads,
-                                                int64_t row_stride = 0) {
-  if (row_stride == 0) row_stride = K;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int warps_per_block = block_threads / 32;
-  const int64_t stride = (int64_t)n_zero_blocks * warps_per_block * 32;
-  for (int64_t r0 = ((int64_t)zero_block * warps_per_block + warp) * 32; r0 < M; r0 += stride) {
-    const int64_t r = r0 + lane;
-    bool empty = false;
-    if (r < M) empty = __ldg(row_ptr + r) == __ldg(row_ptr + r + 1);
-    unsigned m = __ballot_sync(0xffffffffu, empty);
-    while (m) {
-      const int b = __ffs(m) - 1;
-      m &= m - 1;
-      float* crow = C + (r0 + b) * row_stride;
-      if ((K & 3) == 0) {
-        for (int c = lane * 4; c < K; c += 128) st_stream(crow + c, make_float4(0.f, 0.f, 0.f, 0.f));
-      } else {
-        for (int c = lane; c < K; c += 32) crow[c] = 0.f;
-      }
-    }
-  }
-}
-
-// Next non-empty row after `row`, given that entry j (< nnz) follows the end of `row`.
-__device__ __forceinline__ void advance_row(const int* __restrict__ row_ptr, int M, int j,
-                                            int& row, int& row_end) {
-  ++row;
-  int e = __ldg(row_ptr + row + 1);
-  int probes = 0;
-  while (e == j) {
-    if (++probes == 8) {
-      // a long run of empty rows: gallop (8, 16, 32, ... rows ahead) to bracket the row holding j,
-      // then a binary search inside the bracket
-      int lo = row + 1, step = 8, hi;
-      for (;;) {
-        hi = min(lo + step, M);
-        if (hi == M || __ldg(row_ptr + hi) > j) break;
-        lo = hi;
-        step <<= 1;
-      }
-      ++hi;
-      ++lo;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(row_ptr + mid) <= j)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      row = lo - 1;
-      e = __ldg(row_ptr + row + 1);
-      break;
-    }
-    ++row;
-    e = __ldg(row_ptr + row + 1);
-  }
-  row_end = e;
-}
-
-// ---- sub-warp kernel: one W-lane worker per chunk or per row, K = 4 * W * R ----------------
-
-// Row that holds entry j, packed as (row_end << 32) | row.  Kept out of line: it runs once
-// per row, and inlining its search at every unrolled entry bloats the hot loop.  It takes
-// and returns plain integers so that the accumulators never leave registers.
-__device__ __noinline__ unsigned long long next_row_packed(const int* __restrict__ row_ptr, int M,
-                                                           int j, int row) {
-  int row_end;
-  advance_row(row_ptr, M, j, row, row_end);
-  return ((unsigned long long)(unsigned)row_end << 32) | (unsigned)row;
-}
-
-template <int W, int R, int U, int MINB, bool HINT, bool ROWSPLIT>
+// ---- row-split kernel: one W-lane worker per row, K = 4 * W * R --------------------------------
+// HPSPMM_ALGO_ROW_SPLIT: the shape of the reference's GESpMM, every row summed in storage order.
+template <int W, int R, int U, int MINB, bool HINT>
 __global__ void __launch_bounds__(kBlockThreads, MINB)
-spmm_subwarp_kernel(int M, int n_chunks, int n_chunk_blocks, const int* __restrict__ row_ptr,
-                     const int* __restrict__ col_idx, const float* __restrict__ vals,
-                     const float* __restrict__ B, float* __restrict__ C,
-                     const int* __restrict__ chunk_start, const int* __restrict__ chunk_row,
-                     int* __restrict__ carry_row, float* __restrict__ carry_val) {
+spmm_rowsplit_kernel(int M, const int* __restrict__ row_ptr, const int* __restrict__ col_idx,
+                     const float* __restrict__ vals, const float* __restrict__ B, float* __restrict__ C) {
   constexpr int K = 4 * W * R;
   constexpr int T = 32;       // entries per staged (col, val) tile
   constexpr int RT = T / W;   // entries each lane stages per tile
   constexpr int STAGES = 2;
   __shared__ int2 tiles[kBlockThreads / W][STAGES][T];
 
-  if ((int)blockIdx.x >= n_chunk_blocks) {
-    zero_empty_rows(M, K, row_ptr, C, blockIdx.x - n_chunk_blocks, gridDim.x - n_chunk_blocks);
-    return;
-  }
   const int lane = threadIdx.x & (W - 1);
-  const int worker = (int)(((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) / W);
-  if (worker >= n_chunks) return;
+  const int row = (int)(((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) / W);
+  if (row >= M) return;
   const unsigned mask = subwarp_mask<W>();
   const uint64_t policy = HINT ? policy_evict_last() : 0ull;
   int2(*my)[T] = tiles[threadIdx.x / W];
-
-  int n0, n1, row, row_end;
-  if (ROWSPLIT) {
-    row = worker;
-    n0 = __ldg(row_ptr + row);
-    n1 = __ldg(row_ptr + row + 1);
-    row_end = n1;
-  } else {
-    n0 = __ldg(chunk_start + worker);
-    n1 = __ldg(chunk_start + worker + 1);
-    row = __ldg(chunk_row + worker);
-    row_end = __ldg(row_ptr + row + 1);
-  }
+  const int n0 = __ldg(row_ptr + row);
+  const int n1 = __ldg(row_ptr + row + 1);
 
   // (col, val) pairs travel global -> shared with 4-byte asynchronous copies, two tiles
-  // ahead of their use; entries past the end of the chunk are staged as (column 0, 0.0f).
+  // ahead of their use; entries past the end of the row are staged as (column 0, 0.0f).
   auto stage_tile = [&](int stage, int base) {
 #pragma unroll
     for (int t = 0; t < RT; ++t) {
@@ -230,41 +120,11 @@ spmm_subwarp_kernel(int M, int n_chunks, int n_chunk_blocks, const int* __restri
 #pragma unroll
         for (int r = 0; r < R; ++r) b[i][r] = ld_gather<HINT>(p + r * W * 4, policy);
       }
-      if (ROWSPLIT || (j0 + U <= n1 && row_end >= j0 + U)) {
-        // no row ends inside this batch: padded entries (ROWSPLIT tail) carry value 0 and
-        // are skipped below by the same test the slow path uses
-        if (!ROWSPLIT || j0 + U <= n1) {
 #pragma unroll
-          for (int i = 0; i < U; ++i)
+      for (int i = 0; i < U; ++i)
+        if (j0 + i < n1)
 #pragma unroll
-            for (int r = 0; r < R; ++r) fma4(acc[r], v[i], b[i][r]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < U; ++i)
-            if (j0 + i < n1)
-#pragma unroll
-              for (int r = 0; r < R; ++r) fma4(acc[r], v[i], b[i][r]);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-          if (j0 + i < n1) {
-            if (j0 + i == row_end) {
-              float* crow = C + (int64_t)row * K + lane * 4;
-#pragma unroll
-              for (int r = 0; r < R; ++r) {
-                st_stream(crow + r * W * 4, acc[r]);
-                acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-              }
-              const unsigned long long nr = next_row_packed(row_ptr, M, j0 + i, row);
-              row = (int)(unsigned)nr;
-              row_end = (int)(nr >> 32);
-            }
-#pragma unroll
-            for (int r = 0; r < R; ++r) fma4(acc[r], v[i], b[i][r]);
-          }
-        }
-      }
+          for (int r = 0; r < R; ++r) fma4(acc[r], v[i], b[i][r]);
     }
     __syncwarp(mask);
     stage_tile(stage, base + STAGES * T);
@@ -272,323 +132,13 @@ spmm_subwarp_kernel(int M, int n_chunks, int n_chunk_blocks, const int* __restri
   }
   cp_async_wait<0>();
 
-  if (ROWSPLIT || row_end == n1) {
-    float* crow = C + (int64_t)row * K + lane * 4;
+  float* crow = C + (int64_t)row * K + lane * 4;
 #pragma unroll
-    for (int r = 0; r < R; ++r) st_stream(crow + r * W * 4, acc[r]);
-    if (!ROWSPLIT && lane == 0) carry_row[worker] = -1;
-  } else {
-    float* slot = carry_val + (int64_t)worker * K + lane * 4;
-#pragma unroll
-    for (int r = 0; r < R; ++r) *reinterpret_cast<float4*>(slot + r * W * 4) = acc[r];
-    if (lane == 0) carry_row[worker] = row;
-  }
-}
-
-// ---- warp kernel: one warp per chunk, G = 32/W interleaved lane groups, K = 4 * W ---------
-
-template <int W>
-__device__ __forceinline__ float4 reduce_groups(float4 a) {
-  if (W <= 16) {
-    a.x += __shfl_xor_sync(0xffffffffu, a.x, 16);
-    a.y += __shfl_xor_sync(0xffffffffu, a.y, 16);
-    a.z += __shfl_xor_sync(0xffffffffu, a.z, 16);
-    a.w += __shfl_xor_sync(0xffffffffu, a.w, 16);
-  }
-  if (W <= 8) {
-    a.x += __shfl_xor_sync(0xffffffffu, a.x, 8);
-    a.y += __shfl_xor_sync(0xffffffffu, a.y, 8);
-    a.z += __shfl_xor_sync(0xffffffffu, a.z, 8);
-    a.w += __shfl_xor_sync(0xffffffffu, a.w, 8);
-  }
-  return a;
-}
-
-// A finished row: add the groups' partial sums and store the row.  Instead of giving every group the whole
-// sum (reduce_groups: 8 shuffles at W = 8) and letting one group store it, the groups split the work: each
-// exchange hands the partner the half it will own and keeps the other, so W = 8 takes 3 shuffles and every
-// lane stores one float (group g ends up with component g of each float4: 32 lanes, one 128-byte line),
-// W = 16 takes 2 shuffles and every lane stores a float2.  Every kept value is own + partner at each
-// step, in the same pairing as reduce_groups, so the stored bits are the same.
-// ACCUM adds the row into C with reductions (the accumulating COO product) instead of storing it.
-template <int W, bool ACCUM = false>
-__device__ __forceinline__ void store_row_sum(float* __restrict__ crow, const float4& a, int g, int l) {
-  if (W == 8) {
-    const bool up2 = (g & 2) != 0, up1 = (g & 1) != 0;
-    const float s0 = up2 ? a.x : a.z, s1 = up2 ? a.y : a.w;   // the pair the partner (g ^ 2) keeps
-    float k0 = up2 ? a.z : a.x, k1 = up2 ? a.w : a.y;
-    k0 += __shfl_xor_sync(0xffffffffu, s0, 16);
-    k1 += __shfl_xor_sync(0xffffffffu, s1, 16);
-    const float s = up1 ? k0 : k1;                            // the one the partner (g ^ 1) keeps
-    float k = up1 ? k1 : k0;
-    k += __shfl_xor_sync(0xffffffffu, s, 8);
-    if (ACCUM)
-      asm volatile("red.global.add.f32 [%0], %1;" ::"l"(crow + l * 4 + g), "f"(k) : "memory");
-    else
-      asm volatile("st.global.cs.f32 [%0], %1;" ::"l"(crow + l * 4 + g), "f"(k) : "memory");
-  } else if (W == 16) {
-    const bool up = (g & 1) != 0;
-    const float s0 = up ? a.x : a.z, s1 = up ? a.y : a.w;
-    float k0 = up ? a.z : a.x, k1 = up ? a.w : a.y;
-    k0 += __shfl_xor_sync(0xffffffffu, s0, 16);
-    k1 += __shfl_xor_sync(0xffffffffu, s1, 16);
-    if (ACCUM)
-      asm volatile("red.global.add.v2.f32 [%0], {%1,%2};" ::"l"(crow + l * 4 + g * 2), "f"(k0), "f"(k1) : "memory");
-    else
-      asm volatile("st.global.cs.v2.f32 [%0], {%1,%2};" ::"l"(crow + l * 4 + g * 2), "f"(k0), "f"(k1) : "memory");
-  } else {
-    if (ACCUM)
-      red_add_v4(crow + l * 4, a);
-    else
-      st_stream(crow + l * 4, a);
-  }
-}
-
-// In-kernel fix-up of one split row.  A row longer than S is cut at multiples of S only, so its pieces
-// are the chunks first = row_ptr[r] / S .. last = (row_ptr[r+1] - 1) / S: all but the last hand a carry
-// on, the last stores the row.  Every piece bumps the row's counter when its own part is visible
-// device-wide; whoever bumps it last adds the carries, in chunk order, to the stored row.  The sum does
-// not depend on who that is, so results stay bit-reproducible.  No piece ever waits.  Kept out of line
-// so that its registers do not weigh on the gather loop of the caller.
-template <int W>
-__device__ __noinline__ void settle_split_row(int r, int r_end, int S, const int* __restrict__ row_ptr,
-                                              const float* __restrict__ carry_val, float* __restrict__ C,
-                                              int* __restrict__ run_counter, int ld) {
-  const int64_t K = ld;   // row stride of C and of the carry slots (the slab is 4 * W columns wide)
-  constexpr int G = 32 / W;
-  const int lane = threadIdx.x & 31;
-  const int g = lane / W, l = lane % W;
-  const int first = __ldg(row_ptr + r) / S;
-  const int last = (r_end - 1) / S;
-  int seen = 0;
-  if (lane == 0) seen = atomicAdd(run_counter + first, 1);
-  seen = __shfl_sync(0xffffffffu, seen, 0);
-  if (seen != last - first) return;
-  __threadfence();
-  const float* src = carry_val + (int64_t)first * K + l * 4;
-  const int len = last - first;
-  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-  int i = g;
-  for (; i + 7 * G < len; i += 8 * G) {
-    float4 v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = __ldcg(reinterpret_cast<const float4*>(src + (int64_t)(i + u * G) * K));
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      sum.x += v[u].x;
-      sum.y += v[u].y;
-      sum.z += v[u].z;
-      sum.w += v[u].w;
-    }
-  }
-  for (; i < len; i += G) {
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (int64_t)i * K));
-    sum.x += v.x;
-    sum.y += v.y;
-    sum.z += v.z;
-    sum.w += v.w;
-  }
-  sum = reduce_groups<W>(sum);
-  if (g == 0) {
-    float4* out = reinterpret_cast<float4*>(C + (int64_t)r * K + l * 4);
-    float4 o = __ldcg(out);
-    o.x += sum.x;
-    o.y += sum.y;
-    o.z += sum.z;
-    o.w += sum.w;
-    st_stream(reinterpret_cast<float*>(out), o);
-  }
-  if (lane == 0) run_counter[first] = 0;   // ready for the next launch
-}
-
-template <int W, int U, int MINB, bool HINT, int BT, bool SETTLE, bool STRIDED, bool COMPACT>
-__global__ void __launch_bounds__(BT, MINB)
-spmm_warp_kernel(int M, int n_chunks, int n_chunk_blocks, const int* __restrict__ row_ptr,
-                 const int* __restrict__ col_idx, const float* __restrict__ vals,
-                 const float* __restrict__ B, float* __restrict__ C,
-                 const int* __restrict__ chunk_start, const int* __restrict__ chunk_row,
-                 int* __restrict__ carry_row, float* __restrict__ carry_val,
-                 const int* __restrict__ chunk_order, int S, int* __restrict__ run_counter, int ld,
-                 const int* __restrict__ nz_id, const int* __restrict__ nz_end,
-                 const int* __restrict__ chunk_ri) {
-  // COMPACT: the plan lists the rows that hold entries (nz_id, with their ends nz_end) and the position in
-  // that list of every chunk's first row (chunk_ri), so the kernel steps from one such row to the next with
-  // two independent loads and never looks at an empty row.  Without the list it probes row_ptr row by row.
-  // The kernel computes a slab of KW = 4 * W columns.  STRIDED: the slab is part of wider matrices, B, C
-  // and the carry slots have row stride ld; otherwise the stride is the compile-time KW.
-  constexpr int KW = 4 * W;
-  const int64_t K = STRIDED ? (int64_t)ld : (int64_t)KW;
-  constexpr int G = 32 / W;      // lane groups = entries gathered per warp instruction
-  constexpr int T = 32;          // entries per staged tile
-  constexpr int BATCH = U * G;   // entries per batch of gathers
-  constexpr int STAGES = 2;
-  static_assert(BATCH <= T && T % BATCH == 0, "batch must tile the staged tile");
-  __shared__ int2 tiles[BT / 32][STAGES][T];
-
-  if ((int)blockIdx.x >= n_chunk_blocks) {
-    zero_empty_rows(M, KW, row_ptr, C, blockIdx.x - n_chunk_blocks, gridDim.x - n_chunk_blocks, BT, K);
-    return;
-  }
-  const int lane = threadIdx.x & 31;
-  const int g = lane / W;   // group
-  const int l = lane % W;   // position inside the group = float4 column
-  const int slot = (int)(((int64_t)blockIdx.x * BT + threadIdx.x) >> 5);
-  if (slot >= n_chunks) return;
-  // warps take chunks in the plan's order (chunks with many rows first), not in matrix order
-  const int chunk = chunk_order != nullptr ? __ldg(chunk_order + slot) : slot;
-  const uint64_t policy = HINT ? policy_evict_last() : 0ull;
-  int2(*my)[T] = tiles[threadIdx.x >> 5];
-
-  const int n0 = __ldg(chunk_start + chunk);
-  const int n1 = __ldg(chunk_start + chunk + 1);
-  int ri = COMPACT ? __ldg(chunk_ri + chunk) : 0;
-  int row = COMPACT ? __ldg(nz_id + ri) : __ldg(chunk_row + chunk);
-  int row_end = COMPACT ? __ldg(nz_end + ri) : __ldg(row_ptr + row + 1);
-
-  auto stage_tile = [&](int stage, int base) {
-    const int j = base + lane;
-    if (j < n1) {
-      cp_async_4(&my[stage][lane].x, col_idx + j);
-      cp_async_4(&my[stage][lane].y, vals + j);
-    } else {
-      my[stage][lane] = make_int2(0, 0);   // past the chunk: column 0, value 0
-    }
-    cp_async_commit();
-  };
-  stage_tile(0, n0);
-  stage_tile(1, n0 + T);
-
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float* Bl = B + l * 4;
-
-  // the row is complete: combine the groups' partial sums, store, start the next row.
-  // The common case (the next row is not empty, or only a few are) stays inline; a long
-  // run of empty rows falls back to a binary search.
-  auto finish_row = [&](int next_entry) {
-    store_row_sum<W>(C + (int64_t)row * K, acc, g, l);
-    acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (COMPACT) {
-      ++ri;
-      row = __ldg(nz_id + ri);
-      row_end = __ldg(nz_end + ri);
-      return;
-    }
-    int e, probes = 0;
-    do {
-      ++row;
-      e = __ldg(row_ptr + row + 1);
-    } while (e == next_entry && ++probes < 16);
-    if (e == next_entry) {
-      // a long run of empty rows: gallop (16, 32, 64, ... rows ahead) to bracket the row that holds
-      // next_entry, then a binary search inside the bracket
-      int lo = row + 1, step = 16, hi;
-      for (;;) {
-        hi = min(lo + step, M);
-        if (hi == M || __ldg(row_ptr + hi) > next_entry) break;
-        lo = hi;
-        step <<= 1;
-      }
-      ++hi;
-      ++lo;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(row_ptr + mid) <= next_entry)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      row = lo - 1;
-      e = __ldg(row_ptr + row + 1);
-    }
-    row_end = e;
-  };
-
-  int stage = 0;
-  for (int base = n0; base < n1; base += T) {
-    cp_async_wait<STAGES - 1>();
-    __syncwarp();
-    const int2* tile = &my[stage][g];
-    if (base + T <= n1 && row_end >= base + T) {
-      // Fast tile: all 32 entries belong to the current row.  Fully unrolled, every
-      // shared-memory offset is a compile-time constant, no tests between gathers.
-#pragma unroll
-      for (int s0 = 0; s0 < T / G; s0 += U) {
-        float4 b[U];
-        float v[U];
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-          const int2 e = tile[(s0 + i) * G];   // one broadcast per group
-          v[i] = __int_as_float(e.y);
-          b[i] = ld_gather<HINT>(Bl + (int64_t)e.x * K, policy);
-        }
-#pragma unroll
-        for (int i = 0; i < U; ++i) fma4(acc, v[i], b[i]);
-      }
-    } else {
-#pragma unroll 1
-      for (int u0 = 0; u0 < T; u0 += BATCH) {
-        const int j0 = base + u0;
-        if (j0 >= n1) break;
-        float4 b[U];
-        float v[U];
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-          const int2 e = tile[u0 + i * G];
-          v[i] = __int_as_float(e.y);
-          b[i] = ld_gather<HINT>(Bl + (int64_t)e.x * K, policy);
-        }
-        if (j0 + BATCH <= n1 && row_end >= j0 + BATCH) {
-#pragma unroll
-          for (int i = 0; i < U; ++i) fma4(acc, v[i], b[i]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < U; ++i) {
-            const int lo = j0 + i * G;
-            const int hi = min(lo + G, n1);
-            const int mine = lo + g;
-            int cur = lo;
-            while (row_end < hi) {   // warp-uniform: the current row ends inside this step
-              if (mine >= cur && mine < row_end) fma4(acc, v[i], b[i]);
-              cur = row_end;
-              finish_row(cur);
-            }
-            if (mine >= cur && mine < hi) fma4(acc, v[i], b[i]);
-          }
-        }
-      }
-    }
-    __syncwarp();
-    stage_tile(stage, base + STAGES * T);
-    stage ^= 1;
-  }
-  cp_async_wait<0>();
-
-  const bool hands_on = row_end != n1;   // the chunk ends inside `row`
-  if (!hands_on) {
-    store_row_sum<W>(C + (int64_t)row * K, acc, g, l);
-  } else {
-    const float4 t = reduce_groups<W>(acc);
-    if (g == 0) *reinterpret_cast<float4*>(carry_val + (int64_t)chunk * K + l * 4) = t;
-  }
-  if (!SETTLE) {
-    // a separate kernel adds the carries
-    if (lane == 0) carry_row[chunk] = hands_on ? row : -1;
-    return;
-  }
-
-  // the pieces of a split row settle it among themselves (settle_split_row)
-  const int r0 = __ldg(chunk_row + chunk);
-  const int r0_start = __ldg(row_ptr + r0), r0_end = __ldg(row_ptr + r0 + 1);
-  const bool stores_split_row = r0_start < n0 && r0_end <= n1;   // began in an earlier chunk, ends here
-  if (!hands_on && !stores_split_row) return;
-  __threadfence();
-  __syncwarp();   // every lane's part is visible before lane 0 bumps a counter
-  if (stores_split_row) settle_split_row<W>(r0, r0_end, S, row_ptr, carry_val, C, run_counter, (int)K);
-  if (hands_on) settle_split_row<W>(row, row_end, S, row_ptr, carry_val, C, run_counter, (int)K);
+  for (int r = 0; r < R; ++r) st_stream(crow + r * W * 4, acc[r]);
 }
 
 // ---- K = 128 with the rows of B fetched by TMA ----------------------------------------------------
-// Same chunks, same order of additions and same settlement as spmm_warp_kernel<32, ...>; what differs is
+// Same chunks, same order of additions and same settlement as spmm_warp_kernel at K = 128; what differs is
 // how a row of B (512 bytes) reaches the warp.  Lane 0 names four rows at a time to the tensor memory
 // accelerator (cp.async.bulk.tensor ... tile::gather4 on a tensor map of B whose box is one row), which
 // writes them into a ring of kTmaRing 2 KB buffers private to the warp and signals an mbarrier per buffer;
@@ -662,7 +212,7 @@ spmm_tma_kernel(const __grid_constant__ CUtensorMap map_b, int M, int n_chunks, 
   constexpr int64_t K = KW;
   extern __shared__ __align__(1024) unsigned char tma_smem[];
   if ((int)blockIdx.x >= n_chunk_blocks) {
-    zero_empty_rows(M, KW, row_ptr, C, blockIdx.x - n_chunk_blocks, gridDim.x - n_chunk_blocks, kTmaWarps * 32, K);
+    zero_empty_rows<KW>(M, KW, row_ptr, C, blockIdx.x - n_chunk_blocks, gridDim.x - n_chunk_blocks, kTmaWarps * 32);
     return;
   }
   const int lane = threadIdx.x & 31;
@@ -809,46 +359,24 @@ spmm_tma_kernel(const __grid_constant__ CUtensorMap map_b, int M, int n_chunks, 
   const int r0_start = __ldg(row_ptr + r0), r0_end = __ldg(row_ptr + r0 + 1);
   const bool stores_split_row = r0_start < n0 && r0_end <= n1;   // began in an earlier chunk, ends here
   if (!hands_on && !stores_split_row) return;
-  __threadfence();
-  __syncwarp();
-  if (stores_split_row) settle_split_row<32>(r0, r0_end, S, row_ptr, carry_val, C, run_counter, KW);
-  if (hands_on) settle_split_row<32>(row, row_end, S, row_ptr, carry_val, C, run_counter, KW);
+  if (stores_split_row) settle_split_row<4, 32, 1>(r0, r0_start, r0_end, S, carry_val, C, run_counter, KW, KW);
+  if (hands_on)
+    settle_split_row<4, 32, 1>(row, __ldg(row_ptr + row), row_end, S, carry_val, C, run_counter, KW, KW);
 }
 
-// ---- generic kernel: any K -------------------------------------------------------------
-// One warp per chunk; lane l owns columns kb + (s*32 + l)*VEC .. +VEC-1 for s < NS, where
-// kb = blockIdx.y * (32*VEC*NS).  VEC = 4 needs K % 4 == 0.
-template <int VEC, int NS, bool ROWSPLIT>
+// ---- row-split kernel for any other K: one warp per row ------------------------------------------
+// Lane l owns columns kb + (s*32 + l)*VEC .. +VEC-1 for s < NS, where kb = blockIdx.y * (32*VEC*NS).
+// VEC = 4 needs K % 4 == 0.
+template <int VEC, int NS>
 __global__ void __launch_bounds__(kBlockThreads)
-spmm_generic_kernel(int M, int K, int n_chunks, int n_chunk_blocks, const int* __restrict__ row_ptr,
-                    const int* __restrict__ col_idx, const float* __restrict__ vals,
-                    const float* __restrict__ B, float* __restrict__ C,
-                    const int* __restrict__ chunk_start, const int* __restrict__ chunk_row,
-                    int* __restrict__ carry_row, float* __restrict__ carry_val,
-                    const int* __restrict__ chunk_order) {
-  if ((int)blockIdx.x >= n_chunk_blocks) {
-    if (blockIdx.y == 0)
-      zero_empty_rows(M, K, row_ptr, C, blockIdx.x - n_chunk_blocks, gridDim.x - n_chunk_blocks);
-    return;
-  }
+spmm_rowsplit_any_kernel(int M, int K, const int* __restrict__ row_ptr, const int* __restrict__ col_idx,
+                         const float* __restrict__ vals, const float* __restrict__ B, float* __restrict__ C) {
   const int lane = threadIdx.x & 31;
-  const int slot = (int)(((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) >> 5);
-  if (slot >= n_chunks) return;
-  const int worker = (!ROWSPLIT && chunk_order != nullptr) ? __ldg(chunk_order + slot) : slot;
+  const int row = (int)(((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) >> 5);
+  if (row >= M) return;
   const int kb = blockIdx.y * (32 * VEC * NS);
-
-  int n0, n1, row, row_end;
-  if (ROWSPLIT) {
-    row = worker;
-    n0 = __ldg(row_ptr + row);
-    n1 = __ldg(row_ptr + row + 1);
-    row_end = n1;
-  } else {
-    n0 = __ldg(chunk_start + worker);
-    n1 = __ldg(chunk_start + worker + 1);
-    row = __ldg(chunk_row + worker);
-    row_end = __ldg(row_ptr + row + 1);
-  }
+  const int n0 = __ldg(row_ptr + row);
+  const int n1 = __ldg(row_ptr + row + 1);
 
   float acc[NS][VEC];
   int colbase[NS];
@@ -860,21 +388,6 @@ spmm_generic_kernel(int M, int K, int n_chunks, int n_chunk_blocks, const int* _
 #pragma unroll
     for (int x = 0; x < VEC; ++x) acc[s][x] = 0.f;
   }
-
-  auto store_acc = [&](float* dst) {
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      if (!live[s]) continue;
-      if (VEC == 4) {
-        *reinterpret_cast<float4*>(dst + colbase[s]) =
-            make_float4(acc[s][0], acc[s][1], acc[s][2], acc[s][3]);
-      } else {
-#pragma unroll
-        for (int x = 0; x < VEC; ++x) dst[colbase[s] + x] = acc[s][x];
-      }
-    }
-  };
-
   for (int base = n0; base < n1; base += 32) {
     const int jj = base + lane;
     int mycol = 0;
@@ -888,545 +401,60 @@ spmm_generic_kernel(int M, int K, int n_chunks, int n_chunk_blocks, const int* _
       const int c = __shfl_sync(0xffffffffu, mycol, i);
       const float v = __shfl_sync(0xffffffffu, myval, i);
       const float* brow = B + (int64_t)c * K;
-      float bv[NS][VEC];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        if (live[s]) {
-          if (VEC == 4) {
-            const float4 t = __ldg(reinterpret_cast<const float4*>(brow + colbase[s]));
-            bv[s][0] = t.x;
-            bv[s][1] = t.y;
-            bv[s][2] = t.z;
-            bv[s][3] = t.w;
-          } else {
-#pragma unroll
-            for (int x = 0; x < VEC; ++x) bv[s][x] = __ldg(brow + colbase[s] + x);
-          }
-        } else {
-#pragma unroll
-          for (int x = 0; x < VEC; ++x) bv[s][x] = 0.f;
-        }
-      }
-      if (!ROWSPLIT && base + i == row_end) {
-        store_acc(C + (int64_t)row * K);
-#pragma unroll
-        for (int s = 0; s < NS; ++s)
-#pragma unroll
-          for (int x = 0; x < VEC; ++x) acc[s][x] = 0.f;
-        advance_row(row_ptr, M, base + i, row, row_end);
-      }
-#pragma unroll
-      for (int s = 0; s < NS; ++s)
-#pragma unroll
-        for (int x = 0; x < VEC; ++x) acc[s][x] = fmaf(v, bv[s][x], acc[s][x]);
-    }
-  }
-
-  if (ROWSPLIT || row_end == n1) {
-    store_acc(C + (int64_t)row * K);
-    if (!ROWSPLIT && lane == 0 && blockIdx.y == 0) carry_row[worker] = -1;
-  } else {
-    store_acc(carry_val + (int64_t)worker * K);
-    if (lane == 0 && blockIdx.y == 0) carry_row[worker] = row;
-  }
-}
-
-// ---- carries ---------------------------------------------------------------------------
-// Fix-up for K = 4*W in {32, 64, 128} when the nominal chunk size S is known.  A block takes
-// CB = 256 / W consecutive chunks, one group of W lanes per chunk, each lane owning four columns.
-// A row longer than S is cut at multiples of S only, so the carries of row r sit in chunks
-// first = row_ptr[r] / S .. last - 1 with last = (row_ptr[r+1] - 1) / S: the group of chunk `first`
-// needs two loads to know the whole run, where a scan of carry_row would take one round trip per
-// 32 chunks.  Short runs (a row of 300 entries has one or two carries) are summed by that group;
-// tens of thousands of such independent walks hide each other's latency.  A run longer than
-// kLongRun (a row of many thousand entries; at most one can start in a block, since it covers every
-// later chunk of the block) is summed by the whole block: group g takes carries g, g + CB, ..., and
-// the groups are combined pairwise in shared memory in a fixed order.
-// The order of additions depends only on the chunking, never on timing.
-constexpr int kLongRun = 32;
-
-template <int W>
-__global__ void __launch_bounds__(kBlockThreads)
-carry_fixup_grouped_kernel(int n_chunks, int S, const int* __restrict__ row_ptr,
-                           const int* __restrict__ carry_row, const float* __restrict__ carry_val,
-                           float* __restrict__ C, int ld) {
-  const int64_t K = ld;   // row stride of C and of the carry slots; the slab is 4 * W columns wide
-  constexpr int CB = kBlockThreads / W;
-  __shared__ int long_head, long_len, long_row;
-  __shared__ float4 part[CB][W];
-  const int g = threadIdx.x / W, l = threadIdx.x % W;
-  const int64_t c = (int64_t)blockIdx.x * CB + g;
-  if (threadIdx.x == 0) long_len = 0;
-  __syncthreads();
-
-  const int row = c < n_chunks ? carry_row[c] : -1;
-  if (row >= 0) {
-    const int first = __ldg(row_ptr + row) / S;
-    if (c == first) {
-      const int len = (__ldg(row_ptr + row + 1) - 1) / S - first;
-      if (len > kLongRun) {
-        if (l == 0) {
-          long_head = g;
-          long_len = len;
-          long_row = row;
-        }
-      } else {
-        const float* src = carry_val + c * K + l * 4;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        int i = 0;
-        for (; i + 4 <= len; i += 4) {
-          float4 v[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const float4*>(src + (int64_t)(i + u) * K);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            s.x += v[u].x;
-            s.y += v[u].y;
-            s.z += v[u].z;
-            s.w += v[u].w;
-          }
-        }
-        for (; i < len; ++i) {
-          const float4 v = *reinterpret_cast<const float4*>(src + (int64_t)i * K);
-          s.x += v.x;
-          s.y += v.y;
-          s.z += v.z;
-          s.w += v.w;
-        }
-        float4* out = reinterpret_cast<float4*>(C + (int64_t)row * K + l * 4);
-        float4 o = *out;
-        o.x += s.x;
-        o.y += s.y;
-        o.z += s.z;
-        o.w += s.w;
-        *out = o;
-      }
-    }
-  }
-  __syncthreads();
-  const int len = long_len;
-  if (len == 0) return;   // block-uniform
-
-  const float* src = carry_val + ((int64_t)blockIdx.x * CB + long_head) * K + l * 4;
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-  int i = g;
-  for (; i + 3 * CB < len; i += 4 * CB) {
-    float4 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const float4*>(src + (int64_t)(i + u * CB) * K);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      s.x += v[u].x;
-      s.y += v[u].y;
-      s.z += v[u].z;
-      s.w += v[u].w;
-    }
-  }
-  for (; i < len; i += CB) {
-    const float4 v = *reinterpret_cast<const float4*>(src + (int64_t)i * K);
-    s.x += v.x;
-    s.y += v.y;
-    s.z += v.z;
-    s.w += v.w;
-  }
-  part[g][l] = s;
-  __syncthreads();
-#pragma unroll
-  for (int o = CB / 2; o > 0; o >>= 1) {
-    if (g < o) {
-      const float4 a = part[g][l], b = part[g + o][l];
-      part[g][l] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-    }
-    __syncthreads();
-  }
-  if (g == 0) {
-    const float4 t = part[0][l];
-    float4* out = reinterpret_cast<float4*>(C + (int64_t)long_row * K + l * 4);
-    float4 o = *out;
-    o.x += t.x;
-    o.y += t.y;
-    o.z += t.z;
-    o.w += t.w;
-    *out = o;
-  }
-}
-
-// Fix-up for any other K: one lane per chunk finds the first carry of each split row; the warp then
-// counts that row's carries (32 at a time) and sums them in chunk order, lanes owning columns.
-__global__ void __launch_bounds__(kBlockThreads)
-carry_fixup_kernel(int K, int n_chunks, const int* __restrict__ carry_row,
-                   const float* __restrict__ carry_val, float* __restrict__ C) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) >> 5;
-  const int64_t c0 = warp * 32;
-  if (c0 >= n_chunks) return;
-  const int64_t c = c0 + lane;
-  const int row = c < n_chunks ? carry_row[c] : -1;
-  const int prev = (c > 0 && c < n_chunks) ? carry_row[c - 1] : -1;
-  unsigned m = __ballot_sync(0xffffffffu, row >= 0 && row != prev);
-  while (m) {
-    const int bpos = __ffs(m) - 1;
-    m &= m - 1;
-    const int hr = __shfl_sync(0xffffffffu, row, bpos);
-    const int64_t first = c0 + bpos;
-    // length of the run of carries that belong to row hr
-    int64_t len = 0;
-    for (int64_t w = first;; w += 32) {
-      const int64_t cc = w + lane;
-      const bool same = cc < n_chunks && carry_row[cc] == hr;
-      const unsigned bm = __ballot_sync(0xffffffffu, same);
-      if (bm == 0xffffffffu) {
-        len += 32;
-        continue;
-      }
-      len += __ffs(~bm) - 1;
-      break;
-    }
-    float* crow = C + (int64_t)hr * K;
-    const float* src = carry_val + first * K;
-    if ((K & 3) == 0) {
-      for (int col = lane * 4; col < K; col += 128) {
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int64_t i = 0; i < len; ++i) {
-          const float4 t = *reinterpret_cast<const float4*>(src + i * K + col);
-          s.x += t.x;
-          s.y += t.y;
-          s.z += t.z;
-          s.w += t.w;
-        }
-        float4 o = *reinterpret_cast<float4*>(crow + col);
-        o.x += s.x;
-        o.y += s.y;
-        o.z += s.z;
-        o.w += s.w;
-        *reinterpret_cast<float4*>(crow + col) = o;
-      }
-    } else {
-      for (int col = lane; col < K; col += 32) {
-        float s = 0.f;
-        for (int64_t i = 0; i < len; ++i) s += src[i * K + col];
-        crow[col] += s;
-      }
-    }
-  }
-}
-
-// ---- COO, accumulate -------------------------------------------------------------------
-// ---- COO warp kernel: K = 4 * W in {32, 64, 128} --------------------------------------------
-// C += A * B from (row, col, val) triples in any order; zero-valued entries (the padding) are
-// skipped.  Same machinery as the CSR warp kernel: one warp per S consecutive triples, G = 32 / W
-// lane groups that each gather a whole row of B per step, tiles of 32 triples staged global ->
-// shared with cp.async two tiles ahead, U steps of gathers in flight, an unrolled path for tiles
-// that lie inside one row.  Row boundaries come from the staged row ids (one ballot per tile)
-// instead of row_ptr; every run of equal row ids ends in one cross-group reduction and one
-// 16-byte vector reduction per lane of group 0 into C.
-template <int W, int U, int BT, bool STRIDED>
-__global__ void __launch_bounds__(BT, 16)
-spmm_coo_warp_kernel(int64_t nnz, int S, const int* __restrict__ row_idx, const int* __restrict__ col_idx,
-                     const float* __restrict__ vals, const float* __restrict__ B, float* __restrict__ C, int ld) {
-  // a slab of 4 * W columns; STRIDED: part of wider B and C with row stride ld
-  const int64_t K = STRIDED ? (int64_t)ld : (int64_t)(4 * W);
-  constexpr int G = 32 / W;
-  constexpr int T = 32;
-  constexpr int BATCH = U * G;
-  constexpr int STAGES = 2;
-  static_assert(BATCH <= T && T % BATCH == 0, "batch must tile the staged tile");
-  __shared__ int2 cv_tiles[BT / 32][STAGES][T];
-  __shared__ int row_tiles[BT / 32][STAGES][T];
-
-  const int lane = threadIdx.x & 31;
-  const int g = lane / W, l = lane % W;
-  const int64_t worker = ((int64_t)blockIdx.x * BT + threadIdx.x) >> 5;
-  const int64_t n0 = worker * S;
-  if (n0 >= nnz) return;
-  const int64_t n1 = min(nnz, n0 + (int64_t)S);
-  int2(*cv)[T] = cv_tiles[threadIdx.x >> 5];
-  int(*rw)[T] = row_tiles[threadIdx.x >> 5];
-
-  auto stage_tile = [&](int stage, int64_t base) {
-    const int64_t j = base + lane;
-    if (j < n1) {
-      cp_async_4(&cv[stage][lane].x, col_idx + j);
-      cp_async_4(&cv[stage][lane].y, vals + j);
-      cp_async_4(&rw[stage][lane], row_idx + j);
-    } else {
-      cv[stage][lane] = make_int2(0, 0);   // past the chunk: column 0, value 0 (skipped)
-      rw[stage][lane] = -1;
-    }
-    cp_async_commit();
-  };
-  stage_tile(0, n0);
-  stage_tile(1, n0 + T);
-
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float* Bl = B + l * 4;
-  int cur_row = -1;   // row of the run being accumulated
-
-  auto flush = [&]() {
-    if (cur_row >= 0) {   // warp-uniform
-      if (W == 16) {
-        // the groups split the sum and every lane adds a float2: 0.378 -> 0.365 ms at K = 64 on the R-MAT
-        // bench graph.  At K = 32 thirty-two scalar reductions per row cost more than eight 16-byte ones
-        // save in shuffles (0.233 -> 0.236 ms), so that width keeps the full reduction.
-        store_row_sum<W, true>(C + (int64_t)cur_row * K, acc, g, l);
-      } else {
-        const float4 t = reduce_groups<W>(acc);
-        if (g == 0) red_add_v4(C + (int64_t)cur_row * K + l * 4, t);
-      }
-    }
-    acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-
-  int stage = 0;
-  for (int64_t base = n0; base < n1; base += T) {
-    cp_async_wait<STAGES - 1>();
-    __syncwarp();
-    // bit e: triple e of the tile starts a new run (its row differs from its predecessor's);
-    // triples past the chunk carry row -1 and never match, which ends the last run
-    const int my_row = rw[stage][lane];
-    const int prev_row = lane == 0 ? cur_row : rw[stage][lane - 1];
-    unsigned bnd = __ballot_sync(0xffffffffu, my_row != prev_row);
-    const int2* tile = &cv[stage][g];
-    if (bnd == 0u) {
-      // the whole tile continues the current run
-#pragma unroll
-      for (int s0 = 0; s0 < T / G; s0 += U) {
-        float4 b[U];
-        float v[U];
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-          const int2 e = tile[(s0 + i) * G];
-          v[i] = __int_as_float(e.y);
-          b[i] = ld_gather<false>(Bl + (int64_t)e.x * K, 0ull);
-        }
-#pragma unroll
-        for (int i = 0; i < U; ++i)
-          if (v[i] != 0.f) fma4(acc, v[i], b[i]);
-      }
-    } else {
-      const int limit = (int)min((int64_t)T, n1 - base);   // triples of this tile inside the chunk
-#pragma unroll 1
-      for (int u0 = 0; u0 < T; u0 += BATCH) {
-        if (u0 >= limit) break;
-        float4 b[U];
-        float v[U];
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-          const int2 e = tile[u0 + i * G];
-          v[i] = __int_as_float(e.y);
-          b[i] = ld_gather<false>(Bl + (int64_t)e.x * K, 0ull);
-        }
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-          const int lo = u0 + i * G;
-          const int hi = min(lo + G, limit);
-          const int mine = lo + g;
-          int cur = lo;
-          // warp-uniform: runs that start inside this step
-          unsigned m = hi > lo ? (bnd >> lo) & ((1u << (hi - lo)) - 1u) : 0u;
-          while (m) {
-            const int p = lo + __ffs(m) - 1;
-            m &= m - 1;
-            if (mine >= cur && mine < p && v[i] != 0.f) fma4(acc, v[i], b[i]);
-            flush();
-            cur_row = rw[stage][p];
-            cur = p;
-          }
-          if (mine >= cur && mine < hi && v[i] != 0.f) fma4(acc, v[i], b[i]);
-        }
-      }
-    }
-    // the last triple's row carries into the next tile's first comparison
-    __syncwarp();
-    stage_tile(stage, base + STAGES * T);
-    stage ^= 1;
-  }
-  cp_async_wait<0>();
-  flush();
-}
-
-// C += A * B from (row, col, val) triples in any order; zero-valued padding is skipped.
-// One warp per run of S entries; a lane owns columns (s*32 + lane)*VEC of a 128*VEC-wide
-// column block.  Partial sums leave through vector reductions on every row change.
-template <int VEC, int NS>
-__global__ void __launch_bounds__(kBlockThreads)
-spmm_coo_kernel(int K, int64_t nnz, int S, const int* __restrict__ row_idx,
-                const int* __restrict__ col_idx, const float* __restrict__ vals,
-                const float* __restrict__ B, float* __restrict__ C) {
-  const int lane = threadIdx.x & 31;
-  const int64_t worker = ((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) >> 5;
-  const int64_t n0 = worker * S;
-  if (n0 >= nnz) return;
-  const int64_t n1 = min(nnz, n0 + S);
-  const int kb = blockIdx.y * (32 * VEC * NS);
-
-  float acc[NS][VEC];
-  int colbase[NS];
-  bool live[NS];
-#pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    colbase[s] = kb + (s * 32 + lane) * VEC;
-    live[s] = colbase[s] < K;
-#pragma unroll
-    for (int x = 0; x < VEC; ++x) acc[s][x] = 0.f;
-  }
-  int cur_row = -1;
-  bool dirty = false;
-
-  auto flush = [&]() {
-    if (!dirty) return;
-    float* crow = C + (int64_t)cur_row * K;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      if (live[s]) {
-        if (VEC == 4) {
-          red_add_v4(crow + colbase[s], make_float4(acc[s][0], acc[s][1], acc[s][2], acc[s][3]));
-        } else {
-#pragma unroll
-          for (int x = 0; x < VEC; ++x) atomicAdd(crow + colbase[s] + x, acc[s][x]);
-        }
-      }
-#pragma unroll
-      for (int x = 0; x < VEC; ++x) acc[s][x] = 0.f;
-    }
-    dirty = false;
-  };
-
-  for (int64_t base = n0; base < n1; base += 32) {
-    const int64_t jj = base + lane;
-    int myrow = 0, mycol = 0;
-    float myval = 0.f;
-    if (jj < n1) {
-      myrow = ld_stream(row_idx + jj);
-      mycol = ld_stream(col_idx + jj);
-      myval = ld_stream(vals + jj);
-    }
-    const int cnt = (int)min((int64_t)32, n1 - base);
-    for (int i = 0; i < cnt; ++i) {
-      const int r = __shfl_sync(0xffffffffu, myrow, i);
-      const int c = __shfl_sync(0xffffffffu, mycol, i);
-      const float v = __shfl_sync(0xffffffffu, myval, i);
-      if (v == 0.f) continue;  // padding (and explicit zeros) contribute nothing
-      if (r != cur_row) {
-        flush();
-        cur_row = r;
-      }
-      const float* brow = B + (int64_t)c * K;
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
         if (!live[s]) continue;
         if (VEC == 4) {
           const float4 t = __ldg(reinterpret_cast<const float4*>(brow + colbase[s]));
           acc[s][0] = fmaf(v, t.x, acc[s][0]);
-          acc[s][1] = fmaf(v, t.y, acc[s][1]);
-          acc[s][2] = fmaf(v, t.z, acc[s][2]);
-          acc[s][3] = fmaf(v, t.w, acc[s][3]);
+          acc[s][VEC > 1 ? 1 : 0] = fmaf(v, t.y, acc[s][VEC > 1 ? 1 : 0]);
+          acc[s][VEC > 2 ? 2 : 0] = fmaf(v, t.z, acc[s][VEC > 2 ? 2 : 0]);
+          acc[s][VEC > 3 ? 3 : 0] = fmaf(v, t.w, acc[s][VEC > 3 ? 3 : 0]);
         } else {
 #pragma unroll
           for (int x = 0; x < VEC; ++x) acc[s][x] = fmaf(v, __ldg(brow + colbase[s] + x), acc[s][x]);
         }
       }
-      dirty = true;
     }
   }
-  flush();
+  float* dst = C + (int64_t)row * K;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    if (!live[s]) continue;
+#pragma unroll
+    for (int x = 0; x < VEC; ++x) dst[colbase[s] + x] = acc[s][x];
+  }
 }
 
-template <int W, int R, int U, int MINB>
-int launch_balanced(hpspmm_ctx* ctx, bool hint, bool rowsplit, int M, int n_chunks,
-                    const int32_t* row_ptr, const int32_t* col_idx, const float* vals,
-                    const float* B, float* C, const int32_t* chunk_start, const int32_t* chunk_row,
-                    int32_t* carry_row, float* carry_val, cudaStream_t stream) {
-  const int workers_per_block = kBlockThreads / W;
-  const int n_chunk_blocks = (n_chunks + workers_per_block - 1) / workers_per_block;
-  int n_zero_blocks = 0;
-  if (!rowsplit) {
-    n_zero_blocks = (M + kBlockThreads - 1) / kBlockThreads;
-    const int cap = ctx->sm_count * 2;
-    if (n_zero_blocks > cap) n_zero_blocks = cap;
-  }
-  const unsigned grid = (unsigned)(n_chunk_blocks + n_zero_blocks);
-  if (grid == 0) return HPSPMM_OK;
-#define HPSPMM_LAUNCH(H, RS)                                                                   \
-  spmm_subwarp_kernel<W, R, U, MINB, H, RS><<<grid, kBlockThreads, 0, stream>>>(                    \
-      M, n_chunks, n_chunk_blocks, row_ptr, col_idx, vals, B, C, chunk_start, chunk_row,       \
-      carry_row, carry_val)
-  if (rowsplit) {
-    if (hint) HPSPMM_LAUNCH(true, true); else HPSPMM_LAUNCH(false, true);
-  } else {
-    if (hint) HPSPMM_LAUNCH(true, false); else HPSPMM_LAUNCH(false, false);
-  }
-#undef HPSPMM_LAUNCH
-  ctx->launches++;
-  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
-  return HPSPMM_OK;
-}
-
-// rows that hold entries, as a plan lists them (all null without a plan)
-struct row_list {
-  const int32_t* nz_id;
-  const int32_t* nz_end;
-  const int32_t* chunk_ri;
-};
-
-template <int W, int U, int MINB, int BT = kBlockThreads, bool STRIDED = false>
-int launch_warp(hpspmm_ctx* ctx, bool hint, int M, int n_chunks, const int32_t* row_ptr,
-                const int32_t* col_idx, const float* vals, const float* B, float* C,
-                const int32_t* chunk_start, const int32_t* chunk_row, int32_t* carry_row,
-                float* carry_val, const int32_t* chunk_order, int S, int* run_counter, cudaStream_t stream,
-                int ld = 4 * W, row_list rows = row_list{nullptr, nullptr, nullptr}) {
-  const int chunks_per_block = BT / 32;
-  const int n_chunk_blocks = (n_chunks + chunks_per_block - 1) / chunks_per_block;
-  int n_zero_blocks = (M + BT - 1) / BT;
-  const int cap = ctx->sm_count * 2 * (kBlockThreads / BT);
-  if (n_zero_blocks > cap) n_zero_blocks = cap;
-  const unsigned grid = (unsigned)(n_chunk_blocks + n_zero_blocks);
-  if (grid == 0) return HPSPMM_OK;
-#define HPSPMM_LAUNCH_WARP(H, ST, CP)                                                           \
-  spmm_warp_kernel<W, U, MINB, H, BT, ST, STRIDED, CP><<<grid, BT, 0, stream>>>(                   \
-      M, n_chunks, n_chunk_blocks, row_ptr, col_idx, vals, B, C, chunk_start, chunk_row, carry_row, \
-      carry_val, chunk_order, S, run_counter, ld, rows.nz_id, rows.nz_end, rows.chunk_ri)
-  const bool compact = rows.nz_id != nullptr;
-  if (run_counter != nullptr) {
-    if (hint) { if (compact) HPSPMM_LAUNCH_WARP(true, true, true); else HPSPMM_LAUNCH_WARP(true, true, false); }
-    else { if (compact) HPSPMM_LAUNCH_WARP(false, true, true); else HPSPMM_LAUNCH_WARP(false, true, false); }
-  } else {
-    if (hint) { if (compact) HPSPMM_LAUNCH_WARP(true, false, true); else HPSPMM_LAUNCH_WARP(true, false, false); }
-    else { if (compact) HPSPMM_LAUNCH_WARP(false, false, true); else HPSPMM_LAUNCH_WARP(false, false, false); }
-  }
-#undef HPSPMM_LAUNCH_WARP
-  ctx->launches++;
-  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
-  return HPSPMM_OK;
-}
-
-template <int VEC>
-int launch_generic(hpspmm_ctx* ctx, bool rowsplit, int M, int K, int n_chunks,
-                   const int32_t* row_ptr, const int32_t* col_idx, const float* vals,
-                   const float* B, float* C, const int32_t* chunk_start, const int32_t* chunk_row,
-                   int32_t* carry_row, float* carry_val, const int32_t* chunk_order,
-                   cudaStream_t stream) {
-  constexpr int NS = 4;
-  const int kblock = 32 * VEC * NS;
-  const int n_kblocks = (K + kblock - 1) / kblock;
-  const int n_chunk_blocks = (n_chunks + kBlockThreads / 32 - 1) / (kBlockThreads / 32);
-  int n_zero_blocks = 0;
-  if (!rowsplit) {
-    n_zero_blocks = (M + kBlockThreads - 1) / kBlockThreads;
-    const int cap = ctx->sm_count * 2;
-    if (n_zero_blocks > cap) n_zero_blocks = cap;
-  }
-  const dim3 grid((unsigned)(n_chunk_blocks + n_zero_blocks), (unsigned)n_kblocks, 1);
-  if (grid.x == 0) return HPSPMM_OK;
-  if (n_kblocks > 65535) return HPSPMM_ERR_UNSUPPORTED;
-  if (rowsplit)
-    spmm_generic_kernel<VEC, NS, true><<<grid, kBlockThreads, 0, stream>>>(
-        M, K, n_chunks, n_chunk_blocks, row_ptr, col_idx, vals, B, C, chunk_start, chunk_row,
-        carry_row, carry_val, nullptr);
+template <int W>
+void launch_rowsplit(bool hint, int M, const int32_t* row_ptr, const int32_t* col_idx, const float* vals,
+                     const float* B, float* C, cudaStream_t stream) {
+  constexpr int workers_per_block = kBlockThreads / W;
+  const unsigned grid = (unsigned)(((int64_t)M + workers_per_block - 1) / workers_per_block);
+  if (hint)
+    spmm_rowsplit_kernel<W, 1, 8, 4, true><<<grid, kBlockThreads, 0, stream>>>(M, row_ptr, col_idx, vals, B, C);
   else
-    spmm_generic_kernel<VEC, NS, false><<<grid, kBlockThreads, 0, stream>>>(
-        M, K, n_chunks, n_chunk_blocks, row_ptr, col_idx, vals, B, C, chunk_start, chunk_row,
-        carry_row, carry_val, chunk_order);
+    spmm_rowsplit_kernel<W, 1, 8, 4, false><<<grid, kBlockThreads, 0, stream>>>(M, row_ptr, col_idx, vals, B, C);
+}
+
+int run_rowsplit(hpspmm_ctx* ctx, bool hint, int M, int64_t K, const int32_t* row_ptr, const int32_t* col_idx,
+                 const float* vals, const float* B, float* C, cudaStream_t stream) {
+  if (K == 32) {
+    launch_rowsplit<8>(hint, M, row_ptr, col_idx, vals, B, C, stream);
+  } else if (K == 64) {
+    launch_rowsplit<16>(hint, M, row_ptr, col_idx, vals, B, C, stream);
+  } else if (K == 128) {
+    launch_rowsplit<32>(hint, M, row_ptr, col_idx, vals, B, C, stream);
+  } else {
+    const int kblock = 32 * 4 * ((K & 3) == 0 ? 4 : 1);
+    const int64_t n_kblocks = (K + kblock - 1) / kblock;
+    if (n_kblocks > 65535) return HPSPMM_ERR_UNSUPPORTED;
+    const dim3 grid((unsigned)((M + kBlockThreads / 32 - 1) / (kBlockThreads / 32)), (unsigned)n_kblocks, 1);
+    if ((K & 3) == 0)
+      spmm_rowsplit_any_kernel<4, 4><<<grid, kBlockThreads, 0, stream>>>(M, (int)K, row_ptr, col_idx, vals, B, C);
+    else
+      spmm_rowsplit_any_kernel<1, 4><<<grid, kBlockThreads, 0, stream>>>(M, (int)K, row_ptr, col_idx, vals, B, C);
+  }
   ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;
@@ -1457,8 +485,8 @@ tensor_map_encode_fn tensor_map_encoder() {
 int launch_spmm_tma(hpspmm_ctx* ctx, int m, int nc, int64_t rows_b, const int32_t* row_ptr, const int32_t* col_idx,
                     const float* vals, const float* B, float* C, const int32_t* chunk_start,
                     const int32_t* chunk_row, float* carry_val, const int32_t* chunk_order, int S,
-                    int* run_counter, row_list rows, cudaStream_t stream) {
-  if (S <= 0 || S > kTmaMaxS || run_counter == nullptr || rows.nz_id == nullptr || rows_b <= 0) return 1;
+                    int* run_counter, const hpspmm_plan* rows, cudaStream_t stream) {
+  if (S <= 0 || S > kTmaMaxS || rows_b <= 0) return 1;
   tensor_map_encode_fn enc = tensor_map_encoder();
   if (!enc) return 1;
   CUtensorMap map_b;
@@ -1484,7 +512,7 @@ int launch_spmm_tma(hpspmm_ctx* ctx, int m, int nc, int64_t rows_b, const int32_
   if (grid == 0) return 0;
   spmm_tma_kernel<<<grid, kTmaWarps * 32, smem, stream>>>(map_b, m, nc, n_chunk_blocks, row_ptr, col_idx, vals, B, C,
                                                           chunk_start, chunk_row, carry_val, chunk_order, S,
-                                                          run_counter, rows.nz_id, rows.nz_end, rows.chunk_ri,
+                                                          run_counter, rows->nz_id, rows->nz_end, rows->chunk_ri,
                                                           ctx->flag + HPSPMM_FLAG_TMA_FALLBACKS);
   ctx->launches++;
   const cudaError_t e = cudaGetLastError();
@@ -1510,12 +538,19 @@ int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz) {
   // prologue (table loads, pipeline fill) and leave fewer carries.  Measured on B200 (R-MAT scale 20, product
   // time in ms at S = 128 / 256 / 320 / 512 / 1024): K = 32: 0.240 / 0.217 / 0.208 / 0.199 / 0.193;
   // K = 64: 0.356 / 0.314 / 0.307 / 0.310 / 0.306; K = 128: 0.630 / 0.563 / 0.563 / 0.595 / 0.592.
-  // Small matrices keep smaller chunks so that there are still several waves of them
-  // (148 SMs x 40 resident warps x 4).
   // Re-measured at K = 32 after the row-store exchange (S = 384 / 512 / 640 / 768 / 1024 / 1280 / 1536):
   // 0.195 / 0.189 / 0.186 / 0.185 / 0.182 / 0.193 / 0.212 ms.  The default stays at 512 all the same: plans are
   // shared with the SDDMM, which on the same graph takes 0.193 / 0.230 / 0.271 / 0.333 ms at S = 512 / 640 /
   // 768 / 1024.  A caller that builds a plan for products only can ask for 1024 (hpspmm_opts.chunk_nnz).
+  // Below 2.4 M entries there are fewer chunks than warps the GPU can hold, and the time is that of the longest
+  // chunk: a chain of gather round trips.  Measured in us at S = 32 / 64 / 128 / 256, rows of 16 entries on average,
+  // uniform and power-law columns: 12 K entries, K = 32: 3.7 / 4.5 / 6.3 / 10.1 and 6.6 / 7.7 / 10.3 / 13.9;
+  // 300 K, K = 64: 10.2 / 8.3 / 10.3 / 16.3 and 14.2 / 12.9 / 15.6 / 24.2; 1 M, K = 64: 24.3 / 21.0 / 21.4 / 22.7 and
+  // 37.5 / 26.7 / 23.8 / 32.2 (smaller chunks split more rows, and every split costs an exchange through memory).
+  // Beyond 64 columns a split costs as much but saves less, so chunks of 128 begin earlier.
+  if (nnz < 32000) return 32;
+  if (nnz < (K > 64 ? 150000 : 500000)) return 64;
+  if (nnz < 2400000) return 128;
   const int32_t floor_s = probing_chunk_nnz(K);
   const int32_t best = K <= 32 ? 512 : (K <= 64 ? 320 : 256);
   const int64_t want = nnz / 24000 / 32 * 32;
@@ -1524,16 +559,28 @@ int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz) {
   return (int32_t)s;
 }
 
-int hpspmm_launch_chunk_table(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr,
-                              int32_t chunk_nnz, int64_t n_chunks, int32_t* chunk_start,
-                              int32_t* chunk_row, int* split_count, cudaStream_t stream,
-                              int32_t* run_counter) {
-  const unsigned blocks = (unsigned)((n_chunks + 1 + 255) / 256);
-  chunk_table_kernel<<<blocks, 256, 0, stream>>>((int)M, (int)nnz, row_ptr, chunk_nnz, (int)n_chunks,
-                                                 chunk_start, chunk_row, split_count, run_counter);
-  ctx->launches++;
-  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
-  return HPSPMM_OK;
+int32_t hpspmm_coo_chunk_nnz(int64_t K, int64_t nnz) {
+  const int32_t best = probing_chunk_nnz(K);
+  const int64_t want = nnz / 6000 / 32 * 32;
+  return (int32_t)(want < 32 ? 32 : (want > best ? best : want));
+}
+
+int hpspmm_vector_width(int64_t K, uintptr_t addresses) {
+  // K % 4 == 0 is refused by the entry points unless the operands are 16-byte aligned
+  return (K & 3) == 0 ? 4 : ((K & 1) == 0 && (addresses & 7) == 0 ? 2 : 1);
+}
+
+hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, bool hint) {
+  hpspmm_spmm_shape sh;
+  sh.VEC = VEC;
+  sh.hint = hint;
+  sh.lat = false;
+  if (cols > hpspmm_widest_slab(VEC)) cols = hpspmm_widest_slab(VEC);
+  const int vecs = (int)((cols + VEC - 1) / VEC);
+  sh.W = VEC == 1 ? (vecs <= 1 ? 1 : 4) : 2;
+  while (sh.W < 32 && sh.W < vecs) sh.W *= 2;
+  sh.R = (vecs + 31) / 32;
+  return sh;
 }
 
 namespace {
@@ -1559,109 +606,57 @@ int check_spmm_args(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t nn
   return HPSPMM_OK;
 }
 
-// One slab of 4 * W columns with the warp kernel, then its carries.  STRIDED: the slab is part of wider
-// matrices (B, C and the carry slots have row stride ld, the pointers already point at the slab's first
-// column).  With a counter array, slabs of 64 or 128 columns add the carries themselves.  Measured on the
-// R-MAT bench graph against the separate fix-up launch: -6 % at 128 columns, -2 % at 64, but +7 % at 32,
-// where chunks are short and the device-wide fence every piece of a split row takes weighs more than the
-// launch saved.
-// Tuning on B200 (R-MAT scale 20): 64-thread blocks, U = 4 gather steps in flight per lane and at most
-// 51 registers (20 blocks per SM) beat 128/256-thread blocks, U = 2/8/16 and the 32/40/64/80-register
-// builds at every width.
-template <int W, bool STRIDED>
-int run_slab(hpspmm_ctx* ctx, bool hint, int m, int nc, const int32_t* row_ptr, const int32_t* col_idx,
-             const float* vals, const float* B, float* C, const int32_t* chunk_start,
-             const int32_t* chunk_row, int32_t* carry_row, float* carry_val, const int32_t* chunk_order,
-             bool need_fixup, cudaStream_t stream, int S, int* run_counter, int ld, row_list rows) {
-  const bool settle = run_counter != nullptr && W >= 16;
-  // strided slabs carry two more live values (the stride) and spill at 48 registers: 16 blocks per SM
-  // (64 registers) took the K = 256 product from 1.44 to 1.20 ms
-  constexpr int MINB = STRIDED ? 16 : HPSPMM_WARP_MINB;
-  int st = launch_warp<W, 4, MINB, 64, STRIDED>(ctx, hint, m, nc, row_ptr, col_idx, vals, B, C, chunk_start,
-                                                chunk_row, carry_row, carry_val, chunk_order, S,
-                                                settle ? run_counter : nullptr, stream, ld, rows);
-  if (st != HPSPMM_OK) return st;
-  if (need_fixup && nc > 0 && !settle) {
-    if (S > 0) {
-      const unsigned gblocks = (unsigned)(((int64_t)nc * W + kBlockThreads - 1) / kBlockThreads);
-      carry_fixup_grouped_kernel<W><<<gblocks, kBlockThreads, 0, stream>>>(nc, S, row_ptr, carry_row, carry_val,
-                                                                         C, ld);
-    } else {
-      const unsigned blocks = (unsigned)((nc + kBlockThreads - 1) / kBlockThreads);
-      carry_fixup_kernel<<<blocks, kBlockThreads, 0, stream>>>(4 * W, nc, carry_row, carry_val, C);
-    }
-    ctx->launches++;
-    HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
+// shared_counters: the scratch holds one counter per chunk, so the slabs of a wide product run one after the other
+int launch_spmm(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool hint, bool shared_counters, cudaStream_t s) {
+  const int VEC = hpspmm_vector_width(a.K, (uintptr_t)a.B | (uintptr_t)a.C);
+  int32_t* counter = a.counter;
+  a.keep_b = hint ? 1 : 0;
+  for (a.off = 0; a.off < a.K; a.off += a.cols) {
+    a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
+    if (!shared_counters) a.counter = counter + (int64_t)(a.off / 32) * a.n_chunks;
+    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hint);
+    // Few chunks: registers are plenty, so a warp keeps 8 to 32 gather steps in flight instead of 4 (the same order of
+    // additions).  67.6 K entries in chunks of 64: 6.1 -> 5.6 us at K = 64, 9.1 -> 7.2 us at K = 128; with more chunks
+    // than these builds have resident warps they lose (300 K entries, K = 64: 8.3 -> 10.5 us).
+    sh.lat = a.n_chunks <= ctx->sm_count * (sh.W <= 8 ? 24 : 16);
+    const int st = VEC == 4   ? hpspmm_spmm_launch_v4(ctx, a, sh, shared_counters, s)
+                   : VEC == 2 ? hpspmm_spmm_launch_v2(ctx, a, sh, shared_counters, s)
+                              : hpspmm_spmm_launch_v1(ctx, a, sh, shared_counters, s);
+    if (st != HPSPMM_OK) return st;
   }
   return HPSPMM_OK;
 }
 
-int run_spmm(hpspmm_ctx* ctx, bool hint, bool rowsplit, int64_t M, int64_t K, int64_t n_chunks,
-             const int32_t* row_ptr, const int32_t* col_idx, const float* vals, const float* B,
-             float* C, const int32_t* chunk_start, const int32_t* chunk_row, int32_t* carry_row,
-             float* carry_val, const int32_t* chunk_order, bool need_fixup, cudaStream_t stream,
-             int S = 0, int* run_counter = nullptr, row_list rows = row_list{nullptr, nullptr, nullptr},
-             int64_t tma_rows_b = 0) {
-  int st;
-  const int m = (int)M, nc = (int)n_chunks;
-  if (!rowsplit && K == 128 && tma_rows_b > 0) {
-    // B through the tensor memory accelerator (HPSPMM_ALGO_TMA); falls through when that path declines
-    const int r = launch_spmm_tma(ctx, m, nc, tma_rows_b, row_ptr, col_idx, vals, B, C, chunk_start, chunk_row,
-                                  carry_val, chunk_order, S, run_counter, rows, stream);
-    if (r == 0) return HPSPMM_OK;
-    if (r < 0) return HPSPMM_ERR_CUDA;   // the launcher has recorded the message
-  }
-#define HPSPMM_ARGS ctx, hint, rowsplit, m, nc, row_ptr, col_idx, vals, B, C, chunk_start, chunk_row, carry_row, carry_val, stream
-#define HPSPMM_SLAB(W, STRIDED, off) \
-  run_slab<W, STRIDED>(ctx, hint, m, nc, row_ptr, col_idx, vals, B + (off), C + (off), chunk_start, chunk_row, \
-                       carry_row, carry_val + (off), chunk_order, need_fixup, stream, S, run_counter, (int)K, rows)
-  if (rowsplit && (K == 32 || K == 64 || K == 128)) {
-    st = K == 32 ? launch_balanced<8, 1, 8, 4>(HPSPMM_ARGS)
-                 : (K == 64 ? launch_balanced<16, 1, 8, 4>(HPSPMM_ARGS) : launch_balanced<32, 1, 8, 4>(HPSPMM_ARGS));
-    return st;
-  }
-  if (!rowsplit && K == 32) return HPSPMM_SLAB(8, false, 0);
-  if (!rowsplit && K == 64) return HPSPMM_SLAB(16, false, 0);
-  if (!rowsplit && K == 128) return HPSPMM_SLAB(32, false, 0);
-  if (!rowsplit && K % 32 == 0 && S > 0 && K <= 512) {
-    // any other multiple of 32 up to 512: column slabs of 128, then 64 and/or 32, each a strided run of the
-    // warp kernel (the sparse stream is read once per slab, as the reference's K / 32 grid rows read it).
-    // Measured on the R-MAT bench graph against the generic kernel: K = 96 0.73 vs 1.33 ms, 160 0.95 vs 1.49,
-    // 256 1.20 vs 1.61, 512 2.42 vs 2.51; beyond that the generic kernel's 2 KB contiguous gathers win.
-    int64_t off = 0;
-    while (K - off >= 128) {
-      st = HPSPMM_SLAB(32, true, off);
-      if (st != HPSPMM_OK) return st;
-      off += 128;
-    }
-    if (K - off >= 64) {
-      st = HPSPMM_SLAB(16, true, off);
-      if (st != HPSPMM_OK) return st;
-      off += 64;
-    }
-    if (K - off >= 32) {
-      st = HPSPMM_SLAB(8, true, off);
-      if (st != HPSPMM_OK) return st;
-    }
-    return HPSPMM_OK;
-  }
-#undef HPSPMM_ARGS
-#undef HPSPMM_SLAB
-  if ((K & 3) == 0)
-    st = launch_generic<4>(ctx, rowsplit, m, (int)K, nc, row_ptr, col_idx, vals, B, C, chunk_start,
-                           chunk_row, carry_row, carry_val, chunk_order, stream);
-  else
-    st = launch_generic<1>(ctx, rowsplit, m, (int)K, nc, row_ptr, col_idx, vals, B, C, chunk_start,
-                           chunk_row, carry_row, carry_val, chunk_order, stream);
-  if (st != HPSPMM_OK) return st;
-  if (!rowsplit && need_fixup && n_chunks > 0) {
-    const unsigned blocks = (unsigned)((n_chunks + kBlockThreads - 1) / kBlockThreads);
-    carry_fixup_kernel<<<blocks, kBlockThreads, 0, stream>>>((int)K, nc, carry_row, carry_val, C);
-    ctx->launches++;
-    HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
-  }
-  return HPSPMM_OK;
+bool gather_hint(int64_t K, const hpspmm_opts* opts) {
+  // evict-last on the gathers of B, R-MAT bench graph, on / off, one width timed alone: K = 128 0.555 / 0.591 ms,
+  // K = 64 0.307 / 0.304, K = 32 0.189 / 0.1885.  Inside a step of three products run back to back K = 64 measures
+  // the other way round (0.311 on, 0.313 off), so 64 columns stay on.
+  const int mode = opts ? opts->b_l2_hint : 0;
+  return mode == 2 || (mode == 0 && K >= 64);
 }
+
+}  // namespace
+
+namespace {
+
+int32_t planless_chunk_nnz(int64_t K, int64_t nnz, const hpspmm_opts* opts) {
+  const int32_t S = (opts && opts->chunk_nnz > 0) ? opts->chunk_nnz : hpspmm_default_chunk_nnz(K, nnz);
+  return (S + 31) / 32 * 32;
+}
+
+// where a plan-less product keeps what it builds, inside the context's scratch
+struct planless_layout {
+  size_t tiles, counter, rec, nz, carry, bytes;
+  planless_layout(int64_t M, int64_t K, int64_t n_chunks) {
+    bytes = 0;
+    auto take = [&](size_t b) { const size_t at = bytes; bytes += align_up(b, 256); return at; };
+    tiles = take((size_t)hpspmm_row_tiles(M) * 4);
+    counter = take((size_t)(n_chunks + 1) * (size_t)hpspmm_counter_slabs(K) * 4);
+    rec = take((size_t)(n_chunks + 1) * 32);
+    nz = take(hpspmm_nz_bytes(M));
+    carry = take((size_t)(n_chunks + 1) * (size_t)K * 4);
+  }
+};
 
 }  // namespace
 
@@ -1688,50 +683,52 @@ int hpspmm_plan_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const
   p->chunk_nnz = S;
   p->max_K = max_K;
   p->n_chunks = (nnz + S - 1) / S;
-  const size_t b_start = align_up((size_t)(p->n_chunks + 1) * 4, 256);
-  const size_t b_row = align_up((size_t)(p->n_chunks + 1) * 4, 256);
-  const size_t b_crow = align_up((size_t)(p->n_chunks + 1) * 4, 256);
+  const int64_t n_counter = (p->n_chunks + 1) * hpspmm_counter_slabs(max_K);
+  const size_t b_int = align_up((size_t)(p->n_chunks + 1) * 4, 256);
   const size_t b_cval = align_up((size_t)(p->n_chunks + 1) * (size_t)max_K * 4, 256);
-  const size_t b_order = align_up((size_t)(p->n_chunks + 1) * 4, 256);
-  const size_t b_count = align_up((size_t)(p->n_chunks + 1) * 4, 256);
-  const size_t b_nz = align_up((size_t)(M + 2) * 4, 256);          // nz_id, nz_end: one slot per row + sentinel
-  const size_t b_ri = align_up((size_t)(p->n_chunks + 1) * 4, 256);
-  const size_t b_sort = hpspmm_order_scratch_bytes(p->n_chunks);   // only needed while building
-  p->bytes = b_start + b_row + b_crow + b_cval + b_order + b_count + 2 * b_nz + b_ri + b_sort;
+  const size_t b_count = align_up((size_t)n_counter * 4, 256);
+  const size_t b_row = align_up((size_t)(M + 2) * 4, 256);         // one slot per row + sentinel
+  const size_t b_nz = align_up(hpspmm_nz_bytes(M), 256);
+  const size_t b_rec = align_up((size_t)(p->n_chunks + 1) * 32, 256);
+  // the builders' own scratch lives in the context and is free again afterwards
+  const size_t b_sort = hpspmm_order_scratch_bytes(p->n_chunks);
+  const size_t b_tiles = align_up((size_t)hpspmm_row_tiles(M) * 4, 256);
+  p->bytes = 4 * b_int + b_cval + b_count + 2 * b_row + b_nz + b_rec;
   char* base = nullptr;
   cudaError_t e = hpspmm_device_malloc((void**)&base, p->bytes);
   if (e != cudaSuccess) {
     delete p;
     return hpspmm_set_err(ctx, HPSPMM_ERR_OOM, "plan cudaMalloc", e);
   }
-  p->chunk_start = (int32_t*)base;
-  p->chunk_row = (int32_t*)(base + b_start);
-  p->carry_row = (int32_t*)(base + b_start + b_row);
-  p->carry_val = (float*)(base + b_start + b_row + b_crow);
-  p->chunk_order = (int32_t*)(base + b_start + b_row + b_crow + b_cval);
-  p->run_counter = (int32_t*)(base + b_start + b_row + b_crow + b_cval + b_order);
-  p->nz_id = (int32_t*)(base + b_start + b_row + b_crow + b_cval + b_order + b_count);
-  p->nz_end = (int32_t*)(base + b_start + b_row + b_crow + b_cval + b_order + b_count + b_nz);
-  p->chunk_ri = (int32_t*)(base + b_start + b_row + b_crow + b_cval + b_order + b_count + 2 * b_nz);
-  void* sort_scratch = base + b_start + b_row + b_crow + b_cval + b_order + b_count + 2 * b_nz + b_ri;
+  char* at = base;
+  auto take = [&](size_t bytes) { char* r = at; at += bytes; return r; };
+  p->chunk_start = (int32_t*)take(b_int);
+  p->chunk_row = (int32_t*)take(b_int);
+  p->chunk_order = (int32_t*)take(b_int);
+  p->chunk_ri = (int32_t*)take(b_int);
+  p->carry_val = (float*)take(b_cval);
+  p->run_counter = (int32_t*)take(b_count);
+  p->nz_id = (int32_t*)take(b_row);
+  p->nz_end = (int32_t*)take(b_row);
+  p->nz = (int2*)take(b_nz);
+  p->rec = (int4*)take(b_rec);
   cudaStream_t s = (cudaStream_t)stream;
-  int st = HPSPMM_OK;
   int split = 0;
-  e = cudaMemsetAsync(ctx->flag, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(p->run_counter, 0, b_count, s);
-  if (e == cudaSuccess && M > 0)
-    st = hpspmm_launch_chunk_table(ctx, M, nnz, row_ptr, S, p->n_chunks, p->chunk_start,
-                                   p->chunk_row, ctx->flag, s, nullptr);
-  if (e == cudaSuccess && st == HPSPMM_OK && M > 0)
+  int st = hpspmm_ensure_scratch(ctx, b_sort + b_tiles + b_rec);
+  char* scratch = (char*)ctx->scratch;
+  int4* rec_by_chunk = (int4*)(scratch + b_sort + b_tiles);
+  if (st == HPSPMM_OK) e = cudaMemsetAsync(ctx->flag, 0, sizeof(int), s);
+  if (st == HPSPMM_OK && e == cudaSuccess) e = cudaMemsetAsync(p->chunk_start, 0, 4, s);
+  if (st == HPSPMM_OK && e == cudaSuccess)
+    st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, p->n_chunks, p->nz, rec_by_chunk, (int32_t*)(scratch + b_sort),
+                                p->run_counter, n_counter,
+                                hpspmm_structure_tables{p->chunk_start, p->chunk_row, p->chunk_ri, p->nz_id, p->nz_end,
+                                                        ctx->flag}, s);
+  if (st == HPSPMM_OK && e == cudaSuccess && M > 0)
     st = hpspmm_order_chunks_by_cost(ctx, M, N, p->n_chunks, row_ptr, col_idx, p->chunk_start, p->chunk_row,
-                                     p->chunk_order, sort_scratch, s);
-  if (e == cudaSuccess && st == HPSPMM_OK && M > 0) {
-    // the list of rows that hold entries (its scratch lives in the context and is free again afterwards)
-    st = hpspmm_ensure_scratch(ctx, hpspmm_row_list_scratch_bytes(M));
-    if (st == HPSPMM_OK)
-      st = hpspmm_build_row_list(ctx, M, p->n_chunks, row_ptr, p->chunk_row, p->nz_id, p->nz_end, p->chunk_ri,
-                                 ctx->scratch, s);
-  }
+                                     p->chunk_order, scratch, s);
+  if (st == HPSPMM_OK && e == cudaSuccess && M > 0)
+    st = hpspmm_order_records(ctx, p->n_chunks, p->chunk_order, rec_by_chunk, p->rec, s);
   if (e == cudaSuccess && st == HPSPMM_OK)
     e = cudaMemcpyAsync(&split, ctx->flag, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && st == HPSPMM_OK) e = cudaStreamSynchronize(s);
@@ -1766,17 +763,11 @@ int hpspmm_plan_info(const hpspmm_plan* plan, int64_t* n_chunks, int64_t* n_spli
 
 int hpspmm_spmm_kernel_signature(const hpspmm_plan* plan, int64_t K, int32_t b_l2_hint, char* buf, size_t len) {
   if (!buf || len == 0 || K < 1) return HPSPMM_ERR_INVALID;
-  const bool hint = b_l2_hint == 2 || (b_l2_hint == 0 && K >= 64);
-  if (K == 32 || K == 64 || K == 128) {
-    const int W = (int)K / 4;
-    // the template arguments of spmm_warp_kernel as run_slab / launch_warp choose them
-    snprintf(buf, len, "spmm_warp_kernel<%d,4,%d,%d,64,%d,0,1> chunk_nnz=%d", W, HPSPMM_WARP_MINB, hint ? 1 : 0,
-             W >= 16 ? 1 : 0, plan ? (int)plan->chunk_nnz : (int)hpspmm_default_chunk_nnz(K, plan ? plan->nnz : 0));
-  } else if (K % 32 == 0 && K <= 512) {
-    snprintf(buf, len, "spmm_warp_kernel slabs of 128/64/32 columns, strided, K=%lld", (long long)K);
-  } else {
-    snprintf(buf, len, "spmm_generic_kernel<%d,4,0> K=%lld", (K & 3) == 0 ? 4 : 1, (long long)K);
-  }
+  const int64_t nnz = plan ? plan->nnz : 0;
+  const hpspmm_opts o = {0, 0, b_l2_hint, 0};
+  const hpspmm_spmm_shape sh = hpspmm_choose_shape(hpspmm_vector_width(K, 0), K, gather_hint(K, &o));
+  snprintf(buf, len, "spmm_warp_kernel<%d,%d,%d> K=%lld split=%d hint=%d chunk_nnz=%d", sh.VEC, sh.W, sh.R, (long long)K,
+           sh.lat ? 1 : 0, sh.hint ? 1 : 0, plan ? (int)plan->chunk_nnz : (int)hpspmm_default_chunk_nnz(K, nnz));
   return HPSPMM_OK;
 }
 
@@ -1808,64 +799,47 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
   if (M == 0) return HPSPMM_OK;
   hpspmm_device_guard guard(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;
-  const int hint_mode = opts ? opts->b_l2_hint : 0;
-  // evict-last on the gathers of B, R-MAT bench graph, on / off, one width timed alone: K = 128 0.555 / 0.591 ms,
-  // K = 64 0.307 / 0.304, K = 32 0.189 / 0.1885.  Inside a step of three products run back to back K = 64 measures
-  // the other way round (0.311 on, 0.313 off), so 64 columns stay on.
-  const bool hint = hint_mode == 2 || (hint_mode == 0 && K >= 64);
+  const bool hint = gather_hint(K, opts);
   const int algo = opts ? opts->algo : HPSPMM_ALGO_AUTO;
-  if (algo == HPSPMM_ALGO_ROW_SPLIT) {
-    return run_spmm(ctx, hint, true, M, K, M, row_ptr, col_idx, vals, B, C, nullptr, nullptr,
-                    nullptr, nullptr, nullptr, false, s);
-  }
+  if (algo == HPSPMM_ALGO_ROW_SPLIT) return run_rowsplit(ctx, hint, (int)M, K, row_ptr, col_idx, vals, B, C, s);
   HPSPMM_REQUIRE(ctx, algo == HPSPMM_ALGO_AUTO || algo == HPSPMM_ALGO_BALANCED || algo == HPSPMM_ALGO_TMA,
                  "unknown algo");
+  hpspmm_spmm_args a;
+  memset(&a, 0, sizeof(a));
+  a.M = (int)M, a.K = (int)K;
+  a.row_ptr = row_ptr, a.col_idx = col_idx, a.vals = vals, a.B = B, a.C = C;
   if (plan) {
     HPSPMM_REQUIRE(ctx, plan->M == M && plan->nnz == nnz, "plan built for another matrix");
     HPSPMM_REQUIRE(ctx, K <= plan->max_K, "K exceeds the plan's max_K");
     HPSPMM_REQUIRE(ctx, plan->device == ctx->device, "plan built on another device");
-    return run_spmm(ctx, hint, false, M, K, plan->n_chunks, row_ptr, col_idx, vals, B, C,
-                    plan->chunk_start, plan->chunk_row, plan->carry_row, plan->carry_val,
-                    plan->chunk_order, plan->n_split_chunks > 0, s, plan->chunk_nnz, plan->run_counter,
-                    row_list{plan->nz_id, plan->nz_end, plan->chunk_ri}, algo == HPSPMM_ALGO_TMA ? N : 0);
+    if (algo == HPSPMM_ALGO_TMA && K == 128) {
+      // B through the tensor memory accelerator; falls through when that path declines
+      const int r = launch_spmm_tma(ctx, (int)M, (int)plan->n_chunks, N, row_ptr, col_idx, vals, B, C,
+                                    plan->chunk_start, plan->chunk_row, plan->carry_val, plan->chunk_order,
+                                    plan->chunk_nnz, plan->run_counter, plan, s);
+      if (r == 0) return HPSPMM_OK;
+      if (r < 0) return HPSPMM_ERR_CUDA;   // the launcher has recorded the message
+    }
+    a.n_chunks = (int)plan->n_chunks, a.S = plan->chunk_nnz;
+    a.rec = plan->rec, a.nz = plan->nz, a.carry = plan->carry_val, a.counter = plan->run_counter;
+    return launch_spmm(ctx, a, hint, false, s);
   }
-  int32_t S = (opts && opts->chunk_nnz > 0) ? opts->chunk_nnz : hpspmm_default_chunk_nnz(K, nnz);
-  S = (S + 31) / 32 * 32;
+  const int32_t S = planless_chunk_nnz(K, nnz, opts);
   const int64_t n_chunks = (nnz + S - 1) / S;
-  const size_t b_int = align_up((size_t)(n_chunks + 1) * 4, 256);
-  const size_t b_cval = align_up((size_t)(n_chunks + 1) * (size_t)K * 4, 256);
-  const size_t b_sort = hpspmm_order_scratch_bytes(n_chunks);
-  const size_t b_nz = align_up((size_t)(M + 2) * 4, 256);
-  const size_t b_list = hpspmm_row_list_scratch_bytes(M);
-  const size_t b_tmp = b_sort > b_list ? b_sort : b_list;   // the two builders run one after the other
-  st = hpspmm_ensure_scratch(ctx, 6 * b_int + b_cval + 2 * b_nz + b_tmp);
+  const int64_t n_counter = n_chunks * hpspmm_counter_slabs(K);
+  const planless_layout lay(M, K, n_chunks);
+  st = hpspmm_ensure_scratch(ctx, lay.bytes);
   if (st != HPSPMM_OK) return st;
   char* base = (char*)ctx->scratch;
-  int32_t* chunk_start = (int32_t*)base;
-  int32_t* chunk_row = (int32_t*)(base + b_int);
-  int32_t* carry_row = (int32_t*)(base + 2 * b_int);
-  int32_t* chunk_order = (int32_t*)(base + 3 * b_int);
-  int32_t* run_counter = (int32_t*)(base + 4 * b_int);
-  int32_t* chunk_ri = (int32_t*)(base + 5 * b_int);
-  float* carry_val = (float*)(base + 6 * b_int);
-  int32_t* nz_id = (int32_t*)(base + 6 * b_int + b_cval);
-  int32_t* nz_end = (int32_t*)(base + 6 * b_int + b_cval + b_nz);
-  void* tmp = base + 6 * b_int + b_cval + 2 * b_nz;
-  // the table kernel also zeroes the counters of the in-kernel carry settlement
-  st = hpspmm_launch_chunk_table(ctx, M, nnz, row_ptr, S, n_chunks, chunk_start, chunk_row,
-                                 nullptr, s, run_counter);
+  int4* rec = (int4*)(base + lay.rec);
+  int2* nz = (int2*)(base + lay.nz);
+  int32_t* counter = (int32_t*)(base + lay.counter);
+  st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, n_chunks, nz, rec, (int32_t*)(base + lay.tiles), counter,
+                              n_counter, hpspmm_structure_tables{}, s);
   if (st != HPSPMM_OK) return st;
-  // cost order only: the second sort pass of the column-band order costs more per call than it saves
-  st = hpspmm_order_chunks_by_cost(ctx, M, N, n_chunks, row_ptr, nullptr, chunk_start, chunk_row, chunk_order,
-                                   tmp, s);
-  if (st != HPSPMM_OK) return st;
-  // the list of rows that hold entries: a few small launches per call, but without it a chunk in a very
-  // sparse region (entries separated by dozens of empty rows) can outlast the rest of the product
-  st = hpspmm_build_row_list(ctx, M, n_chunks, row_ptr, chunk_row, nz_id, nz_end, chunk_ri, tmp, s);
-  if (st != HPSPMM_OK) return st;
-  return run_spmm(ctx, hint, false, M, K, n_chunks, row_ptr, col_idx, vals, B, C, chunk_start,
-                  chunk_row, carry_row, carry_val, chunk_order, true, s, S, run_counter,
-                  row_list{nz_id, nz_end, chunk_ri});
+  a.n_chunks = (int)n_chunks, a.S = S;
+  a.rec = rec, a.nz = nz, a.carry = (float*)(base + lay.carry), a.counter = counter;
+  return launch_spmm(ctx, a, hint, false, s);
 }
 
 // Host-buffer products, pipelined over column slabs: C[:, s] = A * B[:, s] needs only slab s of B,
@@ -1912,12 +886,8 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
     size_t need = 0;
     for (int i = 0; i < n_slabs; ++i) {
       const int64_t w = slabs[i].width;
-      const int32_t S = (opts && opts->chunk_nnz > 0) ? (opts->chunk_nnz + 31) / 32 * 32 : hpspmm_default_chunk_nnz(w, nnz);
-      const int64_t n_chunks = (nnz + S - 1) / S;
-      const size_t b_int = align_up((size_t)(n_chunks + 1) * 4, 256);
-      const size_t b_sort = hpspmm_order_scratch_bytes(n_chunks), b_list = hpspmm_row_list_scratch_bytes(M);
-      const size_t want = 6 * b_int + align_up((size_t)(n_chunks + 1) * w * 4, 256) +
-                          2 * align_up((size_t)(M + 2) * 4, 256) + (b_sort > b_list ? b_sort : b_list);
+      const int32_t S = planless_chunk_nnz(w, nnz, opts);
+      const size_t want = planless_layout(M, w, (nnz + S - 1) / S).bytes;
       need = want > need ? want : need;
     }
     st = hpspmm_ensure_scratch(ctx, need);
@@ -2095,76 +1065,6 @@ int hpspmm_spmm_csr_f32_host(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t K, i
   return HPSPMM_OK;
 }
 
-int hpspmm_spmm_coo_f32(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t nnz_padded,
-                        const int32_t* row_idx, const int32_t* col_idx, const float* vals,
-                        const float* B, float* C, const hpspmm_opts* opts, hpspmm_stream stream) {
-  HPSPMM_TRACE("hpspmm_spmm_coo_f32");
-  HPSPMM_REQUIRE(ctx, ctx != nullptr, "null context");
-  HPSPMM_REQUIRE(ctx, M >= 0 && N >= 0 && nnz_padded >= 0 && K >= 1, "bad size");
-  if (nnz_padded == 0 || M == 0) return HPSPMM_OK;
-  HPSPMM_REQUIRE(ctx, row_idx && col_idx && vals && B && C, "null operand");
-  if ((K & 3) == 0 && (((uintptr_t)B & 15u) || ((uintptr_t)C & 15u))) {
-    snprintf(ctx->err, sizeof(ctx->err), "dense operands must be 16-byte aligned");
-    return HPSPMM_ERR_INVALID;
-  }
-  hpspmm_device_guard guard(ctx->device);
-  int32_t S = (opts && opts->chunk_nnz > 0) ? opts->chunk_nnz : 128;
-  S = (S + 31) / 32 * 32;
-  const int64_t n_workers = (nnz_padded + S - 1) / S;
-  const int64_t blocks = (n_workers + kBlockThreads / 32 - 1) / (kBlockThreads / 32);
-  if (blocks > 2147483647ll) return HPSPMM_ERR_UNSUPPORTED;
-  cudaStream_t s = (cudaStream_t)stream;
-  if (K % 32 == 0 && K <= 512) {
-    // 32/64/128 directly, other multiples of 32 as column slabs of 128, 64 and 32 (every slab accumulates into
-    // its own columns of C, so the slabs are independent)
-    int32_t Sw = (opts && opts->chunk_nnz > 0) ? opts->chunk_nnz : probing_chunk_nnz(K);
-    Sw = (Sw + 31) / 32 * 32;
-    constexpr int BT = 64;
-    const int64_t n_w = (nnz_padded + Sw - 1) / Sw;
-    const int64_t nb = (n_w + BT / 32 - 1) / (BT / 32);
-    if (nb > 2147483647ll) return HPSPMM_ERR_UNSUPPORTED;
-    const bool whole = K == 32 || K == 64 || K == 128;
-    int64_t off = 0;
-    while (off < K) {
-      const int64_t w = K - off >= 128 ? 128 : (K - off >= 64 ? 64 : 32);
-#define HPSPMM_COO(WW, ST) \
-  spmm_coo_warp_kernel<WW, 4, BT, ST><<<(unsigned)nb, BT, 0, s>>>(nnz_padded, Sw, row_idx, col_idx, vals, B + off, \
-                                                                 C + off, (int)K)
-      if (w == 128) { if (whole) HPSPMM_COO(32, false); else HPSPMM_COO(32, true); }
-      else if (w == 64) { if (whole) HPSPMM_COO(16, false); else HPSPMM_COO(16, true); }
-      else { if (whole) HPSPMM_COO(8, false); else HPSPMM_COO(8, true); }
-#undef HPSPMM_COO
-      ctx->launches++;
-      off += w;
-    }
-    HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
-    return HPSPMM_OK;
-  }
-  if ((K & 3) == 0) {
-    // narrow K keeps one column slab per lane so no lane idles on dead slabs
-    if (K <= 128) {
-      const dim3 grid((unsigned)blocks, 1, 1);
-      spmm_coo_kernel<4, 1><<<grid, kBlockThreads, 0, s>>>((int)K, nnz_padded, S, row_idx, col_idx,
-                                                           vals, B, C);
-    } else {
-      const int kblock = 32 * 4 * 4;
-      const dim3 grid((unsigned)blocks, (unsigned)((K + kblock - 1) / kblock), 1);
-      if (grid.y > 65535) return HPSPMM_ERR_UNSUPPORTED;
-      spmm_coo_kernel<4, 4><<<grid, kBlockThreads, 0, s>>>((int)K, nnz_padded, S, row_idx, col_idx,
-                                                           vals, B, C);
-    }
-  } else {
-    const int kblock = 32 * 4;
-    const dim3 grid((unsigned)blocks, (unsigned)((K + kblock - 1) / kblock), 1);
-    if (grid.y > 65535) return HPSPMM_ERR_UNSUPPORTED;
-    spmm_coo_kernel<1, 4><<<grid, kBlockThreads, 0, s>>>((int)K, nnz_padded, S, row_idx, col_idx,
-                                                         vals, B, C);
-  }
-  ctx->launches++;
-  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
-  return HPSPMM_OK;
-}
-
 }  // extern "C"
 
 // ---- CSR SpMM with its scratch in a static device array -----------------------------------
@@ -2226,14 +1126,21 @@ extern "C" int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
   }
   if (M == 0) return HPSPMM_OK;
 
-  const int32_t S = probing_chunk_nnz(K);
-  const int64_t n_chunks = (nnz + S - 1) / S;
-  const size_t b_int = align_up((size_t)(n_chunks + 1) * 4, 256);
-  const size_t b_cval = align_up((size_t)(n_chunks + 1) * (size_t)K * 4, 256);
-  const size_t need = 4 * b_int + b_cval;
+  // small matrices take the (smaller) chunks of the ordinary entry point where they fit
+  int32_t S = hpspmm_default_chunk_nnz(K, nnz);
+  int64_t n_chunks;
+  size_t b_int, need;
+  for (;;) {
+    if (S > probing_chunk_nnz(K)) S = probing_chunk_nnz(K);
+    n_chunks = (nnz + S - 1) / S;
+    b_int = align_up((size_t)(n_chunks + 1) * 4, 256);
+    need = 3 * b_int + align_up((size_t)(n_chunks + 1) * (size_t)K * 4, 256);
+    if (need <= (size_t)HPSPMM_STATIC_SCRATCH_BYTES || S == probing_chunk_nnz(K)) break;
+    S = probing_chunk_nnz(K);
+  }
   if (need > (size_t)HPSPMM_STATIC_SCRATCH_BYTES) {
     char msg[256];
-    const long long max_chunks = (long long)(HPSPMM_STATIC_SCRATCH_BYTES - 5 * 256) / (16 + 4 * K) - 1;
+    const long long max_chunks = (long long)(HPSPMM_STATIC_SCRATCH_BYTES - 4 * 256) / (12 + 4 * K) - 1;
     snprintf(msg, sizeof(msg),
              "matrix too large for the static scratch: nnz = %lld at K = %lld needs %zu bytes, the "
              "array holds %u (about %lld nnz at this K); use hpspmm_spmm_csr_f32 instead",
@@ -2271,20 +1178,27 @@ extern "C" int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
   }
   local.sm_count = state.sm_count;
 
-  // Every call rewrites the whole chunk table, zeroes the per-row counters (the table kernel does
-  // both) and rewrites every carry_row entry it later reads, and a carry_val slot is read only
-  // where this call hands a carry on, so nothing left over from an earlier call is ever consumed.
+  // Every call rewrites the whole chunk table and zeroes the per-row counters (the table kernel does both), and a
+  // carry slot is read only where this call hands a carry on, so nothing left over from an earlier call is ever
+  // consumed.
   int32_t* chunk_start = (int32_t*)state.base;
   int32_t* chunk_row = (int32_t*)(state.base + b_int);
-  int32_t* carry_row = (int32_t*)(state.base + 2 * b_int);
-  int32_t* run_counter = (int32_t*)(state.base + 3 * b_int);
-  float* carry_val = (float*)(state.base + 4 * b_int);
+  int32_t* run_counter = (int32_t*)(state.base + 2 * b_int);
   cudaStream_t s = (cudaStream_t)stream;
-  st = hpspmm_launch_chunk_table(&local, M, nnz, row_ptr, S, n_chunks, chunk_start, chunk_row,
-                                 nullptr, s, run_counter);
-  if (st == HPSPMM_OK)
-    st = run_spmm(&local, K >= 64, false, M, K, n_chunks, row_ptr, col_idx, vals, B, C, chunk_start,
-                  chunk_row, carry_row, carry_val, /*chunk_order=*/nullptr, true, s, S, run_counter);
+  chunk_table_kernel<<<(unsigned)((n_chunks + 1 + 255) / 256), 256, 0, s>>>((int)M, (int)nnz, row_ptr, S, (int)n_chunks,
+                                                                            chunk_start, chunk_row, run_counter);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    write_err(err_buf, err_len, cudaGetErrorString(e));
+    return HPSPMM_ERR_CUDA;
+  }
+  hpspmm_spmm_args a;
+  memset(&a, 0, sizeof(a));
+  a.M = (int)M, a.K = (int)K, a.n_chunks = (int)n_chunks, a.S = S;
+  a.row_ptr = row_ptr, a.col_idx = col_idx, a.vals = vals, a.B = B, a.C = C;
+  a.chunk_start = chunk_start, a.chunk_row = chunk_row;
+  a.carry = (float*)(state.base + 3 * b_int), a.counter = run_counter;
+  st = launch_spmm(&local, a, gather_hint(K, nullptr), /*shared_counters=*/true, s);
   if (st != HPSPMM_OK) write_err(err_buf, err_len, local.err);
   return st;
 }

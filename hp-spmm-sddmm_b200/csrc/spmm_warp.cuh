@@ -1,0 +1,408 @@
+// The nnz-balanced warp kernel of the CSR product, for every width.
+//
+// One warp owns one chunk of the entry axis.  It stages (col, val) tiles of 32 entries in shared memory with
+// asynchronous copies, two tiles ahead of their use; in every step group g of the warp takes entry G*s+g of the
+// tile, reads its (col, val) pair as one shared-memory broadcast and gathers its fragment of that row of B
+// (warp_frag.cuh), U steps of gathers being in flight before the first FMA.  Row ends are warp-uniform, so groups
+// never diverge.  A finished row is combined across the groups and stored once.
+//
+// A chunk that ends inside a heavy row leaves its partial sum in a carry slot; the pieces of a split row settle it
+// among themselves (settle_split_row).  The order of all additions is fixed by the chunking and the shape, so
+// results are bit-reproducible from run to run.
+#pragma once
+#include "device_utils.cuh"
+#include "hpspmm_internal.h"
+#include "warp_frag.cuh"
+
+namespace hpspmm {
+
+// Writes zeros into the rows that hold no entries: extra blocks of the product's grid walk all rows, 32 at a time,
+// the bounds of the next 32 in flight while the current ones are stored.  KS: the width when it is a compile-time
+// constant (one store instruction then covers 32 * 4 / KS rows), else 0.
+template <int KS>
+__device__ __forceinline__ void zero_empty_rows(int M, int K, const int* __restrict__ row_ptr, float* __restrict__ C,
+                                                int zero_block, int n_zero_blocks, int block_threads) {
+  const int lane = threadIdx.x & 31;
+  const int warps_per_block = block_threads / 32;
+  const int64_t stride = (int64_t)n_zero_blocks * warps_per_block * 32;
+  int64_t r0 = ((int64_t)zero_block * warps_per_block + (threadIdx.x >> 5)) * 32;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto is_empty = [&](int64_t r) { return r < M && __ldg(row_ptr + r) == __ldg(row_ptr + r + 1); };
+  bool next = is_empty(r0 + lane);
+  for (; r0 < M; r0 += stride) {
+    unsigned m = __ballot_sync(0xffffffffu, next);
+    next = is_empty(r0 + stride + lane);
+    if (KS == 32 || KS == 64 || KS == 128) {
+      constexpr int W = KS >= 4 ? KS / 4 : 1;
+      float* c = C + r0 * KS + lane * 4;   // lane / W = row of the store, lane % W = its column
+      m >>= lane / W;
+#pragma unroll 4
+      for (int q = 0; q < W; ++q)
+        if ((m >> (q * (32 / W))) & 1u) st_stream(c + q * 128, zero);
+    } else {
+      while (m) {
+        const int b = __ffs(m) - 1;
+        m &= m - 1;
+        float* crow = C + (r0 + b) * K;
+        if ((K & 3) == 0) {
+          for (int c = lane * 4; c < K; c += 128) st_stream(crow + c, zero);
+        } else {
+          for (int c = lane; c < K; c += 32) crow[c] = 0.f;
+        }
+      }
+    }
+  }
+}
+
+// Next non-empty row after `row`, given that entry j (< nnz) follows the end of `row`, as (row_end << 32) | row.
+// Probes 16 rows, then gallops (16, 32, 64, ... rows ahead) to bracket the row that holds j and searches inside
+// the bracket.  For calls without a list of the rows that hold entries; out of line so that its registers do not
+// weigh on the gather loop of the caller.
+static __device__ __noinline__ unsigned long long probe_next_row(const int* __restrict__ row_ptr, int M, int j, int row) {
+  int e, probes = 0;
+  do {
+    ++row;
+    e = __ldg(row_ptr + row + 1);
+  } while (e == j && ++probes < 16);
+  if (e == j) {
+    int lo = row + 1, step = 16, hi;
+    for (;;) {
+      hi = min(lo + step, M);
+      if (hi == M || __ldg(row_ptr + hi) > j) break;
+      lo = hi;
+      step <<= 1;
+    }
+    ++hi;
+    ++lo;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(row_ptr + mid) <= j)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    row = lo - 1;
+    e = __ldg(row_ptr + row + 1);
+  }
+  return ((unsigned long long)(unsigned)e << 32) | (unsigned)row;
+}
+
+// Adds up one split row.  A row longer than S is cut at multiples of S only, so its pieces are the chunks
+// first = row_ptr[r] / S .. last = (row_ptr[r+1] - 1) / S: all but the last hand a carry on, the last stores the
+// row.  Every piece bumps the row's counter when its own part is visible device-wide; whoever bumps it last adds
+// the carries, in chunk order (the groups summing interleaved carries, combined in a fixed order), to the stored
+// row.  The sum does not depend on who that is.  No piece ever waits.  `C`, `carry` and `counter` are those of the
+// slab: ld is the row stride of C and of the carry slots, kw the slab's width.
+template <int VEC, int W, int R>
+__device__ __forceinline__ void settle_split_row(int r, int r_start, int r_end, int S, const float* __restrict__ carry,
+                                              float* __restrict__ C, int* __restrict__ counter, int ld, int kw) {
+  constexpr int G = 32 / W;
+  const int lane = threadIdx.x & 31;
+  const int g = lane / W, l = lane % W;
+  const int first = r_start / S;
+  const int last = (r_end - 1) / S;
+  __syncwarp();   // every lane's part is written before lane 0 announces it
+  int seen = 0;
+  if (lane == 0) seen = atomic_add_release(counter + first, 1);
+  seen = __shfl_sync(0xffffffffu, seen, 0);
+  if (seen != last - first) return;
+  __threadfence();
+  const int len = last - first;
+  const int64_t K = ld;
+#pragma unroll 1
+  for (int rr = 0; rr < R; ++rr) {
+    const int col = (rr * W + l) * VEC;
+    const bool live = col < kw;
+    const float* src = carry + (int64_t)first * K + (live ? col : 0);
+    float sum[VEC];
+#pragma unroll
+    for (int x = 0; x < VEC; ++x) sum[x] = 0.f;
+    int i = g;
+    for (; i + 7 * G < len; i += 8 * G) {
+      float v[8][VEC];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) load_l2(v[u], src + (int64_t)(i + u * G) * K);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int x = 0; x < VEC; ++x) sum[x] += v[u][x];
+    }
+    for (; i < len; i += G) {
+      float v[VEC];
+      load_l2(v, src + (int64_t)i * K);
+#pragma unroll
+      for (int x = 0; x < VEC; ++x) sum[x] += v[x];
+    }
+    all_reduce_groups<VEC, W>(sum);
+    if (g == 0 && live) {
+      float* out = C + (int64_t)r * K + col;
+      float o[VEC];
+      load_l2(o, out);
+#pragma unroll
+      for (int x = 0; x < VEC; ++x) o[x] += sum[x];
+      store_stream(out, o);
+    }
+  }
+  if (lane == 0) counter[first] = 0;   // ready for the next launch
+}
+
+// Slot of the schedule this warp takes.  Read from the special registers anew at every use (volatile), so that the
+// compiler does not keep it in a register from the prologue to the tail of the kernel.
+template <int BT>
+__device__ __forceinline__ int chunk_slot() {
+  unsigned cta, tid;
+  asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+  return (int)((cta * (unsigned)BT + tid) >> 5);
+}
+
+// KS: row stride of B and C when it is a compile-time constant (the whole width is one full slab), else 0.
+// LIST: the rows that hold entries are listed (a.nz, with records a.rec); without the list the kernel probes row_ptr.
+template <int VEC, int W, int R, int U, int KS, int BT, int MINB, bool HINT, bool LIST>
+__global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_constant__ hpspmm_spmm_args a) {
+  constexpr int CW = VEC * W * R;   // columns a warp covers
+  constexpr int G = 32 / W;         // lane groups = entries gathered per step
+  constexpr int T = 32;             // entries per staged tile
+  constexpr int BATCH = U * G;      // entries per batch of gathers
+  constexpr int STAGES = 2;
+  static_assert(R == 1 || W == 32, "several vectors per lane only when one group is the warp");
+  static_assert(BATCH <= T && T % BATCH == 0, "batch must tile the staged tile");
+  static_assert(KS == 0 || KS == CW, "a fixed stride is the width of the slab");
+  __shared__ int2 tiles[BT / 32][STAGES][T];
+
+  if ((int)blockIdx.x >= a.n_chunk_blocks) {
+    if (blockIdx.y == 0 && a.slab0 == 0 && a.off == 0)
+      zero_empty_rows<KS>(a.M, a.K, a.row_ptr, a.C, blockIdx.x - a.n_chunk_blocks, gridDim.x - a.n_chunk_blocks, BT);
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  const int g = lane / W;   // group
+  const int l = lane % W;   // position inside the group
+  int n1, row, row_end, ri, base;
+  {
+    const int slot = chunk_slot<BT>();
+    if (slot >= a.n_chunks) return;
+    if (LIST) {
+      const int4 p = __ldg(a.rec + 2 * (int64_t)slot);
+      base = p.x, ri = p.y, row = p.z, row_end = p.w;
+      n1 = __ldg(&a.rec[2 * (int64_t)slot + 1].z);
+    } else {
+      ri = 0;
+      base = __ldg(a.chunk_start + slot);
+      n1 = __ldg(a.chunk_start + slot + 1);
+      row = __ldg(a.chunk_row + slot);
+      row_end = __ldg(a.row_ptr + row + 1);
+    }
+  }
+  const int off = KS ? 0 : a.off + (a.slab0 + (int)blockIdx.y) * CW;
+  const int kw = KS ? CW : min(CW, a.cols - (a.slab0 + (int)blockIdx.y) * CW);
+  const uint64_t policy = HINT ? policy_for_gathers(a.keep_b) : 0ull;
+  int2(*my)[T] = tiles[threadIdx.x >> 5];
+
+  // The row after the current one is fetched while the current one is summed, where the registers allow it (R-MAT
+  // scale 18, 64 columns: 0.1009 against 0.1032 ms; scale 20, 128 columns: 0.587 against 0.556 ms, so not there).
+  constexpr bool AHEAD = W <= 16;
+  int2 next = make_int2(0, 0);
+  if (LIST && AHEAD) next = __ldg(a.nz + ri + 1);
+
+  auto stage_tile = [&](int stage, int base) {
+    const int j = base + lane;
+    if (j < n1) {
+      cp_async_4(&my[stage][lane].x, a.col_idx + j);
+      cp_async_4(&my[stage][lane].y, a.vals + j);
+    } else {
+      my[stage][lane] = make_int2(0, 0);   // past the chunk: column 0, value 0
+    }
+    cp_async_commit();
+  };
+  stage_tile(0, base);
+  stage_tile(1, base + T);
+
+  float acc[R][VEC];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int x = 0; x < VEC; ++x) acc[r][x] = 0.f;
+  const bool live_last = KS || ((R - 1) * W + l) * VEC < kw;   // only the last vector of a lane can lie outside
+  const unsigned stride = (KS ? KS : a.K) * 4u;                // bytes
+  const char* Bl = reinterpret_cast<const char*>(a.B + off + ((R > 1 || live_last) ? l * VEC : 0));
+  const char* Bl_last = reinterpret_cast<const char*>(a.B + off + (live_last ? ((R - 1) * W + l) * VEC : 0));
+  using Split = group_split<VEC, W>;
+  const int out_col = Split::column(lane);   // where this lane's share of a finished row goes
+  char* Cl = reinterpret_cast<char*>(a.C + off + out_col);
+
+  auto gather = [&](float (&b)[R][VEC], int col) {
+    const char* p = Bl + (uint64_t)(unsigned)col * stride;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (R > 1 && r == R - 1)
+        gather_vec<VEC, HINT>(b[r], reinterpret_cast<const float*>(Bl_last + (uint64_t)(unsigned)col * stride), policy);
+      else
+        gather_vec<VEC, HINT>(b[r], reinterpret_cast<const float*>(p) + r * W * VEC, policy);
+    }
+  };
+  auto fma = [&](float v, const float (&b)[R][VEC]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int x = 0; x < VEC; ++x) acc[r][x] = fmaf(v, b[r][x], acc[r][x]);
+  };
+  auto store_row = [&]() {
+    float* crow = reinterpret_cast<float*>(Cl + (uint64_t)(unsigned)row * stride);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float v[Split::KEEP];
+      combine_groups<VEC, W>(acc[r], v, lane);
+      if (Split::writes(lane) && (r < R - 1 || live_last)) store_stream(crow + r * W * VEC, v);
+    }
+  };
+  // the row is complete: store it, start the next row that holds entries
+  auto finish_row = [&]() {
+    store_row();
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int x = 0; x < VEC; ++x) acc[r][x] = 0.f;
+    if (LIST) {
+      ++ri;
+      if (!AHEAD) next = __ldg(a.nz + ri);
+      row = next.x;
+      row_end = next.y;
+      if (AHEAD) next = __ldg(a.nz + ri + 1);
+    } else {
+      const unsigned long long nr = probe_next_row(a.row_ptr, a.M, row_end, row);
+      row = (int)(unsigned)nr;
+      row_end = (int)(nr >> 32);
+    }
+  };
+
+  int stage = 0;
+  for (; base < n1; base += T) {
+    cp_async_wait<STAGES - 1>();
+    __syncwarp();
+    const int2* tile = &my[stage][g];
+    if (base + T <= n1 && row_end >= base + T) {
+      // Fast tile: all 32 entries belong to the current row: no tests between gathers.  Not unrolled all the way:
+      // the compiler then hoists gathers of later batches over the FMAs of earlier ones until it has to spill (K = 128
+      // at 48 registers, R-MAT scale 20: 0.700 ms fully unrolled, 0.576 ms two batches at a time, 0.582 ms one).
+#pragma unroll(W == 32 ? 2 : 1)
+      for (int s0 = 0; s0 < T / G; s0 += U) {
+        float b[U][R][VEC];
+        float v[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+          const int2 e = tile[(s0 + i) * G];   // one broadcast per group
+          v[i] = __int_as_float(e.y);
+          gather(b[i], e.x);
+        }
+#pragma unroll
+        for (int i = 0; i < U; ++i) fma(v[i], b[i]);
+      }
+    } else {
+#pragma unroll 1
+      for (int u0 = 0; u0 < T; u0 += BATCH) {
+        const int j0 = base + u0;
+        if (j0 >= n1) break;
+        float b[U][R][VEC];
+        float v[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+          const int2 e = tile[u0 + i * G];
+          v[i] = __int_as_float(e.y);
+          gather(b[i], e.x);
+        }
+        if (j0 + BATCH <= n1 && row_end >= j0 + BATCH) {
+#pragma unroll
+          for (int i = 0; i < U; ++i) fma(v[i], b[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < U; ++i) {
+            const int lo = j0 + i * G;
+            const int hi = min(lo + G, n1);
+            const int mine = lo + g;
+            int cur = lo;
+            while (row_end < hi) {   // warp-uniform: the current row ends inside this step
+              if (mine >= cur && mine < row_end) fma(v[i], b[i]);
+              cur = row_end;
+              finish_row();
+            }
+            if (mine >= cur && mine < hi) fma(v[i], b[i]);
+          }
+        }
+      }
+    }
+    __syncwarp();
+    stage_tile(stage, base + STAGES * T);
+    stage ^= 1;
+  }
+  cp_async_wait<0>();
+
+  // The chunk is read again from its record: nothing of it has to stay in registers through the loop above.
+  const int slot = chunk_slot<BT>();
+  int n0, chunk, r0, r0_start, r0_end;
+  if (LIST) {
+    const int4 p = __ldg(a.rec + 2 * (int64_t)slot);
+    const int2 q = __ldg(reinterpret_cast<const int2*>(a.rec + 2 * (int64_t)slot + 1));
+    n0 = p.x, r0 = p.z, r0_end = p.w;
+    chunk = q.x, r0_start = q.y;
+  } else {
+    chunk = slot;
+    n0 = __ldg(a.chunk_start + slot);
+    r0 = __ldg(a.chunk_row + slot);
+    r0_start = __ldg(a.row_ptr + r0);
+    r0_end = __ldg(a.row_ptr + r0 + 1);
+  }
+  const bool hands_on = row_end != n1;   // the chunk ends inside `row`
+  const int64_t ldc = KS ? KS : a.K;
+  float* carry = a.carry + off;
+  if (!hands_on) {
+    store_row();
+  } else {
+    float* slot_c = carry + (int64_t)chunk * ldc + out_col;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float v[Split::KEEP];
+      combine_groups<VEC, W>(acc[r], v, lane);
+      if (Split::writes(lane) && (r < R - 1 || live_last)) store_plain(slot_c + r * W * VEC, v);
+    }
+  }
+  // the pieces of a split row settle it among themselves
+  const bool stores_split_row = r0_start < n0 && r0_end <= n1;   // began in an earlier chunk, ends here
+  if (!hands_on && !stores_split_row) return;
+  int* counter = a.counter + (int64_t)blockIdx.y * a.n_chunks;
+  if (stores_split_row)
+    settle_split_row<VEC, W, R>(r0, r0_start, r0_end, a.S, carry, a.C + off, counter, (int)ldc, kw);
+  if (hands_on)
+    settle_split_row<VEC, W, R>(row, row == r0 ? r0_start : __ldg(a.row_ptr + row), row_end, a.S, carry, a.C + off,
+                                counter, (int)ldc, kw);
+}
+
+// Launches one shape.  Slabs of the width run as blockIdx.y, each with counters of its own; where the counters are
+// shared (shared_counters: the fixed scratch has room for one set) they run one after the other.
+template <int VEC, int W, int R, int U, int KS, int MINB, bool HINT, int BT = 64>
+int launch_spmm_shape(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool shared_counters, cudaStream_t stream) {
+  constexpr int CW = VEC * W * R;
+  constexpr int per_block = BT / 32;
+  a.n_chunk_blocks = (a.n_chunks + per_block - 1) / per_block;
+  int n_zero_blocks = (a.M + BT - 1) / BT;
+  const int cap = ctx->sm_count * 8;
+  if (n_zero_blocks > cap) n_zero_blocks = cap;
+  const int slabs = (a.cols + CW - 1) / CW;
+  const int64_t grid = (int64_t)a.n_chunk_blocks + n_zero_blocks;
+  if (grid == 0) return HPSPMM_OK;
+  const int step = shared_counters ? 1 : 65535;
+  for (int s = 0; s < slabs; s += step) {
+    a.slab0 = s;
+    const int ny = slabs - s < step ? slabs - s : step;
+    const dim3 g((unsigned)grid, (unsigned)ny);
+    if (a.nz != nullptr)
+      spmm_warp_kernel<VEC, W, R, U, KS, BT, MINB, HINT, true><<<g, BT, 0, stream>>>(a);
+    else   // (the allocation-free entry point only: a runtime stride serves every width)
+      spmm_warp_kernel<VEC, W, R, U, 0, BT, 16, true, false><<<g, BT, 0, stream>>>(a);
+    ctx->launches++;
+  }
+  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
+  return HPSPMM_OK;
+}
+
+}  // namespace hpspmm

@@ -599,56 +599,160 @@ int build_ordered_row_ptr(hpspmm_ctx* ctx, int64_t M, const int32_t* row_ptr, co
 
 }  // namespace
 
-// ---- list of the rows that hold entries -------------------------------------------------------
+// ---- the structure a product walks ---------------------------------------------------------------
+// Rows are cut into at most kRowTiles tiles.  The first kernel counts the rows of every tile that hold entries; in
+// the second, a block adds up the counts of the tiles before its own (at most 4 KB), ranks its rows and writes
+// them, and the thread that owns a row writes the record of every chunk whose cut falls into it.  Two launches
+// instead of a flag pass, a three-kernel scan, a scatter, a binary search per chunk and an index pass.
 namespace {
 
-__global__ void nonempty_flag_kernel(int M, const int* __restrict__ row_ptr, int* __restrict__ flags) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= M; r += stride)
-    flags[r] = r < M ? (row_ptr[r + 1] > row_ptr[r] ? 1 : 0) : 0;
+constexpr int kRowTiles = 1024;
+constexpr int kNzPad = 32;
+
+int row_tile_size(int64_t M) {
+  const int64_t t = ((M + kRowTiles - 1) / kRowTiles + kThreads - 1) / kThreads * kThreads;
+  return (int)(t < kThreads ? kThreads : t);
 }
 
-// rank[r] = number of rows before r that hold entries (rank[M] = their total)
-__global__ void row_list_scatter_kernel(int M, const int* __restrict__ row_ptr, const int* __restrict__ rank,
-                                        int* __restrict__ nz_id, int* __restrict__ nz_end) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= M; r += stride) {
-    if (r == M) {
-      // sentinel after the last row: never a row of C, an end no entry reaches
-      nz_id[rank[M]] = M;
-      nz_end[rank[M]] = 0x7fffffff;
-    } else if (row_ptr[r + 1] > row_ptr[r]) {
-      nz_id[rank[r]] = (int)r;
-      nz_end[rank[r]] = row_ptr[r + 1];
+__global__ void __launch_bounds__(kThreads)
+row_tile_count_kernel(int M, int tile, const int* __restrict__ row_ptr, int* __restrict__ counts,
+                      int* __restrict__ counter, int64_t n_counter) {
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n_counter; i += (int64_t)gridDim.x * kThreads)
+    counter[i] = 0;
+  const int64_t r0 = (int64_t)blockIdx.x * tile;
+  int total = 0;
+  for (int i = 0; i < tile && r0 + i < M; i += kThreads) {
+    const int64_t r = r0 + i + threadIdx.x;
+    total += __syncthreads_count(r < M && __ldg(row_ptr + r + 1) > __ldg(row_ptr + r));
+  }
+  if (threadIdx.x == 0) counts[blockIdx.x] = total;
+}
+
+// the record of chunk c, whose cut falls into row r = [s, e), the rank-th row that holds entries
+__device__ __forceinline__ void write_chunk_record(int c, int S, int n_chunks, int s, int e, int r, int rank,
+                                                   int4* __restrict__ rec, const hpspmm_structure_tables& t) {
+  if (c < 0 || c >= n_chunks) return;   // only a malformed row_ptr gets here
+  const int start = e - s <= S ? s : c * S;
+  rec[2 * (int64_t)c] = make_int4(start, rank, r, e);
+  *reinterpret_cast<int2*>(&rec[2 * (int64_t)c + 1]) = make_int2(c, s);
+  if (c > 0) rec[2 * (int64_t)c - 1].z = start;
+  if (t.chunk_start) {
+    t.chunk_start[c] = start;
+    t.chunk_row[c] = r;
+    t.chunk_ri[c] = rank;
+    if (c > 0 && start != s) atomicAdd(t.split_count, 1);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+row_tile_list_kernel(int M, int nnz, int tile, int S, int n_chunks, const int* __restrict__ row_ptr,
+                     const int* __restrict__ counts, int2* __restrict__ nz, int4* __restrict__ rec,
+                     const hpspmm_structure_tables t) {
+  constexpr int kWarpsHere = kThreads / 32;
+  __shared__ int part[kWarpsHere];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int before = 0;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += kThreads) before += __ldg(counts + i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (lane == 0) part[warp] = before;
+  __syncthreads();
+  int base = 0;
+#pragma unroll
+  for (int w = 0; w < kWarpsHere; ++w) base += part[w];
+  __syncthreads();
+
+  const int64_t r0 = (int64_t)blockIdx.x * tile;
+  for (int i = 0; i < tile && r0 + i < M; i += kThreads) {
+    const int64_t r = r0 + i + threadIdx.x;
+    int s = 0, e = 0;
+    if (r < M) {
+      s = __ldg(row_ptr + r);
+      e = __ldg(row_ptr + r + 1);
+    }
+    const bool has = e > s;
+    const unsigned m = __ballot_sync(0xffffffffu, has);
+    if (lane == 0) part[warp] = __popc(m);
+    __syncthreads();
+    int rank = base + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+    for (int w = 0; w < kWarpsHere; ++w) {
+      if (w < warp) rank += part[w];
+      base += part[w];
+    }
+    __syncthreads();
+    int c_lo = 0, c_n = 0;   // cuts c * S inside [s, e)
+    if (has) {
+      nz[rank] = make_int2((int)r, e);
+      if (t.nz_id) {
+        t.nz_id[rank] = (int)r;
+        t.nz_end[rank] = e;
+      }
+      c_lo = (s + S - 1) / S;
+      c_n = (e - 1) / S - c_lo + 1;
+      if (e == nnz && n_chunks > 0) {
+        rec[2 * (int64_t)n_chunks - 1].z = nnz;
+        if (t.chunk_start) t.chunk_start[n_chunks] = nnz;
+      }
+    }
+    if (c_n > 0 && c_n <= 4)
+      for (int c = c_lo; c < c_lo + c_n; ++c) write_chunk_record(c, S, n_chunks, s, e, (int)r, rank, rec, t);
+    unsigned heavy = __ballot_sync(0xffffffffu, c_n > 4);   // the whole warp writes the records of a long row
+    while (heavy) {
+      const int b = __ffs(heavy) - 1;
+      heavy &= heavy - 1;
+      const int hs = __shfl_sync(0xffffffffu, s, b), he = __shfl_sync(0xffffffffu, e, b);
+      const int hl = __shfl_sync(0xffffffffu, c_lo, b), hn = __shfl_sync(0xffffffffu, c_n, b);
+      const int hk = __shfl_sync(0xffffffffu, rank, b);
+      for (int c = lane; c < hn; c += 32)
+        write_chunk_record(hl + c, S, n_chunks, hs, he, (int)(r - lane + b), hk, rec, t);
+    }
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x < kNzPad) {
+    // sentinels after the last row: never a row of C, an end no entry reaches; a warp reads 32 rows at once
+    nz[base + threadIdx.x] = make_int2(M, 0x7fffffff);
+    if (t.nz_id && threadIdx.x == 0) {
+      t.nz_id[base] = M;
+      t.nz_end[base] = 0x7fffffff;
     }
   }
 }
 
-__global__ void chunk_row_index_kernel(int64_t n_chunks, const int* __restrict__ chunk_row,
-                                       const int* __restrict__ rank, int* __restrict__ chunk_ri) {
+__global__ void order_records_kernel(int64_t n, const int* __restrict__ order, const int4* __restrict__ in,
+                                     int4* __restrict__ out) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n_chunks; c += stride)
-    chunk_ri[c] = rank[chunk_row[c]];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < 2 * n; i += stride)
+    out[i] = __ldg(in + 2 * (int64_t)__ldg(order + (i >> 1)) + (i & 1));
 }
 
 }  // namespace
 
-size_t hpspmm_row_list_scratch_bytes(int64_t M) {
-  return align_up((size_t)(M + 1) * 4, 256) + align_up((size_t)((M + 1 + kScanTile - 1) / kScanTile + 1) * 4, 256);
+size_t hpspmm_nz_bytes(int64_t M) { return (size_t)(M + kNzPad) * 8; }
+
+int64_t hpspmm_row_tiles(int64_t M) {
+  const int64_t tile = row_tile_size(M);
+  const int64_t n = (M + tile - 1) / tile;
+  return n < 1 ? 1 : n;
 }
 
-int hpspmm_build_row_list(hpspmm_ctx* ctx, int64_t M, int64_t n_chunks, const int32_t* row_ptr,
-                          const int32_t* chunk_row, int32_t* nz_id, int32_t* nz_end, int32_t* chunk_ri,
-                          void* scratch, cudaStream_t stream) {
-  int* rank = (int*)scratch;
-  int* totals = (int*)((char*)scratch + align_up((size_t)(M + 1) * 4, 256));
-  nonempty_flag_kernel<<<grid_for(ctx, M + 1), kThreads, 0, stream>>>((int)M, row_ptr, rank);
-  ctx->launches++;
-  exclusive_scan_inplace(ctx, rank, M + 1, totals, stream);
-  row_list_scatter_kernel<<<grid_for(ctx, M + 1), kThreads, 0, stream>>>((int)M, row_ptr, rank, nz_id, nz_end);
-  if (n_chunks > 0)
-    chunk_row_index_kernel<<<grid_for(ctx, n_chunks), kThreads, 0, stream>>>(n_chunks, chunk_row, rank, chunk_ri);
+int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr, int32_t S, int64_t n_chunks,
+                           int2* nz, int4* rec_out, int32_t* counts, int32_t* counter, int64_t n_counter,
+                           const hpspmm_structure_tables& tables, cudaStream_t stream) {
+  const int tile = row_tile_size(M);
+  const unsigned blocks = (unsigned)hpspmm_row_tiles(M);
+  row_tile_count_kernel<<<blocks, kThreads, 0, stream>>>((int)M, tile, row_ptr, counts, counter, n_counter);
+  row_tile_list_kernel<<<blocks, kThreads, 0, stream>>>((int)M, (int)nnz, tile, S, (int)n_chunks, row_ptr, counts, nz,
+                                                        rec_out, tables);
   ctx->launches += 2;
+  HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
+  return HPSPMM_OK;
+}
+
+int hpspmm_order_records(hpspmm_ctx* ctx, int64_t n_chunks, const int32_t* order, const int4* rec_in, int4* rec,
+                         cudaStream_t stream) {
+  if (n_chunks <= 0) return HPSPMM_OK;
+  order_records_kernel<<<grid_for(ctx, 2 * n_chunks), kThreads, 0, stream>>>(n_chunks, order, rec_in, rec);
+  ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;
 }

@@ -61,7 +61,7 @@ enum {
  * in-code heuristics (spmm/mm/spmm_kernel.cu:749-750, :406-420). */
 typedef struct hpspmm_opts {
   int32_t algo;        /* HPSPMM_ALGO_*                                              */
-  int32_t chunk_nnz;   /* nominal nnz per chunk; 0 = chosen from K; multiple of 32   */
+  int32_t chunk_nnz;   /* nominal nnz per chunk; 0 = chosen from K and nnz; multiple of 32 */
   int32_t b_l2_hint;   /* L2 evict-last policy on the gathers of B: 0 = auto (on for
                           K >= 64: +6 % at 128 columns, neutral at 64; off below,
                           where it costs a little), 1 = off, 2 = on                  */
@@ -125,12 +125,12 @@ HPSPMM_API int hpspmm_host_fill_uniform_f32(float* host_ptr, int64_t count, uint
  * Replaces GESpMM (include/spmm/mm/spmm_kernel.h:19, spmm/mm/spmm_kernel.cu:389-426) and
  * the kernels it dispatches to (:247-387).  Argument order follows the reference's
  * kernels: (m, k, row_ptr, col_idx, values, B, C), with N and nnz added.  Overwrites C;
- * empty rows become zeros.  All pointers are device pointers.  K >= 1; K = 32/64/128
- * take the specialised kernels, every other multiple of 32 up to 512 runs them over
- * column slabs of 128, 64 and 32, any other K a generic kernel.
+ * empty rows become zeros.  All pointers are device pointers.  K >= 1: one kernel serves
+ * every width (16-byte gathers when K is a multiple of 4, 8-byte when it is even and the
+ * operands are 8-byte aligned, 4-byte otherwise; wider than 512 columns in slabs).
  *
- * plan may be NULL: the chunk table is then rebuilt into context-owned scratch on
- * every call (one extra small kernel).  The first call that needs more scratch than
+ * plan may be NULL: the structure is then rebuilt into context-owned scratch on
+ * every call (two extra small kernels).  The first call that needs more scratch than
  * the context holds allocates it (cudaMalloc, synchronising); later calls do not.
  * With a plan the call only enqueues kernels (no allocation, no synchronisation), so it can
  * be recorded into a CUDA graph and replayed.
@@ -185,7 +185,7 @@ HPSPMM_API int hpspmm_plan_row_list(const hpspmm_plan* plan, const int32_t** nz_
  * no context.  The chunk table, the carry slots and the per-row counters of the nnz-balanced
  * kernel live in one 16 MiB array inside the library image, so every GPU that loads the library gives up
  * 16 MiB until the process exits.  A matrix whose scratch would not fit -- more than
- * (16 MiB - 1.25 KiB) / (16 + 4 K) chunks (of 128 / 160 / 256 nnz at K = 32 / 64 / 128):
+ * (16 MiB - 1.25 KiB) / (12 + 4 K) chunks (of 128 / 160 / 256 nnz at K = 32 / 64 / 128):
  * about 15 M nnz at K = 32, 10 M at K = 64, 8 M at K = 128 -- is refused with HPSPMM_ERR_UNSUPPORTED and a message in
  * err_buf; use hpspmm_spmm_csr_f32 for it.
  *
