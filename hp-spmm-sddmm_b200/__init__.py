@@ -13,6 +13,8 @@ The directory name contains hyphens, so it is imported by path:
     spec.loader.exec_module(mod)
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 from ctypes import (POINTER, byref, c_char_p, c_double, c_float, c_int, c_int32, c_int64, c_size_t,
                     c_uint64, c_void_p)
@@ -21,6 +23,7 @@ import numpy as np
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "lib", "libhpspmm.so")
+NATIVE_PATH = os.path.join(PKG_DIR, "lib", "_hpspmm_native.so")
 
 OK = 0
 ERR_INVALID = 1
@@ -183,6 +186,33 @@ def load_library(path=None):
     return lib
 
 
+def load_extension(name, path):
+    """A CPython extension module built beside the library."""
+    if not os.path.exists(path):
+        raise RuntimeError("%s not found at %s: build it with `python hp-spmm-sddmm_b200/build.py`" % (name, path))
+    loader = importlib.machinery.ExtensionFileLoader(name, path)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location(name, path, loader=loader))
+    loader.exec_module(mod)
+    return mod
+
+
+_native = None
+
+
+def load_native():
+    """The calls of the hot path with their argument conversion in C (csrc/python_binding.cpp): through ctypes the
+    conversion took longer than a small product."""
+    global _native
+    if _native is None:
+        lib = load_library()
+        mod = load_extension("_hpspmm_native", NATIVE_PATH)
+        mod.bind(*[ctypes.cast(getattr(lib, "hpspmm_" + f), c_void_p).value
+                   for f in ("spmm_csr_f32", "spmm_coo_f32", "sddmm_csr_f32", "fill_f32", "layer_forward",
+                             "layer_backward_features", "layer_backward_weights")])
+        _native = mod
+    return _native
+
+
 def _ptr(a):
     """Address of a numpy array's buffer, or a raw integer address, or NULL."""
     if a is None:
@@ -223,6 +253,7 @@ class Context:
 
     def __init__(self, device=0):
         self.lib = load_library()
+        self._native = load_native()
         h = _P()
         st = self.lib.hpspmm_ctx_create(device, byref(h))
         if st != OK:
@@ -274,8 +305,9 @@ class Context:
         self._check(self.lib.hpspmm_stream_sync(self.handle, stream), "hpspmm_stream_sync")
 
     def fill(self, dev, count, value, stream=None):
-        self._check(self.lib.hpspmm_fill_f32(self.handle, _ptr(dev), count, value, stream),
-                    "hpspmm_fill_f32")
+        st = self._native.fill(self.handle, dev, count, value, stream)
+        if st:
+            self._check(st, "hpspmm_fill_f32")
 
     def fill_uniform(self, dev, count, seed, stream_id, lo, hi, stream=None):
         self._check(self.lib.hpspmm_fill_uniform_f32(self.handle, _ptr(dev), count, seed, stream_id,
@@ -335,10 +367,9 @@ class Context:
         return a.value, b.value, c.value
 
     def spmm_csr(self, M, N, K, nnz, row_ptr, col_idx, vals, B, C, plan=None, opts=None, stream=None):
-        self._check(self.lib.hpspmm_spmm_csr_f32(self.handle, plan, M, N, K, nnz, _ptr(row_ptr),
-                                                 _ptr(col_idx), _ptr(vals), _ptr(B), _ptr(C),
-                                                 byref(opts) if opts else None, stream),
-                    "hpspmm_spmm_csr_f32")
+        st = self._native.spmm_csr(self.handle, plan, M, N, K, nnz, row_ptr, col_idx, vals, B, C, opts, stream)
+        if st:
+            self._check(st, "hpspmm_spmm_csr_f32")
 
     def spmm_csr_host(self, M, N, K, nnz, row_ptr, col_idx, vals, B, C, opts=None):
         self._check(self.lib.hpspmm_spmm_csr_f32_host(self.handle, M, N, K, nnz, _ptr(row_ptr),
@@ -358,16 +389,14 @@ class Context:
                     "hpspmm_spmm_csr_f32_host_multi")
 
     def spmm_coo(self, M, N, K, nnz_padded, row_idx, col_idx, vals, B, C, opts=None, stream=None):
-        self._check(self.lib.hpspmm_spmm_coo_f32(self.handle, M, N, K, nnz_padded, _ptr(row_idx),
-                                                 _ptr(col_idx), _ptr(vals), _ptr(B), _ptr(C),
-                                                 byref(opts) if opts else None, stream),
-                    "hpspmm_spmm_coo_f32")
+        st = self._native.spmm_coo(self.handle, M, N, K, nnz_padded, row_idx, col_idx, vals, B, C, opts, stream)
+        if st:
+            self._check(st, "hpspmm_spmm_coo_f32")
 
     def sddmm_csr(self, M, N, K, nnz, row_ptr, col_idx, X, Y, out, plan=None, opts=None, stream=None):
-        self._check(self.lib.hpspmm_sddmm_csr_f32(self.handle, plan, M, N, K, nnz, _ptr(row_ptr),
-                                                  _ptr(col_idx), _ptr(X), _ptr(Y), _ptr(out),
-                                                  byref(opts) if opts else None, stream),
-                    "hpspmm_sddmm_csr_f32")
+        st = self._native.sddmm_csr(self.handle, plan, M, N, K, nnz, row_ptr, col_idx, X, Y, out, opts, stream)
+        if st:
+            self._check(st, "hpspmm_sddmm_csr_f32")
 
     def csr_transpose(self, M, N, nnz, row_ptr, col_idx, vals, row_ptr_t, col_idx_t, vals_t,
                       perm=None, stream=None):
@@ -476,18 +505,19 @@ class Layer:
         return tuple(x.value for x in v)
 
     def forward(self, K, H, C, stream=None):
-        self.ctx._check(self.ctx.lib.hpspmm_layer_forward(self.ctx.handle, self.handle, K, _ptr(H), _ptr(C),
-                                                          stream), "hpspmm_layer_forward")
+        st = self.ctx._native.layer_forward(self.ctx.handle, self.handle, K, H, C, stream)
+        if st:
+            self.ctx._check(st, "hpspmm_layer_forward")
 
     def backward_features(self, K, dC, dH, stream=None):
-        self.ctx._check(self.ctx.lib.hpspmm_layer_backward_features(self.ctx.handle, self.handle, K, _ptr(dC),
-                                                                    _ptr(dH), stream),
-                        "hpspmm_layer_backward_features")
+        st = self.ctx._native.layer_backward_features(self.ctx.handle, self.handle, K, dC, dH, stream)
+        if st:
+            self.ctx._check(st, "hpspmm_layer_backward_features")
 
     def backward_weights(self, K, dC, H, dA, stream=None):
-        self.ctx._check(self.ctx.lib.hpspmm_layer_backward_weights(self.ctx.handle, self.handle, K, _ptr(dC),
-                                                                   _ptr(H), _ptr(dA), stream),
-                        "hpspmm_layer_backward_weights")
+        st = self.ctx._native.layer_backward_weights(self.ctx.handle, self.handle, K, dC, H, dA, stream)
+        if st:
+            self.ctx._check(st, "hpspmm_layer_backward_weights")
 
     def update_values(self, vals, stream=None):
         self.ctx._check(self.ctx.lib.hpspmm_layer_update_values(self.ctx.handle, self.handle, _ptr(vals), stream),

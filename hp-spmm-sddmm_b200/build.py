@@ -9,6 +9,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
@@ -17,6 +18,8 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_DIR = os.path.join(PKG_DIR, "lib")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libhpspmm.so")
+NATIVE_PATH = os.path.join(LIB_DIR, "_hpspmm_native.so")
+TORCH_PATH = os.path.join(LIB_DIR, "_hpspmm_torch.so")
 TEST_ALL_PATH = os.path.join(LIB_DIR, "test_all")
 
 SOURCES = [
@@ -47,7 +50,7 @@ def _nvcc():
 
 
 def _newest_source_mtime():
-    paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith("_binding.cpp")]
     paths.append(os.path.join(ROOT, "include", "hpspmm.h"))
     paths.append(os.path.abspath(__file__))
     return max(os.path.getmtime(p) for p in paths)
@@ -90,6 +93,38 @@ def build(force=False, verbose=False, ptxas_info=False):
     return LIB_PATH
 
 
+def _cxx():
+    return "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else (shutil.which("g++") or "g++")
+
+
+def _stale(out, *sources):
+    newest = max(os.path.getmtime(p) for p in sources + (os.path.join(ROOT, "include", "hpspmm.h"),))
+    return not os.path.exists(out) or os.path.getmtime(out) < newest
+
+
+def build_bindings(force=False, verbose=False):
+    """Builds the CPython extensions: the hot calls of the C ABI, and the PyTorch operators of the layer."""
+    build(force=force, verbose=verbose)
+    python_inc = ["-I", sysconfig.get_paths()["include"], "-I", os.path.join(ROOT, "include")]
+    common = [_cxx(), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
+    src = os.path.join(CSRC, "python_binding.cpp")
+    if force or _stale(NATIVE_PATH, src):
+        _run(common + python_inc + [src, "-o", NATIVE_PATH], verbose)
+    src = os.path.join(CSRC, "torch_binding.cpp")
+    if force or _stale(TORCH_PATH, src):
+        import torch
+        t = os.path.dirname(torch.__file__)
+        inc = []
+        for d in (os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
+                  os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")):
+            inc += ["-isystem", d]
+        _run(common + python_inc + inc +
+             ["-DTORCH_EXTENSION_NAME=_hpspmm_torch", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()),
+              src, "-o", TORCH_PATH, "-L", LIB_DIR, "-lhpspmm", "-L", os.path.join(t, "lib"), "-lc10", "-lc10_cuda",
+              "-ltorch", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"], verbose)
+    return NATIVE_PATH, TORCH_PATH
+
+
 def build_test_all(force=False, verbose=False):
     """Builds the C++ bench driver (successor of the reference's test/test_all.cpp)."""
     src = os.path.join(PKG_DIR, "host", "test_all.cpp")
@@ -99,8 +134,7 @@ def build_test_all(force=False, verbose=False):
     if (not force and os.path.exists(TEST_ALL_PATH)
             and os.path.getmtime(TEST_ALL_PATH) >= max(os.path.getmtime(src), os.path.getmtime(LIB_PATH))):
         return TEST_ALL_PATH
-    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else (shutil.which("g++") or "g++")
-    _run([cxx, "-O3", "-mavx2", "-mfma", "-std=c++17", "-fopenmp", "-I", os.path.join(ROOT, "include"), src, "-o",
+    _run([_cxx(), "-O3", "-mavx2", "-mfma", "-std=c++17", "-fopenmp", "-I", os.path.join(ROOT, "include"), src, "-o",
           TEST_ALL_PATH, "-L", LIB_DIR, "-lhpspmm", "-Wl,-rpath,$ORIGIN"], verbose)
     return TEST_ALL_PATH
 
@@ -109,6 +143,7 @@ if __name__ == "__main__":
     path = build(force="--force" in sys.argv, verbose="--verbose" in sys.argv,
                  ptxas_info="--ptxas-info" in sys.argv)
     print(path)
+    print(*build_bindings(force="--force" in sys.argv, verbose="--verbose" in sys.argv), sep="\n")
     t = build_test_all(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
     if t:
         print(t)

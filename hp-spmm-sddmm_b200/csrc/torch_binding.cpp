@@ -1,0 +1,177 @@
+// PyTorch operators of the aggregation layer, in C++: registration, autograd formula, stream and memory handling.
+//
+// A training step on a small graph is three or four launches of a few microseconds each; with the operators and the
+// autograd formula in Python the host took 160 us to issue them.  Arithmetic stays in libhpspmm.so, which this file
+// calls through the C ABI; PyTorch supplies memory, streams and the autograd tape.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <memory>
+#include <mutex>
+#include <unordered_map>
+
+#include "hpspmm.h"
+
+namespace {
+
+using at::Tensor;
+
+struct Entry {
+  hpspmm_ctx* ctx;
+  hpspmm_layer* layer;
+  int64_t M, N, nnz;
+  // the weight tensor whose values the layer's transpose holds (kept alive: the layer borrows the device array)
+  Tensor vals;
+  int64_t vals_version;
+};
+
+std::mutex g_mutex;   // guards the registry
+std::unordered_map<int64_t, std::shared_ptr<Entry>> g_layers;
+
+std::shared_ptr<Entry> entry_of(int64_t id) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  auto it = g_layers.find(id);
+  TORCH_CHECK(it != g_layers.end(), "hpspmm: unknown or closed layer id ", id);
+  return it->second;
+}
+
+void check(const Entry& e, int status, const char* what) {
+  TORCH_CHECK(status == HPSPMM_OK, what, " failed with status ", status, ": ", hpspmm_last_error(e.ctx));
+}
+
+Tensor require_cuda_f32(const Tensor& t, int64_t rows, const char* what) {
+  TORCH_CHECK(t.is_cuda(), "hpspmm: ", what, " must be a CUDA tensor (there is no CPU path)");
+  TORCH_CHECK(t.scalar_type() == at::kFloat && t.dim() == 2 && t.size(0) == rows, "hpspmm: ", what,
+              " must be float32 of shape [", rows, ", K], got ", t.scalar_type(), " ", t.sizes());
+  return t.contiguous();
+}
+
+// Re-gathers the transpose's values when the weight tensor moved or was written in place.
+void sync_values(Entry& e, const Tensor& given, cudaStream_t stream) {
+  const Tensor vals = given.contiguous();
+  const int64_t version = vals.is_inference() ? -1 : (int64_t)vals._version();
+  if (version >= 0 && e.vals.defined() && vals.const_data_ptr() == e.vals.const_data_ptr() && version == e.vals_version)
+    return;
+  e.vals = vals.detach();
+  check(e, hpspmm_layer_update_values(e.ctx, e.layer, vals.const_data_ptr<float>(), stream), "hpspmm_layer_update_values");
+  e.vals_version = version;
+}
+
+Tensor forward(const Tensor& H, const Tensor& vals, int64_t id) {
+  auto e = entry_of(id);
+  const Tensor h = require_cuda_f32(H, e->N, "H");
+  const c10::cuda::CUDAGuard guard(h.device());
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  sync_values(*e, vals, stream);
+  Tensor C = at::empty({e->M, h.size(1)}, h.options());
+  check(*e, hpspmm_layer_forward(e->ctx, e->layer, h.size(1), h.const_data_ptr<float>(), C.mutable_data_ptr<float>(), stream),
+        "hpspmm_layer_forward");
+  return C;
+}
+
+Tensor backward_features(const Tensor& grad, const Tensor& vals, int64_t id) {
+  auto e = entry_of(id);
+  const Tensor dC = require_cuda_f32(grad, e->M, "dC");
+  const c10::cuda::CUDAGuard guard(dC.device());
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  sync_values(*e, vals, stream);
+  Tensor dH = at::empty({e->N, dC.size(1)}, dC.options());
+  check(*e, hpspmm_layer_backward_features(e->ctx, e->layer, dC.size(1), dC.const_data_ptr<float>(),
+                                           dH.mutable_data_ptr<float>(), stream), "hpspmm_layer_backward_features");
+  return dH;
+}
+
+Tensor backward_weights(const Tensor& grad, const Tensor& H, int64_t id) {
+  auto e = entry_of(id);
+  const Tensor dC = require_cuda_f32(grad, e->M, "dC");
+  const Tensor h = require_cuda_f32(H, e->N, "H");
+  TORCH_CHECK(h.size(1) == dC.size(1), "hpspmm: dC and H differ in width");
+  const c10::cuda::CUDAGuard guard(dC.device());
+  Tensor dA = at::empty({e->nnz}, dC.options());
+  check(*e, hpspmm_layer_backward_weights(e->ctx, e->layer, dC.size(1), dC.const_data_ptr<float>(),
+                                          h.const_data_ptr<float>(), dA.mutable_data_ptr<float>(),
+                                          c10::cuda::getCurrentCUDAStream().stream()), "hpspmm_layer_backward_weights");
+  return dA;
+}
+
+// the registered operators, for calls that go through the dispatcher (tracing, fake tensors)
+using Op = Tensor(const Tensor&, const Tensor&, int64_t);
+c10::TypedOperatorHandle<Op> find_op(const char* name) {
+  return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Op>();
+}
+const c10::TypedOperatorHandle<Op>& op_forward() {
+  static const auto op = find_op("hpspmm::layer_forward");
+  return op;
+}
+const c10::TypedOperatorHandle<Op>& op_features() {
+  static const auto op = find_op("hpspmm::layer_backward_features");
+  return op;
+}
+const c10::TypedOperatorHandle<Op>& op_weights() {
+  static const auto op = find_op("hpspmm::layer_backward_weights");
+  return op;
+}
+
+struct LayerFunction : public torch::autograd::Function<LayerFunction> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& H, const Tensor& vals, int64_t id) {
+    ctx->saved_data["id"] = id;
+    ctx->save_for_backward({H, vals});
+    at::AutoDispatchBelowADInplaceOrView below;
+    return op_forward().call(H, vals, id);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const int64_t id = ctx->saved_data["id"].toInt();
+    Tensor dH, dvals;
+    if (grads[0].defined()) {
+      if (ctx->needs_input_grad(0)) dH = op_features().call(grads[0], saved[1], id);
+      if (ctx->needs_input_grad(1)) dvals = op_weights().call(grads[0], saved[0], id);
+    }
+    return {dH, dvals, Tensor()};
+  }
+};
+
+Tensor forward_autograd(const Tensor& H, const Tensor& vals, int64_t id) { return LayerFunction::apply(H, vals, id); }
+
+TORCH_LIBRARY(hpspmm, m) {
+  m.def("layer_forward(Tensor H, Tensor vals, int layer_id) -> Tensor");
+  m.def("layer_backward_features(Tensor dC, Tensor vals, int layer_id) -> Tensor");
+  m.def("layer_backward_weights(Tensor dC, Tensor H, int layer_id) -> Tensor");
+}
+// a CPU tensor reaches the same functions, which refuse it by name
+#define HPSPMM_IMPL(KEY)                                  \
+  TORCH_LIBRARY_IMPL(hpspmm, KEY, m) {                    \
+    m.impl("layer_forward", forward);                     \
+    m.impl("layer_backward_features", backward_features); \
+    m.impl("layer_backward_weights", backward_weights);   \
+  }
+HPSPMM_IMPL(CUDA)
+HPSPMM_IMPL(CPU)
+TORCH_LIBRARY_IMPL(hpspmm, Autograd, m) { m.impl("layer_forward", forward_autograd); }
+
+void register_layer(int64_t id, int64_t ctx, int64_t layer, int64_t M, int64_t N, int64_t nnz, const Tensor& vals) {
+  auto e = std::make_shared<Entry>();
+  e->ctx = reinterpret_cast<hpspmm_ctx*>(ctx);
+  e->layer = reinterpret_cast<hpspmm_layer*>(layer);
+  e->M = M, e->N = N, e->nnz = nnz;
+  e->vals = vals.detach();
+  e->vals_version = vals.is_inference() ? -1 : (int64_t)vals._version();
+  std::lock_guard<std::mutex> lock(g_mutex);
+  g_layers[id] = e;
+}
+
+void forget_layer(int64_t id) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  g_layers.erase(id);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_hpspmm_torch, m) {
+  m.def("register_layer", &register_layer);
+  m.def("forget_layer", &forget_layer);
+  m.def("layer_forward", [](const Tensor& H, const Tensor& vals, int64_t id) { return op_forward().call(H, vals, id); },
+        py::call_guard<py::gil_scoped_release>());
+}

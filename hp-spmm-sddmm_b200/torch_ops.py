@@ -4,26 +4,31 @@
     C = layer(H)                                              # C = A·H, differentiable in H and in vals
     C.sum().backward()                                        # dH = Aᵀ·dC (SpMM), dvals = SDDMM(dC, H)
 
-Three operators are registered with torch.library under the namespace ``hpspmm`` (``layer_forward``,
-``layer_backward_features``, ``layer_backward_weights``), with shape functions for tracing and an
-autograd formula that chains them, so the layer can sit inside a compiled or exported module.  Every
-operator calls ``hpspmm_layer_*`` of libhpspmm.so on the current CUDA stream of the input's device; a
-CPU tensor is rejected (there is no fallback).  PyTorch supplies memory, streams and the autograd
+Three operators are registered under the namespace ``hpspmm`` (``layer_forward``,
+``layer_backward_features``, ``layer_backward_weights``) by csrc/torch_binding.cpp, with an autograd
+formula that chains them; the shape functions for tracing are below, so the layer can sit inside a
+compiled or exported module.  Every operator calls ``hpspmm_layer_*`` of libhpspmm.so on the current
+CUDA stream of the input's device; a CPU tensor is rejected (there is no fallback).  PyTorch supplies memory, streams and the autograd
 tape only.
 
 The reference has no framework binding; this is the caller either side of its products
 (test/test_all.cpp:63-107 issues them one at a time from a C++ driver).
 """
 import itertools
-import threading
+import os
 
 import torch
 
-from . import Context, Layer
+from . import PKG_DIR, Context, Layer, load_extension
 
-_layers = {}
+_layers = {}      # what a layer id stands for: the shapes, and what has to stay alive
 _ids = itertools.count(1)
-_lock = threading.Lock()   # guards the registry of layers
+
+_C = load_extension("_hpspmm_torch", os.path.join(PKG_DIR, "lib", "_hpspmm_torch.so"))
+
+layer_forward = torch.ops.hpspmm.layer_forward.default
+layer_backward_features = torch.ops.hpspmm.layer_backward_features.default
+layer_backward_weights = torch.ops.hpspmm.layer_backward_weights.default
 
 
 def _entry(layer_id):
@@ -33,96 +38,19 @@ def _entry(layer_id):
         raise RuntimeError("hpspmm: unknown or closed layer id %d" % layer_id) from None
 
 
-def _require_cuda_f32(t, rows, what):
-    if not t.is_cuda:
-        raise RuntimeError("hpspmm: %s must be a CUDA tensor (there is no CPU path)" % what)
-    if t.dtype != torch.float32 or t.dim() != 2 or t.shape[0] != rows:
-        raise RuntimeError("hpspmm: %s must be float32 of shape [%d, K], got %s %s"
-                           % (what, rows, t.dtype, tuple(t.shape)))
-    return t.contiguous()
-
-
-def _sync_values(e, vals):
-    """Re-gathers the transpose's values when the weight tensor moved or was written in place."""
-    key = (vals.data_ptr(), vals._version)
-    if key != e["vals_key"]:
-        e["vals_ref"] = vals            # keeps the borrowed device array alive
-        e["layer"].update_values(vals.data_ptr(), torch.cuda.current_stream(vals.device).cuda_stream)
-        e["vals_key"] = key
-
-
-@torch.library.custom_op("hpspmm::layer_forward", mutates_args=())
-def layer_forward(H: torch.Tensor, vals: torch.Tensor, layer_id: int) -> torch.Tensor:
-    e = _entry(layer_id)
-    H = _require_cuda_f32(H, e["N"], "H")
-    K = H.shape[1]
-    with torch.cuda.device(H.device):
-        vals = vals.detach().contiguous()
-        _sync_values(e, vals)
-        C = torch.empty((e["M"], K), dtype=torch.float32, device=H.device)
-        e["layer"].forward(K, H.data_ptr(), C.data_ptr(), torch.cuda.current_stream().cuda_stream)
-    return C
-
-
-@layer_forward.register_fake
+@torch.library.register_fake("hpspmm::layer_forward")
 def _(H, vals, layer_id):
     return H.new_empty((_entry(layer_id)["M"], H.shape[1]))
 
 
-@torch.library.custom_op("hpspmm::layer_backward_features", mutates_args=())
-def layer_backward_features(dC: torch.Tensor, vals: torch.Tensor, layer_id: int) -> torch.Tensor:
-    e = _entry(layer_id)
-    dC = _require_cuda_f32(dC, e["M"], "dC")
-    K = dC.shape[1]
-    with torch.cuda.device(dC.device):
-        _sync_values(e, vals.detach().contiguous())
-        dH = torch.empty((e["N"], K), dtype=torch.float32, device=dC.device)
-        e["layer"].backward_features(K, dC.data_ptr(), dH.data_ptr(), torch.cuda.current_stream().cuda_stream)
-    return dH
-
-
-@layer_backward_features.register_fake
+@torch.library.register_fake("hpspmm::layer_backward_features")
 def _(dC, vals, layer_id):
     return dC.new_empty((_entry(layer_id)["N"], dC.shape[1]))
 
 
-@torch.library.custom_op("hpspmm::layer_backward_weights", mutates_args=())
-def layer_backward_weights(dC: torch.Tensor, H: torch.Tensor, layer_id: int) -> torch.Tensor:
-    e = _entry(layer_id)
-    dC = _require_cuda_f32(dC, e["M"], "dC")
-    H = _require_cuda_f32(H, e["N"], "H")
-    K = dC.shape[1]
-    if H.shape[1] != K:
-        raise RuntimeError("hpspmm: dC and H differ in width")
-    with torch.cuda.device(dC.device):
-        dA = torch.empty((e["nnz"],), dtype=torch.float32, device=dC.device)
-        e["layer"].backward_weights(K, dC.data_ptr(), H.data_ptr(), dA.data_ptr(),
-                                    torch.cuda.current_stream().cuda_stream)
-    return dA
-
-
-@layer_backward_weights.register_fake
+@torch.library.register_fake("hpspmm::layer_backward_weights")
 def _(dC, H, layer_id):
     return dC.new_empty((_entry(layer_id)["nnz"],))
-
-
-def _setup_context(ctx, inputs, output):
-    H, vals, layer_id = inputs
-    ctx.layer_id = layer_id
-    ctx.save_for_backward(H, vals)
-
-
-def _backward(ctx, dC):
-    H, vals = ctx.saved_tensors
-    dH = dvals = None
-    if ctx.needs_input_grad[0]:
-        dH = layer_backward_features(dC, vals, ctx.layer_id)
-    if ctx.needs_input_grad[1]:
-        dvals = layer_backward_weights(dC, H, ctx.layer_id)
-    return dH, dvals, None
-
-
-layer_forward.register_autograd(_backward, setup_context=_setup_context)
 
 
 class TorchLayer:
@@ -147,19 +75,22 @@ class TorchLayer:
             v = vals.detach()
             layer = Layer(ctx, self.M, self.N, self.nnz, row_ptr.data_ptr(), col_idx.data_ptr(), v.data_ptr(),
                           self.max_K, torch.cuda.current_stream().cuda_stream)
-        with _lock:
-            self.layer_id = next(_ids)
-            _layers[self.layer_id] = {"layer": layer, "ctx": ctx, "M": self.M, "N": self.N, "nnz": self.nnz,
-                                      "vals_key": (v.data_ptr(), v._version), "vals_ref": v,
-                                      "keep": (row_ptr, col_idx)}
+        self.layer_id = next(_ids)
+        _layers[self.layer_id] = {"layer": layer, "ctx": ctx, "M": self.M, "N": self.N, "nnz": self.nnz,
+                                  "keep": (row_ptr, col_idx)}
+        _C.register_layer(self.layer_id, ctx.handle.value, layer.handle.value, self.M, self.N, self.nnz, v)
 
     def __call__(self, H, vals=None):
-        return layer_forward(H, self.vals if vals is None else vals, self.layer_id)
+        if vals is None:
+            vals = self.vals
+        if torch.compiler.is_compiling():
+            return layer_forward(H, vals, self.layer_id)
+        return _C.layer_forward(H, vals, self.layer_id)    # the same operator without the Python dispatcher's share
 
     def close(self):
-        with _lock:
-            e = _layers.pop(self.layer_id, None)
+        e = _layers.pop(self.layer_id, None)
         if e:
+            _C.forget_layer(self.layer_id)
             e["layer"].close()
             e["ctx"].close()
 
