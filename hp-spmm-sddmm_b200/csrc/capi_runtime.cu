@@ -238,13 +238,14 @@ int hpspmm_event_destroy(hpspmm_ctx* ctx, hpspmm_event ev) {
 
 }  // extern "C"
 
-int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes) {
+static int grow_scratch(hpspmm_ctx* ctx, size_t bytes) {
   if (bytes <= ctx->scratch_bytes) return HPSPMM_OK;
   // grow-only; the old buffer may still be in use by queued kernels
   HPSPMM_CUDA_TRY(ctx, cudaDeviceSynchronize());
   if (ctx->scratch) cudaFree(ctx->scratch);
   ctx->scratch = nullptr;
   ctx->scratch_bytes = 0;
+  ctx->zero_prefix = 0;
   size_t want = bytes + bytes / 4 + 4096;
   cudaError_t e = hpspmm_device_malloc(&ctx->scratch, want);
   if (e != cudaSuccess) {
@@ -253,6 +254,24 @@ int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes) {
   }
   if (e != cudaSuccess) return hpspmm_set_err(ctx, HPSPMM_ERR_OOM, "scratch cudaMalloc", e);
   ctx->scratch_bytes = want;
+  return HPSPMM_OK;
+}
+
+int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes) {
+  ctx->zero_prefix = 0;
+  return grow_scratch(ctx, bytes);
+}
+
+int hpspmm_ensure_scratch_counters(hpspmm_ctx* ctx, size_t bytes, size_t prefix, cudaStream_t stream) {
+  const int st = grow_scratch(ctx, bytes);
+  if (st != HPSPMM_OK) return st;
+  // a graph may be replayed after the scratch has served other calls: a captured call clears the counters itself
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();
+  if (ctx->zero_prefix < prefix || capture != cudaStreamCaptureStatusNone)
+    HPSPMM_CUDA_TRY(ctx, cudaMemsetAsync(ctx->scratch, 0, prefix, stream));
+  // (a shorter prefix than last time: what follows it is about to hold other things)
+  ctx->zero_prefix = prefix;
   return HPSPMM_OK;
 }
 

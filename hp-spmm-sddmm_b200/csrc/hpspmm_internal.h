@@ -19,6 +19,8 @@ struct hpspmm_ctx {
   // scratch for plan-less calls: chunk table and carries
   void* scratch;
   size_t scratch_bytes;
+  size_t zero_prefix;   // leading bytes of scratch that are zero: the split-row counters of plan-less products, which every
+                        // product leaves at zero; any other use of the scratch ends that (hpspmm_ensure_scratch)
   // staging for the host-buffer entry point
   void* stage;
   size_t stage_bytes;
@@ -64,8 +66,7 @@ struct hpspmm_plan {
 //   rec, 32 bytes per slot of the schedule: {n0, ri, row, row_end} {chunk, row_start, n1, -}: entries [n0, n1) of the
 //   chunk, the row holding entry n0 with its bounds and its position in the list of rows.  One aligned load gives a
 //   warp all it needs, where chunk_order -> chunk_start / chunk_ri -> nz_id are three dependent ones.
-//   Null for calls whose scratch has no room: the kernel then reads chunk_start / chunk_row in matrix order, and
-//   with nz null it steps from row to row along row_ptr.
+//   rec and nz null: warps take the chunks in matrix order, search row_ptr for their bounds and step along row_ptr.
 struct hpspmm_spmm_args {
   int M, K, n_chunks, S;
   int off, cols;               // columns of this launch: [off, off + cols), in slabs of the shape's width
@@ -78,8 +79,6 @@ struct hpspmm_spmm_args {
   float* C;
   const int4* rec;
   const int2* nz;
-  const int32_t* chunk_start;
-  const int32_t* chunk_row;
   float* carry;
   int32_t* counter;
 };
@@ -169,6 +168,8 @@ struct hpspmm_trace_range {
 #define HPSPMM_TRACE(name) hpspmm_trace_range hpspmm_trace_range__(name)
 
 int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes);
+// the same for a caller that keeps counters in the first `prefix` bytes and nothing else there: they are zero afterwards
+int hpspmm_ensure_scratch_counters(hpspmm_ctx* ctx, size_t bytes, size_t prefix, cudaStream_t stream);
 int hpspmm_ensure_stage(hpspmm_ctx* ctx, size_t bytes);
 
 // nominal chunk size for a dense width and a matrix of nnz entries
@@ -188,7 +189,7 @@ int hpspmm_order_chunks_by_cost(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t n
 
 // Builds the structure a product walks, in two launches: the list of rows that hold entries (nz, hpspmm_nz_bytes(M)
 // bytes, with sentinels (M, INT_MAX) at its end) and one record per chunk in matrix order (rec_out, 2 * n_chunks int4).
-// counts: hpspmm_row_tiles(M) ints of scratch.  counter (n_counter ints) is zeroed.  The arrays of `tables` are
+// counts: hpspmm_row_tiles(M) ints of scratch.  The arrays of `tables` are
 // filled as well where they are given (a plan exposes them), and split_count receives the number of chunks that
 // begin inside a row.
 struct hpspmm_structure_tables {
@@ -202,8 +203,7 @@ struct hpspmm_structure_tables {
 int64_t hpspmm_row_tiles(int64_t M);
 size_t hpspmm_nz_bytes(int64_t M);
 int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr, int32_t S, int64_t n_chunks,
-                           int2* nz, int4* rec_out, int32_t* counts, int32_t* counter, int64_t n_counter,
-                           const hpspmm_structure_tables& tables, cudaStream_t stream);
+                           int2* nz, int4* rec_out, int32_t* counts, const hpspmm_structure_tables& tables, cudaStream_t stream);
 // rec[slot] = rec_in[order[slot]]
 int hpspmm_order_records(hpspmm_ctx* ctx, int64_t n_chunks, const int32_t* order, const int4* rec_in, int4* rec,
                          cudaStream_t stream);

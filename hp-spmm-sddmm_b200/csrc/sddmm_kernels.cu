@@ -387,7 +387,7 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
     char* base = (char*)ctx->scratch;
     int4* rec = (int4*)(base + b_tiles);
     int2* nz = (int2*)(base + b_tiles + b_rec);
-    st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, n_chunks, nz, rec, (int32_t*)base, nullptr, 0,
+    st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, n_chunks, nz, rec, (int32_t*)base,
                                 hpspmm_structure_tables{}, s);
     if (st != HPSPMM_OK) return st;
     a.n_chunks = (int)n_chunks;

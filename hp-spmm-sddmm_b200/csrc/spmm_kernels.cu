@@ -26,37 +26,6 @@ using namespace hpspmm;
 
 constexpr int kBlockThreads = 256;
 
-// ---- chunk table -----------------------------------------------------------------------
-
-// Used where there is no room for the records of hpspmm_build_structure: first entry of every chunk and the row
-// that holds it, by binary search per cut.
-__global__ void chunk_table_kernel(int M, int nnz, const int* __restrict__ row_ptr, int S,
-                                   int n_chunks, int* __restrict__ chunk_start,
-                                   int* __restrict__ chunk_row, int* __restrict__ run_counter) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > n_chunks) return;
-  run_counter[c] = 0;   // per-row counters of the in-kernel carry settlement
-  if (c == n_chunks) {
-    chunk_start[c] = nnz;
-    return;
-  }
-  const int t = c * S;
-  // first index i in [0, M] with row_ptr[i] > t
-  int lo = 0, hi = M + 1;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(row_ptr + mid) <= t)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  int r = lo - 1;
-  r = r < 0 ? 0 : (r > M - 1 ? M - 1 : r);  // only a malformed row_ptr can need this
-  const int rs = __ldg(row_ptr + r), re = __ldg(row_ptr + r + 1);
-  chunk_start[c] = c == 0 ? 0 : ((re - rs <= S) ? rs : t);
-  chunk_row[c] = r;
-}
-
 // ---- row-split kernel: one W-lane worker per row, K = 4 * W * R --------------------------------
 // HPSPMM_ALGO_ROW_SPLIT: the shape of the reference's GESpMM, every row summed in storage order.
 template <int W, int R, int U, int MINB, bool HINT>
@@ -644,18 +613,27 @@ int32_t planless_chunk_nnz(int64_t K, int64_t nnz, const hpspmm_opts* opts) {
   return (S + 31) / 32 * 32;
 }
 
-// where a plan-less product keeps what it builds, inside the context's scratch
+// Whether a product without a plan lets every warp search row_ptr for its chunk (one launch) instead of building the
+// records and the list of filled rows first (two more).  A search costs a chunk 1 to 2 us of latency, the builders 5 us
+// and more per call; with more chunks than fit on the GPU the searches add up.  With very many empty rows
+// between the entries the list pays for itself.
+bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t n_chunks) {
+  return n_chunks <= ctx->sm_count * 40ll && M <= 8 * nnz;
+}
+
+// where a plan-less product keeps what it builds, inside the context's scratch; the counters come first
 struct planless_layout {
-  size_t tiles, counter, rec, nz, carry, bytes;
-  planless_layout(int64_t M, int64_t K, int64_t n_chunks) {
+  size_t counter, carry, tiles, rec, nz, bytes;
+  planless_layout(int64_t M, int64_t K, int64_t n_chunks, bool search) {
     bytes = 0;
     auto take = [&](size_t b) { const size_t at = bytes; bytes += align_up(b, 256); return at; };
-    tiles = take((size_t)hpspmm_row_tiles(M) * 4);
     counter = take((size_t)(n_chunks + 1) * (size_t)hpspmm_counter_slabs(K) * 4);
-    rec = take((size_t)(n_chunks + 1) * 32);
-    nz = take(hpspmm_nz_bytes(M));
     carry = take((size_t)(n_chunks + 1) * (size_t)K * 4);
+    tiles = search ? 0 : take((size_t)hpspmm_row_tiles(M) * 4);
+    rec = search ? 0 : take((size_t)(n_chunks + 1) * 32);
+    nz = search ? 0 : take(hpspmm_nz_bytes(M));
   }
+  size_t counter_bytes() const { return carry; }
 };
 
 }  // namespace
@@ -719,9 +697,9 @@ int hpspmm_plan_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const
   int4* rec_by_chunk = (int4*)(scratch + b_sort + b_tiles);
   if (st == HPSPMM_OK) e = cudaMemsetAsync(ctx->flag, 0, sizeof(int), s);
   if (st == HPSPMM_OK && e == cudaSuccess) e = cudaMemsetAsync(p->chunk_start, 0, 4, s);
+  if (st == HPSPMM_OK && e == cudaSuccess) e = cudaMemsetAsync(p->run_counter, 0, b_count, s);
   if (st == HPSPMM_OK && e == cudaSuccess)
     st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, p->n_chunks, p->nz, rec_by_chunk, (int32_t*)(scratch + b_sort),
-                                p->run_counter, n_counter,
                                 hpspmm_structure_tables{p->chunk_start, p->chunk_row, p->chunk_ri, p->nz_id, p->nz_end,
                                                         ctx->flag}, s);
   if (st == HPSPMM_OK && e == cudaSuccess && M > 0)
@@ -826,19 +804,21 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
   }
   const int32_t S = planless_chunk_nnz(K, nnz, opts);
   const int64_t n_chunks = (nnz + S - 1) / S;
-  const int64_t n_counter = n_chunks * hpspmm_counter_slabs(K);
-  const planless_layout lay(M, K, n_chunks);
-  st = hpspmm_ensure_scratch(ctx, lay.bytes);
+  const bool search = searches_for_chunks(ctx, M, nnz, n_chunks);
+  const planless_layout lay(M, K, n_chunks, search);
+  st = hpspmm_ensure_scratch_counters(ctx, lay.bytes, lay.counter_bytes(), s);
   if (st != HPSPMM_OK) return st;
   char* base = (char*)ctx->scratch;
-  int4* rec = (int4*)(base + lay.rec);
-  int2* nz = (int2*)(base + lay.nz);
-  int32_t* counter = (int32_t*)(base + lay.counter);
-  st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, n_chunks, nz, rec, (int32_t*)(base + lay.tiles), counter,
-                              n_counter, hpspmm_structure_tables{}, s);
-  if (st != HPSPMM_OK) return st;
   a.n_chunks = (int)n_chunks, a.S = S;
-  a.rec = rec, a.nz = nz, a.carry = (float*)(base + lay.carry), a.counter = counter;
+  a.carry = (float*)(base + lay.carry), a.counter = (int32_t*)(base + lay.counter);
+  if (!search) {
+    int4* rec = (int4*)(base + lay.rec);
+    int2* nz = (int2*)(base + lay.nz);
+    st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, n_chunks, nz, rec, (int32_t*)(base + lay.tiles),
+                                hpspmm_structure_tables{}, s);
+    if (st != HPSPMM_OK) return st;
+    a.rec = rec, a.nz = nz;
+  }
   return launch_spmm(ctx, a, hint, false, s);
 }
 
@@ -887,7 +867,8 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
     for (int i = 0; i < n_slabs; ++i) {
       const int64_t w = slabs[i].width;
       const int32_t S = planless_chunk_nnz(w, nnz, opts);
-      const size_t want = planless_layout(M, w, (nnz + S - 1) / S).bytes;
+      const int64_t n_chunks = (nnz + S - 1) / S;
+      const size_t want = planless_layout(M, w, n_chunks, searches_for_chunks(ctx, M, nnz, n_chunks)).bytes;
       need = want > need ? want : need;
     }
     st = hpspmm_ensure_scratch(ctx, need);
@@ -1134,13 +1115,13 @@ extern "C" int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
     if (S > probing_chunk_nnz(K)) S = probing_chunk_nnz(K);
     n_chunks = (nnz + S - 1) / S;
     b_int = align_up((size_t)(n_chunks + 1) * 4, 256);
-    need = 3 * b_int + align_up((size_t)(n_chunks + 1) * (size_t)K * 4, 256);
+    need = b_int + align_up((size_t)(n_chunks + 1) * (size_t)K * 4, 256);
     if (need <= (size_t)HPSPMM_STATIC_SCRATCH_BYTES || S == probing_chunk_nnz(K)) break;
     S = probing_chunk_nnz(K);
   }
   if (need > (size_t)HPSPMM_STATIC_SCRATCH_BYTES) {
     char msg[256];
-    const long long max_chunks = (long long)(HPSPMM_STATIC_SCRATCH_BYTES - 4 * 256) / (12 + 4 * K) - 1;
+    const long long max_chunks = (long long)(HPSPMM_STATIC_SCRATCH_BYTES - 2 * 256) / (4 + 4 * K) - 1;
     snprintf(msg, sizeof(msg),
              "matrix too large for the static scratch: nnz = %lld at K = %lld needs %zu bytes, the "
              "array holds %u (about %lld nnz at this K); use hpspmm_spmm_csr_f32 instead",
@@ -1178,16 +1159,11 @@ extern "C" int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
   }
   local.sm_count = state.sm_count;
 
-  // Every call rewrites the whole chunk table and zeroes the per-row counters (the table kernel does both), and a
-  // carry slot is read only where this call hands a carry on, so nothing left over from an earlier call is ever
-  // consumed.
-  int32_t* chunk_start = (int32_t*)state.base;
-  int32_t* chunk_row = (int32_t*)(state.base + b_int);
-  int32_t* run_counter = (int32_t*)(state.base + 2 * b_int);
+  // Every call zeroes the per-row counters, and a carry slot is read only where this call hands a carry on, so
+  // nothing left over from an earlier call is ever consumed.
+  int32_t* run_counter = (int32_t*)state.base;
   cudaStream_t s = (cudaStream_t)stream;
-  chunk_table_kernel<<<(unsigned)((n_chunks + 1 + 255) / 256), 256, 0, s>>>((int)M, (int)nnz, row_ptr, S, (int)n_chunks,
-                                                                            chunk_start, chunk_row, run_counter);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = cudaMemsetAsync(run_counter, 0, b_int, s);
   if (e != cudaSuccess) {
     write_err(err_buf, err_len, cudaGetErrorString(e));
     return HPSPMM_ERR_CUDA;
@@ -1196,8 +1172,7 @@ extern "C" int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
   memset(&a, 0, sizeof(a));
   a.M = (int)M, a.K = (int)K, a.n_chunks = (int)n_chunks, a.S = S;
   a.row_ptr = row_ptr, a.col_idx = col_idx, a.vals = vals, a.B = B, a.C = C;
-  a.chunk_start = chunk_start, a.chunk_row = chunk_row;
-  a.carry = (float*)(state.base + 3 * b_int), a.counter = run_counter;
+  a.carry = (float*)(state.base + b_int), a.counter = run_counter;
   st = launch_spmm(&local, a, gather_hint(K, nullptr), /*shared_counters=*/true, s);
   if (st != HPSPMM_OK) write_err(err_buf, err_len, local.err);
   return st;

@@ -54,37 +54,33 @@ __device__ __forceinline__ void zero_empty_rows(int M, int K, const int* __restr
   }
 }
 
-// Next non-empty row after `row`, given that entry j (< nnz) follows the end of `row`, as (row_end << 32) | row.
-// Probes 16 rows, then gallops (16, 32, 64, ... rows ahead) to bracket the row that holds j and searches inside
-// the bracket.  For calls without a list of the rows that hold entries; out of line so that its registers do not
-// weigh on the gather loop of the caller.
-static __device__ __noinline__ unsigned long long probe_next_row(const int* __restrict__ row_ptr, int M, int j, int row) {
-  int e, probes = 0;
-  do {
-    ++row;
-    e = __ldg(row_ptr + row + 1);
-  } while (e == j && ++probes < 16);
-  if (e == j) {
-    int lo = row + 1, step = 16, hi;
-    for (;;) {
-      hi = min(lo + step, M);
-      if (hi == M || __ldg(row_ptr + hi) > j) break;
-      lo = hi;
-      step <<= 1;
-    }
-    ++hi;
-    ++lo;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (__ldg(row_ptr + mid) <= j)
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    row = lo - 1;
-    e = __ldg(row_ptr + row + 1);
+// The row that holds entry t, i.e. the last r in [lo, hi) with row_ptr[r] <= t, given that row_ptr[lo] <= t.  The
+// whole warp searches: 32 probes a round, so a million rows take four rounds of one load.
+__device__ __forceinline__ int find_row(const int* __restrict__ row_ptr, int lo, int hi, int t) {
+  const int lane = threadIdx.x & 31;
+  while (hi - lo > 1) {
+    const int step = (int)(((unsigned)(hi - lo) + 31u) >> 5);
+    const int64_t r = lo + (int64_t)lane * step;
+    const unsigned m = __ballot_sync(0xffffffffu, r < hi && __ldg(row_ptr + r) <= t);
+    lo += (__popc(m | 1u) - 1) * step;   // lane 0 probes lo itself
+    hi = step < hi - lo ? lo + step : hi;
   }
-  return ((unsigned long long)(unsigned)e << 32) | (unsigned)row;
+  return lo;
+}
+
+// The next row that holds entries after `row`, whose end is `row_end` (< nnz): (row, end).  The warp looks at 32 rows
+// at once and searches when all of them are empty.
+__device__ __forceinline__ int2 next_filled_row(const int* __restrict__ row_ptr, int M, int row, int row_end) {
+  const int lane = threadIdx.x & 31;
+  const int r = row + 1 + lane;   // candidate
+  const int e = __ldg(row_ptr + (r + 1 < M ? r + 1 : M));
+  const unsigned m = __ballot_sync(0xffffffffu, e > row_end);
+  if (m) {
+    const int b = __ffs(m) - 1;
+    return make_int2(row + 1 + b, __shfl_sync(0xffffffffu, e, b));
+  }
+  const int f = find_row(row_ptr, row + 32, M, row_end);
+  return make_int2(f, __ldg(row_ptr + f + 1));
 }
 
 // Adds up one split row.  A row longer than S is cut at multiples of S only, so its pieces are the chunks
@@ -146,18 +142,11 @@ __device__ __forceinline__ void settle_split_row(int r, int r_start, int r_end, 
   if (lane == 0) counter[first] = 0;   // ready for the next launch
 }
 
-// Slot of the schedule this warp takes.  Read from the special registers anew at every use (volatile), so that the
-// compiler does not keep it in a register from the prologue to the tail of the kernel.
-template <int BT>
-__device__ __forceinline__ int chunk_slot() {
-  unsigned cta, tid;
-  asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
-  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
-  return (int)((cta * (unsigned)BT + tid) >> 5);
-}
-
 // KS: row stride of B and C when it is a compile-time constant (the whole width is one full slab), else 0.
-// LIST: the rows that hold entries are listed (a.nz, with records a.rec); without the list the kernel probes row_ptr.
+// LIST: the rows that hold entries are listed (a.nz, with records a.rec).  Without the list a warp finds the bounds
+// of its chunk by searching row_ptr and steps from row to row along row_ptr: for calls without a plan whose matrix is
+// so small that the two launches that build the list would cost more than the searches, and for the allocation-free
+// entry point, whose scratch has no room for it.
 template <int VEC, int W, int R, int U, int KS, int BT, int MINB, bool HINT, bool LIST>
 __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_constant__ hpspmm_spmm_args a) {
   constexpr int CW = VEC * W * R;   // columns a warp covers
@@ -169,6 +158,7 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   static_assert(BATCH <= T && T % BATCH == 0, "batch must tile the staged tile");
   static_assert(KS == 0 || KS == CW, "a fixed stride is the width of the slab");
   __shared__ int2 tiles[BT / 32][STAGES][T];
+  __shared__ int meta[BT / 32][8];
 
   if ((int)blockIdx.x >= a.n_chunk_blocks) {
     if (blockIdx.y == 0 && a.slab0 == 0 && a.off == 0)
@@ -180,18 +170,34 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   const int l = lane % W;   // position inside the group
   int n1, row, row_end, ri, base;
   {
-    const int slot = chunk_slot<BT>();
+    const int slot = (int)((blockIdx.x * (unsigned)BT + threadIdx.x) >> 5);
     if (slot >= a.n_chunks) return;
+    int* m = meta[threadIdx.x >> 5];   // what the tail of the kernel needs of the chunk waits in shared memory
     if (LIST) {
-      const int4 p = __ldg(a.rec + 2 * (int64_t)slot);
+      const int4 p = __ldg(a.rec + 2 * (int64_t)slot), q = __ldg(a.rec + 2 * (int64_t)slot + 1);
       base = p.x, ri = p.y, row = p.z, row_end = p.w;
-      n1 = __ldg(&a.rec[2 * (int64_t)slot + 1].z);
+      n1 = q.z;
+      if (lane == 0) m[0] = base, m[1] = q.x, m[2] = row, m[3] = q.y, m[4] = row_end;
     } else {
+      // chunk `slot` begins at the start of the row that holds entry slot * S, or at that entry if the row is longer
+      // than S; it ends where the next one begins
       ri = 0;
-      base = __ldg(a.chunk_start + slot);
-      n1 = __ldg(a.chunk_start + slot + 1);
-      row = __ldg(a.chunk_row + slot);
+      const int t0 = slot * a.S, t1 = t0 + a.S;
+      row = find_row(a.row_ptr, 0, a.M, t0);
+      const int rs = __ldg(a.row_ptr + row);
       row_end = __ldg(a.row_ptr + row + 1);
+      base = slot == 0 ? 0 : (row_end - rs <= a.S ? rs : t0);
+      if (slot + 1 < a.n_chunks) {
+        n1 = t1;
+        if (row_end <= t1) {   // (a row that reaches from t0 over t1 is longer than S and is cut there)
+          const int r1 = find_row(a.row_ptr, row + 1, a.M, t1);
+          const int s1 = __ldg(a.row_ptr + r1), e1 = __ldg(a.row_ptr + r1 + 1);
+          if (e1 - s1 <= a.S) n1 = s1;
+        }
+      } else {
+        n1 = __ldg(a.row_ptr + a.M);
+      }
+      if (lane == 0) m[0] = base, m[1] = slot, m[2] = row, m[3] = rs, m[4] = row_end;
     }
   }
   const int off = KS ? 0 : a.off + (a.slab0 + (int)blockIdx.y) * CW;
@@ -204,6 +210,7 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   constexpr bool AHEAD = W <= 16;
   int2 next = make_int2(0, 0);
   if (LIST && AHEAD) next = __ldg(a.nz + ri + 1);
+  if (!LIST) next.y = __ldg(a.row_ptr + (row + 2 < a.M ? row + 2 : a.M));
 
   auto stage_tile = [&](int stage, int base) {
     const int j = base + lane;
@@ -270,9 +277,16 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
       row_end = next.y;
       if (AHEAD) next = __ldg(a.nz + ri + 1);
     } else {
-      const unsigned long long nr = probe_next_row(a.row_ptr, a.M, row_end, row);
-      row = (int)(unsigned)nr;
-      row_end = (int)(nr >> 32);
+      // next.y: the end of the row below, fetched ahead; the rows below it are looked at when that one is empty
+      if (next.y > row_end) {
+        ++row;
+        row_end = next.y;
+      } else {
+        const int2 f = next_filled_row(a.row_ptr, a.M, row, row_end);
+        row = f.x;
+        row_end = f.y;
+      }
+      next.y = __ldg(a.row_ptr + (row + 2 < a.M ? row + 2 : a.M));
     }
   };
 
@@ -337,21 +351,8 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   }
   cp_async_wait<0>();
 
-  // The chunk is read again from its record: nothing of it has to stay in registers through the loop above.
-  const int slot = chunk_slot<BT>();
-  int n0, chunk, r0, r0_start, r0_end;
-  if (LIST) {
-    const int4 p = __ldg(a.rec + 2 * (int64_t)slot);
-    const int2 q = __ldg(reinterpret_cast<const int2*>(a.rec + 2 * (int64_t)slot + 1));
-    n0 = p.x, r0 = p.z, r0_end = p.w;
-    chunk = q.x, r0_start = q.y;
-  } else {
-    chunk = slot;
-    n0 = __ldg(a.chunk_start + slot);
-    r0 = __ldg(a.chunk_row + slot);
-    r0_start = __ldg(a.row_ptr + r0);
-    r0_end = __ldg(a.row_ptr + r0 + 1);
-  }
+  const int* m = meta[threadIdx.x >> 5];
+  const int n0 = m[0], chunk = m[1], r0 = m[2], r0_start = m[3], r0_end = m[4];
   const bool hands_on = row_end != n1;   // the chunk ends inside `row`
   const int64_t ldc = KS ? KS : a.K;
   float* carry = a.carry + off;
@@ -397,8 +398,8 @@ int launch_spmm_shape(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool shared_counters,
     const dim3 g((unsigned)grid, (unsigned)ny);
     if (a.nz != nullptr)
       spmm_warp_kernel<VEC, W, R, U, KS, BT, MINB, HINT, true><<<g, BT, 0, stream>>>(a);
-    else   // (the allocation-free entry point only: a runtime stride serves every width)
-      spmm_warp_kernel<VEC, W, R, U, 0, BT, 16, true, false><<<g, BT, 0, stream>>>(a);
+    else   // (a runtime stride serves every width)
+      spmm_warp_kernel<VEC, W, R, U, 0, BT, (MINB < 16 ? MINB : 16), true, false><<<g, BT, 0, stream>>>(a);
     ctx->launches++;
   }
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());

@@ -129,8 +129,8 @@ HPSPMM_API int hpspmm_host_fill_uniform_f32(float* host_ptr, int64_t count, uint
  * every width (16-byte gathers when K is a multiple of 4, 8-byte when it is even and the
  * operands are 8-byte aligned, 4-byte otherwise; wider than 512 columns in slabs).
  *
- * plan may be NULL: the structure is then rebuilt into context-owned scratch on
- * every call (two extra small kernels).  The first call that needs more scratch than
+ * plan may be NULL: the warps of a small product then search row_ptr for their part, for a
+ * larger one the structure is rebuilt into context-owned scratch on every call (two extra small kernels).  The first call that needs more scratch than
  * the context holds allocates it (cudaMalloc, synchronising); later calls do not.
  * With a plan the call only enqueues kernels (no allocation, no synchronisation), so it can
  * be recorded into a CUDA graph and replayed.
@@ -185,7 +185,7 @@ HPSPMM_API int hpspmm_plan_row_list(const hpspmm_plan* plan, const int32_t** nz_
  * no context.  The chunk table, the carry slots and the per-row counters of the nnz-balanced
  * kernel live in one 16 MiB array inside the library image, so every GPU that loads the library gives up
  * 16 MiB until the process exits.  A matrix whose scratch would not fit -- more than
- * (16 MiB - 1.25 KiB) / (12 + 4 K) chunks (of 128 / 160 / 256 nnz at K = 32 / 64 / 128):
+ * (16 MiB - 0.5 KiB) / (4 + 4 K) chunks (of 128 / 160 / 256 nnz at K = 32 / 64 / 128):
  * about 15 M nnz at K = 32, 10 M at K = 64, 8 M at K = 128 -- is refused with HPSPMM_ERR_UNSUPPORTED and a message in
  * err_buf; use hpspmm_spmm_csr_f32 for it.
  *
