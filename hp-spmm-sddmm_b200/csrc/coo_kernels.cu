@@ -101,7 +101,7 @@ spmm_coo_warp_kernel(int64_t nnz, int S, const int* __restrict__ row_idx, const 
           if (live) reduce_into(crow + r * W * VEC + group_split<VEC, W>::column(lane), v);
         } else {
           all_reduce_groups<VEC, W>(acc[r]);
-          if (g == 0 && live) reduce_into(crow + l * VEC, acc[r]);
+          if (g == 0 && live) reduce_into(crow + (r * W + l) * VEC, acc[r]);
         }
       }
     }
@@ -190,6 +190,7 @@ int launch_coo(hpspmm_ctx* ctx, const coo_args& a, cudaStream_t s) {
   const int64_t blocks = (workers + BT / 32 - 1) / (BT / 32);
   const int64_t slabs = (a.cols + CW - 1) / CW;
   if (blocks > 2147483647ll || slabs > 65535) return HPSPMM_ERR_UNSUPPORTED;
+  if (!hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
   spmm_coo_warp_kernel<VEC, W, R, U, KS, BT, MINB><<<dim3((unsigned)blocks, (unsigned)slabs), BT, 0, s>>>(
       a.nnz, a.S, a.row_idx, a.col_idx, a.vals, a.B, a.C, a.K, a.off, a.cols);
   ctx->launches++;
@@ -219,6 +220,7 @@ int launch_coo_shape(hpspmm_ctx* ctx, const coo_args& a, const hpspmm_spmm_shape
     if (sh.W == 16) GO(2, 16, 1, 8, 0, 16);
     if (sh.R == 1) GO(2, 32, 1, 8, 0, 16);
     if (sh.R == 2) GO(2, 32, 2, 4, 0, 16);
+    if (sh.R == 3) GO(2, 32, 3, 2, 0, 16);
     GO(2, 32, 4, 2, 0, 16);
   }
   if (sh.W == 1) GO(1, 1, 1, 1, 0, 16);
@@ -227,7 +229,11 @@ int launch_coo_shape(hpspmm_ctx* ctx, const coo_args& a, const hpspmm_spmm_shape
   if (sh.W == 16) GO(1, 16, 1, 8, 0, 16);
   if (sh.R == 1) GO(1, 32, 1, 8, 0, 16);
   if (sh.R == 2) GO(1, 32, 2, 8, 0, 16);
-  if (sh.R <= 4) GO(1, 32, 4, 4, 0, 16);
+  if (sh.R == 3) GO(1, 32, 3, 4, 0, 16);
+  if (sh.R == 4) GO(1, 32, 4, 4, 0, 16);
+  if (sh.R == 5) GO(1, 32, 5, 2, 0, 16);
+  if (sh.R == 6) GO(1, 32, 6, 2, 0, 16);
+  if (sh.R == 7) GO(1, 32, 7, 2, 0, 16);
   GO(1, 32, 8, 2, 0, 16);
 #undef GO
 }

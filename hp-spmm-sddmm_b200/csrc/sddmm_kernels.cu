@@ -295,6 +295,7 @@ template <int VEC, int W, int R, int U, int KS, bool HINT, int MINB>
 int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
   constexpr int BT = 64, CW = VEC * W * R;
   const unsigned grid = (unsigned)((a.n_chunks + BT / 32 - 1) / (BT / 32));
+  if (!hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
   for (int off = a.off; off < a.off + a.cols; off += CW) {
     const int left = a.off + a.cols - off;
     sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, (KS > 0)><<<grid, BT, 0, s>>>(
@@ -331,6 +332,7 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
     if (sh.W == 16) GO(2, 16, 1, 8, 0, true, 16);
     if (sh.R == 1) GO(2, 32, 1, 8, 0, true, 16);
     if (sh.R == 2) GO(2, 32, 2, 4, 0, true, 16);
+    if (sh.R == 3) GO(2, 32, 3, 4, 0, true, 14);
     GO(2, 32, 4, 4, 0, true, 12);
   }
   if (sh.W == 1) GO(1, 1, 1, 1, 0, true, 16);
@@ -339,7 +341,11 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
   if (sh.W == 16) GO(1, 16, 1, 8, 0, true, 16);
   if (sh.R == 1) GO(1, 32, 1, 8, 0, true, 16);
   if (sh.R == 2) GO(1, 32, 2, 8, 0, true, 16);
-  if (sh.R <= 4) GO(1, 32, 4, 4, 0, true, 16);
+  if (sh.R == 3) GO(1, 32, 3, 4, 0, true, 16);
+  if (sh.R == 4) GO(1, 32, 4, 4, 0, true, 16);
+  if (sh.R == 5) GO(1, 32, 5, 4, 0, true, 14);
+  if (sh.R == 6) GO(1, 32, 6, 4, 0, true, 14);
+  if (sh.R == 7) GO(1, 32, 7, 4, 0, true, 12);
   GO(1, 32, 8, 4, 0, true, 12);
 #undef GO
 }

@@ -391,6 +391,7 @@ int launch_spmm_shape(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool shared_counters,
   const int slabs = (a.cols + CW - 1) / CW;
   const int64_t grid = (int64_t)a.n_chunk_blocks + n_zero_blocks;
   if (grid == 0) return HPSPMM_OK;
+  if (!hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
   const int step = shared_counters ? 1 : 65535;
   for (int s = 0; s < slabs; s += step) {
     a.slab0 = s;

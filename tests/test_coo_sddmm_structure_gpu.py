@@ -113,6 +113,38 @@ def test_sddmm(gpu_ctx, pkg, oracle, K, use_plan):
         b.free()
 
 
+@pytest.mark.parametrize("few_entries", [False, True])
+@pytest.mark.parametrize("K", [2, 5, 14, 37, 66, 95, 130, 145, 193, 198, 225, 258, 333, 390, 515])
+def test_coo_and_sddmm_at_every_vector_count(gpu_ctx, pkg, oracle, K, few_entries):
+    """One width for every instance of the two kernels: vectors of 4, 2, 1 floats, 1 to 8 per lane, the last one full
+    or not; with few chunks and with many."""
+    ctx = gpu_ctx
+    g = pkg.gen_rmat(9 if few_entries else 15, 16, seed=95)
+    M, N, nnz = g["M"], g["N"], g["nnz"]
+    X = pkg.host_fill_uniform(M * K, 95, 1, -1.0, 1.0).reshape(M, K)
+    Y = pkg.host_fill_uniform(N * K, 95, 2, -1.0, 1.0).reshape(N, K)
+    d_rp, d_ci, d_X, d_Y = ctx.upload(g["row_ptr"]), ctx.upload(g["col_idx"]), ctx.upload(X), ctx.upload(Y)
+    ref, abs_sum = oracle.sddmm_f64(g["row_ptr"], g["col_idx"], X, Y)
+    for use_plan in (False, True):
+        buf, o_ptr, read = guarded_output(ctx, (nnz,))
+        plan = ctx.plan_create(M, nnz, d_rp, K, N=N, col_idx=d_ci) if use_plan else None
+        ctx.sddmm_csr(M, N, K, nnz, d_rp, d_ci, d_X, d_Y, o_ptr, plan=plan)
+        ctx.stream_sync()
+        check_against_f64(read(), ref, abs_sum, "sddmm K=%d plan=%s" % (K, use_plan))
+        if plan:
+            ctx.plan_destroy(plan)
+        buf.free()
+    r, c, v = oracle.csr_to_coo_padded(g["row_ptr"], g["col_idx"], g["vals"], 32)
+    d_r, d_c, d_v = ctx.upload(r), ctx.upload(c), ctx.upload(v)
+    buf, c_ptr, read = guarded_output(ctx, (M, K), fill=np.float32(0))
+    ctx.spmm_coo(M, N, K, len(r), d_r, d_c, d_v, d_Y, c_ptr)
+    ctx.stream_sync()
+    ref, abs_sum = oracle.spmm_f64(g["row_ptr"], g["col_idx"], g["vals"], Y)
+    check_against_f64(read(), ref, abs_sum, "coo K=%d" % K)
+    for b in (d_rp, d_ci, d_X, d_Y, d_r, d_c, d_v, buf):
+        b.free()
+
+
 def test_sddmm_edge_structures(gpu_ctx, pkg, oracle):
     ctx = gpu_ctx
     rng = np.random.default_rng(3)

@@ -56,6 +56,59 @@ def test_generic_widths(gpu_ctx, pkg, oracle, K):
     _check(gpu_ctx, pkg, oracle, row_ptr, col_idx, vals, B, "generic K=%d" % K)
 
 
+@pytest.mark.parametrize("few_entries", [False, True])
+@pytest.mark.parametrize("K", [2, 5, 9, 14, 23, 34, 37, 66, 70, 95, 97, 130, 145, 193, 198, 225, 255, 258, 333, 386, 390, 515, 1030])
+def test_every_vector_width_and_count(gpu_ctx, pkg, oracle, K, few_entries):
+    """One width for every instance of the product kernel (vectors of 4, 2, 1 floats, 1 to 8 per lane, a last vector
+    that is full or not, more than one slab), with and without a plan, with few chunks and with many; canaries
+    stand on both sides of C, and a store past a row's end would also corrupt the next row."""
+    g = pkg.gen_rmat(9 if few_entries else 15, 16, seed=91)
+    N = g["N"]
+    B = pkg.host_fill_uniform(N * K, 91, K, -1.0, 1.0).reshape(N, K)
+    for use_plan in (False, True):
+        _check(gpu_ctx, pkg, oracle, g["row_ptr"], g["col_idx"], g["vals"], B, "K=%d plan=%s" % (K, use_plan),
+               use_plan=use_plan)
+
+
+@pytest.mark.parametrize("K", [2, 6, 64])
+def test_operands_that_are_only_four_byte_aligned(gpu_ctx, pkg, oracle, K):
+    """An even width with operands off the 8-byte grid takes the 4-byte gathers; a multiple of 4 is refused."""
+    g = pkg.gen_rmat(9, 16, seed=92)
+    M, N, nnz = g["M"], g["N"], g["nnz"]
+    B = pkg.host_fill_uniform(N * K, 92, K, -1.0, 1.0).reshape(N, K)
+    d_rp, d_ci, d_v = (gpu_ctx.upload(g[k]) for k in ("row_ptr", "col_idx", "vals"))
+    d_B = gpu_ctx.upload(np.concatenate([[np.float32(7)], B.reshape(-1)]))
+    d_C = gpu_ctx.alloc((M * K + 1,), np.float32)
+    call = lambda: gpu_ctx.spmm_csr(M, N, K, nnz, d_rp, d_ci, d_v, d_B.ptr + 4, d_C.ptr + 4)
+    if K % 4 == 0:
+        with pytest.raises(pkg.HpspmmError):
+            call()
+    else:
+        call()
+        ref, abs_sum = oracle.spmm_f64(g["row_ptr"], g["col_idx"], g["vals"], B)
+        check_against_f64(d_C.to_host()[1:].reshape(M, K), ref, abs_sum, "four-byte aligned K=%d" % K)
+    for b in (d_rp, d_ci, d_v, d_B, d_C):
+        b.free()
+
+
+def test_calls_without_a_plan_between_other_users_of_the_scratch(gpu_ctx, pkg, oracle):
+    """A plan-less product relies on counters that its predecessors left at zero in the context's scratch: other calls
+    that use the scratch in between, and products of other sizes and widths, must not disturb it."""
+    ctx = gpu_ctx
+    graphs = [pkg.gen_rmat(s, 16, seed=93) for s in (12, 9, 15)]
+    for turn in range(2):
+        for g in graphs:
+            M, N, nnz = g["M"], g["N"], g["nnz"]
+            for K in (64, 7):
+                B = pkg.host_fill_uniform(N * K, 93, K, -1.0, 1.0).reshape(N, K)
+                _check(ctx, pkg, oracle, g["row_ptr"], g["col_idx"], g["vals"], B, "scratch M=%d K=%d" % (M, K))
+            d = [ctx.upload(g[k]) for k in ("row_ptr", "col_idx", "vals")]
+            o = [ctx.alloc((n,), t) for n, t in ((N + 1, np.int32), (nnz, np.int32), (nnz, np.float32))]
+            ctx.csr_transpose(M, N, nnz, *d, *o)          # fills the scratch with sort keys
+            for b in d + o:
+                b.free()
+
+
 @pytest.mark.parametrize("K", [32, 64, 128, 48])
 def test_edge_structures(gpu_ctx, pkg, oracle, K):
     rng = np.random.default_rng(5)
