@@ -529,7 +529,9 @@ int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz) {
 }
 
 int32_t hpspmm_coo_chunk_nnz(int64_t K, int64_t nnz) {
-  const int32_t best = probing_chunk_nnz(K);
+  // 4 M triples of a power-law graph, S = 64 / 128 / 160 / 256: K = 32 56.0 / 56.2 / 57.6 / 63.0 us, K = 64 78.6 / 77.3 /
+  // 78.1 / 83.2; below 768 K triples as many chunks as the GPU has warps, down to 32 triples.
+  const int32_t best = K <= 128 ? 128 : 256;
   const int64_t want = nnz / 6000 / 32 * 32;
   return (int32_t)(want < 32 ? 32 : (want > best ? best : want));
 }
