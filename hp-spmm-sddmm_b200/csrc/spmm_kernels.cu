@@ -930,6 +930,48 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
   return HPSPMM_OK;
 }
 
+// The same for operands so small that issuing the pipeline takes longer than the copies it overlaps: whole products,
+// one stream, one synchronisation.  slabs[i] are whole products (width == K).
+static int host_products_in_turn(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const int32_t* row_ptr,
+                                 const int32_t* col_idx, const float* vals, const host_slab* slabs, int n_slabs,
+                                 const hpspmm_opts* opts, cudaStream_t s) {
+  int64_t wmax = 1;
+  for (int i = 0; i < n_slabs; ++i) wmax = slabs[i].width > wmax ? slabs[i].width : wmax;
+  const size_t b_rp = align_up((size_t)(M + 1) * 4, 256);
+  const size_t b_nz = align_up((size_t)(nnz > 0 ? nnz : 1) * 4, 256);
+  const size_t b_B = align_up((size_t)(N > 0 ? N : 1) * wmax * 4, 256);
+  int st = hpspmm_ensure_stage(ctx, b_rp + 2 * b_nz + b_B + (size_t)M * wmax * 4);
+  if (st != HPSPMM_OK) return st;
+  char* base = (char*)ctx->stage;
+  int32_t* d_rp = (int32_t*)base;
+  int32_t* d_col = (int32_t*)(base + b_rp);
+  float* d_val = (float*)(base + b_rp + b_nz);
+  float* d_B = (float*)(base + b_rp + 2 * b_nz);
+  float* d_C = (float*)(base + b_rp + 2 * b_nz + b_B);
+  cudaError_t e = cudaMemcpyAsync(d_rp, row_ptr, (size_t)(M + 1) * 4, cudaMemcpyHostToDevice, s);
+  if (nnz > 0) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_col, col_idx, (size_t)nnz * 4, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_val, vals, (size_t)nnz * 4, cudaMemcpyHostToDevice, s);
+  }
+  for (int i = 0; i < n_slabs && e == cudaSuccess && st == HPSPMM_OK; ++i) {
+    const host_slab& p = slabs[i];
+    if (nnz > 0 && N > 0) e = cudaMemcpyAsync(d_B, p.B, (size_t)N * p.K * 4, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+      st = hpspmm_spmm_csr_f32(ctx, nullptr, M, N, p.K, nnz, d_rp, d_col, d_val, d_B, d_C, opts, (hpspmm_stream)s);
+    if (e == cudaSuccess && st == HPSPMM_OK)
+      e = cudaMemcpyAsync(p.C, d_C, (size_t)M * p.K * 4, cudaMemcpyDeviceToHost, s);
+  }
+  const cudaError_t e1 = cudaStreamSynchronize(s);   // whatever happened
+  if (st != HPSPMM_OK) return st;
+  if (e == cudaSuccess) e = e1;
+  if (e != cudaSuccess) return hpspmm_set_err(ctx, HPSPMM_ERR_CUDA, "host-buffer products", e);
+  return HPSPMM_OK;
+}
+
+// Up to here the dense operands travel whole, one after the other: at 55 GB/s they take 75 us, and a slab of the
+// pipeline costs about 15 us to issue.
+static const int64_t kHostInTurnBytes = 4 << 20;
+
 // Width of the column slabs a product of width K travels in.  64 columns when they divide K and leave at
 // least two slabs: with both directions busy this link moves 256-byte rows at 50 GB/s each way and 128-byte
 // rows at 36.  `others_overlap` (several products in one call): a 64-column product then travels whole, as
@@ -983,6 +1025,15 @@ int hpspmm_spmm_csr_f32_host_multi(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
     HPSPMM_REQUIRE(ctx, Ks[i] >= 1 && Ks[i] <= 512, "K must be between 1 and 512");
     HPSPMM_REQUIRE(ctx, Cs[i] != nullptr && (nnz == 0 || Bs[i] != nullptr), "null dense operand");
   }
+  int64_t dense = 0;
+  for (int i = 0; i < n_products; ++i) dense += 4 * Ks[i] * (M + N);
+  if (dense <= kHostInTurnBytes) {
+    for (int i = 0; i < n_products; ++i) slabs[i] = host_slab{Bs[i], Cs[i], Ks[i], Ks[i]};
+    hpspmm_device_guard guard(ctx->device);
+    if (!ctx->pipe_streams[0])
+      HPSPMM_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->pipe_streams[0], cudaStreamNonBlocking));
+    return host_products_in_turn(ctx, M, N, nnz, row_ptr, col_idx, vals, slabs, n_products, opts, ctx->pipe_streams[0]);
+  }
   // Order of the products.  Downloads can start only after the first slab has been uploaded and multiplied, and the
   // download of the very last slab overlaps nothing, so the pipeline should begin AND end on a narrow slab: the
   // product with the narrowest slabs goes last, the next narrowest first, the others between them, widest first.
@@ -1019,33 +1070,10 @@ int hpspmm_spmm_csr_f32_host(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t K, i
   if (M == 0) return HPSPMM_OK;
   hpspmm_device_guard guard(ctx->device);
   const int algo = opts ? opts->algo : HPSPMM_ALGO_AUTO;
-  if (nnz > 0 && N > 0 && K >= 64 && K % 32 == 0 && algo != HPSPMM_ALGO_ROW_SPLIT)
+  if (nnz > 0 && N > 0 && K >= 64 && K % 32 == 0 && algo != HPSPMM_ALGO_ROW_SPLIT && 4 * K * (M + N) > kHostInTurnBytes)
     return host_product_slabs(ctx, M, N, K, nnz, row_ptr, col_idx, vals, B, C, opts);
-  const size_t b_rp = align_up((size_t)(M + 1) * 4, 256);
-  const size_t b_nz = align_up((size_t)nnz * 4, 256);
-  const size_t b_B = align_up((size_t)N * (size_t)K * 4, 256);
-  const size_t b_C = align_up((size_t)M * (size_t)K * 4, 256);
-  int st = hpspmm_ensure_stage(ctx, b_rp + 2 * b_nz + b_B + b_C);
-  if (st != HPSPMM_OK) return st;
-  char* base = (char*)ctx->stage;
-  int32_t* d_rp = (int32_t*)base;
-  int32_t* d_col = (int32_t*)(base + b_rp);
-  float* d_val = (float*)(base + b_rp + b_nz);
-  float* d_B = (float*)(base + b_rp + 2 * b_nz);
-  float* d_C = (float*)(base + b_rp + 2 * b_nz + b_B);
-  cudaStream_t s = 0;
-  HPSPMM_CUDA_TRY(ctx, cudaMemcpyAsync(d_rp, row_ptr, (size_t)(M + 1) * 4, cudaMemcpyHostToDevice, s));
-  if (nnz > 0) {
-    HPSPMM_CUDA_TRY(ctx, cudaMemcpyAsync(d_col, col_idx, (size_t)nnz * 4, cudaMemcpyHostToDevice, s));
-    HPSPMM_CUDA_TRY(ctx, cudaMemcpyAsync(d_val, vals, (size_t)nnz * 4, cudaMemcpyHostToDevice, s));
-    HPSPMM_CUDA_TRY(ctx, cudaMemcpyAsync(d_B, B, (size_t)N * (size_t)K * 4, cudaMemcpyHostToDevice, s));
-  }
-  st = hpspmm_spmm_csr_f32(ctx, nullptr, M, N, K, nnz, d_rp, d_col, d_val, d_B, d_C, opts,
-                           (hpspmm_stream)s);
-  if (st != HPSPMM_OK) return st;
-  HPSPMM_CUDA_TRY(ctx, cudaMemcpyAsync(C, d_C, (size_t)M * (size_t)K * 4, cudaMemcpyDeviceToHost, s));
-  HPSPMM_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-  return HPSPMM_OK;
+  const host_slab whole = {B, C, K, K};
+  return host_products_in_turn(ctx, M, N, nnz, row_ptr, col_idx, vals, &whole, 1, opts, /*default stream*/ 0);
 }
 
 }  // extern "C"
