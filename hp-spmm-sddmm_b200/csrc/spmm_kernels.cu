@@ -522,7 +522,10 @@ int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz) {
   if (nnz < 2400000) return 128;
   const int32_t floor_s = probing_chunk_nnz(K);
   const int32_t best = K <= 32 ? 512 : (K <= 64 ? 320 : 256);
-  const int64_t want = nnz / 24000 / 32 * 32;
+  // In between, S grows with the matrix: 4 M / 8 M entries of a power-law graph, K = 32, S = 160 / 192 / 256 / 384 / 512:
+  // 51 / 50 / 48 / 52 / 58 us and 100 / 97 / 93 / 90 / 87 us.  The SDDMM on the same plan turns up sharply a little
+  // later (4 M, K = 32: 43 / 44 / 57 / 52 us at 160 / 192 / 256 / 384), so the line stays below the product's best.
+  const int64_t want = nnz / 20000 / 32 * 32;
   int64_t s = want < floor_s ? floor_s : want;
   if (s > best) s = best;
   return (int32_t)s;
