@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   }
   const int off = KS ? 0 : a.off + (a.slab0 + (int)blockIdx.y) * CW;
   const int kw = KS ? CW : min(CW, a.cols - (a.slab0 + (int)blockIdx.y) * CW);
-  const uint64_t policy = HINT ? policy_for_gathers(a.keep_b) : 0ull;
+  const uint64_t policy = HINT ? (KS ? policy_evict_last() : policy_for_gathers(a.keep_b)) : 0ull;
   int2(*my)[T] = tiles[threadIdx.x >> 5];
 
   // The row after the current one is fetched while the current one is summed, where the registers allow it (R-MAT
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   // the pieces of a split row settle it among themselves
   const bool stores_split_row = r0_start < n0 && r0_end <= n1;   // began in an earlier chunk, ends here
   if (!hands_on && !stores_split_row) return;
-  int* counter = a.counter + (int64_t)blockIdx.y * a.n_chunks;
+  int* counter = KS ? a.counter : a.counter + (int64_t)blockIdx.y * a.n_chunks;
   if (stores_split_row)
     settle_split_row<VEC, W, R>(r0, r0_start, r0_end, a.S, carry, a.C + off, counter, (int)ldc, kw);
   if (hands_on)
