@@ -218,6 +218,7 @@ int launch_coo_shape(hpspmm_ctx* ctx, const coo_args& a, const hpspmm_spmm_shape
     if (sh.W == 2) GO(2, 2, 1, 2, 0, 16);
     if (sh.W == 4) GO(2, 4, 1, 4, 0, 16);
     if (sh.W == 8) GO(2, 8, 1, 8, 0, 16);
+    if (sh.W == 16 && sh.R == 3) GO(2, 16, 3, 4, 0, 16);
     if (sh.W == 16) GO(2, 16, 1, 8, 0, 16);
     if (sh.R == 1) GO(2, 32, 1, 8, 0, 16);
     if (sh.R == 2) GO(2, 32, 2, 4, 0, 16);
@@ -227,6 +228,7 @@ int launch_coo_shape(hpspmm_ctx* ctx, const coo_args& a, const hpspmm_spmm_shape
   if (sh.W == 1) GO(1, 1, 1, 1, 0, 16);
   if (sh.W == 4) GO(1, 4, 1, 4, 0, 16);
   if (sh.W == 8) GO(1, 8, 1, 8, 0, 16);
+  if (sh.W == 16 && sh.R == 3) GO(1, 16, 3, 4, 0, 16);
   if (sh.W == 16) GO(1, 16, 1, 8, 0, 16);
   if (sh.R == 1) GO(1, 32, 1, 8, 0, 16);
   if (sh.R == 2) GO(1, 32, 2, 8, 0, 16);

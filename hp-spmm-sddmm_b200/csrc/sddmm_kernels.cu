@@ -103,12 +103,12 @@ sddmm_warp_kernel(int n_chunks, int ld, int off0, int cols, int add, int keep_y,
   stage_tile(0, n0);
   stage_tile(1, n0 + T);
 
-  // a lane beyond the slab's width works on column 0 of the slab with an x of zero
+  // a lane beyond the slab's width works on the slab's last vector with an x of zero
   const int kw = KS ? CW : cols;
   const bool live_last = KS || ((R - 1) * W + l) * VEC < kw;
   const unsigned stride = (KS ? KS : ld) * 4u;
-  const int o_first = off0 + ((R > 1 || live_last) ? l * VEC : 0);
-  const int o_last = off0 + (live_last ? ((R - 1) * W + l) * VEC : 0);
+  const int o_first = off0 + ((R > 1 || live_last) ? l * VEC : kw - VEC);
+  const int o_last = off0 + (live_last ? ((R - 1) * W + l) * VEC : kw - VEC);
   const char* Yl = reinterpret_cast<const char*>(Y + o_first);
   const char* Yl_last = reinterpret_cast<const char*>(Y + o_last);
   float x[R][VEC];
@@ -322,8 +322,8 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
     if (sh.W == 4) GO(4, 4, 1, 4, 0, true, 16);
     if (sh.W == 8) GO(4, 8, 1, 4, 0, true, 16);
     if (sh.W == 16) GO(4, 16, 1, 4, 0, true, 16);
-    if (sh.R == 1) GO(4, 32, 1, 4, 0, true, 16);
-    if (sh.R == 2) GO(4, 32, 2, 2, 0, true, 16);
+    if (sh.R == 1) GO(4, 32, 1, 4, 0, true, 18);
+    if (sh.R == 2) GO(4, 32, 2, 2, 0, true, 18);
     if (sh.R == 3) GO(4, 32, 3, 2, 0, true, 12);
     GO(4, 32, 4, 2, 0, true, 10);
   }
@@ -331,6 +331,7 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
     if (sh.W == 2) GO(2, 2, 1, 2, 0, true, 16);
     if (sh.W == 4) GO(2, 4, 1, 4, 0, true, 16);
     if (sh.W == 8) GO(2, 8, 1, 8, 0, true, 16);
+    if (sh.W == 16 && sh.R == 3) GO(2, 16, 3, 4, 0, true, 14);
     if (sh.W == 16) GO(2, 16, 1, 8, 0, true, 16);
     if (sh.R == 1) GO(2, 32, 1, 8, 0, true, 16);
     if (sh.R == 2) GO(2, 32, 2, 4, 0, true, 16);
@@ -340,6 +341,7 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
   if (sh.W == 1) GO(1, 1, 1, 1, 0, true, 16);
   if (sh.W == 4) GO(1, 4, 1, 4, 0, true, 16);
   if (sh.W == 8) GO(1, 8, 1, 8, 0, true, 16);
+  if (sh.W == 16 && sh.R == 3) GO(1, 16, 3, 4, 0, true, 18);
   if (sh.W == 16) GO(1, 16, 1, 8, 0, true, 16);
   if (sh.R == 1) GO(1, 32, 1, 8, 0, true, 16);
   if (sh.R == 2) GO(1, 32, 2, 8, 0, true, 16);

@@ -154,7 +154,6 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   constexpr int T = 32;             // entries per staged tile
   constexpr int BATCH = U * G;      // entries per batch of gathers
   constexpr int STAGES = 2;
-  static_assert(R == 1 || W == 32, "several vectors per lane only when one group is the warp");
   static_assert(BATCH <= T && T % BATCH == 0, "batch must tile the staged tile");
   static_assert(KS == 0 || KS == CW, "a fixed stride is the width of the slab");
   __shared__ int2 tiles[BT / 32][STAGES][T];
@@ -232,8 +231,8 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
     for (int x = 0; x < VEC; ++x) acc[r][x] = 0.f;
   const bool live_last = KS || ((R - 1) * W + l) * VEC < kw;   // only the last vector of a lane can lie outside
   const unsigned stride = (KS ? KS : a.K) * 4u;                // bytes
-  const char* Bl = reinterpret_cast<const char*>(a.B + off + ((R > 1 || live_last) ? l * VEC : 0));
-  const char* Bl_last = reinterpret_cast<const char*>(a.B + off + (live_last ? ((R - 1) * W + l) * VEC : 0));
+  const char* Bl = reinterpret_cast<const char*>(a.B + off + ((R > 1 || live_last) ? l * VEC : kw - VEC));
+  const char* Bl_last = reinterpret_cast<const char*>(a.B + off + (live_last ? ((R - 1) * W + l) * VEC : kw - VEC));
   using Split = group_split<VEC, W>;
   const int out_col = Split::column(lane);   // where this lane's share of a finished row goes
   char* Cl = reinterpret_cast<char*>(a.C + off + out_col);

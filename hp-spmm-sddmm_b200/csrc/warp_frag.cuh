@@ -3,9 +3,8 @@
 // A warp is G = 32 / W lane groups of W lanes.  A group covers a slab of CW = VEC * W * R columns of a dense
 // row: lane l of the group owns columns (r * W + l) * VEC .. + VEC - 1 for r < R.  VEC is the widest vector the
 // row stride keeps aligned (K % 4 == 0: 16-byte loads, K even: 8-byte, K odd: 4-byte), W and R are the smallest
-// that cover the slab, and R > 1 only with W = 32.  A slab may be narrower than CW: a lane beyond its width kw
-// gathers column 0 of the slab instead (the same sector as lane 0, so no extra traffic and no predicate in the
-// hot loop) and stores nothing.
+// that cover the slab.  A slab may be narrower than CW: a lane beyond its width kw gathers the slab's last vector
+// instead (a line its neighbours read anyway, so no extra traffic and no predicate in the hot loop) and stores nothing.
 #pragma once
 #include "device_utils.cuh"
 
