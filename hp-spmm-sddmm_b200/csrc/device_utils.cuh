@@ -71,6 +71,9 @@ __device__ __forceinline__ void st_stream(float* p, float4 v) {
                : "memory");
 }
 
+// Asks for the line that holds p to be brought into the L2 cache.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // 16-byte vector reduction into global memory (no return value).
 __device__ __forceinline__ void red_add_v4(float* p, float4 v) {
   asm volatile("red.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(v.x), "f"(v.y),
