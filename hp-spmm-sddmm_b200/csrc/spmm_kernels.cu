@@ -503,14 +503,16 @@ static int32_t probing_chunk_nnz(int64_t K) {
 }
 
 int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz) {
-  // With the list of non-empty rows a row end costs two loads, and larger chunks amortise the per-chunk
-  // prologue (table loads, pipeline fill) and leave fewer carries.  Measured on B200 (R-MAT scale 20, product
-  // time in ms at S = 128 / 256 / 320 / 512 / 1024): K = 32: 0.240 / 0.217 / 0.208 / 0.199 / 0.193;
-  // K = 64: 0.356 / 0.314 / 0.307 / 0.310 / 0.306; K = 128: 0.630 / 0.563 / 0.563 / 0.595 / 0.592.
-  // Re-measured at K = 32 after the row-store exchange (S = 384 / 512 / 640 / 768 / 1024 / 1280 / 1536):
-  // 0.195 / 0.189 / 0.186 / 0.185 / 0.182 / 0.193 / 0.212 ms.  The default stays at 512 all the same: plans are
-  // shared with the SDDMM, which on the same graph takes 0.193 / 0.230 / 0.271 / 0.333 ms at S = 512 / 640 /
-  // 768 / 1024.  A caller that builds a plan for products only can ask for 1024 (hpspmm_opts.chunk_nnz).
+  // Larger chunks amortise the per-chunk prologue and split fewer rows; but the SDDMM shares the plan, and there a chunk
+  // of very short rows waits once per row, so its time turns up with the longest such chunk once chunks are few.
+  // Power-law graphs, S = 128 / 192 / 256 / 320 / 384 / 512 in us, product and SDDMM:
+  //   4 M entries,  K = 64: 83 / 80 / 75 / 79 / 80 / 82        and 75 / 74 / 88 / 103 / 101 / 98
+  //   5 M entries,  K = 32: 66 / 61 / 61 / 57 / 58 / 64        and 57 / 56 / 63 / 77 / 90 / 72
+  //   8 M entries,  K = 32: 110 / 97 / 93 / 93 / 90 / 87       and 94 / 92 / 91 / 92 / 103 / 134
+  //   12 M entries, K = 32: 164 / 144 / 135 / 133 / 133 / 132  and 145 / 138 / 136 / 135 / 135 / 137
+  //   16 M entries, K = 64: 333 / 322 / 305 / 297 / 293 / 297  and 294 / 293 / 292 / 294 / 299 / 303
+  //   16 M entries, K = 128: 566 / 567 / 546 / - / 550 / 526   and 523 / 563 / 572 / 566 / 537 / 561
+  // A caller that builds a plan for products only can ask for more (hpspmm_opts.chunk_nnz).
   // Below 2.4 M entries there are fewer chunks than warps the GPU can hold, and the time is that of the longest
   // chunk: a chain of gather round trips.  Measured in us at S = 32 / 64 / 128 / 256, rows of 16 entries on average,
   // uniform and power-law columns: 12 K entries, K = 32: 3.7 / 4.5 / 6.3 / 10.1 and 6.6 / 7.7 / 10.3 / 13.9;
@@ -521,11 +523,8 @@ int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz) {
   if (nnz < (K > 64 ? 150000 : 500000)) return 64;
   if (nnz < 2400000) return 128;
   const int32_t floor_s = probing_chunk_nnz(K);
-  const int32_t best = K <= 32 ? 512 : (K <= 64 ? 320 : 256);
-  // In between, S grows with the matrix: 4 M / 8 M entries of a power-law graph, K = 32, S = 160 / 192 / 256 / 384 / 512:
-  // 51 / 50 / 48 / 52 / 58 us and 100 / 97 / 93 / 90 / 87 us.  The SDDMM on the same plan turns up sharply a little
-  // later (4 M, K = 32: 43 / 44 / 57 / 52 us at 160 / 192 / 256 / 384), so the line stays below the product's best.
-  const int64_t want = nnz / 20000 / 32 * 32;
+  const int32_t best = K <= 32 ? 384 : (K <= 64 ? 320 : 256);
+  const int64_t want = nnz / 24000 / 32 * 32;
   int64_t s = want < floor_s ? floor_s : want;
   if (s > best) s = best;
   return (int32_t)s;
