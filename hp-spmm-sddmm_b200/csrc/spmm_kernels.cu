@@ -328,9 +328,8 @@ spmm_tma_kernel(const __grid_constant__ CUtensorMap map_b, int M, int n_chunks, 
   const int r0_start = __ldg(row_ptr + r0), r0_end = __ldg(row_ptr + r0 + 1);
   const bool stores_split_row = r0_start < n0 && r0_end <= n1;   // began in an earlier chunk, ends here
   if (!hands_on && !stores_split_row) return;
-  if (stores_split_row) settle_split_row<4, 32, 1>(r0, r0_start, r0_end, S, carry_val, C, run_counter, KW, KW);
-  if (hands_on)
-    settle_split_row<4, 32, 1>(row, __ldg(row_ptr + row), row_end, S, carry_val, C, run_counter, KW, KW);
+  settle_split_rows<4, 32, 1>(stores_split_row, r0, r0_start, r0_end, hands_on, row, __ldg(row_ptr + row), row_end, chunk,
+                              S, carry_val, C, run_counter, KW, KW);
 }
 
 // ---- row-split kernel for any other K: one warp per row ------------------------------------------

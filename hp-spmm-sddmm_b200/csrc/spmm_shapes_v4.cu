@@ -13,7 +13,7 @@ int hpspmm_spmm_launch_v4(hpspmm_ctx* ctx, const hpspmm_spmm_args& a, const hpsp
     if (sh.W == 32 && sh.R == 3) GO(32, 3, 4, 0, 8, true);
     if (sh.W == 32) GO(32, 4, 4, 0, 8, true);
   }
-  if (a.K == 32 && sh.W == 8) { if (sh.hint) GO(8, 1, 4, 32, 20, true); else GO(8, 1, 4, 32, 20, false); }
+  if (a.K == 32 && sh.W == 8) { if (sh.hint) GO(8, 1, 4, 32, 18, true); else GO(8, 1, 4, 32, 18, false); }
   if (a.K == 64 && sh.W == 16) { if (sh.hint) GO(16, 1, 4, 64, 18, true); else GO(16, 1, 4, 64, 18, false); }
   if (a.K == 128 && sh.W == 32 && sh.R == 1) { if (sh.hint) GO(32, 1, 4, 128, 18, true); else GO(32, 1, 4, 128, 18, false); }
   if (sh.W == 2) GO(2, 1, 2, 0, 16, true);

@@ -7,7 +7,7 @@
 // never diverge.  A finished row is combined across the groups and stored once.
 //
 // A chunk that ends inside a heavy row leaves its partial sum in a carry slot; the pieces of a split row settle it
-// among themselves (settle_split_row).  The order of all additions is fixed by the chunking and the shape, so
+// among themselves (settle_split_rows).  The order of all additions is fixed by the chunking and the shape, so
 // results are bit-reproducible from run to run.
 #pragma once
 #include "device_utils.cuh"
@@ -83,63 +83,117 @@ __device__ __forceinline__ int2 next_filled_row(const int* __restrict__ row_ptr,
   return make_int2(f, __ldg(row_ptr + f + 1));
 }
 
-// Adds up one split row.  A row longer than S is cut at multiples of S only, so its pieces are the chunks
-// first = row_ptr[r] / S .. last = (row_ptr[r+1] - 1) / S: all but the last hand a carry on, the last stores the
-// row.  Every piece bumps the row's counter when its own part is visible device-wide; whoever bumps it last adds
-// the carries, in chunk order (the groups summing interleaved carries, combined in a fixed order), to the stored
-// row.  The sum does not depend on who that is.  No piece ever waits.  `C`, `carry` and `counter` are those of the
-// slab: ld is the row stride of C and of the carry slots, kw the slab's width.
-template <int VEC, int W, int R>
-__device__ __forceinline__ void settle_split_row(int r, int r_start, int r_end, int S, const float* __restrict__ carry,
-                                              float* __restrict__ C, int* __restrict__ counter, int ld, int kw) {
+// Adds up the split rows that a chunk has a piece of: row r0, whose last piece the chunk has stored (`stored`), and row
+// r1, whose partial sum it has left in its carry slot (`handed_on`).
+//
+// A row longer than S is cut at multiples of S only, so its pieces are the chunks first = row_ptr[r] / S .. last =
+// (row_ptr[r+1] - 1) / S: all but the last hand a carry on, the last stores the row.  A piece bumps a counter when its
+// own part is visible device-wide, and whoever bumps it last adds the carries up: nobody waits, and the order of the
+// additions does not depend on who that is.  Up to kCarryGroup carries meet at one counter (counter[first]) and are
+// added to the stored row.  More meet in groups: the last of a group (counter[first + 16 q]) leaves the group's sum in
+// the group's first slot, and the groups and the stored row meet at counter[first + 1].  A row of 40,000 entries has 250
+// carries; added by one warp they were a chain of 16 memory round trips at the end of the launch.
+// Both rows are announced by one instruction (lane 0 and lane 1), so a chunk that has a piece of two rows pays for one
+// release and one round trip.  Power-law graphs, one row at a time and all carries by one warp -> this: 4 M entries,
+// K = 64 79.3 -> 76.5 us, K = 128 132.6 -> 126.5 us; 16 M entries, K = 64 291.9 -> 283.4 us, K = 128 517 -> 505 us.
+// `C`, `carry` and `counter` are those of the slab: ld is the row stride of C and of the carry slots, kw the width.
+constexpr int kCarryGroup = 16;
+
+// sum of slots 0, step, 2 * step, .. of n, the lane groups taking them in turn; every lane gets the total
+template <int VEC, int W>
+__device__ __forceinline__ void sum_carries(float (&sum)[VEC], const float* src, int n, int64_t step) {
   constexpr int G = 32 / W;
+  constexpr int BATCH = kCarryGroup / G < 1 ? 1 : (kCarryGroup / G > 8 ? 8 : kCarryGroup / G);   // loads in flight
+  const int g = (threadIdx.x & 31) / W;
+#pragma unroll
+  for (int x = 0; x < VEC; ++x) sum[x] = 0.f;
+#pragma unroll 1
+  for (int i = g; i < n; i += BATCH * G) {
+    float v[BATCH][VEC];
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u) {
+#pragma unroll
+      for (int x = 0; x < VEC; ++x) v[u][x] = 0.f;
+      if (i + u * G < n) load_l2(v[u], src + (int64_t)(i + u * G) * step);
+    }
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u)
+#pragma unroll
+      for (int x = 0; x < VEC; ++x) sum[x] += v[u][x];
+  }
+  all_reduce_groups<VEC, W>(sum);
+}
+
+template <int VEC, int W, int R>
+__device__ __forceinline__ void settle_split_rows(bool stored, int r0, int r0_start, int r0_end, bool handed_on, int r1,
+                                                  int r1_start, int r1_end, int chunk, int S, float* __restrict__ carry,
+                                                  float* __restrict__ C, int* __restrict__ counter, int ld, int kw) {
   const int lane = threadIdx.x & 31;
   const int g = lane / W, l = lane % W;
-  const int first = r_start / S;
-  const int last = (r_end - 1) / S;
-  __syncwarp();   // every lane's part is written before lane 0 announces it
-  int seen = 0;
-  if (lane == 0) seen = atomic_add_release(counter + first, 1);
-  seen = __shfl_sync(0xffffffffu, seen, 0);
-  if (seen != last - first) return;
+  const int my_row = lane == 0 ? r0 : r1;
+  const int my_first = (lane == 0 ? r0_start : r1_start) / S;
+  const int my_len = ((lane == 0 ? r0_end : r1_end) - 1) / S - my_first;   // carries of the row
+  const int my_group = (chunk - my_first) / kCarryGroup * kCarryGroup;      // first carry of this piece's group
+  __syncwarp();   // every lane's part is written before lanes 0 and 1 announce it
+  bool complete = false;
+  if (lane == 0 ? stored : (lane == 1 && handed_on)) {
+    int at = my_first, others = my_len;
+    if (my_len > kCarryGroup) {
+      at += lane == 0 ? 1 : my_group;
+      others = lane == 0 ? (my_len + kCarryGroup - 1) / kCarryGroup : min(kCarryGroup, my_len - my_group) - 1;
+    }
+    complete = atomic_add_release(counter + at, 1) == others;
+  }
+  const unsigned todo = __ballot_sync(0xffffffffu, complete);
+  if (todo == 0) return;
   __threadfence();
-  const int len = last - first;
   const int64_t K = ld;
 #pragma unroll 1
-  for (int rr = 0; rr < R; ++rr) {
-    const int col = (rr * W + l) * VEC;
-    const bool live = col < kw;
-    const float* src = carry + (int64_t)first * K + (live ? col : 0);
-    float sum[VEC];
-#pragma unroll
-    for (int x = 0; x < VEC; ++x) sum[x] = 0.f;
-    int i = g;
-    for (; i + 7 * G < len; i += 8 * G) {
-      float v[8][VEC];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) load_l2(v[u], src + (int64_t)(i + u * G) * K);
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int x = 0; x < VEC; ++x) sum[x] += v[u][x];
+  for (int t = 0; t < 2; ++t) {
+    if (!((todo >> t) & 1u)) continue;
+    const int row = __shfl_sync(0xffffffffu, my_row, t), first = __shfl_sync(0xffffffffu, my_first, t);
+    const int len = __shfl_sync(0xffffffffu, my_len, t), group = __shfl_sync(0xffffffffu, my_group, t);
+    const bool grouped = len > kCarryGroup;
+    const int n_groups = (len + kCarryGroup - 1) / kCarryGroup;
+    const int at = first + (grouped ? 1 : 0);
+    if (grouped && t == 1) {
+      // the group is complete: its sum replaces its first carry
+      float* slot = carry + (int64_t)(first + group) * K;
+#pragma unroll 1
+      for (int rr = 0; rr < R; ++rr) {
+        const int col = (rr * W + l) * VEC;
+        const bool live = col < kw;
+        float sum[VEC];
+        sum_carries<VEC, W>(sum, slot + (live ? col : 0), min(kCarryGroup, len - group), K);
+        if (g == 0 && live) store_plain(slot + col, sum);
+      }
+      __syncwarp();
+      bool all = false;
+      if (lane == 0) {
+        counter[first + group] = 0;
+        all = atomic_add_release(counter + at, 1) == n_groups;
+      }
+      if (!__shfl_sync(0xffffffffu, (int)all, 0)) continue;
+      __threadfence();
     }
-    for (; i < len; i += G) {
-      float v[VEC];
-      load_l2(v, src + (int64_t)i * K);
+#pragma unroll 1
+    for (int rr = 0; rr < R; ++rr) {
+      const int col = (rr * W + l) * VEC;
+      const bool live = col < kw;
+      float sum[VEC];
+      sum_carries<VEC, W>(sum, carry + (int64_t)first * K + (live ? col : 0), grouped ? n_groups : len,
+                          grouped ? K * kCarryGroup : K);
+      if (g == 0 && live) {
+        float* out = C + (int64_t)row * K + col;
+        float o[VEC];
+        load_l2(o, out);
 #pragma unroll
-      for (int x = 0; x < VEC; ++x) sum[x] += v[x];
+        for (int x = 0; x < VEC; ++x) o[x] += sum[x];
+        store_stream(out, o);
+      }
     }
-    all_reduce_groups<VEC, W>(sum);
-    if (g == 0 && live) {
-      float* out = C + (int64_t)r * K + col;
-      float o[VEC];
-      load_l2(o, out);
-#pragma unroll
-      for (int x = 0; x < VEC; ++x) o[x] += sum[x];
-      store_stream(out, o);
-    }
+    if (lane == 0) counter[at] = 0;   // ready for the next launch
   }
-  if (lane == 0) counter[first] = 0;   // ready for the next launch
 }
 
 // KS: row stride of B and C when it is a compile-time constant (the whole width is one full slab), else 0.
@@ -370,11 +424,9 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   const bool stores_split_row = r0_start < n0 && r0_end <= n1;   // began in an earlier chunk, ends here
   if (!hands_on && !stores_split_row) return;
   int* counter = KS ? a.counter : a.counter + (int64_t)blockIdx.y * a.n_chunks;
-  if (stores_split_row)
-    settle_split_row<VEC, W, R>(r0, r0_start, r0_end, a.S, carry, a.C + off, counter, (int)ldc, kw);
-  if (hands_on)
-    settle_split_row<VEC, W, R>(row, row == r0 ? r0_start : __ldg(a.row_ptr + row), row_end, a.S, carry, a.C + off,
-                                counter, (int)ldc, kw);
+  settle_split_rows<VEC, W, R>(stores_split_row, r0, r0_start, r0_end, hands_on, row,
+                               row == r0 ? r0_start : __ldg(a.row_ptr + row), row_end, chunk, a.S, carry, a.C + off,
+                               counter, (int)ldc, kw);
 }
 
 // Launches one shape.  Slabs of the width run as blockIdx.y, each with counters of its own; where the counters are
