@@ -295,6 +295,8 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct sddmm_args {
   int n_chunks, K, off, cols, keep_y;
+  bool waves;       // four waves of chunks and more
+  bool long_rows;   // rows are long enough that waiting for each row of X costs little
   const int32_t* col_idx;
   const float *X, *Y;
   float* out;
@@ -303,14 +305,14 @@ struct sddmm_args {
 };
 
 // one launch per slab of the width: the first writes the partial dot products, the others add theirs
-template <int VEC, int W, int R, int U, int KS, bool HINT, int MINB>
+template <int VEC, int W, int R, int U, int KS, bool HINT, int MINB, bool SERIAL>
 int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
   constexpr int BT = 64, CW = VEC * W * R;
   const unsigned grid = (unsigned)((a.n_chunks + BT / 32 - 1) / (BT / 32));
   if (!hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
   for (int off = a.off; off < a.off + a.cols; off += CW) {
     const int left = a.off + a.cols - off;
-    sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, (KS > 0)><<<grid, BT, 0, s>>>(
+    sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, SERIAL><<<grid, BT, 0, s>>>(
         a.n_chunks, a.K, off, left < CW ? left : CW, off > 0 ? 1 : 0, a.keep_y, a.col_idx, a.X, a.Y, a.out, a.rec, a.nz);
     ctx->launches++;
   }
@@ -318,16 +320,42 @@ int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
   return HPSPMM_OK;
 }
 
-// 20 resident blocks per SM (48 registers) measured 0.193 / 0.318 / 0.542 ms at K = 32 / 64 / 128 on the R-MAT
-// scale-20 graph against 0.204 / 0.318 / 0.555 ms at 18 (56 registers)
+// Shapes.  With few chunks (lat) a group is as wide as the slab.  With many chunks the shared-memory and shuffle pipe
+// that also carries the gathers decides, and narrow groups with several vectors per lane use it less: W = 8 instead of 16
+// halves the broadcast reads of an entry and the exchanges of its sum, and R = 3 leaves fewer lanes idle than the next
+// power of two.  R-MAT scale 20, 16 M entries, before -> after in us:
+//   K = 48 360 -> 309, 64 294 -> 281, 96 606 -> 424, 100 617 -> 515, 128 521 -> 490, 160 1055 -> 743, 192 1083 -> 792,
+//   256 1187 -> 1029; uniform columns, K = 64 551 -> 520, 96 984 -> 882, 160 1794 -> 1564
+//   2-float vectors: K = 46 407 -> 321, 62 419 -> 363, 126 694 -> 577; 4-byte: K = 13 205 -> 193, 23 306 -> 253, 31 310 -> 279
+// K = 32 stays at W = 8, R = 1 (185 us; 193 to 218 with other shapes).  16 blocks per SM (64 registers) where two or three
+// vectors per lane are in flight; 20 (48 registers) at K = 32: 193 against 204 us at 18.
+// Which of them are SERIAL: 16-byte vectors fill the registers that the other path needs (K = 96 424 against 477 us); with
+// narrower vectors it costs more than it saves except where noted by the shape.  Where rows are short the waits do not
+// pay (uniform rows of 4 entries, K = 100: 176 against 159 us; of 8: 130 against 119; of 12: 110 against 105, but K = 96 92
+// against 103 and K = 160 158 against 185): from 10 entries per row on, or on matrices with many split rows.  Where the
+// gain is small it also takes enough chunks to cover the waits (12,500 chunks: K = 48 38.9 against 41.4 us, K = 62 45.7
+// against 55.1; 31,000: 105 against 97 and 110 against 97).
 int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_shape& sh, cudaStream_t s) {
-#define GO(V, W, R, U, KS, H, MINB) return launch_sddmm<V, W, R, U, KS, H, MINB>(ctx, a, s)
+#define GO(V, W, R, U, KS, H, MINB) return launch_sddmm<V, W, R, U, KS, H, MINB, false>(ctx, a, s)
+#define GO_SERIAL(V, W, R, U, KS, H, MINB) return launch_sddmm<V, W, R, U, KS, H, MINB, true>(ctx, a, s)
   if (sh.VEC == 4) {
-    // (the fixed strides are the SERIAL form)
+    const int vecs = a.cols / 4;
     if (sh.lat) {
-    } else if (a.K == 32) { if (sh.hint) GO(4, 8, 1, 4, 32, true, 20); else GO(4, 8, 1, 4, 32, false, 20); }
-    else if (a.K == 64) { if (sh.hint) GO(4, 16, 1, 4, 64, true, 20); else GO(4, 16, 1, 4, 64, false, 20); }
-    else if (a.K == 128) { if (sh.hint) GO(4, 32, 1, 4, 128, true, 20); else GO(4, 32, 1, 4, 128, false, 20); }
+    } else if (a.K == 32) {
+      if (sh.hint) GO_SERIAL(4, 8, 1, 4, 32, true, 20); else GO_SERIAL(4, 8, 1, 4, 32, false, 20);
+    } else if (a.K == 64) {
+      if (sh.hint) GO_SERIAL(4, 8, 2, 4, 64, true, 16); else GO_SERIAL(4, 8, 2, 4, 64, false, 16);
+    } else if (a.K == 128) {
+      if (sh.hint) GO_SERIAL(4, 16, 2, 4, 128, true, 16); else GO_SERIAL(4, 16, 2, 4, 128, false, 16);
+    } else if (a.long_rows && vecs > 8 && vecs <= 64) {
+      if (vecs <= 16) {
+        if (a.waves) GO_SERIAL(4, 8, 2, 4, 0, true, 16); else GO(4, 16, 1, 4, 0, true, 16);
+      }
+      if (vecs <= 24) GO_SERIAL(4, 8, 3, 2, 0, true, 16);
+      if (vecs <= 32) GO_SERIAL(4, 16, 2, 4, 0, true, 16);
+      if (vecs <= 48) GO_SERIAL(4, 16, 3, 2, 0, true, 16);
+      GO_SERIAL(4, 16, 4, 2, 0, true, 14);
+    }
     if (sh.W == 2) GO(4, 2, 1, 2, 0, true, 16);
     if (sh.W == 4) GO(4, 4, 1, 4, 0, true, 16);
     if (sh.W == 8) GO(4, 8, 1, 4, 0, true, 16);
@@ -338,6 +366,10 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
     GO(4, 32, 4, 2, 0, true, 10);
   }
   if (sh.VEC == 2) {
+    const int vecs = (a.cols + 1) / 2;
+    if (!sh.lat && vecs > 16 && vecs <= 24) GO(2, 8, 3, 4, 0, true, 16);
+    if (!sh.lat && a.long_rows && a.waves && vecs > 24 && vecs <= 32) GO_SERIAL(2, 16, 2, 8, 0, true, 16);
+    if (!sh.lat && a.long_rows && vecs > 48 && vecs <= 64) GO_SERIAL(2, 16, 4, 4, 0, true, 16);
     if (sh.W == 2) GO(2, 2, 1, 2, 0, true, 16);
     if (sh.W == 4) GO(2, 4, 1, 4, 0, true, 16);
     if (sh.W == 8) GO(2, 8, 1, 8, 0, true, 16);
@@ -347,6 +379,12 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
     if (sh.R == 2) GO(2, 32, 2, 4, 0, true, 16);
     if (sh.R == 3) GO(2, 32, 3, 4, 0, true, 14);
     GO(2, 32, 4, 4, 0, true, 12);
+  }
+  if (!sh.lat) {
+    if (a.cols > 8 && a.cols <= 16) GO(1, 8, 2, 4, 0, true, 18);
+    if (a.cols > 16 && a.cols <= 24) GO(1, 8, 3, 4, 0, true, 18);
+    if (a.cols > 24 && a.cols <= 32) GO(1, 16, 2, 8, 0, true, 16);
+    if (a.cols > 48 && a.cols <= 64) GO(1, 16, 4, 4, 0, true, 16);
   }
   if (sh.W == 1) GO(1, 1, 1, 1, 0, true, 16);
   if (sh.W == 4) GO(1, 4, 1, 4, 0, true, 16);
@@ -362,6 +400,7 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
   if (sh.R == 7) GO(1, 32, 7, 4, 0, true, 12);
   GO(1, 32, 8, 4, 0, true, 12);
 #undef GO
+#undef GO_SERIAL
 }
 
 }  // namespace
@@ -389,11 +428,14 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   cudaStream_t s = (cudaStream_t)stream;
   const int hint_mode = opts ? opts->b_l2_hint : 0;
   const bool hint = hint_mode == 2 || (hint_mode == 0 && K >= 64);
-  sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, col_idx, X, Y, out_vals, nullptr, nullptr};
+  sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, false, nnz >= 10 * M, col_idx, X, Y, out_vals, nullptr, nullptr};
   if (plan) {
     HPSPMM_REQUIRE(ctx, plan->M == M && plan->nnz == nnz, "plan built for another matrix");
     HPSPMM_REQUIRE(ctx, plan->device == ctx->device, "plan built on another device");
     a.n_chunks = (int)plan->n_chunks;
+    // The average says nothing about a skewed matrix, most of whose entries lie in long rows; there many rows are split.
+    // (power-law graph of 1 M rows, 5 M entries, K = 96: serial 175 us, mask 230 us)
+    a.long_rows = a.long_rows || plan->n_split_chunks * 8 >= plan->n_chunks;
     a.rec = plan->rec;
     a.nz = plan->nz;
   } else {
@@ -414,11 +456,13 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
     a.rec = rec;
     a.nz = nz;
   }
+  a.waves = a.n_chunks > ctx->sm_count * 160;
   const int VEC = hpspmm_vector_width(K, (uintptr_t)X | (uintptr_t)Y);
   for (a.off = 0; a.off < a.K; a.off += a.cols) {
     a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
     hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hint);
     sh.lat = a.n_chunks <= ctx->sm_count * 80;   // up to about two waves of resident warps
+    if (sh.VEC == 4 && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;
     const int st = launch_sddmm_shape(ctx, a, sh, s);
     if (st != HPSPMM_OK) return st;
   }

@@ -145,6 +145,55 @@ def test_coo_and_sddmm_at_every_vector_count(gpu_ctx, pkg, oracle, K, few_entrie
         b.free()
 
 
+@pytest.mark.parametrize("short_rows", [False, True])
+@pytest.mark.parametrize("K", [9, 16, 17, 23, 25, 31, 34, 36, 46, 49, 50, 62, 63, 64, 68, 96, 98, 100, 126, 128, 132, 160, 192,
+                               196, 256])
+def test_shapes_for_many_chunks(gpu_ctx, pkg, oracle, K, short_rows):
+    """Narrow lane groups with several vectors per lane, which the kernels take when there are many chunks: the first and
+    last width of every shape, rows that are split and rows of a few entries."""
+    ctx = gpu_ctx
+    if short_rows:
+        rng = np.random.default_rng(7)
+        M, N = 150_000, 40_000
+        rp = np.concatenate([[0], np.cumsum(rng.integers(0, 8, M))]).astype(np.int32)
+        ci = rng.integers(0, N, rp[-1]).astype(np.int32)
+        vals = rng.random(rp[-1], dtype=np.float32)
+    else:
+        g = pkg.gen_rmat(16, 16, seed=97)
+        M, N, rp, ci, vals = g["M"], g["N"], g["row_ptr"], g["col_idx"], g["vals"]
+    nnz = len(ci)
+    opts = pkg.Opts(algo=pkg.ALGO_BALANCED, chunk_nnz=32)
+    assert nnz // 32 > 80 * 148
+    X = pkg.host_fill_uniform(M * K, 97, 1, -1.0, 1.0).reshape(M, K)
+    Y = pkg.host_fill_uniform(N * K, 97, 2, -1.0, 1.0).reshape(N, K)
+    d = [ctx.upload(x) for x in (rp, ci, vals, X, Y)]
+    d_rp, d_ci, d_v, d_X, d_Y = d
+    ref, abs_sum = oracle.sddmm_f64(rp, ci, X, Y)
+    for use_plan in (False, True):
+        buf, o_ptr, read = guarded_output(ctx, (nnz,))
+        plan = ctx.plan_create(M, nnz, d_rp, K, N=N, col_idx=d_ci, opts=opts) if use_plan else None
+        ctx.sddmm_csr(M, N, K, nnz, d_rp, d_ci, d_X, d_Y, o_ptr, plan=plan, opts=opts)
+        ctx.stream_sync()
+        check_against_f64(read(), ref, abs_sum, "sddmm K=%d plan=%s" % (K, use_plan))
+        buf.free()
+        if plan:
+            buf, c_ptr, read = guarded_output(ctx, (M, K))
+            ctx.spmm_csr(M, N, K, nnz, d_rp, d_ci, d_v, d_Y, c_ptr, plan=plan)
+            ctx.stream_sync()
+            ref_c, abs_c = oracle.spmm_f64(rp, ci, vals, Y)
+            check_against_f64(read(), ref_c, abs_c, "spmm K=%d" % K)
+            buf.free()
+            ctx.plan_destroy(plan)
+    r, c, v = oracle.csr_to_coo_padded(rp, ci, vals, 32)
+    e = [ctx.upload(x) for x in (r, c, v)]
+    buf, c_ptr, read = guarded_output(ctx, (M, K), fill=np.float32(0))
+    ctx.spmm_coo(M, N, K, len(r), e[0], e[1], e[2], d_Y, c_ptr)
+    ctx.stream_sync()
+    check_against_f64(read(), ref_c, abs_c, "coo K=%d" % K)
+    for b in d + e + [buf]:
+        b.free()
+
+
 def test_sddmm_edge_structures(gpu_ctx, pkg, oracle):
     ctx = gpu_ctx
     rng = np.random.default_rng(3)
