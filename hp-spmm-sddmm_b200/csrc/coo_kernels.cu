@@ -208,6 +208,7 @@ int launch_coo_shape(hpspmm_ctx* ctx, const coo_args& a, const hpspmm_spmm_shape
     if (sh.W == 2) GO(4, 2, 1, 2, 0, 16);
     if (sh.W == 4) GO(4, 4, 1, 4, 0, 16);
     if (sh.W == 8) GO(4, 8, 1, 4, 0, 16);
+    if (sh.W == 16 && sh.R == 3) GO(4, 16, 3, 2, 0, 16);
     if (sh.W == 16) GO(4, 16, 1, 4, 0, 16);
     if (sh.R == 1) GO(4, 32, 1, 4, 0, 16);
     if (sh.R == 2) GO(4, 32, 2, 2, 0, 16);
@@ -263,7 +264,15 @@ extern "C" int hpspmm_spmm_coo_f32(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
   const int VEC = hpspmm_vector_width(K, (uintptr_t)B | (uintptr_t)C);
   for (a.off = 0; a.off < a.K; a.off += a.cols) {   // every slab accumulates into its own columns
     a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
-    const int st = launch_coo_shape(ctx, a, hpspmm_choose_shape(VEC, a.cols, false), (cudaStream_t)stream);
+    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, false);
+    // Three vectors per lane as in the CSR product, but only from 33 vectors on: every run of equal rows is combined over
+    // the groups before it goes to C, and over four groups that costs more than the idle lanes of one (1 M entries of a
+    // power-law graph, K = 96: 49.0 -> 56.0 us).  With few warps the exchange is not covered either (100 K entries,
+    // K = 160: 15.1 -> 16.2 us); 8 M uniform entries, K = 160: 516 -> 442 us.
+    const int64_t warps = (nnz_padded + a.S - 1) / a.S;
+    if (VEC == 4 && sh.R == 3 && sh.W < 32 && (sh.W == 8 || warps < (int64_t)ctx->sm_count * 24))
+      sh.R = sh.W / 8, sh.W = 32;
+    const int st = launch_coo_shape(ctx, a, sh, (cudaStream_t)stream);
     if (st != HPSPMM_OK) return st;
   }
   return HPSPMM_OK;

@@ -554,7 +554,11 @@ hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, bool hint) {
   sh.R = (vecs + 31) / 32;
   // 33 to 48 narrow vectors: two groups of 16 lanes with three vectors each leave no lane idle and read two entries per
   // step (4 M entries, uniform columns: K = 47 107 -> 89 us, K = 66 148 -> 132 us; a power-law graph gains nothing)
-  if (VEC < 4 && vecs > 32 && vecs <= 48) sh.W = 16, sh.R = 3;
+  if (vecs > 32 && vecs <= 48) sh.W = 16, sh.R = 3;
+  // 17 to 24 wide vectors: four groups of 8 lanes, for the same reason.  R-MAT scale 20 / 8 M uniform entries: K = 96
+  // 484 -> 440 / 200 -> 175 us; and with 16 lanes K = 160 812 -> 707 / 467 -> 378 us, K = 192 875 -> 796 / 548 -> 482 us.
+  // (25 to 32 vectors lose: K = 100 516 -> 529 us, K = 128 524 -> 544 us, the rows' ends then cost exchanges.)
+  if (VEC == 4 && vecs > 16 && vecs <= 24) sh.W = 8, sh.R = 3;
   return sh;
 }
 
@@ -594,7 +598,7 @@ int launch_spmm(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool hint, bool shared_coun
     // additions).  67.6 K entries in chunks of 64: 6.1 -> 5.6 us at K = 64, 9.1 -> 7.2 us at K = 128; with more chunks
     // than these builds have resident warps they lose (300 K entries, K = 64: 8.3 -> 10.5 us).
     sh.lat = a.n_chunks <= ctx->sm_count * (sh.W <= 8 ? 24 : 16);
-    if (sh.lat && sh.R == 3 && sh.W == 16) sh.W = 32, sh.R = 2;   // (one group: rows end without an exchange)
+    if (sh.lat && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;   // (one group: rows end without an exchange)
     const int st = VEC == 4   ? hpspmm_spmm_launch_v4(ctx, a, sh, shared_counters, s)
                    : VEC == 2 ? hpspmm_spmm_launch_v2(ctx, a, sh, shared_counters, s)
                               : hpspmm_spmm_launch_v1(ctx, a, sh, shared_counters, s);

@@ -18,7 +18,9 @@ int hpspmm_spmm_launch_v4(hpspmm_ctx* ctx, const hpspmm_spmm_args& a, const hpsp
   if (a.K == 128 && sh.W == 32 && sh.R == 1) { if (sh.hint) GO(32, 1, 4, 128, 18, true); else GO(32, 1, 4, 128, 18, false); }
   if (sh.W == 2) GO(2, 1, 2, 0, 16, true);
   if (sh.W == 4) GO(4, 1, 4, 0, 16, true);
+  if (sh.W == 8 && sh.R == 3) GO(8, 3, 2, 0, 16, true);
   if (sh.W == 8) GO(8, 1, 4, 0, 16, true);
+  if (sh.W == 16 && sh.R == 3) GO(16, 3, 2, 0, 16, true);
   if (sh.W == 16) GO(16, 1, 4, 0, 18, true);
   if (sh.R == 1) GO(32, 1, 4, 0, 18, true);
   if (sh.R == 2) GO(32, 2, 2, 0, 18, true);
