@@ -295,6 +295,7 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct sddmm_args {
   int n_chunks, K, off, cols, keep_y;
+  bool few;         // at most one wave of chunks
   bool waves;       // four waves of chunks and more
   bool long_rows;   // rows are long enough that waiting for each row of X costs little
   const int32_t* col_idx;
@@ -320,7 +321,7 @@ int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
   return HPSPMM_OK;
 }
 
-// Shapes.  With few chunks (lat) a group is as wide as the slab.  With many chunks the shared-memory and shuffle pipe
+// Shapes.  With many chunks the shared-memory and shuffle pipe
 // that also carries the gathers decides, and narrow groups with several vectors per lane use it less: W = 8 instead of 16
 // halves the broadcast reads of an entry and the exchanges of its sum, and R = 3 leaves fewer lanes idle than the next
 // power of two.  R-MAT scale 20, 16 M entries, before -> after in us:
@@ -329,6 +330,13 @@ int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
 //   2-float vectors: K = 46 407 -> 321, 62 419 -> 363, 126 694 -> 577; 4-byte: K = 13 205 -> 193, 23 306 -> 253, 31 310 -> 279
 // K = 32 stays at W = 8, R = 1 (185 us; 193 to 218 with other shapes).  16 blocks per SM (64 registers) where two or three
 // vectors per lane are in flight; 20 (48 registers) at K = 32: 193 against 204 us at 18.
+// With few chunks (lat) a chunk's chain of batches decides, and several groups make it shorter: a batch holds U entries
+// of each, and every load of its rows of X is waited for once.  There registers are plenty, so more of it is in flight.
+// Power-law graph of 300 K entries / uniform columns, 300 K / power-law, 1 M: K = 96 29.1 -> 14.8 / 23.0 -> 14.8 / 44.8 ->
+// 34.9 us, K = 128 29.1 -> 18.8 / 27.1 -> 19.4 us, K = 160 49.7 -> 22.0 / 45.6 -> 24.8 / 77.4 -> 58.5 us, K = 256 50.8 ->
+// 25.1 / 48.7 -> 41.4 / 80.6 -> 76.9 us, K = 126 29.2 -> 18.9 / 25.1 -> 19.6 us, K = 23, 1 M 25.1 -> 20.9 us.  Shapes that
+// lose with more than one wave of chunks (1 M uniform entries, K = 128: 55 against 60 us) end there (few), those that lose
+// on short rows (500 K entries in 100 K rows, K = 128: 42 against 49 us) want long ones; at 9 to 16 vectors and at K = 62 and 63 a wide group stays ahead.
 // Which of them are SERIAL: 16-byte vectors fill the registers that the other path needs (K = 96 424 against 477 us); with
 // narrower vectors it costs more than it saves except where noted by the shape.  Where rows are short the waits do not
 // pay (uniform rows of 4 entries, K = 100: 176 against 159 us; of 8: 130 against 119; of 12: 110 against 105, but K = 96 92
@@ -341,6 +349,11 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
   if (sh.VEC == 4) {
     const int vecs = a.cols / 4;
     if (sh.lat) {
+      if (a.few && vecs > 16 && vecs <= 24) GO(4, 8, 3, 4, 0, true, 8);
+      if (vecs > 16 && vecs <= 24) GO(4, 8, 3, 2, 0, true, 10);
+      if (a.few && a.long_rows && vecs > 24 && vecs <= 32) GO(4, 8, 4, 2, 0, true, 8);
+      if (vecs > 32 && vecs <= 48) GO(4, 16, 3, 4, 0, true, 8);
+      if (a.long_rows && vecs > 48 && vecs <= 64) GO(4, 16, 4, 4, 0, true, 6);
     } else if (a.K == 32) {
       if (sh.hint) GO_SERIAL(4, 8, 1, 4, 32, true, 20); else GO_SERIAL(4, 8, 1, 4, 32, false, 20);
     } else if (a.K == 64) {
@@ -367,6 +380,8 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
   }
   if (sh.VEC == 2) {
     const int vecs = (a.cols + 1) / 2;
+    if (a.few && vecs > 16 && vecs <= 24) GO(2, 8, 3, 4, 0, true, 8);
+    if (a.few && a.long_rows && vecs > 48 && vecs <= 64) GO(2, 16, 4, 4, 0, true, 6);
     if (!sh.lat && vecs > 16 && vecs <= 24) GO(2, 8, 3, 4, 0, true, 16);
     if (!sh.lat && a.long_rows && a.waves && vecs > 24 && vecs <= 32) GO_SERIAL(2, 16, 2, 8, 0, true, 16);
     if (!sh.lat && a.long_rows && vecs > 48 && vecs <= 64) GO_SERIAL(2, 16, 4, 4, 0, true, 16);
@@ -380,6 +395,7 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
     if (sh.R == 3) GO(2, 32, 3, 4, 0, true, 14);
     GO(2, 32, 4, 4, 0, true, 12);
   }
+  if (sh.lat && a.cols > 16 && a.cols <= 24) GO(1, 8, 3, 4, 0, true, 8);
   if (!sh.lat) {
     if (a.cols > 8 && a.cols <= 16) GO(1, 8, 2, 4, 0, true, 18);
     if (a.cols > 16 && a.cols <= 24) GO(1, 8, 3, 4, 0, true, 18);
@@ -428,7 +444,7 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   cudaStream_t s = (cudaStream_t)stream;
   const int hint_mode = opts ? opts->b_l2_hint : 0;
   const bool hint = hint_mode == 2 || (hint_mode == 0 && K >= 64);
-  sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, false, nnz >= 10 * M, col_idx, X, Y, out_vals, nullptr, nullptr};
+  sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, false, false, nnz >= 10 * M, col_idx, X, Y, out_vals, nullptr, nullptr};
   if (plan) {
     HPSPMM_REQUIRE(ctx, plan->M == M && plan->nnz == nnz, "plan built for another matrix");
     HPSPMM_REQUIRE(ctx, plan->device == ctx->device, "plan built on another device");
@@ -456,6 +472,7 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
     a.rec = rec;
     a.nz = nz;
   }
+  a.few = a.n_chunks <= ctx->sm_count * 32;
   a.waves = a.n_chunks > ctx->sm_count * 160;
   const int VEC = hpspmm_vector_width(K, (uintptr_t)X | (uintptr_t)Y);
   for (a.off = 0; a.off < a.K; a.off += a.cols) {

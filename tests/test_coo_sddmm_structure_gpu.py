@@ -148,9 +148,9 @@ def test_coo_and_sddmm_at_every_vector_count(gpu_ctx, pkg, oracle, K, few_entrie
 @pytest.mark.parametrize("short_rows", [False, True])
 @pytest.mark.parametrize("K", [9, 16, 17, 23, 25, 31, 34, 36, 46, 49, 50, 62, 63, 64, 68, 96, 98, 100, 126, 128, 132, 160, 192,
                                196, 256])
-def test_shapes_for_many_chunks(gpu_ctx, pkg, oracle, K, short_rows):
-    """Narrow lane groups with several vectors per lane, which the kernels take when there are many chunks: the first and
-    last width of every shape, rows that are split and rows of a few entries."""
+def test_shapes_by_number_of_chunks(gpu_ctx, pkg, oracle, K, short_rows):
+    """Narrow lane groups with several vectors per lane, which the kernels take by width and by number of chunks: the first
+    and last width of every shape, rows that are split and rows of a few entries."""
     ctx = gpu_ctx
     if short_rows:
         rng = np.random.default_rng(7)
@@ -184,6 +184,12 @@ def test_shapes_for_many_chunks(gpu_ctx, pkg, oracle, K, short_rows):
             check_against_f64(read(), ref_c, abs_c, "spmm K=%d" % K)
             buf.free()
             ctx.plan_destroy(plan)
+    for chunk in (96, 512):   # one to two waves of chunks, and less than one
+        buf, o_ptr, read = guarded_output(ctx, (nnz,))
+        ctx.sddmm_csr(M, N, K, nnz, d_rp, d_ci, d_X, d_Y, o_ptr, opts=pkg.Opts(algo=pkg.ALGO_BALANCED, chunk_nnz=chunk))
+        ctx.stream_sync()
+        check_against_f64(read(), ref, abs_sum, "sddmm K=%d chunk=%d" % (K, chunk))
+        buf.free()
     r, c, v = oracle.csr_to_coo_padded(rp, ci, vals, 32)
     e = [ctx.upload(x) for x in (r, c, v)]
     buf, c_ptr, read = guarded_output(ctx, (M, K), fill=np.float32(0))
