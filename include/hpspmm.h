@@ -207,7 +207,7 @@ HPSPMM_API int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
 /* Same product with HOST buffers: copies A and B to the device, runs the product,
  * copies C back, synchronises.  When K is a multiple of 32 and at least 64 the call is
  * pipelined over 32- or 64-column slabs of B and C (uploads, products and downloads overlap on
- * three internal streams, PCIe being full duplex); each slab is a product of the slab's width, so
+ * three internal streams, PCIe being full duplex; dense operands of up to 4 MB go whole); each slab is a product of the slab's width, so
  * the rounding of rows split across chunks can differ from the device-pointer entry point in
  * the last bits.  The overlap needs page-locked host buffers (hpspmm_host_alloc_pinned or the
  * caller's own): from pageable memory the copies are staged and serialised by the driver and the
