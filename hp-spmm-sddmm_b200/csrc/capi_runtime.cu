@@ -166,6 +166,7 @@ int hpspmm_ctx_destroy(hpspmm_ctx* ctx) {
     if (--g_pool[ctx->device].contexts == 0) flush_pool_locked(g_pool[ctx->device]);
   }
   if (ctx->scratch) cudaFree(ctx->scratch);
+  if (ctx->counters) cudaFree(ctx->counters);
   if (ctx->stage) cudaFree(ctx->stage);
   if (ctx->flag) cudaFree(ctx->flag);
   for (int i = 0; i < 3; ++i)
@@ -321,14 +322,13 @@ int hpspmm_event_destroy(hpspmm_ctx* ctx, hpspmm_event ev) {
 
 }  // extern "C"
 
-static int grow_scratch(hpspmm_ctx* ctx, size_t bytes) {
+int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes) {
   if (bytes <= ctx->scratch_bytes) return HPSPMM_OK;
   // grow-only; the old buffer may still be in use by queued kernels
   HPSPMM_CUDA_TRY(ctx, cudaDeviceSynchronize());
   if (ctx->scratch) cudaFree(ctx->scratch);
   ctx->scratch = nullptr;
   ctx->scratch_bytes = 0;
-  ctx->zero_prefix = 0;
   size_t want = bytes + bytes / 4 + 4096;
   cudaError_t e = hpspmm_device_malloc(&ctx->scratch, want);
   if (e != cudaSuccess) {
@@ -340,22 +340,42 @@ static int grow_scratch(hpspmm_ctx* ctx, size_t bytes) {
   return HPSPMM_OK;
 }
 
-int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes) {
-  ctx->zero_prefix = 0;
-  return grow_scratch(ctx, bytes);
+int hpspmm_ensure_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream) {
+  if (n > ctx->counter_cap) {
+    HPSPMM_CUDA_TRY(ctx, cudaDeviceSynchronize());
+    if (ctx->counters) cudaFree(ctx->counters);
+    ctx->counters = nullptr;
+    ctx->counter_cap = 0;
+    const int64_t cap = (n + n / 4 + 1023) / 1024 * 1024;
+    const cudaError_t e = hpspmm_device_malloc(&ctx->counters, (size_t)cap * 8);
+    if (e != cudaSuccess) return hpspmm_set_err(ctx, HPSPMM_ERR_OOM, "counter cudaMalloc", e);
+    ctx->counter_cap = cap;
+    ctx->counters_unknown = true;
+  }
+  if (ctx->counters_unknown) {
+    HPSPMM_CUDA_TRY(ctx, cudaMemsetAsync(ctx->counters, 0, (size_t)ctx->counter_cap * 8, stream));
+    ctx->counter_used[0] = ctx->counter_used[1] = 0;
+    ctx->counters_unknown = false;
+  }
+  return HPSPMM_OK;
 }
 
-int hpspmm_ensure_scratch_counters(hpspmm_ctx* ctx, size_t bytes, size_t prefix, cudaStream_t stream) {
-  const int st = grow_scratch(ctx, bytes);
+int hpspmm_take_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream, int32_t** set, int32_t** clear, int* n_clear) {
+  const int st = hpspmm_ensure_counters(ctx, n, stream);
   if (st != HPSPMM_OK) return st;
-  // a graph may be replayed after the scratch has served other calls: a captured call clears the counters itself
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();
-  if (ctx->zero_prefix < prefix || capture != cudaStreamCaptureStatusNone)
-    HPSPMM_CUDA_TRY(ctx, cudaMemsetAsync(ctx->scratch, 0, prefix, stream));
-  // (a shorter prefix than last time: what follows it is about to hold other things)
-  ctx->zero_prefix = prefix;
+  const int turn = ctx->counter_turn;
+  *set = ctx->counters + turn * ctx->counter_cap;
+  *clear = ctx->counters + (1 - turn) * ctx->counter_cap;
+  *n_clear = (int)ctx->counter_used[1 - turn];
   return HPSPMM_OK;
+}
+
+void hpspmm_counters_used(hpspmm_ctx* ctx, int64_t n, bool launched) {
+  const int turn = ctx->counter_turn;
+  ctx->counter_used[turn] = n;
+  ctx->counter_used[1 - turn] = 0;
+  ctx->counter_turn = 1 - turn;
+  ctx->counters_unknown = !launched;
 }
 
 int hpspmm_ensure_stage(hpspmm_ctx* ctx, size_t bytes) {

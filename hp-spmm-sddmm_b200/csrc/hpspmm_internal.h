@@ -19,8 +19,14 @@ struct hpspmm_ctx {
   // scratch for plan-less calls: chunk table and carries
   void* scratch;
   size_t scratch_bytes;
-  size_t zero_prefix;   // leading bytes of scratch that are zero: the split-row counters of plan-less products, which every
-                        // product leaves at zero; any other use of the scratch ends that (hpspmm_ensure_scratch)
+  // split-row counters of plan-less products that run as one launch: two sets of counter_cap ints in a block that
+  // nothing else writes.  A product counts in one set and clears what the one before it may have left in the other
+  // (hpspmm_take_counters).
+  int32_t* counters;
+  int64_t counter_cap;
+  int64_t counter_used[2];
+  int counter_turn;
+  bool counters_unknown;   // a launch failed between the two: both sets are cleared before the next use
   // staging for the host-buffer entry point
   void* stage;
   size_t stage_bytes;
@@ -81,6 +87,8 @@ struct hpspmm_spmm_args {
   const int2* nz;
   float* carry;
   int32_t* counter;
+  int32_t* clear;   // n_clear ints that the kernel without a list sets to zero, for the next product (hpspmm_take_counters)
+  int n_clear;
 };
 // Shape of the kernel for `cols` columns: VEC-wide vectors, W lanes and R vectors per lane to a group (warp_frag.cuh).
 struct hpspmm_spmm_shape {
@@ -178,8 +186,12 @@ struct hpspmm_trace_range {
 #define HPSPMM_TRACE(name) hpspmm_trace_range hpspmm_trace_range__(name)
 
 int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes);
-// the same for a caller that keeps counters in the first `prefix` bytes and nothing else there: they are zero afterwards
-int hpspmm_ensure_scratch_counters(hpspmm_ctx* ctx, size_t bytes, size_t prefix, cudaStream_t stream);
+// `n` counters that are zero when work queued on `stream` starts, for one product whose kernel clears the first
+// `*n_clear` ints at `*clear`; hpspmm_counters_used tells how its launch went.  Not for captured calls: a graph may be
+// replayed between any two products, so a captured call keeps its counters in the scratch and clears them itself.
+int hpspmm_ensure_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream);
+int hpspmm_take_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream, int32_t** set, int32_t** clear, int* n_clear);
+void hpspmm_counters_used(hpspmm_ctx* ctx, int64_t n, bool launched);
 int hpspmm_ensure_stage(hpspmm_ctx* ctx, size_t bytes);
 
 // nominal chunk size for a dense width and a matrix of nnz entries
@@ -199,7 +211,7 @@ int hpspmm_order_chunks_by_cost(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t n
 
 // Builds the structure a product walks, in two launches: the list of rows that hold entries (nz, hpspmm_nz_bytes(M)
 // bytes, with sentinels (M, INT_MAX) at its end) and one record per chunk in matrix order (rec_out, 2 * n_chunks int4).
-// counts: hpspmm_row_tiles(M) ints of scratch.  The arrays of `tables` are
+// counts: hpspmm_row_tiles(M) ints of scratch.  The first launch also sets `n_clear` ints at `clear` to zero.  The arrays of `tables` are
 // filled as well where they are given (a plan exposes them), and split_count receives the number of chunks that
 // begin inside a row.
 struct hpspmm_structure_tables {
@@ -213,7 +225,8 @@ struct hpspmm_structure_tables {
 int64_t hpspmm_row_tiles(int64_t M);
 size_t hpspmm_nz_bytes(int64_t M);
 int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr, int32_t S, int64_t n_chunks,
-                           int2* nz, int4* rec_out, int32_t* counts, const hpspmm_structure_tables& tables, cudaStream_t stream);
+                           int2* nz, int4* rec_out, int32_t* counts, const hpspmm_structure_tables& tables, cudaStream_t stream,
+                           int32_t* clear = nullptr, int64_t n_clear = 0);
 // rec[slot] = rec_in[order[slot]]
 int hpspmm_order_records(hpspmm_ctx* ctx, int64_t n_chunks, const int32_t* order, const int4* rec_in, int4* rec,
                          cudaStream_t stream);

@@ -632,19 +632,20 @@ bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t 
   return n_chunks <= ctx->sm_count * 40ll && M <= 8 * nnz;
 }
 
-// where a plan-less product keeps what it builds, inside the context's scratch; the counters come first
+// where a plan-less product keeps what it builds, inside the context's scratch
 struct planless_layout {
+  int64_t n_counter;
   size_t counter, carry, tiles, rec, nz, bytes;
   planless_layout(int64_t M, int64_t K, int64_t n_chunks, bool search) {
     bytes = 0;
     auto take = [&](size_t b) { const size_t at = bytes; bytes += align_up(b, 256); return at; };
-    counter = take((size_t)(n_chunks + 1) * (size_t)hpspmm_counter_slabs(K) * 4);
+    n_counter = (n_chunks + 1) * hpspmm_counter_slabs(K);
+    counter = take((size_t)n_counter * 4);
     carry = take((size_t)(n_chunks + 1) * (size_t)K * 4);
     tiles = search ? 0 : take((size_t)hpspmm_row_tiles(M) * 4);
     rec = search ? 0 : take((size_t)(n_chunks + 1) * 32);
     nz = search ? 0 : take(hpspmm_nz_bytes(M));
   }
-  size_t counter_bytes() const { return carry; }
 };
 
 }  // namespace
@@ -817,20 +818,34 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
   const int64_t n_chunks = (nnz + S - 1) / S;
   const bool search = searches_for_chunks(ctx, M, nnz, n_chunks);
   const planless_layout lay(M, K, n_chunks, search);
-  st = hpspmm_ensure_scratch_counters(ctx, lay.bytes, lay.counter_bytes(), s);
+  st = hpspmm_ensure_scratch(ctx, lay.bytes);
   if (st != HPSPMM_OK) return st;
   char* base = (char*)ctx->scratch;
   a.n_chunks = (int)n_chunks, a.S = S;
   a.carry = (float*)(base + lay.carry), a.counter = (int32_t*)(base + lay.counter);
+  // The counters of split rows have to be zero when the product starts.  Where the structure is built first, that clears
+  // them.  A product of one launch takes them from sets of their own, cleared by the product before it (a memset in front
+  // costs 2 us of a product of 8), unless the call is being captured.
   if (!search) {
     int4* rec = (int4*)(base + lay.rec);
     int2* nz = (int2*)(base + lay.nz);
     st = hpspmm_build_structure(ctx, M, nnz, row_ptr, S, n_chunks, nz, rec, (int32_t*)(base + lay.tiles),
-                                hpspmm_structure_tables{}, s);
+                                hpspmm_structure_tables{}, s, a.counter, lay.n_counter);
     if (st != HPSPMM_OK) return st;
     a.rec = rec, a.nz = nz;
+    return launch_spmm(ctx, a, hint, false, s);
   }
-  return launch_spmm(ctx, a, hint, false, s);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
+  if (capture != cudaStreamCaptureStatusNone) {
+    HPSPMM_CUDA_TRY(ctx, cudaMemsetAsync(a.counter, 0, (size_t)lay.n_counter * 4, s));
+    return launch_spmm(ctx, a, hint, false, s);
+  }
+  st = hpspmm_take_counters(ctx, lay.n_counter, s, &a.counter, &a.clear, &a.n_clear);
+  if (st != HPSPMM_OK) return st;
+  st = launch_spmm(ctx, a, hint, false, s);
+  hpspmm_counters_used(ctx, lay.n_counter, st == HPSPMM_OK);
+  return st;
 }
 
 // Host-buffer products, pipelined over column slabs: C[:, s] = A * B[:, s] needs only slab s of B,
@@ -875,14 +890,18 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
   // size the kernel scratch before anything is queued (growing it synchronises the device)
   {
     size_t need = 0;
+    int64_t need_counters = 0;
     for (int i = 0; i < n_slabs; ++i) {
       const int64_t w = slabs[i].width;
       const int32_t S = planless_chunk_nnz(w, nnz, opts);
       const int64_t n_chunks = (nnz + S - 1) / S;
-      const size_t want = planless_layout(M, w, n_chunks, searches_for_chunks(ctx, M, nnz, n_chunks)).bytes;
-      need = want > need ? want : need;
+      const bool search = searches_for_chunks(ctx, M, nnz, n_chunks);
+      const planless_layout lay(M, w, n_chunks, search);
+      need = lay.bytes > need ? lay.bytes : need;
+      if (search && lay.n_counter > need_counters) need_counters = lay.n_counter;
     }
     st = hpspmm_ensure_scratch(ctx, need);
+    if (st == HPSPMM_OK) st = hpspmm_ensure_counters(ctx, need_counters, s_run);
     if (st != HPSPMM_OK) return st;
   }
   char* base = (char*)ctx->stage;

@@ -214,8 +214,13 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   __shared__ int meta[BT / 32][8];
 
   if ((int)blockIdx.x >= a.n_chunk_blocks) {
-    if (blockIdx.y == 0 && a.slab0 == 0 && a.off == 0)
+    if (blockIdx.y == 0 && a.slab0 == 0 && a.off == 0) {
+      if (!LIST)
+        for (int i = ((int)blockIdx.x - a.n_chunk_blocks) * BT + (int)threadIdx.x; i < a.n_clear;
+             i += ((int)gridDim.x - a.n_chunk_blocks) * BT)
+          a.clear[i] = 0;
       zero_empty_rows<KS>(a.M, a.K, a.row_ptr, a.C, blockIdx.x - a.n_chunk_blocks, gridDim.x - a.n_chunk_blocks, BT);
+    }
     return;
   }
   const int lane = threadIdx.x & 31;

@@ -615,7 +615,9 @@ int row_tile_size(int64_t M) {
 }
 
 __global__ void __launch_bounds__(kThreads)
-row_tile_count_kernel(int M, int tile, const int* __restrict__ row_ptr, int* __restrict__ counts) {
+row_tile_count_kernel(int M, int tile, const int* __restrict__ row_ptr, int* __restrict__ counts, int* __restrict__ clear,
+                      int64_t n_clear) {
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n_clear; i += (int64_t)gridDim.x * kThreads) clear[i] = 0;
   const int64_t r0 = (int64_t)blockIdx.x * tile;
   int total = 0;
   for (int i = 0; i < tile && r0 + i < M; i += kThreads) {
@@ -733,10 +735,11 @@ int64_t hpspmm_row_tiles(int64_t M) {
 }
 
 int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr, int32_t S, int64_t n_chunks,
-                           int2* nz, int4* rec_out, int32_t* counts, const hpspmm_structure_tables& tables, cudaStream_t stream) {
+                           int2* nz, int4* rec_out, int32_t* counts, const hpspmm_structure_tables& tables, cudaStream_t stream,
+                           int32_t* clear, int64_t n_clear) {
   const int tile = row_tile_size(M);
   const unsigned blocks = (unsigned)hpspmm_row_tiles(M);
-  row_tile_count_kernel<<<blocks, kThreads, 0, stream>>>((int)M, tile, row_ptr, counts);
+  row_tile_count_kernel<<<blocks, kThreads, 0, stream>>>((int)M, tile, row_ptr, counts, clear, n_clear);
   row_tile_list_kernel<<<blocks, kThreads, 0, stream>>>((int)M, (int)nnz, tile, S, (int)n_chunks, row_ptr, counts, nz,
                                                         rec_out, tables);
   ctx->launches += 2;

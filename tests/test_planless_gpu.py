@@ -1,0 +1,119 @@
+"""Products without a plan between other users of the context: the counters of split rows start at zero in every call
+(needs a B200)."""
+import numpy as np
+import pytest
+
+from helpers import check_against_f64, random_csr
+
+pytestmark = pytest.mark.gpu
+
+
+class _Work:
+    """Operands of one plan-less product whose rows are longer than a chunk, with its reference."""
+
+    def __init__(self, pkg, oracle, degrees, N, K, seed):
+        import torch
+        self.rp_h, self.ci_h, self.v_h = random_csr(len(degrees), N, degrees, seed=seed)
+        self.M, self.N, self.K, self.nnz = len(degrees), N, K, len(self.ci_h)
+        B = pkg.host_fill_uniform(N * K, seed, 1, -1.0, 1.0).reshape(N, K)
+        self.ref, self.abs_sum = oracle.spmm_f64(self.rp_h, self.ci_h, self.v_h, B)
+        self.rp, self.ci, self.v, self.B = (torch.from_numpy(x).cuda() for x in (self.rp_h, self.ci_h, self.v_h, B))
+        self.C = torch.empty((self.M, K), device="cuda")
+
+    def call(self, ctx, stream, opts=None):
+        self.C.fill_(7.0)
+        ctx.spmm_csr(self.M, self.N, self.K, self.nnz, self.rp.data_ptr(), self.ci.data_ptr(), self.v.data_ptr(),
+                     self.B.data_ptr(), self.C.data_ptr(), opts=opts, stream=stream)
+
+    def check(self, what):
+        import torch
+        torch.cuda.synchronize()
+        check_against_f64(self.C.cpu().numpy(), self.ref, self.abs_sum, what)
+
+
+def _dirty_scratch(ctx, w, stream):
+    """A transpose keeps its own tables where plan-less products keep theirs."""
+    import torch
+    rpt = torch.empty(w.N + 1, dtype=torch.int32, device="cuda")
+    cit, vt = torch.empty_like(w.ci), torch.empty_like(w.v)
+    ctx.csr_transpose(w.M, w.N, w.nnz, w.rp.data_ptr(), w.ci.data_ptr(), w.v.data_ptr(), rpt.data_ptr(), cit.data_ptr(),
+                      vt.data_ptr(), stream=stream)
+    return rpt, cit, vt
+
+
+DEGREES = [5000, 1, 700, 0, 33, 9000, 64, 65, 2, 3000] * 3
+
+
+@pytest.mark.parametrize("chunk", [0, 32])
+def test_eager_products_around_a_capture(pkg, oracle, chunk):
+    """Eager products before the first replay, between replays of narrower and wider captured ones, and beside a
+    captured SDDMM and transpose: a replay writes the scratch without the host knowing."""
+    import torch
+    opts = pkg.Opts(chunk_nnz=chunk)
+    N = 20000
+    small = _Work(pkg, oracle, DEGREES[:10], N, 32, 101)
+    wide = _Work(pkg, oracle, DEGREES, N, 128, 102)
+    with pkg.Context(0) as ctx:
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            s = side.cuda_stream
+            out = torch.empty(wide.nnz, device="cuda")
+            X = torch.rand((wide.M, 32), device="cuda")
+
+            def sddmm():
+                ctx.sddmm_csr(wide.M, N, 32, wide.nnz, wide.rp.data_ptr(), wide.ci.data_ptr(), X.data_ptr(),
+                              wide.B.data_ptr(), out.data_ptr(), opts=opts, stream=s)
+
+            keep = _dirty_scratch(ctx, wide, s)
+            for w in (wide, small):                       # sizes the scratch for every call below
+                w.call(ctx, s, opts)
+                w.check("warm-up")
+            sddmm()
+            keep = _dirty_scratch(ctx, wide, s)           # the counters' old place now holds sort keys
+            side.synchronize()
+            g_small, g_sddmm, g_wide = (torch.cuda.CUDAGraph() for _ in range(3))
+            with torch.cuda.graph(g_small, stream=side):
+                small.call(ctx, s, opts)
+            small.call(ctx, s, opts)                      # before the first replay: only recorded so far
+            small.check("eager product after a capture")
+            with torch.cuda.graph(g_sddmm, stream=side):
+                sddmm()
+            with torch.cuda.graph(g_wide, stream=side):
+                wide.call(ctx, s, opts)
+            for turn in range(3):
+                wide.call(ctx, s, opts)
+                wide.check("wide, eager, turn %d" % turn)
+                g_small.replay()
+                small.check("small, replayed, turn %d" % turn)
+                wide.call(ctx, s, opts)
+                wide.check("wide after a replay of small, turn %d" % turn)
+                g_sddmm.replay()
+                wide.call(ctx, s, opts)
+                wide.check("wide after a replayed SDDMM, turn %d" % turn)
+                small.call(ctx, s, opts)
+                small.check("small, eager, turn %d" % turn)
+                keep = _dirty_scratch(ctx, wide, s)
+                g_wide.replay()
+                wide.check("wide, replayed, turn %d" % turn)
+                g_wide.replay()
+                wide.check("wide, replayed twice, turn %d" % turn)
+            del g_small, g_sddmm, g_wide, keep
+
+
+def test_products_of_changing_sizes_without_a_plan(pkg, oracle):
+    """One launch per product, then with the structure built first (many empty rows), in turn: each kind keeps its
+    counters elsewhere, and the sets grow between calls."""
+    import torch
+    N = 20000
+    works = [_Work(pkg, oracle, DEGREES[:10], N, 32, 103), _Work(pkg, oracle, DEGREES, N, 96, 104),
+             _Work(pkg, oracle, ([0] * 30000 + [900]) * 3, N, 64, 105), _Work(pkg, oracle, DEGREES, N, 600, 106),
+             _Work(pkg, oracle, [4000], N, 5, 107)]
+    assert works[2].M > 8 * works[2].nnz                 # this one has its structure built
+    with pkg.Context(0) as ctx:
+        s = torch.cuda.current_stream().cuda_stream
+        for turn in range(3):
+            for i, w in enumerate(works):
+                for rep in range(2):
+                    w.call(ctx, s)
+                    w.check("product %d, turn %d, call %d" % (i, turn, rep))
