@@ -135,6 +135,25 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
 
 Tensor forward_autograd(const Tensor& H, const Tensor& vals, int64_t id) { return LayerFunction::apply(H, vals, id); }
 
+// The two gradients have no derivative of their own.  Without a formula on the autograd key PyTorch would only warn and
+// leave their terms out of a second derivative, so differentiating them is an error.
+template <const c10::TypedOperatorHandle<Op>& (*OP)()>
+struct NoDerivative : public torch::autograd::Function<NoDerivative<OP>> {
+  static Tensor forward(torch::autograd::AutogradContext*, const Tensor& a, const Tensor& b, int64_t id) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return OP().call(a, b, id);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext*, torch::autograd::variable_list) {
+    TORCH_CHECK(false, "hpspmm: no derivative of ", OP().schema().name(), " is implemented (a second derivative of the layer)");
+  }
+};
+template <const c10::TypedOperatorHandle<Op>& (*OP)()>
+Tensor gradient_autograd(const Tensor& a, const Tensor& b, int64_t id) {
+  if (at::GradMode::is_enabled() && (a.requires_grad() || b.requires_grad())) return NoDerivative<OP>::apply(a, b, id);
+  at::AutoDispatchBelowADInplaceOrView below;
+  return OP().call(a, b, id);
+}
+
 TORCH_LIBRARY(hpspmm, m) {
   m.def("layer_forward(Tensor H, Tensor vals, int layer_id) -> Tensor");
   m.def("layer_backward_features(Tensor dC, Tensor vals, int layer_id) -> Tensor");
@@ -149,7 +168,11 @@ TORCH_LIBRARY(hpspmm, m) {
   }
 HPSPMM_IMPL(CUDA)
 HPSPMM_IMPL(CPU)
-TORCH_LIBRARY_IMPL(hpspmm, Autograd, m) { m.impl("layer_forward", forward_autograd); }
+TORCH_LIBRARY_IMPL(hpspmm, Autograd, m) {
+  m.impl("layer_forward", forward_autograd);
+  m.impl("layer_backward_features", gradient_autograd<op_features>);
+  m.impl("layer_backward_weights", gradient_autograd<op_weights>);
+}
 
 void register_layer(int64_t id, int64_t ctx, int64_t layer, int64_t M, int64_t N, int64_t nnz, const Tensor& vals) {
   auto e = std::make_shared<Entry>();
