@@ -18,12 +18,15 @@ namespace {
 using at::Tensor;
 
 struct Entry {
+  // Held while a call uses the handles and the fields below: the interpreter lock is not held then, and threads may meet
+  // on one layer (the autograd engine's and the caller's at least).
+  std::mutex use;
   hpspmm_ctx* ctx;
-  hpspmm_layer* layer;
+  hpspmm_layer* layer;   // null once the layer is closed
   int64_t M, N, nnz;
   // the weight tensor whose values the layer's transpose holds (kept alive: the layer borrows the device array)
   Tensor vals;
-  int64_t vals_version;
+  int64_t vals_version;   // of `vals` when the transpose was filled; -1: unknown, fill it again
 };
 
 std::mutex g_mutex;   // guards the registry
@@ -36,6 +39,8 @@ std::shared_ptr<Entry> entry_of(int64_t id) {
   return it->second;
 }
 
+void check_open(const Entry& e, int64_t id) { TORCH_CHECK(e.layer, "hpspmm: unknown or closed layer id ", id); }
+
 void check(const Entry& e, int status, const char* what) {
   TORCH_CHECK(status == HPSPMM_OK, what, " failed with status ", status, ": ", hpspmm_last_error(e.ctx));
 }
@@ -47,24 +52,36 @@ Tensor require_cuda_f32(const Tensor& t, int64_t rows, const char* what) {
   return t.contiguous();
 }
 
-// Re-gathers the transpose's values when the weight tensor moved or was written in place.
-void sync_values(Entry& e, const Tensor& given, cudaStream_t stream) {
-  const Tensor vals = given.contiguous();
+Tensor require_weights(const Tensor& t, const Entry& e, const at::Device& device) {
+  TORCH_CHECK(t.is_cuda() && t.device() == device && t.scalar_type() == at::kFloat && t.numel() >= e.nnz,
+              "hpspmm: vals must be ", e.nnz, " float32 values on ", device, ", got ", t.scalar_type(), " ", t.sizes(), " on ",
+              t.device());
+  return t.contiguous();
+}
+
+// Re-gathers the transpose's values when the weight tensor moved or was written in place.  What was held goes to `old`, to
+// be released after the lock.
+void sync_values(Entry& e, const Tensor& vals, cudaStream_t stream, Tensor& old) {
   const int64_t version = vals.is_inference() ? -1 : (int64_t)vals._version();
   if (version >= 0 && e.vals.defined() && vals.const_data_ptr() == e.vals.const_data_ptr() && version == e.vals_version)
     return;
-  e.vals = vals.detach();
+  e.vals_version = -1;   // until the update has succeeded
   check(e, hpspmm_layer_update_values(e.ctx, e.layer, vals.const_data_ptr<float>(), stream), "hpspmm_layer_update_values");
+  old = std::move(e.vals);
+  e.vals = vals.detach();
   e.vals_version = version;
 }
 
 Tensor forward(const Tensor& H, const Tensor& vals, int64_t id) {
   auto e = entry_of(id);
-  const Tensor h = require_cuda_f32(H, e->N, "H");
+  const Tensor h = require_cuda_f32(H, e->N, "H"), v = require_weights(vals, *e, H.device());
   const c10::cuda::CUDAGuard guard(h.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-  sync_values(*e, vals, stream);
   Tensor C = at::empty({e->M, h.size(1)}, h.options());
+  Tensor old;
+  std::lock_guard<std::mutex> lock(e->use);
+  check_open(*e, id);
+  sync_values(*e, v, stream, old);
   check(*e, hpspmm_layer_forward(e->ctx, e->layer, h.size(1), h.const_data_ptr<float>(), C.mutable_data_ptr<float>(), stream),
         "hpspmm_layer_forward");
   return C;
@@ -72,11 +89,14 @@ Tensor forward(const Tensor& H, const Tensor& vals, int64_t id) {
 
 Tensor backward_features(const Tensor& grad, const Tensor& vals, int64_t id) {
   auto e = entry_of(id);
-  const Tensor dC = require_cuda_f32(grad, e->M, "dC");
+  const Tensor dC = require_cuda_f32(grad, e->M, "dC"), v = require_weights(vals, *e, grad.device());
   const c10::cuda::CUDAGuard guard(dC.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-  sync_values(*e, vals, stream);
   Tensor dH = at::empty({e->N, dC.size(1)}, dC.options());
+  Tensor old;
+  std::lock_guard<std::mutex> lock(e->use);
+  check_open(*e, id);
+  sync_values(*e, v, stream, old);
   check(*e, hpspmm_layer_backward_features(e->ctx, e->layer, dC.size(1), dC.const_data_ptr<float>(),
                                            dH.mutable_data_ptr<float>(), stream), "hpspmm_layer_backward_features");
   return dH;
@@ -89,6 +109,8 @@ Tensor backward_weights(const Tensor& grad, const Tensor& H, int64_t id) {
   TORCH_CHECK(h.size(1) == dC.size(1), "hpspmm: dC and H differ in width");
   const c10::cuda::CUDAGuard guard(dC.device());
   Tensor dA = at::empty({e->nnz}, dC.options());
+  std::lock_guard<std::mutex> lock(e->use);
+  check_open(*e, id);
   check(*e, hpspmm_layer_backward_weights(e->ctx, e->layer, dC.size(1), dC.const_data_ptr<float>(),
                                           h.const_data_ptr<float>(), dA.mutable_data_ptr<float>(),
                                           c10::cuda::getCurrentCUDAStream().stream()), "hpspmm_layer_backward_weights");
@@ -185,16 +207,25 @@ void register_layer(int64_t id, int64_t ctx, int64_t layer, int64_t M, int64_t N
   g_layers[id] = e;
 }
 
+// The caller destroys the handles next: calls in flight end first, later ones find the layer closed.
 void forget_layer(int64_t id) {
-  std::lock_guard<std::mutex> lock(g_mutex);
-  g_layers.erase(id);
+  std::shared_ptr<Entry> e;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    auto it = g_layers.find(id);
+    if (it == g_layers.end()) return;
+    e = std::move(it->second);
+    g_layers.erase(it);
+  }
+  std::lock_guard<std::mutex> lock(e->use);
+  e->layer = nullptr;
 }
 
 }  // namespace
 
 PYBIND11_MODULE(_hpspmm_torch, m) {
   m.def("register_layer", &register_layer);
-  m.def("forget_layer", &forget_layer);
+  m.def("forget_layer", &forget_layer, py::call_guard<py::gil_scoped_release>());
   m.def("layer_forward", [](const Tensor& H, const Tensor& vals, int64_t id) { return op_forward().call(H, vals, id); },
         py::call_guard<py::gil_scoped_release>());
 }

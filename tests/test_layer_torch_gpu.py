@@ -60,3 +60,72 @@ def test_second_derivatives_are_refused(work):
         with torch.no_grad():
             assert not op(dC, other, work.layer.layer_id).requires_grad
         assert not op(dC.detach(), other, work.layer.layer_id).requires_grad
+
+
+def test_weights_that_cannot_be_used_are_refused_every_time(work):
+    import torch
+    bad = [work.v.double(), work.v.cpu(), work.v[:-1].clone()]
+    for vals in bad:
+        for attempt in range(2):            # a refused tensor is not remembered as the one in use
+            with pytest.raises(RuntimeError):
+                work.layer(work.H, vals)
+            with pytest.raises(RuntimeError):
+                work.ops.layer_backward_features(torch.ones((work.M, work.K), device="cuda"), vals, work.layer.layer_id)
+    assert _close(work.layer(work.H), work.product(work.v, work.H))
+    two = torch.stack([work.v, work.v * 2], 1)
+    assert _close(work.layer(work.H, two[:, 1]), work.product(work.v * 2, work.H))      # strided
+    assert _close(work.layer(work.H, (work.v * 3)[None]), work.product(work.v * 3, work.H))
+
+
+def test_threads_meet_on_one_layer(work):
+    """Three threads on one stream, each with weights of its own that change in every step, beside the engine's."""
+    import threading
+
+    import torch
+    want, errors = [work.product(work.v * (t + 1), work.H) for t in range(3)], []
+    want_dH = [work.dense(work.v * (t + 1)).T @ torch.ones((work.M, work.K), device="cuda", dtype=torch.float64)
+               for t in range(3)]
+    torch.cuda.synchronize()
+
+    def steps(t):
+        try:
+            for i in range(60):
+                H = work.H.clone().requires_grad_()
+                W = (work.v * (t + 1)).requires_grad_()
+                C = work.layer(H, W)
+                C.sum().backward()
+                if i % 6 == 0:
+                    assert _close(C.detach(), want[t]) and _close(H.grad, want_dH[t])
+        except BaseException as e:      # noqa: B902 -- a thread's failure is the test's
+            errors.append(e)
+
+    threads = [threading.Thread(target=steps, args=(t,)) for t in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
+
+
+def test_closing_under_calls(pkg):
+    """close() waits for the call in flight; later calls find the layer closed."""
+    import threading
+    w = _Layer(pkg)
+    ends = []
+
+    def calls():
+        try:
+            for _ in range(2000):
+                w.layer(w.H)
+        except RuntimeError as e:
+            ends.append(str(e))
+
+    threads = [threading.Thread(target=calls) for _ in range(2)]
+    for t in threads:
+        t.start()
+    w.layer.close()
+    for t in threads:
+        t.join()
+    assert all("unknown or closed" in e for e in ends)
+    with pytest.raises(RuntimeError, match="unknown or closed"):
+        w.layer(w.H)
