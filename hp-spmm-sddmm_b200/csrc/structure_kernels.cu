@@ -687,7 +687,7 @@ row_tile_list_kernel(int M, int nnz, int tile, int S, int n_chunks, const int* _
         t.nz_id[rank] = (int)r;
         t.nz_end[rank] = e;
       }
-      c_lo = (s + S - 1) / S;
+      c_lo = s == 0 ? 0 : (s - 1) / S + 1;   // (s + S - 1 would overflow for the largest S)
       c_n = (e - 1) / S - c_lo + 1;
       if (e == nnz && n_chunks > 0) {
         rec[2 * (int64_t)n_chunks - 1].z = nnz;

@@ -117,3 +117,33 @@ def test_products_of_changing_sizes_without_a_plan(pkg, oracle):
                 for rep in range(2):
                     w.call(ctx, s)
                     w.check("product %d, turn %d, call %d" % (i, turn, rep))
+
+
+@pytest.mark.parametrize("chunk", [1 << 20, (1 << 31) - 64, (1 << 31) - 32])
+def test_chunks_larger_than_any_matrix(pkg, oracle, chunk):
+    """One chunk for the whole matrix, up to the largest size that can be asked for, with the structure built."""
+    import torch
+    opts = pkg.Opts(chunk_nnz=chunk)
+    w = _Work(pkg, oracle, [40, 0, 1, 700, 33, 5000], 8000, 32, 110)
+    sparse = _Work(pkg, oracle, ([0] * 30000 + [900]) * 3, 8000, 64, 111)
+    with pkg.Context(0) as ctx:
+        s = torch.cuda.current_stream().cuda_stream
+        for x in (w, sparse):
+            x.call(ctx, s, opts)
+            x.check("without a plan, chunk %d" % chunk)
+            plan = ctx.plan_create(x.M, x.nnz, x.rp.data_ptr(), x.K, opts, N=x.N, col_idx=x.ci.data_ptr(), stream=s)
+            assert ctx.plan_info(plan)["n_chunks"] == 1
+            x.C.fill_(7.0)
+            ctx.spmm_csr(x.M, x.N, x.K, x.nnz, x.rp.data_ptr(), x.ci.data_ptr(), x.v.data_ptr(), x.B.data_ptr(),
+                         x.C.data_ptr(), plan=plan, stream=s)
+            x.check("with a plan, chunk %d" % chunk)
+            X = torch.rand((x.M, x.K), device="cuda")
+            out = torch.empty(x.nnz, device="cuda")
+            rows = torch.repeat_interleave(torch.arange(x.M, device="cuda"), (x.rp[1:] - x.rp[:-1]).long())
+            want = (X[rows].double() * x.B[x.ci.long()].double()).sum(1)
+            for p in (plan, None):
+                out.fill_(7.0)
+                ctx.sddmm_csr(x.M, x.N, x.K, x.nnz, x.rp.data_ptr(), x.ci.data_ptr(), X.data_ptr(), x.B.data_ptr(),
+                              out.data_ptr(), plan=p, opts=opts, stream=s)
+                assert float((out.double() - want).abs().max()) <= 2e-5      # 64 terms of at most 1, in 32 bits
+            ctx.plan_destroy(plan)
