@@ -3,7 +3,6 @@
 // operators (include/starml/basic/matrix.h:14-77, spmm/starml/basic/allocator_cuda.cpp:5-24,
 // spmm/starml/basic/handle_cuda.cpp:4-23, spmm/starml/operators/cuda/copy_kernel.cu:7-41).
 #include <atomic>
-#include <mutex>
 #include <new>
 
 #include "hpspmm_internal.h"
@@ -12,91 +11,17 @@
 static std::atomic<int64_t> g_fail_skip{0};
 static std::atomic<int64_t> g_fail_count{0};
 
-static bool injected_failure(void** out) {
-  if (g_fail_count.load(std::memory_order_relaxed) <= 0) return false;
-  if (g_fail_skip.load(std::memory_order_relaxed) > 0) {
-    g_fail_skip.fetch_sub(1, std::memory_order_relaxed);
-    return false;
-  }
-  g_fail_count.fetch_sub(1, std::memory_order_relaxed);
-  if (out) *out = nullptr;
-  return true;
-}
-
 cudaError_t hpspmm_device_malloc(void** out, size_t bytes) {
-  return injected_failure(out) ? cudaErrorMemoryAllocation : cudaMalloc(out, bytes);
-}
-
-// Blocks of destroyed plans and layers, for the next ones: cudaMalloc and cudaFree of a block beyond 1 MB take 0.25 to
-// 0.35 ms each, most of what building a plan takes (1.8 M entries, K = 32: plan 0.48 -> 0.12 ms, its end 0.27 -> 0.00).
-// Per device at most kPoolBlocks blocks and kPoolBytes bytes, none larger than kPoolLargest; all given back when the
-// last context on the device goes.  A block enters the pool only after the device is idle (as with cudaFree), so
-// whatever stream used it last is done with it.
-namespace {
-constexpr int kPoolDevices = 64, kPoolBlocks = 8;
-constexpr size_t kPoolSmallest = 256u << 10, kPoolLargest = 32u << 20, kPoolBytes = 64u << 20;
-struct device_pool {
-  int contexts, n;
-  size_t held;
-  struct {
-    void* p;
-    size_t bytes;
-  } block[kPoolBlocks];
-};
-device_pool g_pool[kPoolDevices];
-std::mutex g_pool_mutex;
-
-void flush_pool_locked(device_pool& d) {   // the device is current
-  for (int i = 0; i < d.n; ++i) cudaFree(d.block[i].p);
-  d.n = 0;
-  d.held = 0;
-}
-}  // namespace
-
-cudaError_t hpspmm_pool_malloc(int device, void** out, size_t bytes, size_t* got) {
-  *got = bytes;
-  if (injected_failure(out)) return cudaErrorMemoryAllocation;
-  if (device < 0 || device >= kPoolDevices || bytes < kPoolSmallest || bytes > kPoolLargest) return cudaMalloc(out, bytes);
-  {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    device_pool& d = g_pool[device];
-    int best = -1;
-    for (int i = 0; i < d.n; ++i)
-      if (d.block[i].bytes >= bytes && d.block[i].bytes <= 2 * bytes &&
-          (best < 0 || d.block[i].bytes < d.block[best].bytes))
-        best = i;
-    if (best >= 0) {
-      *out = d.block[best].p;
-      *got = d.block[best].bytes;
-      d.held -= *got;
-      d.block[best] = d.block[--d.n];
-      return cudaSuccess;
+  if (g_fail_count.load(std::memory_order_relaxed) > 0) {
+    if (g_fail_skip.load(std::memory_order_relaxed) > 0) {
+      g_fail_skip.fetch_sub(1, std::memory_order_relaxed);
+    } else {
+      g_fail_count.fetch_sub(1, std::memory_order_relaxed);
+      if (out) *out = nullptr;
+      return cudaErrorMemoryAllocation;
     }
   }
-  cudaError_t e = cudaMalloc(out, bytes);
-  if (e == cudaErrorMemoryAllocation) {   // what the pool holds may be what is missing
-    cudaGetLastError();
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    flush_pool_locked(g_pool[device]);
-    e = cudaMalloc(out, bytes);
-  }
-  return e;
-}
-
-void hpspmm_pool_free(int device, void* p, size_t bytes) {
-  if (!p) return;
-  if (device >= 0 && device < kPoolDevices && bytes >= kPoolSmallest && bytes <= kPoolLargest &&
-      cudaDeviceSynchronize() == cudaSuccess) {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    device_pool& d = g_pool[device];
-    if (d.contexts > 0 && d.n < kPoolBlocks && d.held + bytes <= kPoolBytes) {
-      d.block[d.n].p = p;
-      d.block[d.n++].bytes = bytes;
-      d.held += bytes;
-      return;
-    }
-  }
-  cudaFree(p);
+  return cudaMalloc(out, bytes);
 }
 
 extern "C" {
@@ -149,10 +74,6 @@ int hpspmm_ctx_create(int device_ordinal, hpspmm_ctx** out) {
     return e == cudaErrorMemoryAllocation ? HPSPMM_ERR_OOM : HPSPMM_ERR_CUDA;
   }
   cudaMemset(ctx->flag, 0, 256);
-  if (device_ordinal < kPoolDevices) {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    g_pool[device_ordinal].contexts++;
-  }
   *out = ctx;
   return HPSPMM_OK;
 }
@@ -161,10 +82,6 @@ int hpspmm_ctx_destroy(hpspmm_ctx* ctx) {
   if (!ctx) return HPSPMM_OK;
   hpspmm_device_guard guard(ctx->device);
   cudaDeviceSynchronize();
-  if (ctx->device < kPoolDevices) {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (--g_pool[ctx->device].contexts == 0) flush_pool_locked(g_pool[ctx->device]);
-  }
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->counters) cudaFree(ctx->counters);
   if (ctx->stage) cudaFree(ctx->stage);

@@ -27,7 +27,6 @@ struct hpspmm_layer {
   hpspmm_plan* plan[3];
   hpspmm_plan* plan_t[3];
   size_t bytes;
-  size_t block_bytes[4];   // of the four arrays of the transpose
 };
 
 namespace {
@@ -47,10 +46,10 @@ void release(hpspmm_ctx* ctx, hpspmm_layer* g) {
     if (g->plan[i]) hpspmm_plan_destroy(ctx, g->plan[i]);
     if (g->plan_t[i]) hpspmm_plan_destroy(ctx, g->plan_t[i]);
   }
-  hpspmm_pool_free(g->device, g->row_ptr_t, g->block_bytes[0]);
-  hpspmm_pool_free(g->device, g->col_idx_t, g->block_bytes[1]);
-  hpspmm_pool_free(g->device, g->vals_t, g->block_bytes[2]);
-  hpspmm_pool_free(g->device, g->perm, g->block_bytes[3]);
+  cudaFree(g->row_ptr_t);
+  cudaFree(g->col_idx_t);
+  cudaFree(g->vals_t);
+  cudaFree(g->perm);
   delete g;
 }
 
@@ -99,10 +98,10 @@ int hpspmm_layer_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, cons
   g->col_idx = col_idx;
   g->vals = vals;
   const size_t b_rp = (size_t)(N + 1) * 4, b_e = (size_t)(nnz > 0 ? nnz : 1) * 4;
-  cudaError_t e = hpspmm_pool_malloc(g->device, (void**)&g->row_ptr_t, b_rp, &g->block_bytes[0]);
-  if (e == cudaSuccess) e = hpspmm_pool_malloc(g->device, (void**)&g->col_idx_t, b_e, &g->block_bytes[1]);
-  if (e == cudaSuccess) e = hpspmm_pool_malloc(g->device, (void**)&g->vals_t, b_e, &g->block_bytes[2]);
-  if (e == cudaSuccess) e = hpspmm_pool_malloc(g->device, (void**)&g->perm, b_e, &g->block_bytes[3]);
+  cudaError_t e = hpspmm_device_malloc((void**)&g->row_ptr_t, b_rp);
+  if (e == cudaSuccess) e = hpspmm_device_malloc((void**)&g->col_idx_t, b_e);
+  if (e == cudaSuccess) e = hpspmm_device_malloc((void**)&g->vals_t, b_e);
+  if (e == cudaSuccess) e = hpspmm_device_malloc((void**)&g->perm, b_e);
   if (e != cudaSuccess) {
     release(ctx, g);
     return hpspmm_set_err(ctx, HPSPMM_ERR_OOM, "layer cudaMalloc", e);

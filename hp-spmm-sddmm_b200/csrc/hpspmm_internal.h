@@ -65,7 +65,7 @@ struct hpspmm_plan {
   int32_t* chunk_ri;
   int2* nz;        // (nz_id, nz_end) as one word per row: what the product kernels step through
   int4* rec;
-  size_t bytes, block_bytes;   // needed, and what the block behind it holds
+  size_t bytes;
 };
 
 // What the CSR product kernels are launched with.
@@ -167,11 +167,6 @@ template <typename T>
 static inline cudaError_t hpspmm_device_malloc(T** out, size_t bytes) {
   return hpspmm_device_malloc(reinterpret_cast<void**>(out), bytes);
 }
-
-// The same for the blocks of plans and layers, which are kept for the next ones (a bounded pool per device).  `got` is
-// what hpspmm_pool_free wants back as `bytes`; the device is current.
-cudaError_t hpspmm_pool_malloc(int device, void** out, size_t bytes, size_t* got);
-void hpspmm_pool_free(int device, void* p, size_t bytes);
 
 // A named range around an entry point for timeline tools (NVTX 3, header-only: nothing to link, and a call is a
 // null-pointer test when no tool is attached).  The reference has no tracing beyond its event timer

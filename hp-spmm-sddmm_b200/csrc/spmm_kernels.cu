@@ -685,7 +685,7 @@ int hpspmm_plan_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const
   const size_t b_tiles = align_up((size_t)hpspmm_row_tiles(M) * 4, 256);
   p->bytes = 4 * b_int + b_cval + b_count + 2 * b_row + b_nz + b_rec;
   char* base = nullptr;
-  cudaError_t e = hpspmm_pool_malloc(ctx->device, (void**)&base, p->bytes, &p->block_bytes);
+  cudaError_t e = hpspmm_device_malloc((void**)&base, p->bytes);
   if (e != cudaSuccess) {
     delete p;
     return hpspmm_set_err(ctx, HPSPMM_ERR_OOM, "plan cudaMalloc", e);
@@ -723,7 +723,7 @@ int hpspmm_plan_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const
     e = cudaMemcpyAsync(&split, ctx->flag, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && st == HPSPMM_OK) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess || st != HPSPMM_OK) {
-    hpspmm_pool_free(ctx->device, base, p->block_bytes);
+    cudaFree(base);
     delete p;
     return e != cudaSuccess ? hpspmm_set_err(ctx, HPSPMM_ERR_CUDA, "plan build", e) : st;
   }
@@ -735,7 +735,7 @@ int hpspmm_plan_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const
 int hpspmm_plan_destroy(hpspmm_ctx* ctx, hpspmm_plan* plan) {
   if (!plan) return HPSPMM_OK;
   hpspmm_device_guard guard(plan->device);
-  hpspmm_pool_free(plan->device, plan->chunk_start, plan->block_bytes);
+  if (plan->chunk_start) cudaFree(plan->chunk_start);
   delete plan;
   (void)ctx;
   return HPSPMM_OK;

@@ -147,3 +147,57 @@ def test_chunks_larger_than_any_matrix(pkg, oracle, chunk):
                               out.data_ptr(), plan=p, opts=opts, stream=s)
                 assert float((out.double() - want).abs().max()) <= 2e-5      # 64 terms of at most 1, in 32 bits
             ctx.plan_destroy(plan)
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_plans_come_and_go_beside_a_capture_in_another_thread(pkg, oracle, mode):
+    """A plan destroyed and another built here while a thread records a graph of its own: neither disturbs the other."""
+    import threading
+
+    import torch
+    w = _Work(pkg, oracle, [3000] * 40, 20000, 64, 112)     # the plan's block is well over 256 KB
+    with pkg.Context(0) as ctx:
+        s = torch.cuda.current_stream().cuda_stream
+
+        def build():
+            return ctx.plan_create(w.M, w.nnz, w.rp.data_ptr(), w.K, pkg.Opts(chunk_nnz=32), N=w.N,
+                                   col_idx=w.ci.data_ptr(), stream=s)
+
+        plan = build()
+        x = torch.zeros(1000, device="cuda")
+        torch.cuda.synchronize()
+        begun, go_on, result = threading.Event(), threading.Event(), []
+
+        def record():
+            try:
+                graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+                with torch.cuda.stream(side):
+                    graph.capture_begin(capture_error_mode=mode)
+                    x.add_(1)
+                    begun.set()
+                    go_on.wait(30)
+                    x.add_(1)
+                    graph.capture_end()
+                graph.replay()
+                torch.cuda.synchronize()
+                result.append(float(x[0]))
+            except BaseException as e:      # noqa: B902 -- a thread's failure is the test's
+                result.append(e)
+            finally:
+                begun.set()
+
+        t = threading.Thread(target=record)
+        t.start()
+        begun.wait(30)
+        try:
+            ctx.plan_destroy(plan)
+            plan = build()
+        finally:
+            go_on.set()
+            t.join()
+        assert result == [2.0]
+        w.C.fill_(7.0)
+        ctx.spmm_csr(w.M, w.N, w.K, w.nnz, w.rp.data_ptr(), w.ci.data_ptr(), w.v.data_ptr(), w.B.data_ptr(),
+                     w.C.data_ptr(), plan=plan, stream=s)
+        w.check("product with the plan built meanwhile")
+        ctx.plan_destroy(plan)
