@@ -8,8 +8,8 @@ Three operators are registered under the namespace ``hpspmm`` (``layer_forward``
 ``layer_backward_features``, ``layer_backward_weights``) by csrc/torch_binding.cpp, with an autograd
 formula that chains them; the shape functions for tracing are below, so the layer can sit inside a
 compiled or exported module.  Every operator calls ``hpspmm_layer_*`` of libhpspmm.so on the current
-CUDA stream of the input's device; a CPU tensor is rejected (there is no fallback).  PyTorch supplies memory, streams and the autograd
-tape only.
+CUDA stream of the input's device; a CPU tensor is rejected (there is no fallback).  PyTorch supplies
+memory, streams and the autograd tape only.
 
 The reference has no framework binding; this is the caller either side of its products
 (test/test_all.cpp:63-107 issues them one at a time from a C++ driver).
@@ -18,6 +18,7 @@ import itertools
 import os
 
 import torch
+from torch.overrides import has_torch_function_variadic
 
 from . import PKG_DIR, Context, Layer, load_extension
 
@@ -83,7 +84,9 @@ class TorchLayer:
     def __call__(self, H, vals=None):
         if vals is None:
             vals = self.vals
-        if torch.compiler.is_compiling():
+        # tracers, tensor subclasses and function modes see the call through __torch_function__
+        if (torch.compiler.is_compiling() or not isinstance(H, torch.Tensor) or not isinstance(vals, torch.Tensor)
+                or has_torch_function_variadic(H, vals)):
             return layer_forward(H, vals, self.layer_id)
         return _C.layer_forward(H, vals, self.layer_id)    # the same operator without the Python dispatcher's share
 

@@ -129,3 +129,40 @@ def test_closing_under_calls(pkg):
     assert all("unknown or closed" in e for e in ends)
     with pytest.raises(RuntimeError, match="unknown or closed"):
         w.layer(w.H)
+
+
+def test_tracers_modes_and_subclasses_see_the_operator(work):
+    import torch
+    from torch.overrides import TorchFunctionMode
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.w = torch.nn.Parameter(work.v.clone())
+
+        def forward(self, h):
+            return work.layer(h * 2, self.w)
+
+    traced = torch.fx.symbolic_trace(Net())
+    assert any("layer_forward" in str(n.target) for n in traced.graph.nodes)
+    assert _close(traced(work.H).detach(), 2 * work.product(work.v, work.H))
+
+    seen = []
+
+    class Mode(TorchFunctionMode):
+        def __torch_function__(self, f, types, args=(), kwargs=None):
+            seen.append(str(f))
+            return f(*args, **(kwargs or {}))
+
+    with Mode():
+        work.layer(work.H)
+    assert any("layer_forward" in s for s in seen)
+
+    class Sub(torch.Tensor):
+        pass
+
+    assert type(work.layer(work.H.as_subclass(Sub))) is Sub
+    assert type(work.layer(work.H, work.v.as_subclass(Sub))) is Sub
+    assert type(work.layer(torch.nn.Parameter(work.H))) is torch.Tensor
+    with pytest.raises(RuntimeError):
+        work.layer(work.H.cpu().numpy())
