@@ -208,7 +208,8 @@ def load_native():
         mod = load_extension("_hpspmm_native", NATIVE_PATH)
         mod.bind(*[ctypes.cast(getattr(lib, "hpspmm_" + f), c_void_p).value
                    for f in ("spmm_csr_f32", "spmm_coo_f32", "sddmm_csr_f32", "fill_f32", "layer_forward",
-                             "layer_backward_features", "layer_backward_weights")])
+                             "layer_backward_features", "layer_backward_weights")],
+                 np.ndarray, DeviceBuffer, Opts)
         _native = mod
     return _native
 
