@@ -996,6 +996,12 @@ static int host_products_in_turn(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t 
   return HPSPMM_OK;
 }
 
+static int first_pipe_stream(hpspmm_ctx* ctx) {   // the device is current
+  if (!ctx->pipe_streams[0])
+    HPSPMM_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->pipe_streams[0], cudaStreamNonBlocking));
+  return HPSPMM_OK;
+}
+
 // Up to here the dense operands travel whole, one after the other: at 55 GB/s they take 75 us, and a slab of the
 // pipeline costs about 15 us to issue.
 static const int64_t kHostInTurnBytes = 4 << 20;
@@ -1058,8 +1064,8 @@ int hpspmm_spmm_csr_f32_host_multi(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
   if (dense <= kHostInTurnBytes) {
     for (int i = 0; i < n_products; ++i) slabs[i] = host_slab{Bs[i], Cs[i], Ks[i], Ks[i]};
     hpspmm_device_guard guard(ctx->device);
-    if (!ctx->pipe_streams[0])
-      HPSPMM_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->pipe_streams[0], cudaStreamNonBlocking));
+    const int st = first_pipe_stream(ctx);
+    if (st != HPSPMM_OK) return st;
     return host_products_in_turn(ctx, M, N, nnz, row_ptr, col_idx, vals, slabs, n_products, opts, ctx->pipe_streams[0]);
   }
   // Order of the products.  Downloads can start only after the first slab has been uploaded and multiplied, and the
@@ -1097,10 +1103,16 @@ int hpspmm_spmm_csr_f32_host(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t K, i
   HPSPMM_REQUIRE(ctx, M == 0 || C != nullptr, "null output");
   if (M == 0) return HPSPMM_OK;
   hpspmm_device_guard guard(ctx->device);
+  int st = HPSPMM_OK;
   const int algo = opts ? opts->algo : HPSPMM_ALGO_AUTO;
-  if (nnz > 0 && N > 0 && K >= 64 && K % 32 == 0 && algo != HPSPMM_ALGO_ROW_SPLIT && 4 * K * (M + N) > kHostInTurnBytes)
-    return host_product_slabs(ctx, M, N, K, nnz, row_ptr, col_idx, vals, B, C, opts);
   const host_slab whole = {B, C, K, K};
+  if (nnz > 0 && N > 0 && K >= 64 && K % 32 == 0 && algo != HPSPMM_ALGO_ROW_SPLIT) {
+    if (4 * K * (M + N) > kHostInTurnBytes)
+      return host_product_slabs(ctx, M, N, K, nnz, row_ptr, col_idx, vals, B, C, opts);
+    // these widths run beside the default stream, whatever their size
+    if ((st = first_pipe_stream(ctx)) != HPSPMM_OK) return st;
+    return host_products_in_turn(ctx, M, N, nnz, row_ptr, col_idx, vals, &whole, 1, opts, ctx->pipe_streams[0]);
+  }
   return host_products_in_turn(ctx, M, N, nnz, row_ptr, col_idx, vals, &whole, 1, opts, /*default stream*/ 0);
 }
 

@@ -228,6 +228,35 @@ def test_host_buffer_entry_point(gpu_ctx, pkg, oracle, K):
     check_against_f64(C, ref, abs_sum, "host entry")
 
 
+@pytest.mark.parametrize("K", [64, 128])
+@pytest.mark.parametrize("several", [False, True])
+def test_host_entry_does_not_wait_for_the_default_stream(pkg, oracle, K, several):
+    """Widths of the slab pipeline run on streams of the context's own, small operands included."""
+    torch = pytest.importorskip("torch")
+    g = pkg.gen_rmat(9, 8, seed=4)
+    B = pkg.host_fill_uniform(g["N"] * K, 4, 1, -1.0, 1.0).reshape(g["N"], K)
+    C = np.full((g["M"], K), np.nan, dtype=np.float32)
+    with pkg.Context(0) as ctx:
+        def call():
+            if several:
+                ctx.spmm_csr_host_multi(g["M"], g["N"], g["nnz"], g["row_ptr"], g["col_idx"], g["vals"], [K], [B], [C])
+            else:
+                ctx.spmm_csr_host(g["M"], g["N"], K, g["nnz"], g["row_ptr"], g["col_idx"], g["vals"], B, C)
+        call()                                                      # allocates what the next call needs
+        C[:] = np.nan
+        torch.cuda.synchronize()
+        busy = torch.cuda.Event()
+        with torch.cuda.stream(torch.cuda.default_stream()):
+            torch.cuda._sleep(1_000_000_000)                        # half a second and more
+            busy.record()
+        call()
+        still_busy = not busy.query()
+        torch.cuda.synchronize()
+        assert still_busy
+    ref, abs_sum = oracle.spmm_f64(g["row_ptr"], g["col_idx"], g["vals"], B)
+    check_against_f64(C, ref, abs_sum, "host entry beside a busy default stream")
+
+
 def test_argument_errors_return_codes(gpu_ctx, pkg):
     lib = pkg.load_library()
     d = gpu_ctx.alloc((64,), np.float32)
