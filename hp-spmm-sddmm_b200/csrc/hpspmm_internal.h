@@ -68,6 +68,10 @@ struct hpspmm_plan {
   size_t bytes;
 };
 
+// Whether the rows of the plan's matrix are of even length: few of them are longer than a chunk.  A power-law graph has
+// a chunk in two to a chunk in four beginning inside a row, uniform rows have none.
+static inline bool hpspmm_even_rows(const hpspmm_plan* p) { return p->n_split_chunks * 8 < p->n_chunks; }
+
 // What the CSR product kernels are launched with.
 //   rec, 32 bytes per slot of the schedule: {n0, ri, row, row_end} {chunk, row_start, n1, -}: entries [n0, n1) of the
 //   chunk, the row holding entry n0 with its bounds and its position in the list of rows.  One aligned load gives a

@@ -419,6 +419,22 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
 #undef GO_SERIAL
 }
 
+// Up to about two waves of resident warps (80 chunks per SM) a call takes the shapes for few chunks -- except that at 32,
+// 64 and 128 columns the SERIAL kernel of a fixed width is ahead from some number of chunks on.  With rows of even length
+// no chunk has many more row ends to wait at than the others; a power-law graph (even: false, also where there is no plan
+// to tell) needs more chunks to cover its worst one.  Uniform rows, shapes for few chunks -> SERIAL in us:
+//   K = 32:  300 K entries 8.3 -> 8.3, 600 K 14.4 -> 12.4, 1.3 M 24.7 -> 20.7, 1.5 M 20.9 -> 17.7; rows of 4 or 5 entries
+//            lose (400 K 13.8 -> 15.3, 1 M 23.2 -> 27.6), as does a power-law graph at any size (1.5 M 20.6 -> 23.7)
+//   K = 64:  150 K 10.3 -> 8.3, 1.3 M 37.0 -> 30.8, 1.5 M 32.9 -> 26.7; 67.6 K 8.3 -> 8.3; power-law, 1 M 26.7 -> 28.8
+//   K = 128: 400 K 24.7 -> 20.6, 1 M 49.6 -> 43.0, 1.5 M 59.5 -> 49.2, 3 M 135 -> 109; 300 K 16.3 -> 18.5;
+//            power-law, 1 M 43.5 -> 40.9, 3 M 120 -> 94, but 600 K 26.7 -> 36.9
+bool serial_when_few(int64_t K, int64_t n_chunks, bool long_rows, bool even, int sm_count) {
+  if (K == 32) return even && long_rows && n_chunks > sm_count * 30;
+  if (K == 64) return even && n_chunks > sm_count * 12;
+  if (K == 128) return n_chunks > sm_count * (even ? 20 : 48);
+  return false;
+}
+
 }  // namespace
 
 extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int64_t N,
@@ -445,13 +461,15 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   const int hint_mode = opts ? opts->b_l2_hint : 0;
   const bool hint = hint_mode == 2 || (hint_mode == 0 && K >= 64);
   sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, false, false, nnz >= 10 * M, col_idx, X, Y, out_vals, nullptr, nullptr};
+  bool even = false;   // rows are known to be of even length
   if (plan) {
     HPSPMM_REQUIRE(ctx, plan->M == M && plan->nnz == nnz, "plan built for another matrix");
     HPSPMM_REQUIRE(ctx, plan->device == ctx->device, "plan built on another device");
     a.n_chunks = (int)plan->n_chunks;
     // The average says nothing about a skewed matrix, most of whose entries lie in long rows; there many rows are split.
     // (power-law graph of 1 M rows, 5 M entries, K = 96: serial 175 us, mask 230 us)
-    a.long_rows = a.long_rows || plan->n_split_chunks * 8 >= plan->n_chunks;
+    even = hpspmm_even_rows(plan);
+    a.long_rows = a.long_rows || !even;
     a.rec = plan->rec;
     a.nz = plan->nz;
   } else {
@@ -478,7 +496,7 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   for (a.off = 0; a.off < a.K; a.off += a.cols) {
     a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
     hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hint);
-    sh.lat = a.n_chunks <= ctx->sm_count * 80;   // up to about two waves of resident warps
+    sh.lat = a.n_chunks <= ctx->sm_count * 80 && !serial_when_few(K, a.n_chunks, nnz >= 10 * M, even, ctx->sm_count);
     if (sh.VEC == 4 && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;
     const int st = launch_sddmm_shape(ctx, a, sh, s);
     if (st != HPSPMM_OK) return st;

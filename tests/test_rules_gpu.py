@@ -1,0 +1,62 @@
+"""Rules that choose a kernel by the number of chunks, the evenness of the rows and the width: both sides of every line,
+with a plan of rows of even length, a plan of rows longer than a chunk, and without a plan (needs a B200)."""
+import numpy as np
+import pytest
+
+from helpers import check_against_f64, random_csr
+
+pytestmark = pytest.mark.gpu
+
+CHUNK = 32
+SMS = 148     # the lines lie at multiples of the number of SMs
+
+
+def _matrix(n_chunks, even, N=4000, seed=0):
+    """CSR of about n_chunks chunks of 32 entries: rows of 4 to 28 entries and empty ones, or some of them far longer
+    than a chunk (every chunk of those begins inside a row)."""
+    rng = np.random.default_rng(seed + n_chunks)
+    nnz = n_chunks * CHUNK - 5
+    degrees = []
+    if not even:
+        degrees = [900] * max(1, nnz // 1800) + [0, 33, 64]
+    left = nnz - sum(degrees)
+    while left > 0:
+        d = int(rng.integers(4, 29)) if rng.random() > 0.05 else 0
+        d = min(d, left)
+        degrees.append(d)
+        left -= d
+    order = rng.permutation(len(degrees))
+    return random_csr(len(degrees), N, [degrees[i] for i in order], seed=seed)
+
+
+def _operands(pkg, rp, K, N=4000):
+    M = len(rp) - 1
+    X = pkg.host_fill_uniform(M * K, 7, 1, -1.0, 1.0).reshape(M, K)
+    Y = pkg.host_fill_uniform(N * K, 7, 2, -1.0, 1.0).reshape(N, K)
+    return M, X, Y
+
+
+@pytest.mark.parametrize("K", [32, 64, 128])
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("per_sm", [12, 20, 30, 48, 80])
+def test_sddmm_of_fixed_widths_with_few_chunks(gpu_ctx, pkg, oracle, K, even, per_sm):
+    ctx, N = gpu_ctx, 4000
+    assert ctx.lib.hpspmm_ctx_sm_count(ctx.handle) == SMS
+    opts = pkg.Opts(chunk_nnz=CHUNK)
+    for n_chunks in (per_sm * SMS, per_sm * SMS + 1):
+        rp, ci, _ = _matrix(n_chunks, even)
+        M, X, Y = _operands(pkg, rp, K)
+        nnz = len(ci)
+        ref, abs_sum = oracle.sddmm_f64(rp, ci, X, Y)
+        d_rp, d_ci, d_X, d_Y = (ctx.upload(x) for x in (rp, ci, X, Y))
+        d_out = ctx.alloc((nnz,), np.float32)
+        plan = ctx.plan_create(M, nnz, d_rp, K, opts, N=N, col_idx=d_ci)
+        info = ctx.plan_info(plan)
+        assert info["n_chunks"] == n_chunks and (info["n_split_chunks"] * 8 < n_chunks) == even
+        for p in (plan, None):
+            ctx.fill(d_out, nnz, 7.0)
+            ctx.sddmm_csr(M, N, K, nnz, d_rp, d_ci, d_X, d_Y, d_out, plan=p, opts=opts)
+            check_against_f64(d_out.to_host(), ref, abs_sum, "sddmm K=%d chunks=%d plan=%s" % (K, n_chunks, p is not None))
+        ctx.plan_destroy(plan)
+        for b in (d_rp, d_ci, d_X, d_Y, d_out):
+            b.free()
