@@ -263,8 +263,8 @@ extern "C" int hpspmm_spmm_coo_f32(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
   coo_args a = {nnz_padded, S, (int)K, 0, 0, row_idx, col_idx, vals, B, C};
   const int VEC = hpspmm_vector_width(K, (uintptr_t)B | (uintptr_t)C);
   for (a.off = 0; a.off < a.K; a.off += a.cols) {   // every slab accumulates into its own columns
-    a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
-    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, false);
+    a.cols = hpspmm_launch_cols(a.K, a.off, hpspmm_widest_slab(VEC));
+    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hpspmm_widest_slab(VEC), false);
     // Three vectors per lane as in the CSR product, but only from 33 vectors on: every run of equal rows is combined over
     // the groups before it goes to C, and over four groups that costs more than the idle lanes of one (1 M entries of a
     // power-law graph, K = 96: 49.0 -> 56.0 us).  With few warps the exchange is not covered either (100 K entries,

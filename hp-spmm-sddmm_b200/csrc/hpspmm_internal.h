@@ -102,7 +102,7 @@ struct hpspmm_spmm_shape {
 };
 // widest vector the rows of the dense operands keep aligned; addresses: bitwise or of the operands' addresses
 int hpspmm_vector_width(int64_t K, uintptr_t addresses);
-hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, bool hint);
+hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, int widest, bool hint);
 // Widest slab one shape covers (four vectors per lane, eight of 4 bytes).  A wider product runs as that many full
 // slabs and one launch for the rest, so that only the last vector of a lane can ever lie outside a slab.
 static inline int hpspmm_widest_slab(int VEC) { return VEC == 1 ? 256 : 128 * VEC; }
@@ -111,8 +111,8 @@ static inline bool hpspmm_shape_covers(int VEC, int W, int R, int cols) {
   const int cw = VEC * W * R, last = cols % cw == 0 ? cw : cols % cw;
   return cols > 0 && last > VEC * W * (R - 1);
 }
-static inline int hpspmm_launch_cols(int VEC, int K, int off) {
-  const int widest = hpspmm_widest_slab(VEC), left = K - off;
+static inline int hpspmm_launch_cols(int K, int off, int widest) {
+  const int left = K - off;
   return left < widest ? left : left / widest * widest;
 }
 // triples per warp of the COO product

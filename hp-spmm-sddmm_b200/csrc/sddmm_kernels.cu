@@ -494,8 +494,8 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   a.waves = a.n_chunks > ctx->sm_count * 160;
   const int VEC = hpspmm_vector_width(K, (uintptr_t)X | (uintptr_t)Y);
   for (a.off = 0; a.off < a.K; a.off += a.cols) {
-    a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
-    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hint);
+    a.cols = hpspmm_launch_cols(a.K, a.off, hpspmm_widest_slab(VEC));
+    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hpspmm_widest_slab(VEC), hint);
     sh.lat = a.n_chunks <= ctx->sm_count * 80 && !serial_when_few(K, a.n_chunks, nnz >= 10 * M, even, ctx->sm_count);
     if (sh.VEC == 4 && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;
     const int st = launch_sddmm_shape(ctx, a, sh, s);

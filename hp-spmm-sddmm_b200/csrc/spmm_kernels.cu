@@ -542,12 +542,12 @@ int hpspmm_vector_width(int64_t K, uintptr_t addresses) {
   return (K & 3) == 0 ? 4 : ((K & 1) == 0 && (addresses & 7) == 0 ? 2 : 1);
 }
 
-hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, bool hint) {
+hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, int widest, bool hint) {
   hpspmm_spmm_shape sh;
   sh.VEC = VEC;
   sh.hint = hint;
   sh.lat = false;
-  if (cols > hpspmm_widest_slab(VEC)) cols = hpspmm_widest_slab(VEC);
+  if (cols > widest) cols = widest;
   const int vecs = (int)((cols + VEC - 1) / VEC);
   sh.W = VEC == 1 ? (vecs <= 1 ? 1 : 4) : 2;
   while (sh.W < 32 && sh.W < vecs) sh.W *= 2;
@@ -585,15 +585,33 @@ int check_spmm_args(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t nn
   return HPSPMM_OK;
 }
 
+// Widest slab of a product's columns.  With wide vectors one pass over up to 512 columns holds two to four vectors of a
+// row per lane, so only one or two entries are in flight, and all of B competes for the L2 cache.  Passes of 128 columns
+// read the small sparse operand again instead, keep four entries in flight and need a part of B at a time.
+// One pass -> passes in us:
+//   uniform rows:     1 M entries, 62.5 K rows, K = 448 202 -> 129;  2 M, 200 K rows, K = 256 236 -> 195, 320 347 -> 258,
+//                     448 554 -> 364;  4 M, 250 K rows, K = 256 483 -> 417, 320 685 -> 488, 512 1189 -> 798
+//   power-law graphs: 1.2 M, 60 K rows, K = 392 136 -> 141, 512 148 -> 142;  4 M, 250 K rows, K = 392 479 -> 446, 512 548 ->
+//                     501, and without a plan 590 -> 557; below 384 columns about level with a plan, and without one, where the
+//                     chunks are not ordered by cost and every pass ends on its own last ones, behind (4 M, K = 300 +6 %)
+// 300 K entries, K = 512: 37 -> 47, so with few chunks one pass stays.
+int widest_slab(const hpspmm_ctx* ctx, int VEC, int64_t K, int64_t n_chunks, bool even) {
+  if (VEC == 4 && ((K > 384 && n_chunks > ctx->sm_count * 48ll) || (K >= 256 && even && n_chunks > ctx->sm_count * 64ll)))
+    return 128;
+  return hpspmm_widest_slab(VEC);
+}
+
 // shared_counters: the scratch holds one counter per chunk, so the slabs of a wide product run one after the other
-int launch_spmm(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool hint, bool shared_counters, cudaStream_t s) {
+// even: the rows are known to be of even length (hpspmm_even_rows)
+int launch_spmm(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool hint, bool even, bool shared_counters, cudaStream_t s) {
   const int VEC = hpspmm_vector_width(a.K, (uintptr_t)a.B | (uintptr_t)a.C);
+  const int widest = widest_slab(ctx, VEC, a.K, a.n_chunks, even);
   int32_t* counter = a.counter;
   a.keep_b = hint ? 1 : 0;
   for (a.off = 0; a.off < a.K; a.off += a.cols) {
-    a.cols = hpspmm_launch_cols(VEC, a.K, a.off);
+    a.cols = hpspmm_launch_cols(a.K, a.off, widest);
     if (!shared_counters) a.counter = counter + (int64_t)(a.off / 32) * a.n_chunks;
-    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hint);
+    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, widest, hint);
     // Few chunks: registers are plenty, so a warp keeps 8 to 32 gather steps in flight instead of 4 (the same order of
     // additions).  67.6 K entries in chunks of 64: 6.1 -> 5.6 us at K = 64, 9.1 -> 7.2 us at K = 128; with more chunks
     // than these builds have resident warps they lose (300 K entries, K = 64: 8.3 -> 10.5 us).
@@ -755,7 +773,7 @@ int hpspmm_spmm_kernel_signature(const hpspmm_plan* plan, int64_t K, int32_t b_l
   if (!buf || len == 0 || K < 1) return HPSPMM_ERR_INVALID;
   const int64_t nnz = plan ? plan->nnz : 0;
   const hpspmm_opts o = {0, 0, b_l2_hint, 0};
-  const hpspmm_spmm_shape sh = hpspmm_choose_shape(hpspmm_vector_width(K, 0), K, gather_hint(K, &o));
+  const hpspmm_spmm_shape sh = hpspmm_choose_shape(hpspmm_vector_width(K, 0), K, hpspmm_widest_slab(hpspmm_vector_width(K, 0)), gather_hint(K, &o));
   snprintf(buf, len, "spmm_warp_kernel<%d,%d,%d> K=%lld split=%d hint=%d chunk_nnz=%d", sh.VEC, sh.W, sh.R, (long long)K,
            sh.lat ? 1 : 0, sh.hint ? 1 : 0, plan ? (int)plan->chunk_nnz : (int)hpspmm_default_chunk_nnz(K, nnz));
   return HPSPMM_OK;
@@ -812,7 +830,7 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
     }
     a.n_chunks = (int)plan->n_chunks, a.S = plan->chunk_nnz;
     a.rec = plan->rec, a.nz = plan->nz, a.carry = plan->carry_val, a.counter = plan->run_counter;
-    return launch_spmm(ctx, a, hint, false, s);
+    return launch_spmm(ctx, a, hint, hpspmm_even_rows(plan), false, s);
   }
   const int32_t S = planless_chunk_nnz(K, nnz, opts);
   const int64_t n_chunks = (nnz + S - 1) / S;
@@ -833,17 +851,17 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
                                 hpspmm_structure_tables{}, s, a.counter, lay.n_counter);
     if (st != HPSPMM_OK) return st;
     a.rec = rec, a.nz = nz;
-    return launch_spmm(ctx, a, hint, false, s);
+    return launch_spmm(ctx, a, hint, false, false, s);
   }
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
   if (capture != cudaStreamCaptureStatusNone) {
     HPSPMM_CUDA_TRY(ctx, cudaMemsetAsync(a.counter, 0, (size_t)lay.n_counter * 4, s));
-    return launch_spmm(ctx, a, hint, false, s);
+    return launch_spmm(ctx, a, hint, false, false, s);
   }
   st = hpspmm_take_counters(ctx, lay.n_counter, s, &a.counter, &a.clear, &a.n_clear);
   if (st != HPSPMM_OK) return st;
-  st = launch_spmm(ctx, a, hint, false, s);
+  st = launch_spmm(ctx, a, hint, false, false, s);
   hpspmm_counters_used(ctx, lay.n_counter, st == HPSPMM_OK);
   return st;
 }
@@ -1243,7 +1261,7 @@ extern "C" int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
   a.M = (int)M, a.K = (int)K, a.n_chunks = (int)n_chunks, a.S = S;
   a.row_ptr = row_ptr, a.col_idx = col_idx, a.vals = vals, a.B = B, a.C = C;
   a.carry = (float*)(state.base + b_int), a.counter = run_counter;
-  st = launch_spmm(&local, a, gather_hint(K, nullptr), /*shared_counters=*/true, s);
+  st = launch_spmm(&local, a, gather_hint(K, nullptr), /*even=*/false, /*shared_counters=*/true, s);
   if (st != HPSPMM_OK) write_err(err_buf, err_len, local.err);
   return st;
 }

@@ -3,7 +3,7 @@ with a plan of rows of even length, a plan of rows longer than a chunk, and with
 import numpy as np
 import pytest
 
-from helpers import check_against_f64, random_csr
+from helpers import check_against_f64, guarded_output, random_csr
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +60,34 @@ def test_sddmm_of_fixed_widths_with_few_chunks(gpu_ctx, pkg, oracle, K, even, pe
         ctx.plan_destroy(plan)
         for b in (d_rp, d_ci, d_X, d_Y, d_out):
             b.free()
+
+
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("K", [252, 256, 260, 288, 384, 388, 448, 512, 640])
+def test_wide_products_in_one_pass_and_in_several(gpu_ctx, pkg, oracle, K, even):
+    """Passes of 128 columns beyond 384 columns, and from 256 on where the rows are even: the last pass is as narrow as
+    the width leaves it."""
+    ctx, N = gpu_ctx, 4000
+    opts = pkg.Opts(chunk_nnz=CHUNK)
+    for per_sm in (48, 64):
+        for n_chunks in (per_sm * SMS, per_sm * SMS + 1):
+            rp, ci, v = _matrix(n_chunks, even)
+            M, nnz = len(rp) - 1, len(ci)
+            B = pkg.host_fill_uniform(N * K, 8, 1, -1.0, 1.0).reshape(N, K)
+            ref, abs_sum = oracle.spmm_f64(rp, ci, v, B)
+            d_rp, d_ci, d_v, d_B = (ctx.upload(x) for x in (rp, ci, v, B))
+            buf, c_ptr, read = guarded_output(ctx, (M, K))
+            plan = ctx.plan_create(M, nnz, d_rp, K, opts, N=N, col_idx=d_ci)
+            assert ctx.plan_info(plan)["n_chunks"] == n_chunks
+            for p in (plan, None):
+                passes = (K > 384 and n_chunks > 48 * SMS) or (K >= 256 and even and p is not None and n_chunks > 64 * SMS)
+                before = ctx.launch_count()
+                ctx.spmm_csr(M, N, K, nnz, d_rp, d_ci, d_v, d_B, c_ptr, plan=p, opts=opts)
+                launches = ctx.launch_count() - before - (0 if p is not None else 2 if n_chunks > 40 * SMS else 0)
+                widest = 128 if passes else 512
+                assert launches == (K >= widest) + (K % widest > 0)
+                ctx.stream_sync()
+                check_against_f64(read(), ref, abs_sum, "K=%d chunks=%d plan=%s" % (K, n_chunks, p is not None))
+            ctx.plan_destroy(plan)
+            for b in (d_rp, d_ci, d_v, d_B, buf):
+                b.free()
