@@ -305,18 +305,15 @@ struct sddmm_args {
   const int2* nz;
 };
 
-// one launch per slab of the width: the first writes the partial dot products, the others add theirs
+// one slab of the width: the first writes the partial dot products, the others add theirs
 template <int VEC, int W, int R, int U, int KS, bool HINT, int MINB, bool SERIAL>
 int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
-  constexpr int BT = 64, CW = VEC * W * R;
+  constexpr int BT = 64;
   const unsigned grid = (unsigned)((a.n_chunks + BT / 32 - 1) / (BT / 32));
-  if (!hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
-  for (int off = a.off; off < a.off + a.cols; off += CW) {
-    const int left = a.off + a.cols - off;
-    sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, SERIAL><<<grid, BT, 0, s>>>(
-        a.n_chunks, a.K, off, left < CW ? left : CW, off > 0 ? 1 : 0, a.keep_y, a.col_idx, a.X, a.Y, a.out, a.rec, a.nz);
-    ctx->launches++;
-  }
+  if (a.cols > VEC * W * R || !hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
+  sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, SERIAL><<<grid, BT, 0, s>>>(
+      a.n_chunks, a.K, a.off, a.cols, a.off > 0 ? 1 : 0, a.keep_y, a.col_idx, a.X, a.Y, a.out, a.rec, a.nz);
+  ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;
 }
@@ -419,6 +416,24 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
 #undef GO_SERIAL
 }
 
+// Widest slab of the SDDMM's columns.  289 to 512 columns in one pass are three or four vectors of 32 lanes with one or two
+// entries in flight; two passes of at most 256 columns run the shapes of 16 lanes, and the second adds its part.  A short
+// rest is a cheap second pass on any graph; a long one pays on rows of even length only, once there are enough chunks or
+// Y is too large for the L2 cache anyway.  One pass -> two in us:
+//   K = 288: uniform, 1 M entries 137 -> 127, 2.5 M 322 -> 304, 4 M 671 -> 600;  power-law, 4 M 411 -> 329
+//   K = 384: uniform, 2 M 416 -> 391, 4 M in 100 K rows 612 -> 484;  power-law, 4 M without a plan +10 %
+//   K = 448: uniform, 2.5 M 515 -> 463, 4 M 1005 -> 896, but 1.5 M, whose Y fits the cache, 210 -> 220
+//   K = 512: uniform, 2 M 566 -> 513, 4 M 1123 -> 998
+int widest_sddmm_slab(const hpspmm_ctx* ctx, int VEC, int64_t N, int64_t K, int64_t n_chunks, bool even) {
+  if (VEC == 4 && K > 256 && K <= 512) {
+    if (K <= 288 && n_chunks > ctx->sm_count * 48ll) return 256;
+    const bool many = n_chunks > ctx->sm_count * 80ll;
+    const bool large = n_chunks > ctx->sm_count * 48ll && 4 * N * K > ctx->l2_bytes;
+    if (K >= 320 && even && (many || large)) return 256;
+  }
+  return hpspmm_widest_slab(VEC);
+}
+
 // Up to about two waves of resident warps (80 chunks per SM) a call takes the shapes for few chunks -- except that at 32,
 // 64 and 128 columns the SERIAL kernel of a fixed width is ahead from some number of chunks on.  With rows of even length
 // no chunk has many more row ends to wait at than the others; a power-law graph (even: false, also where there is no plan
@@ -493,9 +508,10 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   a.few = a.n_chunks <= ctx->sm_count * 32;
   a.waves = a.n_chunks > ctx->sm_count * 160;
   const int VEC = hpspmm_vector_width(K, (uintptr_t)X | (uintptr_t)Y);
+  const int widest = widest_sddmm_slab(ctx, VEC, N, K, a.n_chunks, even);
   for (a.off = 0; a.off < a.K; a.off += a.cols) {
-    a.cols = hpspmm_launch_cols(a.K, a.off, hpspmm_widest_slab(VEC));
-    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, hpspmm_widest_slab(VEC), hint);
+    a.cols = a.K - a.off < widest ? a.K - a.off : widest;
+    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, widest, hint);
     sh.lat = a.n_chunks <= ctx->sm_count * 80 && !serial_when_few(K, a.n_chunks, nnz >= 10 * M, even, ctx->sm_count);
     if (sh.VEC == 4 && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;
     const int st = launch_sddmm_shape(ctx, a, sh, s);

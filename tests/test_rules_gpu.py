@@ -91,3 +91,34 @@ def test_wide_products_in_one_pass_and_in_several(gpu_ctx, pkg, oracle, K, even)
             ctx.plan_destroy(plan)
             for b in (d_rp, d_ci, d_v, d_B, buf):
                 b.free()
+
+
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("K", [256, 260, 288, 292, 320, 448, 512, 516])
+def test_wide_sddmm_in_one_pass_and_in_several(gpu_ctx, pkg, oracle, K, even):
+    """Passes of 256 columns where they are ahead; the second adds to what the first has written."""
+    ctx = gpu_ctx
+    opts = pkg.Opts(chunk_nnz=CHUNK)
+    l2 = ctx.lib.hpspmm_ctx_l2_bytes(ctx.handle)
+    for per_sm, N in ((48, 4000), (80, 4000), (48, 140000)):
+        for n_chunks in (per_sm * SMS, per_sm * SMS + 1):
+            rp, ci, _ = _matrix(n_chunks, even, N=N)
+            M, X, Y = _operands(pkg, rp, K, N)
+            nnz = len(ci)
+            ref, abs_sum = oracle.sddmm_f64(rp, ci, X, Y)
+            d_rp, d_ci, d_X, d_Y = (ctx.upload(x) for x in (rp, ci, X, Y))
+            d_out = ctx.alloc((nnz,), np.float32)
+            plan = ctx.plan_create(M, nnz, d_rp, K, opts, N=N, col_idx=d_ci)
+            for p in (plan, None):
+                two = 256 < K <= 288 and n_chunks > 48 * SMS
+                if 320 <= K <= 512 and even and p is not None:
+                    two = n_chunks > 80 * SMS or (n_chunks > 48 * SMS and 4 * N * K > l2)
+                before = ctx.launch_count()
+                ctx.fill(d_out, nnz, 7.0)
+                ctx.sddmm_csr(M, N, K, nnz, d_rp, d_ci, d_X, d_Y, d_out, plan=p, opts=opts)
+                launches = ctx.launch_count() - before - 1 - (0 if p is not None else 2)
+                assert launches == (2 if two else -(-K // 512))
+                check_against_f64(d_out.to_host(), ref, abs_sum, "K=%d chunks=%d plan=%s" % (K, n_chunks, p is not None))
+            ctx.plan_destroy(plan)
+            for b in (d_rp, d_ci, d_X, d_Y, d_out):
+                b.free()
