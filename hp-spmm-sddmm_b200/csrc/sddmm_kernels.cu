@@ -337,7 +337,7 @@ int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
 // Which of them are SERIAL: 16-byte vectors fill the registers that the other path needs (K = 96 424 against 477 us); with
 // narrower vectors it costs more than it saves except where noted by the shape.  Where rows are short the waits do not
 // pay (uniform rows of 4 entries, K = 100: 176 against 159 us; of 8: 130 against 119; of 12: 110 against 105, but K = 96 92
-// against 103 and K = 160 158 against 185): from 10 entries per row on, or on matrices with many split rows.  Where the
+// against 103 and K = 160 158 against 185): rows_are_long.  Where the
 // gain is small it also takes enough chunks to cover the waits (12,500 chunks: K = 48 38.9 against 41.4 us, K = 62 45.7
 // against 55.1; 31,000: 105 against 97 and 110 against 97).
 int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_shape& sh, cudaStream_t s) {
@@ -416,6 +416,19 @@ int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_s
 #undef GO_SERIAL
 }
 
+// Whether the rows are long enough on average for the SERIAL shapes.  At 129 to 160 columns they pay early (uniform rows of
+// 9 entries, K = 160: 435 -> 401 us; of 5 about level; of 4: 519 -> 534).  Without a plan nothing tells a skewed matrix, most
+// of whose entries lie in long rows whatever the average, so there the line lies where a uniform one loses little:
+//   power-law, 4 M entries in 1 M rows: K = 96 273 -> 233, 160 420 -> 333, 192 451 -> 356 us
+//   uniform, the same sizes:            K = 96 322 -> 331, 160 544 -> 554, 192 609 -> 643 us; rows of 8, K = 160 224 -> 200 us
+bool rows_are_long(int VEC, int64_t M, int64_t K, int64_t nnz, bool has_plan) {
+  if (VEC == 4) {
+    if (!has_plan && ((K > 64 && K <= 96) || (K > 128 && K <= 192))) return nnz >= 4 * M;
+    if (K > 128 && K <= 160) return nnz >= 5 * M;
+  }
+  return nnz >= 10 * M;
+}
+
 // Widest slab of the SDDMM's columns.  289 to 512 columns in one pass are three or four vectors of 32 lanes with one or two
 // entries in flight; two passes of at most 256 columns run the shapes of 16 lanes, and the second adds its part.  A short
 // rest is a cheap second pass on any graph; a long one pays on rows of even length only, once there are enough chunks or
@@ -475,7 +488,9 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   cudaStream_t s = (cudaStream_t)stream;
   const int hint_mode = opts ? opts->b_l2_hint : 0;
   const bool hint = hint_mode == 2 || (hint_mode == 0 && K >= 64);
-  sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, false, false, nnz >= 10 * M, col_idx, X, Y, out_vals, nullptr, nullptr};
+  sddmm_args a = {0, (int)K, 0, 0, hint ? 1 : 0, false, false, false, col_idx, X, Y, out_vals, nullptr, nullptr};
+  const int VEC = hpspmm_vector_width(K, (uintptr_t)X | (uintptr_t)Y);
+  a.long_rows = rows_are_long(VEC, M, K, nnz, plan != nullptr);
   bool even = false;   // rows are known to be of even length
   if (plan) {
     HPSPMM_REQUIRE(ctx, plan->M == M && plan->nnz == nnz, "plan built for another matrix");
@@ -507,7 +522,6 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
   }
   a.few = a.n_chunks <= ctx->sm_count * 32;
   a.waves = a.n_chunks > ctx->sm_count * 160;
-  const int VEC = hpspmm_vector_width(K, (uintptr_t)X | (uintptr_t)Y);
   const int widest = widest_sddmm_slab(ctx, VEC, N, K, a.n_chunks, even);
   for (a.off = 0; a.off < a.K; a.off += a.cols) {
     a.cols = a.K - a.off < widest ? a.K - a.off : widest;

@@ -122,3 +122,39 @@ def test_wide_sddmm_in_one_pass_and_in_several(gpu_ctx, pkg, oracle, K, even):
             ctx.plan_destroy(plan)
             for b in (d_rp, d_ci, d_X, d_Y, d_out):
                 b.free()
+
+
+@pytest.mark.parametrize("K", [68, 96, 100, 132, 164, 196])
+def test_sddmm_on_both_sides_of_the_row_length_lines(gpu_ctx, pkg, oracle, K):
+    """Average row lengths of just under and just over 4, 5 and 10 entries, with enough chunks for the shapes of many."""
+    ctx, N = gpu_ctx, 3000
+    opts = pkg.Opts(chunk_nnz=CHUNK)
+    n_chunks = 80 * SMS + 40
+    for length in (4, 5, 10):
+        for rows_more in (0, 1):      # nnz = length * M, and one row too many for that
+            M = n_chunks * CHUNK // length
+            nnz = length * M
+            rng = np.random.default_rng(length)
+            degrees = np.full(M, length)
+            move = rng.integers(0, length - 1, M // 2)
+            degrees[:M // 2] -= move
+            degrees[M - M // 2:] += move[::-1]
+            degrees = np.concatenate([rng.permutation(degrees), np.zeros(rows_more, int)])
+            M += rows_more
+            rp = np.concatenate([[0], np.cumsum(degrees)]).astype(np.int32)
+            first = rng.integers(0, N - 64, M)
+            within = np.arange(nnz) - np.repeat(rp[:-1], degrees)
+            ci = (np.repeat(first, degrees) + within * 3 % 64).astype(np.int32)
+            assert (nnz >= length * M) == (rows_more == 0)
+            M_, X, Y = _operands(pkg, rp, K, N)
+            ref, abs_sum = oracle.sddmm_f64(rp, ci, X, Y)
+            d_rp, d_ci, d_X, d_Y = (ctx.upload(x) for x in (rp, ci, X, Y))
+            d_out = ctx.alloc((nnz,), np.float32)
+            plan = ctx.plan_create(M, nnz, d_rp, K, opts, N=N, col_idx=d_ci)
+            for p in (plan, None):
+                ctx.fill(d_out, nnz, 7.0)
+                ctx.sddmm_csr(M, N, K, nnz, d_rp, d_ci, d_X, d_Y, d_out, plan=p, opts=opts)
+                check_against_f64(d_out.to_host(), ref, abs_sum, "K=%d rows of %d plan=%s" % (K, length, p is not None))
+            ctx.plan_destroy(plan)
+            for b in (d_rp, d_ci, d_X, d_Y, d_out):
+                b.free()
