@@ -48,6 +48,7 @@ struct hpspmm_ctx {
 //   rec             the same per chunk in the order in which warps take them, see hpspmm_spmm_args
 struct hpspmm_plan {
   int device;
+  int sm_count;
   int64_t M, nnz;
   int32_t chunk_nnz;
   int64_t n_chunks;
@@ -97,7 +98,7 @@ struct hpspmm_spmm_args {
 // Shape of the kernel for `cols` columns: VEC-wide vectors, W lanes and R vectors per lane to a group (warp_frag.cuh).
 struct hpspmm_spmm_shape {
   int VEC, W, R;
-  bool lat;    // few chunks: columns split over more warps, more gathers in flight per warp
+  bool lat;    // few chunks: more gathers in flight per warp
   bool hint;
 };
 // widest vector the rows of the dense operands keep aligned; addresses: bitwise or of the operands' addresses

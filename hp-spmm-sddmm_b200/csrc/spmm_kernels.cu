@@ -595,28 +595,34 @@ int check_spmm_args(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t nn
 //                     501, and without a plan 590 -> 557; below 384 columns about level with a plan, and without one, where the
 //                     chunks are not ordered by cost and every pass ends on its own last ones, behind (4 M, K = 300 +6 %)
 // 300 K entries, K = 512: 37 -> 47, so with few chunks one pass stays.
-int widest_slab(const hpspmm_ctx* ctx, int VEC, int64_t K, int64_t n_chunks, bool even) {
-  if (VEC == 4 && ((K > 384 && n_chunks > ctx->sm_count * 48ll) || (K >= 256 && even && n_chunks > ctx->sm_count * 64ll)))
-    return 128;
+int widest_slab(int sm_count, int VEC, int64_t K, int64_t n_chunks, bool even) {
+  if (VEC == 4 && ((K > 384 && n_chunks > sm_count * 48ll) || (K >= 256 && even && n_chunks > sm_count * 64ll))) return 128;
   return hpspmm_widest_slab(VEC);
+}
+
+// The launch of a product that begins at column `off`: how many columns it takes (*cols) and its shape.
+hpspmm_spmm_shape shape_of_launch(int sm_count, int VEC, int K, int off, int64_t n_chunks, bool even, bool hint, int* cols) {
+  const int widest = widest_slab(sm_count, VEC, K, n_chunks, even);
+  *cols = hpspmm_launch_cols(K, off, widest);
+  hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, *cols, widest, hint);
+  // Few chunks: registers are plenty, so a warp keeps 8 to 32 gather steps in flight instead of 4 (the additions keep
+  // their order).  67.6 K entries in chunks of 64: 6.1 -> 5.6 us at K = 64, 9.1 -> 7.2 us at K = 128; with more chunks
+  // than these builds have resident warps they lose (300 K entries, K = 64: 8.3 -> 10.5 us).
+  sh.lat = n_chunks <= sm_count * (sh.W <= 8 ? 24 : 16);
+  // (one group instead of several of three vectors: rows end without an exchange, and are added up in another order)
+  if (sh.lat && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;
+  return sh;
 }
 
 // shared_counters: the scratch holds one counter per chunk, so the slabs of a wide product run one after the other
 // even: the rows are known to be of even length (hpspmm_even_rows)
 int launch_spmm(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool hint, bool even, bool shared_counters, cudaStream_t s) {
   const int VEC = hpspmm_vector_width(a.K, (uintptr_t)a.B | (uintptr_t)a.C);
-  const int widest = widest_slab(ctx, VEC, a.K, a.n_chunks, even);
   int32_t* counter = a.counter;
   a.keep_b = hint ? 1 : 0;
   for (a.off = 0; a.off < a.K; a.off += a.cols) {
-    a.cols = hpspmm_launch_cols(a.K, a.off, widest);
+    const hpspmm_spmm_shape sh = shape_of_launch(ctx->sm_count, VEC, a.K, a.off, a.n_chunks, even, hint, &a.cols);
     if (!shared_counters) a.counter = counter + (int64_t)(a.off / 32) * a.n_chunks;
-    hpspmm_spmm_shape sh = hpspmm_choose_shape(VEC, a.cols, widest, hint);
-    // Few chunks: registers are plenty, so a warp keeps 8 to 32 gather steps in flight instead of 4 (the same order of
-    // additions).  67.6 K entries in chunks of 64: 6.1 -> 5.6 us at K = 64, 9.1 -> 7.2 us at K = 128; with more chunks
-    // than these builds have resident warps they lose (300 K entries, K = 64: 8.3 -> 10.5 us).
-    sh.lat = a.n_chunks <= ctx->sm_count * (sh.W <= 8 ? 24 : 16);
-    if (sh.lat && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;   // (one group: rows end without an exchange)
     const int st = VEC == 4   ? hpspmm_spmm_launch_v4(ctx, a, sh, shared_counters, s)
                    : VEC == 2 ? hpspmm_spmm_launch_v2(ctx, a, sh, shared_counters, s)
                               : hpspmm_spmm_launch_v1(ctx, a, sh, shared_counters, s);
@@ -686,6 +692,7 @@ int hpspmm_plan_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const
   if (!p) return HPSPMM_ERR_OOM;
   memset(p, 0, sizeof(*p));
   p->device = ctx->device;
+  p->sm_count = ctx->sm_count;
   p->M = M;
   p->nnz = nnz;
   p->chunk_nnz = S;
@@ -771,11 +778,16 @@ int hpspmm_plan_info(const hpspmm_plan* plan, int64_t* n_chunks, int64_t* n_spli
 
 int hpspmm_spmm_kernel_signature(const hpspmm_plan* plan, int64_t K, int32_t b_l2_hint, char* buf, size_t len) {
   if (!buf || len == 0 || K < 1) return HPSPMM_ERR_INVALID;
-  const int64_t nnz = plan ? plan->nnz : 0;
+  const int VEC = hpspmm_vector_width(K, 0);
   const hpspmm_opts o = {0, 0, b_l2_hint, 0};
-  const hpspmm_spmm_shape sh = hpspmm_choose_shape(hpspmm_vector_width(K, 0), K, hpspmm_widest_slab(hpspmm_vector_width(K, 0)), gather_hint(K, &o));
-  snprintf(buf, len, "spmm_warp_kernel<%d,%d,%d> K=%lld split=%d hint=%d chunk_nnz=%d", sh.VEC, sh.W, sh.R, (long long)K,
-           sh.lat ? 1 : 0, sh.hint ? 1 : 0, plan ? (int)plan->chunk_nnz : (int)hpspmm_default_chunk_nnz(K, nnz));
+  const bool hint = gather_hint(K, &o);
+  int cols = 0;
+  const bool fits = plan != nullptr && K <= plan->max_K && K <= (1 << 20);
+  const hpspmm_spmm_shape sh =
+      fits ? shape_of_launch(plan->sm_count, VEC, (int)K, 0, plan->n_chunks, hpspmm_even_rows(plan), hint, &cols)
+           : hpspmm_choose_shape(VEC, K, hpspmm_widest_slab(VEC), hint);
+  snprintf(buf, len, "spmm_warp_kernel<%d,%d,%d> K=%lld few=%d hint=%d chunk_nnz=%d", sh.VEC, sh.W, sh.R, (long long)K,
+           sh.lat ? 1 : 0, sh.hint ? 1 : 0, plan ? (int)plan->chunk_nnz : (int)hpspmm_default_chunk_nnz(K, 0));
   return HPSPMM_OK;
 }
 

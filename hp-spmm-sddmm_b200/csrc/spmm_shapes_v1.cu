@@ -1,4 +1,4 @@
-// Instances of the CSR product kernel for odd widths (4-byte gathers), and of its column-split form.
+// Instances of the CSR product kernel for odd widths (4-byte gathers).
 #include "spmm_warp.cuh"
 using namespace hpspmm;
 

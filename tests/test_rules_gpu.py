@@ -158,3 +158,26 @@ def test_sddmm_on_both_sides_of_the_row_length_lines(gpu_ctx, pkg, oracle, K):
             ctx.plan_destroy(plan)
             for b in (d_rp, d_ci, d_X, d_Y, d_out):
                 b.free()
+
+
+def test_the_signature_names_the_shape_that_is_launched(gpu_ctx, pkg):
+    ctx, N = gpu_ctx, 4000
+    opts = pkg.Opts(chunk_nnz=CHUNK)
+
+    def signature(n_chunks, K, even=True):
+        rp, ci, _ = _matrix(n_chunks, even)
+        d_rp, d_ci = ctx.upload(rp), ctx.upload(ci)
+        plan = ctx.plan_create(len(rp) - 1, len(ci), d_rp, K, opts, N=N, col_idx=d_ci)
+        try:
+            return ctx.kernel_signature(plan, K)
+        finally:
+            ctx.plan_destroy(plan)
+            d_rp.free()
+            d_ci.free()
+
+    for K, few, many, line in ((128, "<4,32,1>", "<4,32,1>", 16), (96, "<4,32,1>", "<4,8,3>", 24),
+                               (160, "<4,32,2>", "<4,16,3>", 16), (32, "<4,8,1>", "<4,8,1>", 24)):
+        assert few in signature(line * SMS, K) and "few=1" in signature(line * SMS, K)
+        assert many in signature(line * SMS + 1, K) and "few=0" in signature(line * SMS + 1, K)
+    assert "<4,32,3>" in signature(64 * SMS, 384) and "<4,32,3>" in signature(64 * SMS + 1, 384, even=False)
+    assert "<4,32,1>" in signature(64 * SMS + 1, 384)
