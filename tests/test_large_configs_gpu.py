@@ -149,9 +149,9 @@ def test_cfg5_gnn_layer_full_size(gpu_ctx, pkg, oracle):
         b.free()
 
 
-def test_cfg2_graph_at_k256_runs_as_two_slabs(gpu_ctx, pkg, oracle):
-    """The R-MAT scale-20 graph at K = 256 (two strided 128-column slabs): the product against the oracle, the COO
-    product and the SDDMM on the same operands."""
+def test_cfg2_graph_at_k256(gpu_ctx, pkg, oracle):
+    """The R-MAT scale-20 graph at K = 256 (one pass, several vectors per lane): the product against the oracle, the
+    COO product and the SDDMM on the same operands."""
     ctx = gpu_ctx
     K = 256
     g = pkg.gen_rmat(20, 16, seed=2)

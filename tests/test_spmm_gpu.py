@@ -200,7 +200,7 @@ def test_full_size_cfg2(gpu_ctx, pkg, oracle, K):
 
 
 def test_host_entry_with_several_products(gpu_ctx, pkg, oracle):
-    """hpspmm_spmm_csr_f32_host_multi: A uploaded once, the slabs of all products through one pipeline."""
+    """hpspmm_spmm_csr_f32_host_multi: A uploaded once, the slabs of all products (11.8 MB) through one pipeline."""
     g = pkg.gen_rmat(12, 16, seed=6)
     M, N, nnz = g["M"], g["N"], g["nnz"]
     Ks = [32, 64, 128, 40, 96]
@@ -217,15 +217,40 @@ def test_host_entry_with_several_products(gpu_ctx, pkg, oracle):
     assert e.value.status == pkg.ERR_INVALID
 
 
+@pytest.mark.parametrize("scale", [12, 14])
 @pytest.mark.parametrize("K", [32, 64, 128, 192, 96, 40])
-def test_host_buffer_entry_point(gpu_ctx, pkg, oracle, K):
-    """K = 64 / 96 / 128 / 192 take the slab pipeline (32- or 64-column slabs), the others the plain path."""
-    g = pkg.gen_rmat(12, 16, seed=4)
+def test_host_buffer_entry_point(gpu_ctx, pkg, oracle, K, scale):
+    """Multiples of 32 from 64 columns on take the slab pipeline (32- or 64-column slabs) once the dense operands are
+    larger than 4 MB: at scale 14 all of those, at scale 12 K = 192 alone.  The others go whole."""
+    g = pkg.gen_rmat(scale, 16, seed=4)
+    assert (4 * K * (g["M"] + g["N"]) > 4 << 20) == (K == 192 or (scale == 14 and K > 32))
     B = pkg.host_fill_uniform(g["N"] * K, 4, 1, -1.0, 1.0).reshape(g["N"], K)
     C = np.full((g["M"], K), np.nan, dtype=np.float32)
     gpu_ctx.spmm_csr_host(g["M"], g["N"], K, g["nnz"], g["row_ptr"], g["col_idx"], g["vals"], B, C)
     ref, abs_sum = oracle.spmm_f64(g["row_ptr"], g["col_idx"], g["vals"], B)
     check_against_f64(C, ref, abs_sum, "host entry")
+
+
+@pytest.mark.parametrize("more", [-1, 0, 1])
+@pytest.mark.parametrize("Ks", [[64], [128], [32, 32], [17, 40, 1, 6]])
+def test_host_entries_around_the_size_that_goes_whole(gpu_ctx, pkg, oracle, Ks, more):
+    """4 * K * (M + N) of all products just below, at and just above 4 MB, through both host entries."""
+    per_row = 4 * sum(Ks)
+    M = 3000
+    N = (4 << 20) // per_row - M + more
+    assert (per_row * (M + N) > 4 << 20) == (more > 0)
+    g = pkg.gen_uniform_degree(M, N, 0, 24, seed=9, vals_kind=pkg.VALS_UPM1)
+    nnz = g["nnz"]
+    Bs = [pkg.host_fill_uniform(N * K, 9, K, -1.0, 1.0).reshape(N, K) for K in Ks]
+    refs = [oracle.spmm_f64(g["row_ptr"], g["col_idx"], g["vals"], B) for B in Bs]
+    Cs = [np.full((M, K), np.nan, dtype=np.float32) for K in Ks]
+    gpu_ctx.spmm_csr_host_multi(M, N, nnz, g["row_ptr"], g["col_idx"], g["vals"], Ks, Bs, Cs)
+    for K, C, (ref, abs_sum) in zip(Ks, Cs, refs):
+        check_against_f64(C, ref, abs_sum, "several products, K=%d" % K)
+    for K, B, (ref, abs_sum) in zip(Ks, Bs, refs):
+        C = np.full((M, K), np.nan, dtype=np.float32)
+        gpu_ctx.spmm_csr_host(M, N, K, nnz, g["row_ptr"], g["col_idx"], g["vals"], B, C)
+        check_against_f64(C, ref, abs_sum, "one product, K=%d" % K)
 
 
 @pytest.mark.parametrize("K", [64, 128])
@@ -328,7 +353,7 @@ def test_plan_tables_tile_the_matrix_and_schedule_every_chunk_once(gpu_ctx, pkg,
 @pytest.mark.parametrize("K", [64, 128])
 @pytest.mark.parametrize("chunk", [32, 256])
 def test_split_rows_settled_inside_the_kernel_on_repeated_calls(gpu_ctx, pkg, oracle, K, chunk):
-    """With a plan, K = 64/128 add the carries of split rows inside the product kernel, through per-row
+    """With a plan the carries of split rows are added inside the product kernel, through per-row
     counters that must be back at zero after every launch: three calls on one plan, rows of 1 to 20,000
     entries (up to 625 pieces), each call checked."""
     ctx = gpu_ctx
@@ -352,7 +377,7 @@ def test_split_rows_settled_inside_the_kernel_on_repeated_calls(gpu_ctx, pkg, or
         if first is None:
             first = got
         assert np.array_equal(got, first)            # bit-reproducible from call to call
-    # the same plan at a narrower width takes the separate fix-up kernel and leaves the counters alone
+    # the same plan at a narrower width uses the same counters
     B32 = np.ascontiguousarray(B[:, :32])
     d_B32, d_C32 = ctx.upload(B32), ctx.alloc((M, 32), np.float32)
     ctx.spmm_csr(M, N, 32, nnz, d_rp, d_ci, d_v, d_B32, d_C32, plan=plan, opts=opts)
@@ -442,16 +467,14 @@ def test_products_with_a_plan_can_be_captured_in_a_cuda_graph(pkg, oracle):
 
 @pytest.mark.parametrize("K", [96, 160, 192, 224, 256, 320, 512])
 @pytest.mark.parametrize("use_plan", [False, True])
-def test_other_multiples_of_32_run_as_column_slabs(gpu_ctx, pkg, oracle, K, use_plan):
-    """K = 32·m beyond 32/64/128 runs the specialised kernel over column slabs of 128, 64 and 32 (strided B, C and
-    carry slots); heavy rows make every slab hand on and settle carries; canaries guard the neighbouring columns."""
+def test_other_multiples_of_32(gpu_ctx, pkg, oracle, K, use_plan):
+    """K = 32·m beyond 32/64/128: several vectors per lane; heavy rows make every chunk hand on and settle carries;
+    canaries guard what lies around the result."""
     g = pkg.gen_rmat(12, 16, seed=81)
     N = g["N"]
     B = pkg.host_fill_uniform(N * K, 81, K, -1.0, 1.0).reshape(N, K)
     for chunk in (0, 32):
         opts = pkg.Opts(algo=pkg.ALGO_BALANCED, chunk_nnz=chunk)
-        C, _ = _check(gpu_ctx, pkg, oracle, g["row_ptr"], g["col_idx"], g["vals"], B, "slabs K=%d S=%d" % (K, chunk),
+        C, _ = _check(gpu_ctx, pkg, oracle, g["row_ptr"], g["col_idx"], g["vals"], B, "K=%d S=%d" % (K, chunk),
                       opts=opts, use_plan=use_plan)
-        # a slab is the product with that slab of B: columns 0..31 equal the K = 32 product bit for bit when the
-        # first slab is 32 wide... not in general (slab widths differ), but every slab must agree with the oracle
         assert np.all(np.isfinite(C))
