@@ -259,8 +259,10 @@ int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes) {
 
 int hpspmm_ensure_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream) {
   if (n > ctx->counter_cap) {
-    HPSPMM_CUDA_TRY(ctx, cudaDeviceSynchronize());
-    if (ctx->counters) cudaFree(ctx->counters);
+    if (ctx->counters) {   // the old ones may still be in use by queued kernels
+      HPSPMM_CUDA_TRY(ctx, cudaDeviceSynchronize());
+      cudaFree(ctx->counters);
+    }
     ctx->counters = nullptr;
     ctx->counter_cap = 0;
     const int64_t cap = (n + n / 4 + 1023) / 1024 * 1024;
@@ -277,14 +279,11 @@ int hpspmm_ensure_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream) {
   return HPSPMM_OK;
 }
 
-int hpspmm_take_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream, int32_t** set, int32_t** clear, int* n_clear) {
-  const int st = hpspmm_ensure_counters(ctx, n, stream);
-  if (st != HPSPMM_OK) return st;
+void hpspmm_take_counters(hpspmm_ctx* ctx, int32_t** set, int32_t** clear, int* n_clear) {
   const int turn = ctx->counter_turn;
   *set = ctx->counters + turn * ctx->counter_cap;
   *clear = ctx->counters + (1 - turn) * ctx->counter_cap;
   *n_clear = (int)ctx->counter_used[1 - turn];
-  return HPSPMM_OK;
 }
 
 void hpspmm_counters_used(hpspmm_ctx* ctx, int64_t n, bool launched) {

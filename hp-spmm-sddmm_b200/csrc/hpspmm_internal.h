@@ -186,11 +186,12 @@ struct hpspmm_trace_range {
 #define HPSPMM_TRACE(name) hpspmm_trace_range hpspmm_trace_range__(name)
 
 int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes);
-// `n` counters that are zero when work queued on `stream` starts, for one product whose kernel clears the first
-// `*n_clear` ints at `*clear`; hpspmm_counters_used tells how its launch went.  Not for captured calls: a graph may be
-// replayed between any two products, so a captured call keeps its counters in the scratch and clears them itself.
+// Two sets of at least `n` counters, zero when work queued on `stream` starts.  hpspmm_take_counters hands out the set for
+// one product, whose kernel clears the first `*n_clear` ints at `*clear`; hpspmm_counters_used tells how many it counts in
+// and how its launch went.  Not for captured calls: a graph may be replayed between any two products, so a captured call
+// keeps its counters in the scratch and clears them itself.
 int hpspmm_ensure_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream);
-int hpspmm_take_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream, int32_t** set, int32_t** clear, int* n_clear);
+void hpspmm_take_counters(hpspmm_ctx* ctx, int32_t** set, int32_t** clear, int* n_clear);
 void hpspmm_counters_used(hpspmm_ctx* ctx, int64_t n, bool launched);
 int hpspmm_ensure_stage(hpspmm_ctx* ctx, size_t bytes);
 

@@ -512,8 +512,8 @@ int32_t hpspmm_default_chunk_nnz(int64_t K, int64_t nnz) {
   //   16 M entries, K = 64: 333 / 322 / 305 / 297 / 293 / 297  and 294 / 293 / 292 / 294 / 299 / 303
   //   16 M entries, K = 128: 566 / 567 / 546 / - / 550 / 526   and 523 / 563 / 572 / 566 / 537 / 561
   // A caller that builds a plan for products only can ask for more (hpspmm_opts.chunk_nnz).
-  // Below 2.4 M entries there are fewer chunks than warps the GPU can hold, and the time is that of the longest
-  // chunk: a chain of gather round trips.  Measured in us at S = 32 / 64 / 128 / 256, rows of 16 entries on average,
+  // Below 2.4 M entries there are at most a few waves of chunks (5,300 warps of the fixed widths are resident), and the
+  // time is that of the longest chunk: a chain of gather round trips.  Measured in us at S = 32 / 64 / 128 / 256, rows of 16 entries on average,
   // uniform and power-law columns: 12 K entries, K = 32: 3.7 / 4.5 / 6.3 / 10.1 and 6.6 / 7.7 / 10.3 / 13.9;
   // 300 K, K = 64: 10.2 / 8.3 / 10.3 / 16.3 and 14.2 / 12.9 / 15.6 / 24.2; 1 M, K = 64: 24.3 / 21.0 / 21.4 / 22.7 and
   // 37.5 / 26.7 / 23.8 / 32.2 (smaller chunks split more rows, and every split costs an exchange through memory).
@@ -654,6 +654,13 @@ int32_t planless_chunk_nnz(int64_t K, int64_t nnz, const hpspmm_opts* opts) {
 // between the entries the list pays for itself.
 bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t n_chunks) {
   return n_chunks <= ctx->sm_count * 40ll && M <= 8 * nnz;
+}
+
+// Counters that are set aside at the first product of a width: enough for any later one of up to that width, so that a
+// smaller call never allocates.  Beyond 512 columns as many as the call needs.
+int64_t counters_to_keep(const hpspmm_ctx* ctx, int64_t K, int64_t n_counter, bool search) {
+  const int64_t most = (ctx->sm_count * 40ll + 1) * hpspmm_counter_slabs(K < 512 ? K : 512);
+  return search && n_counter > most ? n_counter : most;
 }
 
 // where a plan-less product keeps what it builds, inside the context's scratch
@@ -848,7 +855,11 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
   const int64_t n_chunks = (nnz + S - 1) / S;
   const bool search = searches_for_chunks(ctx, M, nnz, n_chunks);
   const planless_layout lay(M, K, n_chunks, search);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
+  const bool eager = capture == cudaStreamCaptureStatusNone;
   st = hpspmm_ensure_scratch(ctx, lay.bytes);
+  if (st == HPSPMM_OK && eager) st = hpspmm_ensure_counters(ctx, counters_to_keep(ctx, K, lay.n_counter, search), s);
   if (st != HPSPMM_OK) return st;
   char* base = (char*)ctx->scratch;
   a.n_chunks = (int)n_chunks, a.S = S;
@@ -865,14 +876,11 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
     a.rec = rec, a.nz = nz;
     return launch_spmm(ctx, a, hint, false, false, s);
   }
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
-  if (capture != cudaStreamCaptureStatusNone) {
+  if (!eager) {
     HPSPMM_CUDA_TRY(ctx, cudaMemsetAsync(a.counter, 0, (size_t)lay.n_counter * 4, s));
     return launch_spmm(ctx, a, hint, false, false, s);
   }
-  st = hpspmm_take_counters(ctx, lay.n_counter, s, &a.counter, &a.clear, &a.n_clear);
-  if (st != HPSPMM_OK) return st;
+  hpspmm_take_counters(ctx, &a.counter, &a.clear, &a.n_clear);
   st = launch_spmm(ctx, a, hint, false, false, s);
   hpspmm_counters_used(ctx, lay.n_counter, st == HPSPMM_OK);
   return st;
@@ -928,7 +936,8 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
       const bool search = searches_for_chunks(ctx, M, nnz, n_chunks);
       const planless_layout lay(M, w, n_chunks, search);
       need = lay.bytes > need ? lay.bytes : need;
-      if (search && lay.n_counter > need_counters) need_counters = lay.n_counter;
+      const int64_t keep = counters_to_keep(ctx, w, lay.n_counter, search);
+      need_counters = keep > need_counters ? keep : need_counters;
     }
     st = hpspmm_ensure_scratch(ctx, need);
     if (st == HPSPMM_OK) st = hpspmm_ensure_counters(ctx, need_counters, s_run);

@@ -201,3 +201,23 @@ def test_plans_come_and_go_beside_a_capture_in_another_thread(pkg, oracle, mode)
                      w.C.data_ptr(), plan=plan, stream=s)
         w.check("product with the plan built meanwhile")
         ctx.plan_destroy(plan)
+
+
+def test_only_the_first_product_of_a_width_allocates(pkg, oracle):
+    """After a large product without a plan, smaller ones of up to its width find all they need."""
+    import torch
+    lib = pkg.load_library()
+    N = 20000
+    large = _Work(pkg, oracle, [300] * 3000, N, 96, 120)                        # has its structure built
+    works = [_Work(pkg, oracle, DEGREES, N, K, 121) for K in (96, 64, 5)]      # one launch each
+    with pkg.Context(0) as ctx:
+        s = torch.cuda.current_stream().cuda_stream
+        large.call(ctx, s)
+        large.check("large")
+        lib.hpspmm_debug_fail_device_alloc(1, 1000)
+        try:
+            for w in works + [large]:
+                w.call(ctx, s)
+                w.check("K=%d, no allocation possible" % w.K)
+        finally:
+            lib.hpspmm_debug_fail_device_alloc(0, 0)
