@@ -337,8 +337,9 @@ int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
 // Which of them are SERIAL: 16-byte vectors fill the registers that the other path needs (K = 96 424 against 477 us); with
 // narrower vectors it costs more than it saves except where noted by the shape.  Where rows are short the waits do not
 // pay (uniform rows of 4 entries, K = 100: 176 against 159 us; of 8: 130 against 119; of 12: 110 against 105, but K = 96 92
-// against 103 and K = 160 158 against 185): rows_are_long.  Where the
-// gain is small it also takes enough chunks to cover the waits (12,500 chunks: K = 48 38.9 against 41.4 us, K = 62 45.7
+// against 103 and K = 160 158 against 185): rows_are_long.  K = 32, 64 and 128 take SERIAL at any row length; on short rows
+// that is compared with the kernel before it only (4 M uniform entries in rows of 4: K = 32 164 -> 134 us, 64 234 ->
+// 193, 128 401 -> 398).  Where the gain is small it also takes enough chunks to cover the waits (12,500 chunks: K = 48 38.9 against 41.4 us, K = 62 45.7
 // against 55.1; 31,000: 105 against 97 and 110 against 97).
 int launch_sddmm_shape(hpspmm_ctx* ctx, const sddmm_args& a, const hpspmm_spmm_shape& sh, cudaStream_t s) {
 #define GO(V, W, R, U, KS, H, MINB) return launch_sddmm<V, W, R, U, KS, H, MINB, false>(ctx, a, s)

@@ -127,13 +127,16 @@ HPSPMM_API int hpspmm_host_fill_uniform_f32(float* host_ptr, int64_t count, uint
  * kernels: (m, k, row_ptr, col_idx, values, B, C), with N and nnz added.  Overwrites C;
  * empty rows become zeros.  All pointers are device pointers.  K >= 1: one kernel serves
  * every width (16-byte gathers when K is a multiple of 4, 8-byte when it is even and the
- * operands are 8-byte aligned, 4-byte otherwise; wider than 512 columns in slabs).
+ * operands are 8-byte aligned, 4-byte otherwise; wide operands in passes of 128 or slabs
+ * of 512 columns).
  *
  * plan may be NULL: the warps of a small product then search row_ptr for their part, for a
- * larger one the structure is rebuilt into context-owned scratch on every call (two extra small kernels).  The first call that needs more scratch than
- * the context holds allocates it (cudaMalloc, synchronising); later calls do not.
+ * larger one the structure is rebuilt into context-owned scratch on every call (two extra
+ * small kernels).  The first call that needs more scratch than the context holds allocates
+ * it (cudaMalloc, synchronising); later calls do not.
  * With a plan the call only enqueues kernels (no allocation, no synchronisation), so it can
- * be recorded into a CUDA graph and replayed.
+ * be recorded into a CUDA graph and replayed.  So can a call without one, once the same call
+ * has run outside the capture and as long as the context's scratch does not grow.
  * Calls that share a context or a plan must not overlap on the GPU. */
 HPSPMM_API int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M,
                                    int64_t N, int64_t K, int64_t nnz, const int32_t* row_ptr,
@@ -183,11 +186,10 @@ HPSPMM_API int hpspmm_plan_row_list(const hpspmm_plan* plan, const int32_t** nz_
  * cannot take the device-wide synchronisation an allocation may bring.
  *
  * This entry point calls no cudaMalloc, cudaFree or allocating library routine, and needs
- * no context.  The chunk table, the carry slots and the per-row counters of the nnz-balanced
- * kernel live in one 16 MiB array inside the library image, so every GPU that loads the library gives up
+ * no context.  The carry slots and the per-row counters of the nnz-balanced kernel live in one 16 MiB array inside the library image, so every GPU that loads the library gives up
  * 16 MiB until the process exits.  A matrix whose scratch would not fit -- more than
  * (16 MiB - 0.5 KiB) / (4 + 4 K) chunks (of 128 / 160 / 256 nnz at K = 32 / 64 / 128):
- * about 15 M nnz at K = 32, 10 M at K = 64, 8 M at K = 128 -- is refused with HPSPMM_ERR_UNSUPPORTED and a message in
+ * about 16 M nnz at K = 32, 10 M at K = 64, 8 M at K = 128 -- is refused with HPSPMM_ERR_UNSUPPORTED and a message in
  * err_buf; use hpspmm_spmm_csr_f32 for it.
  *
  * The first call on a device looks up the array's device address (cudaGetSymbolAddress,
@@ -208,8 +210,9 @@ HPSPMM_API int hpspmm_spmm_csr_f32_static_scratch(int device_ordinal, int64_t M,
 /* Same product with HOST buffers: copies A and B to the device, runs the product,
  * copies C back, synchronises.  When K is a multiple of 32 and at least 64 the call is
  * pipelined over 32- or 64-column slabs of B and C (uploads, products and downloads overlap on
- * three internal streams, PCIe being full duplex; dense operands of up to 4 MB go whole); each slab is a product of the slab's width, so
- * the rounding of rows split across chunks can differ from the device-pointer entry point in
+ * three internal streams, PCIe being full duplex; dense operands of up to 4 MB go whole through
+ * one of them); other widths run on the default stream.  Each slab is a product of the slab's
+ * width, so the rounding of rows split across chunks can differ from the device-pointer entry point in
  * the last bits.  The overlap needs page-locked host buffers (hpspmm_host_alloc_pinned or the
  * caller's own): from pageable memory the copies are staged and serialised by the driver and the
  * call degrades to upload, product, download one after the other.  It is what the reference's
