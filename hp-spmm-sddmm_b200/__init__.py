@@ -116,6 +116,8 @@ PROTOTYPES = {
     "hpspmm_layer_info": (c_int, [_P, POINTER(_I64), POINTER(_I64), POINTER(_I64), POINTER(_I64),
                                   POINTER(_I64)]),
     "hpspmm_layer_transposed": (c_int, [_P, POINTER(_P), POINTER(_P), POINTER(_P), POINTER(_P)]),
+    "hpspmm_layer_forward_values": (c_int, [_P, _P, _I64, _P, _P, _P, _P]),
+    "hpspmm_layer_backward": (c_int, [_P, _P, _I64, _P, _P, _P, _P, _P, _P]),
     "hpspmm_layer_forward": (c_int, [_P, _P, _I64, _P, _P, _P]),
     "hpspmm_layer_backward_features": (c_int, [_P, _P, _I64, _P, _P, _P]),
     "hpspmm_layer_backward_weights": (c_int, [_P, _P, _I64, _P, _P, _P, _P]),

@@ -30,6 +30,7 @@ SOURCES = [
     "spmm_shapes_v1.cu",
     "coo_kernels.cu",
     "sddmm_kernels.cu",
+    "layer_grad_kernels.cu",
     "structure_kernels.cu",
     "graph_layer.cu",
     "probe_kernels.cu",

@@ -2,6 +2,7 @@
 //   forward            C  = A  · H          (CSR SpMM, cached plan)
 //   backward, features dH = Aᵀ · dC         (SpMM on the device-built transpose, cached plan)
 //   backward, weights  dA = pattern(A) ⊙ (dC · Hᵀ)   (SDDMM, same plan as forward)
+//   backward, both     one pass over the transpose     (layer_grad_kernels.cu, the transpose's plan)
 // The reference has no such layer: its driver calls one product at a time
 // (test/test_all.cpp:63-107) and ships neither a transpose nor an SDDMM.  What the
 // handle owns is what a training loop would otherwise rebuild every step: the two
@@ -150,13 +151,19 @@ int hpspmm_layer_transposed(const hpspmm_layer* g, const int32_t** row_ptr_t, co
 
 int hpspmm_layer_forward(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, const float* H, float* C,
                          hpspmm_stream stream) {
+  HPSPMM_REQUIRE(ctx, ctx != nullptr && g != nullptr, "null context or layer");
+  return hpspmm_layer_forward_values(ctx, g, K, g->vals, H, C, stream);
+}
+
+int hpspmm_layer_forward_values(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, const float* vals, const float* H,
+                                float* C, hpspmm_stream stream) {
   HPSPMM_TRACE("hpspmm_layer_forward");
   HPSPMM_REQUIRE(ctx, ctx != nullptr && g != nullptr, "null context or layer");
   HPSPMM_REQUIRE(ctx, K >= 1 && K <= g->max_K, "K outside [1, max_K] of the layer");
   int cls;
   const int st = plans_for(ctx, g, K, stream, &cls);
   if (st != HPSPMM_OK) return st;
-  return hpspmm_spmm_csr_f32(ctx, g->plan[cls], g->M, g->N, K, g->nnz, g->row_ptr, g->col_idx, g->vals, H, C,
+  return hpspmm_spmm_csr_f32(ctx, g->plan[cls], g->M, g->N, K, g->nnz, g->row_ptr, g->col_idx, vals, H, C,
                              nullptr, stream);
 }
 
@@ -182,6 +189,31 @@ int hpspmm_layer_backward_weights(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, c
   if (st != HPSPMM_OK) return st;
   return hpspmm_sddmm_csr_f32(ctx, g->plan[cls], g->M, g->N, K, g->nnz, g->row_ptr, g->col_idx, dC, H, dA, nullptr,
                               stream);
+}
+
+int hpspmm_layer_backward(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, const float* vals, const float* dC,
+                          const float* H, float* dH, float* dA, hpspmm_stream stream) {
+  HPSPMM_TRACE("hpspmm_layer_backward");
+  HPSPMM_REQUIRE(ctx, ctx != nullptr && g != nullptr, "null context or layer");
+  HPSPMM_REQUIRE(ctx, K >= 1 && K <= g->max_K, "K outside [1, max_K] of the layer");
+  if (g->nnz == 0 || g->M == 0 || g->N == 0 || K > 256) return HPSPMM_ERR_UNSUPPORTED;
+  HPSPMM_REQUIRE(ctx, vals && dC && H && dH && dA, "null operand");
+  if ((K & 3) == 0) HPSPMM_REQUIRE(ctx, (((uintptr_t)dC | (uintptr_t)H | (uintptr_t)dH) & 15u) == 0,
+                                   "dense operands must be 16-byte aligned");
+  hpspmm_device_guard guard(ctx->device);
+  int cls;
+  const int st = plans_for(ctx, g, K, stream, &cls);
+  if (st != HPSPMM_OK) return st;
+  const hpspmm_plan* p = g->plan_t[cls];
+  if (!hpspmm_layer_grad_pays(ctx, g->nnz, hpspmm_even_rows(p))) return HPSPMM_ERR_UNSUPPORTED;
+  hpspmm_layer_grad_args a;
+  memset(&a, 0, sizeof(a));
+  a.rows = (int)g->N, a.K = (int)K, a.n_chunks = (int)p->n_chunks, a.S = p->chunk_nnz;
+  a.keep = K >= 64 ? 1 : 0;   // as in the product
+  a.row_ptr = g->row_ptr_t, a.col_idx = g->col_idx_t, a.perm = g->perm;
+  a.vals = vals, a.dC = dC, a.H = H, a.dH = dH, a.dA = dA;
+  a.rec = p->rec, a.nz = p->nz, a.carry = p->carry_val, a.counter = p->run_counter;
+  return hpspmm_layer_grad_launch(ctx, a, (cudaStream_t)stream);
 }
 
 int hpspmm_layer_update_values(hpspmm_ctx* ctx, hpspmm_layer* g, const float* vals, hpspmm_stream stream) {

@@ -127,6 +127,29 @@ int hpspmm_spmm_launch_v1(hpspmm_ctx* ctx, const hpspmm_spmm_args& a, const hpsp
 // sets of per-chunk counters a product of up to K columns may need: one per slab, no slab narrower than 32 columns
 static inline int64_t hpspmm_counter_slabs(int64_t K) { return (K + 31) / 32; }
 
+// What the kernel of both layer gradients is launched with: the transpose of A by rows (row_ptr, col_idx, and perm, the
+// position of every entry in A's order) with its plan's tables, and the dense operands, K columns wide.
+struct hpspmm_layer_grad_args {
+  int rows, K, n_chunks, S;
+  int n_chunk_blocks;   // filled in by the launcher
+  int keep;             // L2 evict-last on the gathers of dC
+  const int32_t* row_ptr;
+  const int32_t* col_idx;
+  const int32_t* perm;
+  const float* vals;    // weights in A's order
+  const float* dC;
+  const float* H;
+  float* dH;
+  float* dA;
+  const int4* rec;
+  const int2* nz;
+  float* carry;
+  int32_t* counter;
+};
+// whether the one kernel beats the three it replaces; even: rows of even length (hpspmm_even_rows)
+bool hpspmm_layer_grad_pays(const hpspmm_ctx* ctx, int64_t nnz, bool even);
+int hpspmm_layer_grad_launch(hpspmm_ctx* ctx, const hpspmm_layer_grad_args& a, cudaStream_t s);
+
 static inline int hpspmm_set_err(hpspmm_ctx* ctx, int status, const char* what, cudaError_t e) {
   if (ctx) snprintf(ctx->err, sizeof(ctx->err), "%s: %s", what, cudaGetErrorString(e));
   return status;

@@ -78,12 +78,10 @@ Tensor forward(const Tensor& H, const Tensor& vals, int64_t id) {
   const c10::cuda::CUDAGuard guard(h.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
   Tensor C = at::empty({e->M, h.size(1)}, h.options());
-  Tensor old;
   std::lock_guard<std::mutex> lock(e->use);
   check_open(*e, id);
-  sync_values(*e, v, stream, old);
-  check(*e, hpspmm_layer_forward(e->ctx, e->layer, h.size(1), h.const_data_ptr<float>(), C.mutable_data_ptr<float>(), stream),
-        "hpspmm_layer_forward");
+  check(*e, hpspmm_layer_forward_values(e->ctx, e->layer, h.size(1), v.const_data_ptr<float>(), h.const_data_ptr<float>(),
+                                        C.mutable_data_ptr<float>(), stream), "hpspmm_layer_forward");
   return C;
 }
 
@@ -117,6 +115,28 @@ Tensor backward_weights(const Tensor& grad, const Tensor& H, int64_t id) {
   return dA;
 }
 
+// Both gradients: one pass over the transpose where the library has a kernel for the width, else the two above.
+std::tuple<Tensor, Tensor> backward(const Tensor& grad, const Tensor& H, const Tensor& vals, int64_t id) {
+  auto e = entry_of(id);
+  const Tensor dC = require_cuda_f32(grad, e->M, "dC"), h = require_cuda_f32(H, e->N, "H");
+  const Tensor v = require_weights(vals, *e, grad.device());
+  TORCH_CHECK(h.size(1) == dC.size(1) && h.device() == dC.device(), "hpspmm: dC and H differ in width or device");
+  {
+    const c10::cuda::CUDAGuard guard(dC.device());
+    Tensor dH = at::empty({e->N, dC.size(1)}, dC.options()), dA = at::empty({e->nnz}, dC.options());
+    std::lock_guard<std::mutex> lock(e->use);
+    check_open(*e, id);
+    const int st = hpspmm_layer_backward(e->ctx, e->layer, dC.size(1), v.const_data_ptr<float>(), dC.const_data_ptr<float>(),
+                                         h.const_data_ptr<float>(), dH.mutable_data_ptr<float>(),
+                                         dA.mutable_data_ptr<float>(), c10::cuda::getCurrentCUDAStream().stream());
+    if (st != HPSPMM_ERR_UNSUPPORTED) {
+      check(*e, st, "hpspmm_layer_backward");
+      return {dH, dA};
+    }
+  }
+  return {backward_features(dC, v, id), backward_weights(dC, h, id)};
+}
+
 // the registered operators, for calls that go through the dispatcher (tracing, fake tensors)
 using Op = Tensor(const Tensor&, const Tensor&, int64_t);
 c10::TypedOperatorHandle<Op> find_op(const char* name) {
@@ -135,6 +155,12 @@ const c10::TypedOperatorHandle<Op>& op_weights() {
   return op;
 }
 
+using OpBoth = std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, int64_t);
+const c10::TypedOperatorHandle<OpBoth>& op_both() {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("hpspmm::layer_backward", "").typed<OpBoth>();
+  return op;
+}
+
 struct LayerFunction : public torch::autograd::Function<LayerFunction> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& H, const Tensor& vals, int64_t id) {
     ctx->saved_data["id"] = id;
@@ -148,8 +174,13 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
     const int64_t id = ctx->saved_data["id"].toInt();
     Tensor dH, dvals;
     if (grads[0].defined()) {
-      if (ctx->needs_input_grad(0)) dH = op_features().call(grads[0], saved[1], id);
-      if (ctx->needs_input_grad(1)) dvals = op_weights().call(grads[0], saved[0], id);
+      const bool features = ctx->needs_input_grad(0), weights = ctx->needs_input_grad(1);
+      if (features && weights)
+        std::tie(dH, dvals) = op_both().call(grads[0], saved[0], saved[1], id);
+      else if (features)
+        dH = op_features().call(grads[0], saved[1], id);
+      else if (weights)
+        dvals = op_weights().call(grads[0], saved[0], id);
     }
     return {dH, dvals, Tensor()};
   }
@@ -176,10 +207,32 @@ Tensor gradient_autograd(const Tensor& a, const Tensor& b, int64_t id) {
   return OP().call(a, b, id);
 }
 
+struct NoDerivativeOfBoth : public torch::autograd::Function<NoDerivativeOfBoth> {
+  static torch::autograd::variable_list forward(torch::autograd::AutogradContext*, const Tensor& dC, const Tensor& H,
+                                                const Tensor& vals, int64_t id) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto out = op_both().call(dC, H, vals, id);
+    return {std::get<0>(out), std::get<1>(out)};
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext*, torch::autograd::variable_list) {
+    TORCH_CHECK(false, "hpspmm: no derivative of ", op_both().schema().name(),
+                " is implemented (a second derivative of the layer)");
+  }
+};
+std::tuple<Tensor, Tensor> both_autograd(const Tensor& dC, const Tensor& H, const Tensor& vals, int64_t id) {
+  if (at::GradMode::is_enabled() && (dC.requires_grad() || H.requires_grad() || vals.requires_grad())) {
+    auto out = NoDerivativeOfBoth::apply(dC, H, vals, id);
+    return {out[0], out[1]};
+  }
+  at::AutoDispatchBelowADInplaceOrView below;
+  return op_both().call(dC, H, vals, id);
+}
+
 TORCH_LIBRARY(hpspmm, m) {
   m.def("layer_forward(Tensor H, Tensor vals, int layer_id) -> Tensor");
   m.def("layer_backward_features(Tensor dC, Tensor vals, int layer_id) -> Tensor");
   m.def("layer_backward_weights(Tensor dC, Tensor H, int layer_id) -> Tensor");
+  m.def("layer_backward(Tensor dC, Tensor H, Tensor vals, int layer_id) -> (Tensor, Tensor)");
 }
 // a CPU tensor reaches the same functions, which refuse it by name
 #define HPSPMM_IMPL(KEY)                                  \
@@ -187,6 +240,7 @@ TORCH_LIBRARY(hpspmm, m) {
     m.impl("layer_forward", forward);                     \
     m.impl("layer_backward_features", backward_features); \
     m.impl("layer_backward_weights", backward_weights);   \
+    m.impl("layer_backward", backward);                   \
   }
 HPSPMM_IMPL(CUDA)
 HPSPMM_IMPL(CPU)
@@ -194,6 +248,7 @@ TORCH_LIBRARY_IMPL(hpspmm, Autograd, m) {
   m.impl("layer_forward", forward_autograd);
   m.impl("layer_backward_features", gradient_autograd<op_features>);
   m.impl("layer_backward_weights", gradient_autograd<op_weights>);
+  m.impl("layer_backward", both_autograd);
 }
 
 void register_layer(int64_t id, int64_t ctx, int64_t layer, int64_t M, int64_t N, int64_t nnz, const Tensor& vals) {

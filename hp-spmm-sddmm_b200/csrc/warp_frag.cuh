@@ -135,4 +135,42 @@ __device__ __forceinline__ void combine_groups(const float (&a)[VEC], float (&ou
   for (int x = 0; x < S::KEEP; ++x) out[x] = k[x];
 }
 
+// log2 of a power of two
+__host__ __device__ constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
+
+// Sums p[0..U-1] over the W lanes of a group.  While values remain to be split, each exchange hands the partner
+// half of them; afterwards lane l holds in the return value the total of entry `which(l)`.
+template <int U, int W>
+__device__ __forceinline__ float reduce_transposed(float (&p)[U], int lane) {
+  int n = U, d = 1;
+#pragma unroll
+  for (int s = 0; s < ilog2(U); ++s) {
+    const bool up = (lane & d) != 0;
+    n >>= 1;
+#pragma unroll
+    for (int i = 0; i < U / 2; ++i)
+      if (i < n) {
+        const float send = up ? p[i] : p[i + n];
+        const float keep = up ? p[i + n] : p[i];
+        p[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+      }
+    d <<= 1;
+  }
+  float total = p[0];
+#pragma unroll
+  for (int s = ilog2(U); s < ilog2(W); ++s) {
+    total += __shfl_xor_sync(0xffffffffu, total, d);
+    d <<= 1;
+  }
+  return total;
+}
+
+template <int U>
+__device__ __forceinline__ int reduced_entry(int l) {   // the entry whose total lane l < U holds: l with its bits reversed
+  int w = 0;
+#pragma unroll
+  for (int s = 0; s < ilog2(U); ++s) w |= ((l >> s) & 1) << (ilog2(U) - 1 - s);
+  return w;
+}
+
 }  // namespace hpspmm

@@ -4,9 +4,9 @@
     C = layer(H)                                              # C = A·H, differentiable in H and in vals
     C.sum().backward()                                        # dH = Aᵀ·dC (SpMM), dvals = SDDMM(dC, H)
 
-Three operators are registered under the namespace ``hpspmm`` (``layer_forward``,
-``layer_backward_features``, ``layer_backward_weights``) by csrc/torch_binding.cpp, with an autograd
-formula that chains them; the shape functions for tracing are below, so the layer can sit inside a
+Four operators are registered under the namespace ``hpspmm`` (``layer_forward``,
+``layer_backward_features``, ``layer_backward_weights``, and ``layer_backward`` for both gradients at
+once) by csrc/torch_binding.cpp, with an autograd formula that chains them; the shape functions for tracing are below, so the layer can sit inside a
 compiled or exported module.  Every operator calls ``hpspmm_layer_*`` of libhpspmm.so on the current
 CUDA stream of the input's device; a CPU tensor is rejected (there is no fallback).  PyTorch supplies
 memory, streams and the autograd tape only.
@@ -30,6 +30,7 @@ _C = load_extension("_hpspmm_torch", os.path.join(PKG_DIR, "lib", "_hpspmm_torch
 layer_forward = torch.ops.hpspmm.layer_forward.default
 layer_backward_features = torch.ops.hpspmm.layer_backward_features.default
 layer_backward_weights = torch.ops.hpspmm.layer_backward_weights.default
+layer_backward = torch.ops.hpspmm.layer_backward.default
 
 
 def _entry(layer_id):
@@ -52,6 +53,12 @@ def _(dC, vals, layer_id):
 @torch.library.register_fake("hpspmm::layer_backward_weights")
 def _(dC, H, layer_id):
     return dC.new_empty((_entry(layer_id)["nnz"],))
+
+
+@torch.library.register_fake("hpspmm::layer_backward")
+def _(dC, H, vals, layer_id):
+    e = _entry(layer_id)
+    return dC.new_empty((e["N"], dC.shape[1])), dC.new_empty((e["nnz"],))
 
 
 class TorchLayer:

@@ -279,6 +279,11 @@ HPSPMM_API int hpspmm_csr_transpose(hpspmm_ctx* ctx, int64_t M, int64_t N, int64
  *   backward_features  dH = A^T * dC      dC is M x K, dH is N x K
  *   backward_weights   dA[j] = dot(dC[row(j),:], H[col[j],:])   (nnz values, CSR order)
  *   update_values      new vals pointer; the transpose's values are re-gathered from it
+ *   forward_values     forward with weights given for this call; the handle's own stay as they are
+ *   backward           both gradients at once for weights given in A's order, in one pass over the transpose;
+ *                      HPSPMM_ERR_UNSUPPORTED, with nothing launched, where one launch does not cover the rows of dC
+ *                      (more than 256 columns, 128 where rows are only 4-byte aligned) or would be slower than two
+ *                      (matrices whose weights fill the L2 cache): call the other two then
  * The best chunk size depends on K, so the handle keeps one pair of plans per width class
  * (K <= 32, K <= 64, wider).  create builds the pair for max_K and synchronises the stream;
  * the first product at a width of another class builds that pair (synchronising once more);
@@ -303,6 +308,12 @@ HPSPMM_API int hpspmm_layer_backward_features(hpspmm_ctx* ctx, hpspmm_layer* lay
 HPSPMM_API int hpspmm_layer_backward_weights(hpspmm_ctx* ctx, hpspmm_layer* layer,
                                              int64_t K, const float* dC, const float* H,
                                              float* dA, hpspmm_stream stream);
+HPSPMM_API int hpspmm_layer_forward_values(hpspmm_ctx* ctx, hpspmm_layer* layer, int64_t K,
+                                           const float* vals, const float* H, float* C,
+                                           hpspmm_stream stream);
+HPSPMM_API int hpspmm_layer_backward(hpspmm_ctx* ctx, hpspmm_layer* layer, int64_t K, const float* vals,
+                                     const float* dC, const float* H, float* dH, float* dA,
+                                     hpspmm_stream stream);
 HPSPMM_API int hpspmm_layer_update_values(hpspmm_ctx* ctx, hpspmm_layer* layer,
                                           const float* vals, hpspmm_stream stream);
 

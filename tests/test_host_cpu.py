@@ -133,11 +133,11 @@ def test_context_needs_a_gpu_or_fails_loudly(pkg):
 
 
 def test_torch_front_end_registers_and_has_no_cpu_path(pkg):
-    """The autograd front-end imports without a GPU, registers its three operators, and refuses CPU tensors."""
+    """The autograd front-end imports without a GPU, registers its operators, and refuses CPU tensors."""
     import importlib
     import torch
     ops = importlib.import_module(pkg.__name__ + ".torch_ops")
-    for name in ("layer_forward", "layer_backward_features", "layer_backward_weights"):
+    for name in ("layer_forward", "layer_backward_features", "layer_backward_weights", "layer_backward"):
         assert hasattr(torch.ops.hpspmm, name)
     rp = torch.zeros(5, dtype=torch.int32)
     ci = torch.zeros(0, dtype=torch.int32)
@@ -154,6 +154,8 @@ def test_torch_front_end_registers_and_has_no_cpu_path(pkg):
             assert ops.layer_forward(H, torch.empty(9), -1).shape == (7, 32)
             assert ops.layer_backward_features(torch.empty(7, 32), torch.empty(9), -1).shape == (4, 32)
             assert ops.layer_backward_weights(torch.empty(7, 32), H, -1).shape == (9,)
+            both = ops.layer_backward(torch.empty(7, 32), H, torch.empty(9), -1)
+            assert both[0].shape == (4, 32) and both[1].shape == (9,)
     finally:
         del ops._layers[-1]
 

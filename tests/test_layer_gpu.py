@@ -6,7 +6,7 @@ import importlib
 import numpy as np
 import pytest
 
-from helpers import check_against_f64
+from helpers import check_against_f64, guarded_output
 
 pytestmark = pytest.mark.gpu
 
@@ -111,6 +111,43 @@ def test_empty_layer(gpu_ctx, pkg):
         b.free()
 
 
+# every instance of the one-pass kernel: full and ragged widths of 16-, 8- and 4-byte vectors, and the first widths it refuses
+@pytest.mark.parametrize("K", [4, 16, 28, 32, 52, 64, 96, 116, 128, 160, 196, 256, 2, 6, 14, 30, 46, 62, 94, 126, 190, 254,
+                               1, 3, 7, 15, 23, 31, 47, 63, 95, 127, 129, 260])
+def test_both_gradients_in_one_pass(gpu_ctx, pkg, oracle, K):
+    """hpspmm_layer_backward against the oracle, rows split over several carry groups and empty rows among them."""
+    ctx = gpu_ctx
+    for g in (pkg.gen_rmat(10, 24, seed=41), _rect_graph(pkg, 700, 333, 42)):
+        M, N, nnz = g["M"], g["N"], g["nnz"]
+        H = pkg.host_fill_uniform(N * K, 41, 1, -1.0, 1.0).reshape(N, K)
+        dC = pkg.host_fill_uniform(M * K, 41, 2, -1.0, 1.0).reshape(M, K)
+        v2 = pkg.host_fill_uniform(nnz, 41, 3, -2.0, 2.0)
+        bufs = [ctx.upload(a) for a in (g["row_ptr"], g["col_idx"], g["vals"], H, dC, v2)]
+        d_rp, d_ci, d_v, d_H, d_dC, d_v2 = bufs
+        layer = pkg.Layer(ctx, M, N, nnz, d_rp, d_ci, d_v, 260)
+        out_H, p_H, read_H = guarded_output(ctx, (N, K))
+        out_A, p_A, read_A = guarded_output(ctx, (nnz,))
+
+        def call(width=K, a=p_A):
+            return ctx.lib.hpspmm_layer_backward(ctx.handle, layer.handle, width, d_v2.ptr, d_dC.ptr, d_H.ptr, p_H, a, None)
+
+        if K in (129, 260):
+            assert call() == pkg.ERR_UNSUPPORTED
+        else:
+            for _ in range(2):                  # the counters of split rows are zero again afterwards
+                assert call() == 0
+                ctx.stream_sync()
+                rpt, cit, vt, _ = oracle.csr_transpose(M, N, g["row_ptr"], g["col_idx"], v2)
+                ref, abs_sum = oracle.spmm_f64(rpt, cit, vt, dC)
+                check_against_f64(read_H(), ref, abs_sum, "dH")
+                ref, abs_sum = oracle.sddmm_f64(g["row_ptr"], g["col_idx"], dC, H)
+                check_against_f64(read_A(), ref, abs_sum, "dA")
+            assert call(width=261) == pkg.ERR_INVALID and call(a=None) == pkg.ERR_INVALID
+        layer.close()
+        for b in bufs + [out_H, out_A]:
+            b.free()
+
+
 @pytest.mark.parametrize("K", [64, 48])
 def test_torch_autograd_front_end(pkg, oracle, K):
     torch = pytest.importorskip("torch")
@@ -150,6 +187,9 @@ def test_torch_autograd_front_end(pkg, oracle, K):
 
     # registration: schema and shape function agree with the real operator
     torch.library.opcheck(ops.layer_forward, (H.detach(), vals.detach(), layer.layer_id),
+                          test_utils=("test_schema", "test_faketensor"))
+
+    torch.library.opcheck(ops.layer_backward, (G, H.detach(), vals.detach(), layer.layer_id),
                           test_utils=("test_schema", "test_faketensor"))
 
     # no CPU path

@@ -60,6 +60,10 @@ def test_second_derivatives_are_refused(work):
         with torch.no_grad():
             assert not op(dC, other, work.layer.layer_id).requires_grad
         assert not op(dC.detach(), other, work.layer.layer_id).requires_grad
+    for out in work.ops.layer_backward(dC, work.H, work.v, work.layer.layer_id):
+        assert out.requires_grad
+        with pytest.raises(RuntimeError, match="no derivative"):
+            out.sum().backward()
 
 
 def test_weights_that_cannot_be_used_are_refused_every_time(work):
