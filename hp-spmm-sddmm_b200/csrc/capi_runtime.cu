@@ -5,6 +5,7 @@
 #include <atomic>
 #include <new>
 
+#include "device_utils.cuh"
 #include "hpspmm_internal.h"
 
 // Allocation-failure seam for tests: g_fail_skip allocations still succeed, then g_fail_count fail.
@@ -309,6 +310,7 @@ int hpspmm_ensure_stage(hpspmm_ctx* ctx, size_t bytes) {
 // ---- dense factories -------------------------------------------------------------------
 
 __global__ void fill_f32_kernel(float* __restrict__ x, int64_t n, float v) {
+  hpspmm::chain_grid();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i] = v;
 }
@@ -332,7 +334,7 @@ int hpspmm_fill_f32(hpspmm_ctx* ctx, float* dev_ptr, int64_t count, float value,
   int64_t blocks = (count + 1023) / 1024;
   const int64_t cap = (int64_t)ctx->sm_count * 16;
   if (blocks > cap) blocks = cap;
-  fill_f32_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(dev_ptr, count, value);
+  hpspmm_launch(fill_f32_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, dev_ptr, count, value);
   ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;

@@ -27,6 +27,7 @@ spmm_coo_warp_kernel(int64_t nnz, int S, const int* __restrict__ row_idx, const 
   __shared__ int2 cv_tiles[BT / 32][STAGES][T];
   __shared__ int row_tiles[BT / 32][STAGES][T];
 
+  chain_grid();
   const int lane = threadIdx.x & 31;
   const int g = lane / W, l = lane % W;
   const int64_t worker = ((int64_t)blockIdx.x * BT + threadIdx.x) >> 5;
@@ -192,8 +193,8 @@ int launch_coo(hpspmm_ctx* ctx, const coo_args& a, cudaStream_t s) {
   const int64_t slabs = (a.cols + CW - 1) / CW;
   if (blocks > 2147483647ll || slabs > 65535) return HPSPMM_ERR_UNSUPPORTED;
   if (!hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
-  spmm_coo_warp_kernel<VEC, W, R, U, KS, BT, MINB><<<dim3((unsigned)blocks, (unsigned)slabs), BT, 0, s>>>(
-      a.nnz, a.S, a.row_idx, a.col_idx, a.vals, a.B, a.C, a.K, a.off, a.cols);
+  hpspmm_launch(spmm_coo_warp_kernel<VEC, W, R, U, KS, BT, MINB>, dim3((unsigned)blocks, (unsigned)slabs), BT, 0, s,
+                a.nnz, a.S, a.row_idx, a.col_idx, a.vals, a.B, a.C, a.K, a.off, a.cols);
   ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;

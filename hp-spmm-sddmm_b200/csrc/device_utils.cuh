@@ -105,4 +105,11 @@ __device__ __forceinline__ unsigned subwarp_mask() {
   return ((1u << W) - 1u) << (lane & ~(unsigned)(W - 1));
 }
 
+// The first statement of every kernel that hpspmm_launch starts: waits until all that came before in the stream is done
+// and visible.
+// (No griddepcontrol.launch_dependents: with it the next kernel's blocks move in as soon as all of this one have started,
+// and a grid of less than a wave then crowds onto the SMs that drained first.  334 K entries without a plan, K = 256: 39.9 us
+// with ordinary launches, 38.0 like this, 44.7 with the early start; never ahead by more than 2 %.)
+__device__ __forceinline__ void chain_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace hpspmm

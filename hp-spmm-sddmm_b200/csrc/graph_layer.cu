@@ -9,6 +9,7 @@
 // chunk tables, Aᵀ, and the permutation that carries new edge weights into Aᵀ.
 #include <new>
 
+#include "device_utils.cuh"
 #include "hpspmm_internal.h"
 
 struct hpspmm_layer {
@@ -36,6 +37,7 @@ constexpr int kThreads = 256;
 
 __global__ void gather_by_perm_kernel(int64_t n, const int* __restrict__ perm, const float* __restrict__ src,
                                       float* __restrict__ dst) {
+  hpspmm::chain_grid();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride)
     dst[t] = __ldg(src + perm[t]);
@@ -225,8 +227,8 @@ int hpspmm_layer_update_values(hpspmm_ctx* ctx, hpspmm_layer* g, const float* va
   int64_t blocks = (g->nnz + kThreads - 1) / kThreads;
   const int64_t cap = (int64_t)ctx->sm_count * 32;
   if (blocks > cap) blocks = cap;
-  gather_by_perm_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(g->nnz, g->perm, vals,
-                                                                                g->vals_t);
+  hpspmm_launch(gather_by_perm_kernel, (unsigned)blocks, kThreads, 0, (cudaStream_t)stream, g->nnz, g->perm, vals,
+                g->vals_t);
   ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;

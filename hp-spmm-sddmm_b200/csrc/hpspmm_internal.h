@@ -255,6 +255,24 @@ int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_
 int hpspmm_order_records(hpspmm_ctx* ctx, int64_t n_chunks, const int32_t* order, const int4* rec_in, int4* rec,
                          cudaStream_t stream);
 
+#if defined(__CUDACC__)
+// Launches a kernel whose blocks may be set up before the kernel in front of it in the stream has ended (programmatic
+// stream serialisation).  The kernel begins with chain_grid() (device_utils.cuh), so it touches no memory earlier than an
+// ordinary launch would; what is saved is the time from the end of one kernel to the first instruction of the next.
+// Passes back to back, ordinary launches -> these, us: product of 67.6 K entries, K = 32 10.6 -> 9.4, 1 M, K = 32 16.8 -> 14.4;
+// without a plan 300 K, K = 100 24.3 -> 22.2, 1 M, K = 32 (three launches) 25.0 -> 18.8, 4 M, K = 64 101.2 -> 95.9; SDDMM of
+// 100 K entries, K = 64 9.4 -> 7.8, 280 K, K = 160 18.9 -> 16.5; COO product of 280 K, K = 160 with its fill 20.9 -> 17.2.
+template <typename... P, typename... A>
+static inline void hpspmm_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid, c.blockDim = block, c.dynamicSmemBytes = smem, c.stream = s, c.attrs = &attr, c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);   // (the caller asks cudaGetLastError)
+}
+#endif
+
 // ---- counter-based PRNG shared by host and device --------------------------------------
 // splitmix64 finaliser over (seed, stream, index); 24 high bits -> [0, 1).
 #if defined(__CUDACC__)

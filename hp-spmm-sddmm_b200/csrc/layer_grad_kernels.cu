@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(BT, MINB) layer_grad_kernel(const __grid_const
   __shared__ int perms[BT / 32][STAGES][T];
   __shared__ int meta[BT / 32][8];
 
+  chain_grid();
   if ((int)blockIdx.x >= a.n_chunk_blocks) {
     zero_empty_rows<KS>(a.rows, a.K, a.row_ptr, a.dH, blockIdx.x - a.n_chunk_blocks, gridDim.x - a.n_chunk_blocks, BT);
     return;
@@ -218,7 +219,7 @@ int launch(hpspmm_ctx* ctx, hpspmm_layer_grad_args a, cudaStream_t s) {
   const int cap = ctx->sm_count * 8;
   if (n_zero_blocks > cap) n_zero_blocks = cap;
   const unsigned grid = (unsigned)(a.n_chunk_blocks + n_zero_blocks);
-  layer_grad_kernel<VEC, W, R, U, KS, BT, MINB><<<grid, BT, 0, s>>>(a);
+  hpspmm_launch(layer_grad_kernel<VEC, W, R, U, KS, BT, MINB>, grid, BT, 0, s, a);
   ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;

@@ -39,6 +39,7 @@ sddmm_warp_kernel(int n_chunks, int ld, int off0, int cols, int add, int keep_y,
   static_assert(T % BATCH == 0 && (U <= W || W == 1), "batch must tile the staged tile; a lane holds one total");
   __shared__ int tiles[BT / 32][STAGES][T];
 
+  chain_grid();
   const int lane = threadIdx.x & 31;
   const int g = lane / W;
   const int l = lane % W;
@@ -273,8 +274,8 @@ int launch_sddmm(hpspmm_ctx* ctx, const sddmm_args& a, cudaStream_t s) {
   constexpr int BT = 64;
   const unsigned grid = (unsigned)((a.n_chunks + BT / 32 - 1) / (BT / 32));
   if (a.cols > VEC * W * R || !hpspmm_shape_covers(VEC, W, R, a.cols)) return HPSPMM_ERR_INVALID;
-  sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, SERIAL><<<grid, BT, 0, s>>>(
-      a.n_chunks, a.K, a.off, a.cols, a.off > 0 ? 1 : 0, a.keep_y, a.col_idx, a.X, a.Y, a.out, a.rec, a.nz);
+  hpspmm_launch(sddmm_warp_kernel<VEC, W, R, U, KS, HINT, BT, MINB, SERIAL>, grid, BT, 0, s, a.n_chunks, a.K, a.off,
+                a.cols, a.off > 0 ? 1 : 0, a.keep_y, a.col_idx, a.X, a.Y, a.out, a.rec, a.nz);
   ctx->launches++;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;

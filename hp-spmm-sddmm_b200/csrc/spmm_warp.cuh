@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
   __shared__ int2 tiles[BT / 32][STAGES][T];
   __shared__ int meta[BT / 32][8];
 
+  chain_grid();
   if ((int)blockIdx.x >= a.n_chunk_blocks) {
     if (blockIdx.y == 0 && a.slab0 == 0 && a.off == 0) {
       if (!LIST)
@@ -454,9 +455,9 @@ int launch_spmm_shape(hpspmm_ctx* ctx, hpspmm_spmm_args a, bool shared_counters,
     const int ny = slabs - s < step ? slabs - s : step;
     const dim3 g((unsigned)grid, (unsigned)ny);
     if (a.nz != nullptr)
-      spmm_warp_kernel<VEC, W, R, U, KS, BT, MINB, HINT, true><<<g, BT, 0, stream>>>(a);
+      hpspmm_launch(spmm_warp_kernel<VEC, W, R, U, KS, BT, MINB, HINT, true>, g, BT, 0, stream, a);
     else   // (a runtime stride serves every width)
-      spmm_warp_kernel<VEC, W, R, U, 0, BT, (MINB < 16 ? MINB : 16), true, false><<<g, BT, 0, stream>>>(a);
+      hpspmm_launch(spmm_warp_kernel<VEC, W, R, U, 0, BT, (MINB < 16 ? MINB : 16), true, false>, g, BT, 0, stream, a);
     ctx->launches++;
   }
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());

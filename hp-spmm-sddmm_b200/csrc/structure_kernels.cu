@@ -2,6 +2,7 @@
 // expansion (the device form of spmm/mm/spmm_common.cpp:210-226), and a deterministic CSR
 // transpose (stable LSD radix sort of the entry positions by column index).  All outputs
 // are integer-exact and independent of thread scheduling.
+#include "device_utils.cuh"
 #include "hpspmm_internal.h"
 
 namespace {
@@ -617,6 +618,7 @@ int row_tile_size(int64_t M) {
 __global__ void __launch_bounds__(kThreads)
 row_tile_count_kernel(int M, int tile, const int* __restrict__ row_ptr, int* __restrict__ counts, int* __restrict__ clear,
                       int64_t n_clear) {
+  hpspmm::chain_grid();
   for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n_clear; i += (int64_t)gridDim.x * kThreads) clear[i] = 0;
   const int64_t r0 = (int64_t)blockIdx.x * tile;
   int total = 0;
@@ -649,6 +651,7 @@ row_tile_list_kernel(int M, int nnz, int tile, int S, int n_chunks, const int* _
                      const hpspmm_structure_tables t) {
   constexpr int kWarpsHere = kThreads / 32;
   __shared__ int part[kWarpsHere];
+  hpspmm::chain_grid();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int before = 0;
   for (int i = threadIdx.x; i < (int)blockIdx.x; i += kThreads) before += __ldg(counts + i);
@@ -739,9 +742,9 @@ int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_
                            int32_t* clear, int64_t n_clear) {
   const int tile = row_tile_size(M);
   const unsigned blocks = (unsigned)hpspmm_row_tiles(M);
-  row_tile_count_kernel<<<blocks, kThreads, 0, stream>>>((int)M, tile, row_ptr, counts, clear, n_clear);
-  row_tile_list_kernel<<<blocks, kThreads, 0, stream>>>((int)M, (int)nnz, tile, S, (int)n_chunks, row_ptr, counts, nz,
-                                                        rec_out, tables);
+  hpspmm_launch(row_tile_count_kernel, blocks, kThreads, 0, stream, (int)M, tile, row_ptr, counts, clear, n_clear);
+  hpspmm_launch(row_tile_list_kernel, blocks, kThreads, 0, stream, (int)M, (int)nnz, tile, S, (int)n_chunks, row_ptr, counts, nz,
+                rec_out, tables);
   ctx->launches += 2;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;
