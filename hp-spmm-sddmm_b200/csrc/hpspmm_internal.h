@@ -234,8 +234,9 @@ int hpspmm_order_chunks_by_cost(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t n
                                 cudaStream_t stream);
 
 // Builds the structure a product walks, in two launches: the list of rows that hold entries (nz, hpspmm_nz_bytes(M)
-// bytes, with sentinels (M, INT_MAX) at its end) and one record per chunk in matrix order (rec_out, 2 * n_chunks int4).
-// counts: hpspmm_row_tiles(M) ints of scratch.  The first launch also sets `n_clear` ints at `clear` to zero.  The arrays of `tables` are
+// bytes, with sentinels (M, INT_MAX) at its end) and one record per chunk (rec_out, 2 * n_chunks int4): in matrix order with
+// `tables`, without them the chunks that lie inside one row after all others.
+// counts: hpspmm_row_tile_ints(M) ints of scratch.  The first launch also sets `n_clear` ints at `clear` to zero.  The arrays of `tables` are
 // filled as well where they are given (a plan exposes them), and split_count receives the number of chunks that
 // begin inside a row.
 struct hpspmm_structure_tables {
@@ -246,7 +247,7 @@ struct hpspmm_structure_tables {
   int32_t* nz_end;
   int* split_count;
 };
-int64_t hpspmm_row_tiles(int64_t M);
+int64_t hpspmm_row_tile_ints(int64_t M);
 size_t hpspmm_nz_bytes(int64_t M);
 int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr, int32_t S, int64_t n_chunks,
                            int2* nz, int4* rec_out, int32_t* counts, const hpspmm_structure_tables& tables, cudaStream_t stream,

@@ -470,7 +470,7 @@ extern "C" int hpspmm_sddmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, in
     int32_t S = (opts && opts->chunk_nnz > 0) ? opts->chunk_nnz : hpspmm_default_chunk_nnz(K, nnz);
     S = (S + 31) / 32 * 32;
     const int64_t n_chunks = (nnz + S - 1) / S;
-    const size_t b_tiles = align_up((size_t)hpspmm_row_tiles(M) * 4, 256);
+    const size_t b_tiles = align_up((size_t)hpspmm_row_tile_ints(M) * 4, 256);
     const size_t b_rec = align_up((size_t)n_chunks * 32, 256);
     int st = hpspmm_ensure_scratch(ctx, b_tiles + b_rec + hpspmm_nz_bytes(M));
     if (st != HPSPMM_OK) return st;

@@ -673,7 +673,7 @@ struct planless_layout {
     n_counter = (n_chunks + 1) * hpspmm_counter_slabs(K);
     counter = take((size_t)n_counter * 4);
     carry = take((size_t)(n_chunks + 1) * (size_t)K * 4);
-    tiles = search ? 0 : take((size_t)hpspmm_row_tiles(M) * 4);
+    tiles = search ? 0 : take((size_t)hpspmm_row_tile_ints(M) * 4);
     rec = search ? 0 : take((size_t)(n_chunks + 1) * 32);
     nz = search ? 0 : take(hpspmm_nz_bytes(M));
   }
@@ -714,7 +714,7 @@ int hpspmm_plan_create(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_t nnz, const
   const size_t b_rec = align_up((size_t)(p->n_chunks + 1) * 32, 256);
   // the builders' own scratch lives in the context and is free again afterwards
   const size_t b_sort = hpspmm_order_scratch_bytes(p->n_chunks);
-  const size_t b_tiles = align_up((size_t)hpspmm_row_tiles(M) * 4, 256);
+  const size_t b_tiles = align_up((size_t)hpspmm_row_tile_ints(M) * 4, 256);
   p->bytes = 4 * b_int + b_cval + b_count + 2 * b_row + b_nz + b_rec;
   char* base = nullptr;
   cudaError_t e = hpspmm_device_malloc((void**)&base, p->bytes);

@@ -602,8 +602,8 @@ int build_ordered_row_ptr(hpspmm_ctx* ctx, int64_t M, const int32_t* row_ptr, co
 
 // ---- the structure a product walks ---------------------------------------------------------------
 // Rows are cut into at most kRowTiles tiles.  The first kernel counts the rows of every tile that hold entries; in
-// the second, a block adds up the counts of the tiles before its own (at most 4 KB), ranks its rows and writes
-// them, and the thread that owns a row writes the record of every chunk whose cut falls into it.  Two launches
+// the second, a block adds up the counts of the tiles before its own (at most 8 KB), ranks its rows and writes
+// them, and then the record of every chunk whose cut falls into them.  Two launches
 // instead of a flag pass, a three-kernel scan, a scatter, a binary search per chunk and an index pass.
 namespace {
 
@@ -615,28 +615,74 @@ int row_tile_size(int64_t M) {
   return (int)(t < kThreads ? kThreads : t);
 }
 
+// x / S for 0 <= x < 2^31 as a multiplication (Granlund and Montgomery, Division by Invariant Integers Using
+// Multiplication, 1994): with l = ceil(log2 S), floor(x * (floor(2^(31 + l) / S) + 1) / 2^(31 + l)).  S >= 32.
+struct chunk_size {
+  int S, shift;
+  unsigned factor;
+  explicit chunk_size(int32_t s) : S(s), shift(0) {
+    int l = 0;
+    while (((int64_t)1 << l) < s) ++l;
+    factor = (unsigned)(((uint64_t)1 << (31 + l)) / (uint64_t)s + 1);
+    shift = l - 1;
+  }
+  __device__ __forceinline__ int quotient(int x) const { return (int)(__umulhi((unsigned)x, factor) >> shift); }
+};
+
+// Cuts c * S inside a row [s, e): the first one and how many.  All chunks that begin at one of them but the last lie
+// inside the row (its pieces).
+struct row_cuts {
+  int lo, n;
+  __device__ __forceinline__ row_cuts(int s, int e, const chunk_size& cs) {
+    lo = s == 0 ? 0 : cs.quotient(s - 1) + 1;   // (s + S - 1 would overflow for the largest S)
+    n = e > s ? cs.quotient(e - 1) - lo + 1 : 0;
+  }
+  __device__ __forceinline__ int pieces() const { return n > 1 ? n - 1 : 0; }
+};
+
+// PIECES: also the number of pieces of long rows per tile, behind the counts of rows
+template <bool PIECES>
 __global__ void __launch_bounds__(kThreads)
-row_tile_count_kernel(int M, int tile, const int* __restrict__ row_ptr, int* __restrict__ counts, int* __restrict__ clear,
-                      int64_t n_clear) {
+row_tile_count_kernel(int M, int tile, const chunk_size cs, const int* __restrict__ row_ptr, int* __restrict__ counts,
+                      int* __restrict__ clear, int64_t n_clear) {
+  __shared__ int part[kThreads / 32];
   hpspmm::chain_grid();
   for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n_clear; i += (int64_t)gridDim.x * kThreads) clear[i] = 0;
   const int64_t r0 = (int64_t)blockIdx.x * tile;
-  int total = 0;
+  int total = 0, pieces = 0;
   for (int i = 0; i < tile && r0 + i < M; i += kThreads) {
     const int64_t r = r0 + i + threadIdx.x;
-    total += __syncthreads_count(r < M && __ldg(row_ptr + r + 1) > __ldg(row_ptr + r));
+    int s = 0, e = 0;
+    if (r < M) {
+      s = __ldg(row_ptr + r);
+      e = __ldg(row_ptr + r + 1);
+    }
+    total += __syncthreads_count(e > s);
+    if (PIECES) pieces += row_cuts(s, e, cs).pieces();
   }
-  if (threadIdx.x == 0) counts[blockIdx.x] = total;
+  if (PIECES) {
+    pieces = __reduce_add_sync(0xffffffffu, pieces);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = pieces;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    counts[blockIdx.x] = total;
+    if (PIECES) {
+      for (int w = 1; w < kThreads / 32; ++w) pieces += part[w];
+      counts[gridDim.x + blockIdx.x] = pieces;
+    }
+  }
 }
 
-// the record of chunk c, whose cut falls into row r = [s, e), the rank-th row that holds entries
-__device__ __forceinline__ void write_chunk_record(int c, int S, int n_chunks, int s, int e, int r, int rank,
-                                                   int4* __restrict__ rec, const hpspmm_structure_tables& t) {
-  if (c < 0 || c >= n_chunks) return;   // only a malformed row_ptr gets here
+// the record of chunk c, whose cut falls into row r = [s, e), the rank-th row that holds entries: in slot `slot`, with the
+// end of the chunk before it, which is in slot `before`
+__device__ __forceinline__ void write_chunk_record(int c, int slot, int before, int S, int n_chunks, int s, int e, int r,
+                                                   int rank, int4* __restrict__ rec, const hpspmm_structure_tables& t) {
+  if (c < 0 || c >= n_chunks || slot < 0 || slot >= n_chunks) return;   // only a malformed row_ptr gets here
   const int start = e - s <= S ? s : c * S;
-  rec[2 * (int64_t)c] = make_int4(start, rank, r, e);
-  *reinterpret_cast<int2*>(&rec[2 * (int64_t)c + 1]) = make_int2(c, s);
-  if (c > 0) rec[2 * (int64_t)c - 1].z = start;
+  rec[2 * (int64_t)slot] = make_int4(start, rank, r, e);
+  *reinterpret_cast<int2*>(&rec[2 * (int64_t)slot + 1]) = make_int2(c, s);
+  if (c > 0 && before >= 0 && before < n_chunks) rec[2 * (int64_t)before + 1].z = start;
   if (t.chunk_start) {
     t.chunk_start[c] = start;
     t.chunk_row[c] = r;
@@ -645,35 +691,83 @@ __device__ __forceinline__ void write_chunk_record(int c, int S, int n_chunks, i
   }
 }
 
+// Bound by latency (4 M entries in 250 K rows: 977 blocks, 5.7 us, 4.2 MB): loads are issued before they are needed, chunks
+// are spread over the threads of a block (the longest rows of a power-law graph often stand side by side) and divided by
+// multiplication.  16 M entries in 1 M rows: 16.5 us for matrix order with a warp per long row, 13.7 like this.
+//
+// PIECES: the chunks that lie inside one row come after all others, both in matrix order; else all in matrix order.
+// Chunk c = lo + i of a row (row_cuts) with `h` pieces in the rows above it is a piece for i < n - 1, the h + i-th of the
+// matrix, and otherwise has c - h - (n - 1) chunks of its kind before it.  The chunk before the first one of a row is none:
+// the next cut lies in another row.
+// Why pieces come last: chunks full of short rows take longest, and started last they leave the GPU draining.  Product without
+// a plan, matrix order -> this, kernel alone in us: power-law, 4 M entries, K = 32 57.5 -> 49.4, K = 64 88 -> 77; 16 M, K = 32
+// 201 -> 178; uniform columns 49.7 -> 49.5.
+template <bool PIECES>
 __global__ void __launch_bounds__(kThreads)
-row_tile_list_kernel(int M, int nnz, int tile, int S, int n_chunks, const int* __restrict__ row_ptr,
+row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks, const int* __restrict__ row_ptr,
                      const int* __restrict__ counts, int2* __restrict__ nz, int4* __restrict__ rec,
                      const hpspmm_structure_tables t) {
   constexpr int kWarpsHere = kThreads / 32;
-  __shared__ int part[kWarpsHere];
+  __shared__ int part[kWarpsHere], part_h[kWarpsHere], part_all[kWarpsHere];
+  __shared__ int bound[kThreads + 1], ranks[kThreads], above[kThreads];   // of the rows at hand: first entries, rank, pieces above
   hpspmm::chain_grid();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int before = 0;
-  for (int i = threadIdx.x; i < (int)blockIdx.x; i += kThreads) before += __ldg(counts + i);
+  const int64_t r0 = (int64_t)blockIdx.x * tile;
+  auto row_start = [&](int64_t r) { return __ldg(row_ptr + (r < M ? r : M)); };
+  int s = row_start(r0 + threadIdx.x), e = row_start(r0 + threadIdx.x + 1);   // in flight while the counts are added up
+  // rows that hold entries and pieces in the tiles above, pieces in all tiles: every load of a thread in flight at once
+  constexpr int kPer = kRowTiles / kThreads;   // at most kRowTiles tiles
+  int rows_of[kPer], pieces_of[kPer];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-  if (lane == 0) part[warp] = before;
+  for (int q = 0; q < kPer; ++q) {
+    const int i = q * kThreads + threadIdx.x;
+    rows_of[q] = i < (int)gridDim.x ? __ldg(counts + i) : 0;
+    pieces_of[q] = PIECES && i < (int)gridDim.x ? __ldg(counts + gridDim.x + i) : 0;
+  }
+  int before = 0, before_h = 0, all_h = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const bool above_me = q * kThreads + (int)threadIdx.x < (int)blockIdx.x;
+    before += above_me ? rows_of[q] : 0;
+    before_h += above_me ? pieces_of[q] : 0;
+    all_h += pieces_of[q];
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (PIECES) {
+    before_h = __reduce_add_sync(0xffffffffu, before_h);
+    all_h = __reduce_add_sync(0xffffffffu, all_h);
+  }
+  if (lane == 0) part[warp] = before, part_h[warp] = before_h, part_all[warp] = all_h;
   __syncthreads();
-  int base = 0;
+  int base = 0, base_h = 0, whole = n_chunks;   // whole: chunks that are no pieces
 #pragma unroll
-  for (int w = 0; w < kWarpsHere; ++w) base += part[w];
+  for (int w = 0; w < kWarpsHere; ++w) {
+    base += part[w];
+    if (PIECES) base_h += part_h[w], whole -= part_all[w];
+  }
   __syncthreads();
 
-  const int64_t r0 = (int64_t)blockIdx.x * tile;
-  for (int i = 0; i < tile && r0 + i < M; i += kThreads) {
-    const int64_t r = r0 + i + threadIdx.x;
-    int s = 0, e = 0;
-    if (r < M) {
-      s = __ldg(row_ptr + r);
-      e = __ldg(row_ptr + r + 1);
-    }
+  for (int i0 = 0; i0 < tile && r0 + i0 < M; i0 += kThreads) {
+    const int64_t r = r0 + i0 + threadIdx.x;
+    if (i0 > 0) s = row_start(r), e = row_start(r + 1);
     const bool has = e > s;
+    const row_cuts cuts(s, e, cs);
     const unsigned m = __ballot_sync(0xffffffffu, has);
+    int h = cuts.pieces();   // becomes the pieces in the rows above this one
+    if (PIECES) {
+      const int mine = h;
+      if (__any_sync(0xffffffffu, h > 0)) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, h, o);
+          if (lane >= o) h += v;
+        }
+      }
+      if (lane == 31) part_h[warp] = h;
+      h += base_h - mine;
+    } else {
+      h = 0;
+    }
     if (lane == 0) part[warp] = __popc(m);
     __syncthreads();
     int rank = base + __popc(m & ((1u << lane) - 1u));
@@ -681,34 +775,48 @@ row_tile_list_kernel(int M, int nnz, int tile, int S, int n_chunks, const int* _
     for (int w = 0; w < kWarpsHere; ++w) {
       if (w < warp) rank += part[w];
       base += part[w];
+      if (PIECES) {
+        if (w < warp) h += part_h[w];
+        base_h += part_h[w];
+      }
     }
+    if (threadIdx.x == 0) bound[0] = s;
+    bound[threadIdx.x + 1] = e;
+    ranks[threadIdx.x] = rank;
+    above[threadIdx.x] = h;
     __syncthreads();
-    int c_lo = 0, c_n = 0;   // cuts c * S inside [s, e)
     if (has) {
       nz[rank] = make_int2((int)r, e);
       if (t.nz_id) {
         t.nz_id[rank] = (int)r;
         t.nz_end[rank] = e;
       }
-      c_lo = s == 0 ? 0 : (s - 1) / S + 1;   // (s + S - 1 would overflow for the largest S)
-      c_n = (e - 1) / S - c_lo + 1;
       if (e == nnz && n_chunks > 0) {
-        rec[2 * (int64_t)n_chunks - 1].z = nnz;
+        const int last = PIECES ? whole - 1 : n_chunks - 1;   // the matrix ends with a chunk that is no piece
+        if (last >= 0) rec[2 * (int64_t)last + 1].z = nnz;
         if (t.chunk_start) t.chunk_start[n_chunks] = nnz;
       }
     }
-    if (c_n > 0 && c_n <= 4)
-      for (int c = c_lo; c < c_lo + c_n; ++c) write_chunk_record(c, S, n_chunks, s, e, (int)r, rank, rec, t);
-    unsigned heavy = __ballot_sync(0xffffffffu, c_n > 4);   // the whole warp writes the records of a long row
-    while (heavy) {
-      const int b = __ffs(heavy) - 1;
-      heavy &= heavy - 1;
-      const int hs = __shfl_sync(0xffffffffu, s, b), he = __shfl_sync(0xffffffffu, e, b);
-      const int hl = __shfl_sync(0xffffffffu, c_lo, b), hn = __shfl_sync(0xffffffffu, c_n, b);
-      const int hk = __shfl_sync(0xffffffffu, rank, b);
-      for (int c = lane; c < hn; c += 32)
-        write_chunk_record(hl + c, S, n_chunks, hs, he, (int)(r - lane + b), hk, rec, t);
+    // a thread a chunk
+    const int first = bound[0], end = bound[kThreads];
+    const row_cuts all(first, end, cs);
+#pragma unroll 4
+    for (int k = threadIdx.x; k < all.n; k += kThreads) {
+      const int c = all.lo + k;
+      int at = 0;   // the row that holds entry c * S: the last one that begins at or before it
+#pragma unroll
+      for (int d = kThreads / 2; d >= 1; d >>= 1)
+        if (bound[at + d] <= c * cs.S) at += d;
+      const row_cuts own(bound[at], bound[at + 1], cs);
+      const int i = c - own.lo, h = above[at];
+      int slot = c, prev = c - 1;
+      if (PIECES) {
+        slot = i < own.n - 1 ? whole + h + i : c - h - (own.n - 1);
+        prev = i > 0 ? whole + h + i - 1 : c - 1 - h;
+      }
+      write_chunk_record(c, slot, prev, cs.S, n_chunks, bound[at], bound[at + 1], (int)(r0 + i0 + at), ranks[at], rec, t);
     }
+    __syncthreads();
   }
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x < kNzPad) {
     // sentinels after the last row: never a row of C, an end no entry reaches; a warp reads 32 rows at once
@@ -731,20 +839,25 @@ __global__ void order_records_kernel(int64_t n, const int* __restrict__ order, c
 
 size_t hpspmm_nz_bytes(int64_t M) { return (size_t)(M + kNzPad) * 8; }
 
-int64_t hpspmm_row_tiles(int64_t M) {
+static int64_t row_tiles(int64_t M) {
   const int64_t tile = row_tile_size(M);
   const int64_t n = (M + tile - 1) / tile;
   return n < 1 ? 1 : n;
 }
 
+int64_t hpspmm_row_tile_ints(int64_t M) { return 2 * row_tiles(M); }
+
 int hpspmm_build_structure(hpspmm_ctx* ctx, int64_t M, int64_t nnz, const int32_t* row_ptr, int32_t S, int64_t n_chunks,
                            int2* nz, int4* rec_out, int32_t* counts, const hpspmm_structure_tables& tables, cudaStream_t stream,
                            int32_t* clear, int64_t n_clear) {
   const int tile = row_tile_size(M);
-  const unsigned blocks = (unsigned)hpspmm_row_tiles(M);
-  hpspmm_launch(row_tile_count_kernel, blocks, kThreads, 0, stream, (int)M, tile, row_ptr, counts, clear, n_clear);
-  hpspmm_launch(row_tile_list_kernel, blocks, kThreads, 0, stream, (int)M, (int)nnz, tile, S, (int)n_chunks, row_ptr, counts, nz,
-                rec_out, tables);
+  const unsigned blocks = (unsigned)row_tiles(M);
+  const chunk_size cs(S);
+  const bool plan = tables.chunk_start != nullptr;   // a plan orders its records by cost afterwards
+  hpspmm_launch(plan ? row_tile_count_kernel<false> : row_tile_count_kernel<true>, blocks, kThreads, 0, stream, (int)M, tile, cs,
+                row_ptr, counts, clear, n_clear);
+  hpspmm_launch(plan ? row_tile_list_kernel<false> : row_tile_list_kernel<true>, blocks, kThreads, 0, stream, (int)M, (int)nnz,
+                tile, cs, (int)n_chunks, row_ptr, counts, nz, rec_out, tables);
   ctx->launches += 2;
   HPSPMM_CUDA_TRY(ctx, cudaGetLastError());
   return HPSPMM_OK;

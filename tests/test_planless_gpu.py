@@ -221,3 +221,32 @@ def test_only_the_first_product_of_a_width_allocates(pkg, oracle):
                 w.check("K=%d, no allocation possible" % w.K)
         finally:
             lib.hpspmm_debug_fail_device_alloc(0, 0)
+
+
+@pytest.mark.parametrize("seed", [0, 1, 2])
+def test_pieces_of_long_rows_come_last(gpu_ctx, pkg, oracle, seed):
+    """The records of a call without a plan: rows that end on, just before and just after a cut, rows of one to many
+    pieces side by side and across the builder's tiles of rows, the first and last row among them."""
+    ctx, S, K, M, N = gpu_ctx, 32, 20, 9000, 600
+    rng = np.random.default_rng(seed)
+    n = rng.choice([0, 1, 3, 31, 32, 33, 64, 65, 96, 130, 500], size=M)
+    n[[0, -1]] = [(700, 0), (0, 321), (64, 64)][seed]
+    row_ptr = np.concatenate([[0], np.cumsum(n)]).astype(np.int32)
+    nnz = int(row_ptr[-1])
+    col_idx = rng.integers(0, N, size=nnz).astype(np.int32)
+    vals = rng.uniform(-1, 1, size=nnz).astype(np.float32)
+    B = rng.uniform(-1, 1, size=(N, K)).astype(np.float32)
+    X = rng.uniform(-1, 1, size=(M, K)).astype(np.float32)
+    bufs = [ctx.upload(a) for a in (row_ptr, col_idx, vals, B, X)]
+    d_C, d_o = ctx.alloc((M, K), np.float32), ctx.alloc((nnz,), np.float32)
+    opts = pkg.Opts(chunk_nnz=S)
+    assert nnz > 40 * 160 * S           # more chunks than the warps of the GPU search for by themselves
+    for _ in range(2):
+        ctx.spmm_csr(M, N, K, nnz, bufs[0], bufs[1], bufs[2], bufs[3], d_C, opts=opts)
+        ref, abs_sum = oracle.spmm_f64(row_ptr, col_idx, vals, B)
+        check_against_f64(d_C.to_host(), ref, abs_sum, "product without a plan")
+    ctx.sddmm_csr(M, N, K, nnz, bufs[0], bufs[1], bufs[4], bufs[3], d_o, opts=opts)
+    ref, abs_sum = oracle.sddmm_f64(row_ptr, col_idx, X, B)
+    check_against_f64(d_o.to_host(), ref, abs_sum, "SDDMM without a plan")
+    for b in bufs + [d_C, d_o]:
+        b.free()
