@@ -649,11 +649,17 @@ int32_t planless_chunk_nnz(int64_t K, int64_t nnz, const hpspmm_opts* opts) {
 }
 
 // Whether a product without a plan lets every warp search row_ptr for its chunk (one launch) instead of building the
-// records and the list of filled rows first (two more).  A search costs a chunk 1 to 2 us of latency, the builders 5 us
-// and more per call; with more chunks than fit on the GPU the searches add up.  With very many empty rows
-// between the entries the list pays for itself.
-bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t n_chunks) {
-  return n_chunks <= ctx->sm_count * 40ll && M <= 8 * nnz;
+// records and the list of filled rows first (two more).  A search costs a chunk 1 to 2 us of latency and the product its
+// steps along row_ptr, the builders 4 to 8 us a call; with more chunks than fit on the GPU the searches add up, and long
+// rows gain by the records' order (pieces last).  Search -> records in us:
+//   chunks of 128: 700 K entries (37 chunks per SM), power-law K = 32 / 64 / 128 31.2 -> 21.3 / 35.0 -> 25.6 / 45.0 -> 32.6,
+//                  uniform K = 32 16.7 -> 16.6, in 170 K rows 25.6 -> 24.4; 335 K, K = 100 (18 per SM), power-law 31.9 -> 27.7;
+//                  300 K, K = 100 (16 per SM), uniform 16.4 -> 19.4; 150 K, K = 100 (8 per SM), power-law 23.2 -> 22.0, uniform 13.2 -> 16.2
+//   chunks of 64:  335 K (35 per SM), power-law K = 64 20.6 -> 22.1; 300 K (32 per SM), uniform 10.0 -> 13.4
+// (the figures beyond K = 32 with builders that took 1 to 2 us longer).  With very many empty rows between the entries the list
+// pays for itself.
+bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t n_chunks, int32_t S) {
+  return n_chunks <= ctx->sm_count * (S < 128 ? 40ll : 16ll) && M <= 8 * nnz;
 }
 
 // Counters that are set aside at the first product of a width: enough for any later one of up to that width, so that a
@@ -853,7 +859,7 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
   }
   const int32_t S = planless_chunk_nnz(K, nnz, opts);
   const int64_t n_chunks = (nnz + S - 1) / S;
-  const bool search = searches_for_chunks(ctx, M, nnz, n_chunks);
+  const bool search = searches_for_chunks(ctx, M, nnz, n_chunks, S);
   const planless_layout lay(M, K, n_chunks, search);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
@@ -933,7 +939,7 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
       const int64_t w = slabs[i].width;
       const int32_t S = planless_chunk_nnz(w, nnz, opts);
       const int64_t n_chunks = (nnz + S - 1) / S;
-      const bool search = searches_for_chunks(ctx, M, nnz, n_chunks);
+      const bool search = searches_for_chunks(ctx, M, nnz, n_chunks, S);
       const planless_layout lay(M, w, n_chunks, search);
       need = lay.bytes > need ? lay.bytes : need;
       const int64_t keep = counters_to_keep(ctx, w, lay.n_counter, search);
