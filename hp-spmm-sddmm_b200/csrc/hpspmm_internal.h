@@ -99,6 +99,7 @@ struct hpspmm_spmm_args {
 struct hpspmm_spmm_shape {
   int VEC, W, R;
   bool lat;    // few chunks: more gathers in flight per warp
+  bool mid;    // one or two waves of 24 warps per SM: twice the gathers in flight (wide groups of 16-byte vectors)
   bool hint;
 };
 // widest vector the rows of the dense operands keep aligned; addresses: bitwise or of the operands' addresses

@@ -547,6 +547,7 @@ hpspmm_spmm_shape hpspmm_choose_shape(int VEC, int64_t cols, int widest, bool hi
   sh.VEC = VEC;
   sh.hint = hint;
   sh.lat = false;
+  sh.mid = false;
   if (cols > widest) cols = widest;
   const int vecs = (int)((cols + VEC - 1) / VEC);
   sh.W = VEC == 1 ? (vecs <= 1 ? 1 : 4) : 2;
@@ -609,6 +610,15 @@ hpspmm_spmm_shape shape_of_launch(int sm_count, int VEC, int K, int off, int64_t
   // their order).  67.6 K entries in chunks of 64: 6.1 -> 5.6 us at K = 64, 9.1 -> 7.2 us at K = 128; with more chunks
   // than these builds have resident warps they lose (300 K entries, K = 64: 8.3 -> 10.5 us).
   sh.lat = n_chunks <= sm_count * (sh.W <= 8 ? 24 : 16);
+  // A warp over 97 to 128 or 193 to 256 columns has four or two entries in flight.  With twice as many 24 warps fit on an SM
+  // instead of 36, which pays where the chunks are about one or two waves of those.  Chunks per SM: 17.7 to 22 / 37 to 42,
+  // power-law and uniform graphs of 335 K to 800 K entries, plan, 36 -> 24 warps in us:
+  //   K = 100  23.2 -> 21.3, 17.0 -> 15.5 / 28.0 -> 25.6, 42.8 -> 38.5;   K = 128  22.9 -> 21.3, 16.8 -> 15.7 / 31.0 -> 29.3, 46.9 -> 41.7
+  //   K = 224  34.3 -> 28.2, 29.0 -> 23.6 / 57.0 -> 48.3, 49.5 -> 42.7;   K = 256  34.4 -> 28.6, 29.6 -> 25.8 / 59.8 -> 51.2, 53.9 -> 47.0
+  // Between (30 per SM) uniform rows lose (K = 128 19.9 -> 25.4), from 53 on it is level or behind, and at up to 64 columns
+  // uniform rows lose everywhere (335 K, K = 64: 8.4 -> 10.4).
+  sh.mid = !sh.lat && VEC == 4 && sh.W == 32 && sh.R <= 2 &&
+           (n_chunks <= sm_count * 24ll || (n_chunks > sm_count * 36ll && n_chunks <= sm_count * 48ll));
   // (one group instead of several of three vectors: rows end without an exchange, and are added up in another order)
   if (sh.lat && sh.R == 3 && sh.W < 32) sh.R = sh.W / 8, sh.W = 32;
   return sh;

@@ -13,6 +13,10 @@ int hpspmm_spmm_launch_v4(hpspmm_ctx* ctx, const hpspmm_spmm_args& a, const hpsp
     if (sh.W == 32 && sh.R == 3) GO(32, 3, 4, 0, 8, true);
     if (sh.W == 32) GO(32, 4, 4, 0, 8, true);
   }
+  if (sh.mid) {
+    if (sh.R == 1) GO(32, 1, 8, 0, 12, true);
+    GO(32, 2, 4, 0, 12, true);
+  }
   if (a.K == 32 && sh.W == 8) { if (sh.hint) GO(8, 1, 4, 32, 18, true); else GO(8, 1, 4, 32, 18, false); }
   if (a.K == 64 && sh.W == 16) { if (sh.hint) GO(16, 1, 4, 64, 18, true); else GO(16, 1, 4, 64, 18, false); }
   if (a.K == 128 && sh.W == 32 && sh.R == 1) { if (sh.hint) GO(32, 1, 4, 128, 18, true); else GO(32, 1, 4, 128, 18, false); }

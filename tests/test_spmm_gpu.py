@@ -478,3 +478,24 @@ def test_other_multiples_of_32(gpu_ctx, pkg, oracle, K, use_plan):
         C, _ = _check(gpu_ctx, pkg, oracle, g["row_ptr"], g["col_idx"], g["vals"], B, "K=%d S=%d" % (K, chunk),
                       opts=opts, use_plan=use_plan)
         assert np.all(np.isfinite(C))
+
+
+@pytest.mark.parametrize("K", [100, 128, 196, 256])
+@pytest.mark.parametrize("per_sm", [16.5, 24, 36.5, 48])
+def test_one_or_two_waves_of_wide_products(gpu_ctx, pkg, oracle, K, per_sm):
+    """The builds with twice the gathers in flight, at both ends of their ranges: split rows, empty rows, a ragged last
+    chunk; on a GPU of 148 SMs."""
+    ctx, S, M, N = gpu_ctx, 32, 6000, 900
+    rng = np.random.default_rng(K)
+    nnz = int(per_sm * 148) * S - 7
+    cuts = np.sort(rng.integers(0, nnz + 1, size=M - 1))
+    cuts[100:140] = cuts[100]                       # empty rows
+    cuts[:60] = 0                                   # a long first row behind them
+    row_ptr = np.concatenate([[0], np.sort(cuts), [nnz]]).astype(np.int32)
+    col_idx = rng.integers(0, N, size=nnz).astype(np.int32)
+    vals = rng.uniform(-1, 1, size=nnz).astype(np.float32)
+    B = rng.uniform(-1, 1, size=(N, K)).astype(np.float32)
+    ref, abs_sum = oracle.spmm_f64(row_ptr, col_idx, vals, B)
+    for use_plan in (True, False):
+        C = gpu_spmm(ctx, pkg, row_ptr, col_idx, vals, B, opts=pkg.Opts(chunk_nnz=S), use_plan=use_plan)
+        check_against_f64(C, ref, abs_sum, "K=%d, %g chunks per SM" % (K, per_sm))
