@@ -809,8 +809,10 @@ int hpspmm_spmm_kernel_signature(const hpspmm_plan* plan, int64_t K, int32_t b_l
   const hpspmm_spmm_shape sh =
       fits ? shape_of_launch(plan->sm_count, VEC, (int)K, 0, plan->n_chunks, hpspmm_even_rows(plan), hint, &cols)
            : hpspmm_choose_shape(VEC, K, hpspmm_widest_slab(VEC), hint);
-  snprintf(buf, len, "spmm_warp_kernel<%d,%d,%d> K=%lld few=%d hint=%d chunk_nnz=%d", sh.VEC, sh.W, sh.R, (long long)K,
-           sh.lat ? 1 : 0, sh.hint ? 1 : 0, plan ? (int)plan->chunk_nnz : (int)hpspmm_default_chunk_nnz(K, 0));
+  // (mid only where it is set: captures on file were taken of builds without it)
+  snprintf(buf, len, "spmm_warp_kernel<%d,%d,%d> K=%lld few=%d%s hint=%d chunk_nnz=%d", sh.VEC, sh.W, sh.R, (long long)K,
+           sh.lat ? 1 : 0, sh.mid ? " mid=1" : "", sh.hint ? 1 : 0,
+           plan ? (int)plan->chunk_nnz : (int)hpspmm_default_chunk_nnz(K, 0));
   return HPSPMM_OK;
 }
 

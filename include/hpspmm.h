@@ -163,7 +163,8 @@ HPSPMM_API int hpspmm_plan_info(const hpspmm_plan* plan, int64_t* n_chunks,
                                 int64_t* scratch_bytes);
 /* Name and shape (vector width, lanes, vectors per lane) of the kernel hpspmm_spmm_csr_f32 launches for
  * the first columns of width K with this plan and L2 hint setting, as a string: profiler captures are filed
- * under it.  few=1: the build for few chunks.  Without a plan (NULL) the number of chunks is left out of it. */
+ * under it.  few=1: the build for few chunks; mid=1 (left out where it is not): the one with twice the gathers in
+ * flight for one or two waves of wide chunks.  Without a plan (NULL) the number of chunks is left out of it. */
 HPSPMM_API int hpspmm_spmm_kernel_signature(const hpspmm_plan* plan, int64_t K, int32_t b_l2_hint,
                                             char* buf, size_t len);
 /* Device pointers to the plan's tables, for inspection: chunk_start[n_chunks + 1] (first

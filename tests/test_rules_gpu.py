@@ -181,3 +181,10 @@ def test_the_signature_names_the_shape_that_is_launched(gpu_ctx, pkg):
         assert many in signature(line * SMS + 1, K) and "few=0" in signature(line * SMS + 1, K)
     assert "<4,32,3>" in signature(64 * SMS, 384) and "<4,32,3>" in signature(64 * SMS + 1, 384, even=False)
     assert "<4,32,1>" in signature(64 * SMS + 1, 384)
+    # twice the gathers in flight from 16 to 24 and from 36 to 48 chunks per SM, over 97 to 128 and 193 to 256 columns
+    for K in (100, 128, 196, 256):
+        for line, below, above in ((16, "few=1 hint", "few=0 mid=1 hint"), (24, "few=0 mid=1 hint", "few=0 hint"),
+                                   (36, "few=0 hint", "few=0 mid=1 hint"), (48, "few=0 mid=1 hint", "few=0 hint")):
+            assert below in signature(line * SMS, K) and above in signature(line * SMS + 1, K)
+    for K in (64, 96, 98, 132, 192, 260):
+        assert "mid" not in signature(17 * SMS, K) and "mid" not in signature(48 * SMS, K)

@@ -484,10 +484,10 @@ def test_other_multiples_of_32(gpu_ctx, pkg, oracle, K, use_plan):
 @pytest.mark.parametrize("per_sm", [16.5, 24, 36.5, 48])
 def test_one_or_two_waves_of_wide_products(gpu_ctx, pkg, oracle, K, per_sm):
     """The builds with twice the gathers in flight, at both ends of their ranges: split rows, empty rows, a ragged last
-    chunk; on a GPU of 148 SMs."""
+    chunk."""
     ctx, S, M, N = gpu_ctx, 32, 6000, 900
     rng = np.random.default_rng(K)
-    nnz = int(per_sm * 148) * S - 7
+    nnz = int(per_sm * ctx.lib.hpspmm_ctx_sm_count(ctx.handle)) * S - 7
     cuts = np.sort(rng.integers(0, nnz + 1, size=M - 1))
     cuts[100:140] = cuts[100]                       # empty rows
     cuts[:60] = 0                                   # a long first row behind them
@@ -495,6 +495,12 @@ def test_one_or_two_waves_of_wide_products(gpu_ctx, pkg, oracle, K, per_sm):
     col_idx = rng.integers(0, N, size=nnz).astype(np.int32)
     vals = rng.uniform(-1, 1, size=nnz).astype(np.float32)
     B = rng.uniform(-1, 1, size=(N, K)).astype(np.float32)
+    d_rp, d_ci = ctx.upload(row_ptr), ctx.upload(col_idx)
+    plan = ctx.plan_create(M, nnz, d_rp, K, pkg.Opts(chunk_nnz=S), N=N, col_idx=d_ci)
+    assert "few=0 mid=1" in ctx.kernel_signature(plan, K)
+    ctx.plan_destroy(plan)
+    d_rp.free()
+    d_ci.free()
     ref, abs_sum = oracle.spmm_f64(row_ptr, col_idx, vals, B)
     for use_plan in (True, False):
         C = gpu_spmm(ctx, pkg, row_ptr, col_idx, vals, B, opts=pkg.Opts(chunk_nnz=S), use_plan=use_plan)
