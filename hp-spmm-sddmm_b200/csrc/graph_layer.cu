@@ -60,6 +60,7 @@ int width_class(int64_t K) { return K <= 32 ? 0 : (K <= 64 ? 1 : 2); }
 
 // plans of A and of its transpose for the width class of K, built on first use
 int plans_for(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, hpspmm_stream stream, int* cls_out) {
+  HPSPMM_REQUIRE(ctx, g->device == ctx->device, "layer built on another device");
   const int cls = width_class(K);
   *cls_out = cls;
   if (g->plan[cls] && g->plan_t[cls]) return HPSPMM_OK;
@@ -198,6 +199,7 @@ int hpspmm_layer_backward(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, const flo
   HPSPMM_TRACE("hpspmm_layer_backward");
   HPSPMM_REQUIRE(ctx, ctx != nullptr && g != nullptr, "null context or layer");
   HPSPMM_REQUIRE(ctx, K >= 1 && K <= g->max_K, "K outside [1, max_K] of the layer");
+  HPSPMM_REQUIRE(ctx, g->device == ctx->device, "layer built on another device");
   if (g->nnz == 0 || g->M == 0 || g->N == 0 || K > 256) return HPSPMM_ERR_UNSUPPORTED;
   HPSPMM_REQUIRE(ctx, vals && dC && H && dH && dA, "null operand");
   if ((K & 3) == 0) HPSPMM_REQUIRE(ctx, (((uintptr_t)dC | (uintptr_t)H | (uintptr_t)dH) & 15u) == 0,

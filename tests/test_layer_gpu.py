@@ -148,6 +148,34 @@ def test_both_gradients_in_one_pass(gpu_ctx, pkg, oracle, K):
             b.free()
 
 
+def test_a_layer_is_refused_by_the_context_of_another_device(gpu_ctx, pkg):
+    """Every product of the handle, also of a width whose plans are still to be built.  (One GPU is enough: the handle
+    begins with its device's ordinal, which is set to another one here.)"""
+    ctx, K = gpu_ctx, 32
+    g = pkg.gen_rmat(8, 8, seed=43)
+    M, N, nnz = g["M"], g["N"], g["nnz"]
+    bufs = [ctx.upload(a) for a in (g["row_ptr"], g["col_idx"], g["vals"])]
+    x, dA = ctx.alloc((M, 64), np.float32), ctx.alloc((nnz,), np.float32)
+    layer = pkg.Layer(ctx, M, N, nnz, *bufs, 64)
+    device = ctypes.c_int.from_address(layer.handle.value)
+    assert device.value == 0
+    lib, h = ctx.lib, ctx.handle
+    device.value = 1
+    try:
+        for width in (64, K):
+            assert lib.hpspmm_layer_backward(h, layer.handle, width, bufs[2].ptr, x.ptr, x.ptr, x.ptr, dA.ptr,
+                                             None) == pkg.ERR_INVALID
+            assert lib.hpspmm_layer_forward(h, layer.handle, width, x.ptr, x.ptr, None) == pkg.ERR_INVALID
+            assert lib.hpspmm_layer_forward_values(h, layer.handle, width, bufs[2].ptr, x.ptr, x.ptr, None) == pkg.ERR_INVALID
+            assert lib.hpspmm_layer_backward_features(h, layer.handle, width, x.ptr, x.ptr, None) == pkg.ERR_INVALID
+            assert lib.hpspmm_layer_backward_weights(h, layer.handle, width, x.ptr, x.ptr, dA.ptr, None) == pkg.ERR_INVALID
+    finally:
+        device.value = 0
+    layer.close()
+    for b in bufs + [x, dA]:
+        b.free()
+
+
 @pytest.mark.parametrize("K", [64, 48])
 def test_torch_autograd_front_end(pkg, oracle, K):
     torch = pytest.importorskip("torch")
