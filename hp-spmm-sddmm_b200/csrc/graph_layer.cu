@@ -200,10 +200,14 @@ int hpspmm_layer_backward(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, const flo
   HPSPMM_REQUIRE(ctx, ctx != nullptr && g != nullptr, "null context or layer");
   HPSPMM_REQUIRE(ctx, K >= 1 && K <= g->max_K, "K outside [1, max_K] of the layer");
   HPSPMM_REQUIRE(ctx, g->device == ctx->device, "layer built on another device");
-  if (g->nnz == 0 || g->M == 0 || g->N == 0 || K > 256) return HPSPMM_ERR_UNSUPPORTED;
+  if (g->nnz == 0 || g->M == 0 || g->N == 0) return HPSPMM_ERR_UNSUPPORTED;
   HPSPMM_REQUIRE(ctx, vals && dC && H && dH && dA, "null operand");
   if ((K & 3) == 0) HPSPMM_REQUIRE(ctx, (((uintptr_t)dC | (uintptr_t)H | (uintptr_t)dH) & 15u) == 0,
                                    "dense operands must be 16-byte aligned");
+  // what no plan can change is refused before one is built (rows of uneven length have the higher limit)
+  if (!hpspmm_layer_grad_covers(K, (uintptr_t)dC | (uintptr_t)H | (uintptr_t)dH) ||
+      !hpspmm_layer_grad_pays(ctx, g->nnz, false))
+    return HPSPMM_ERR_UNSUPPORTED;
   hpspmm_device_guard guard(ctx->device);
   int cls;
   const int st = plans_for(ctx, g, K, stream, &cls);

@@ -147,6 +147,8 @@ struct hpspmm_layer_grad_args {
   float* carry;
   int32_t* counter;
 };
+// whether the kernel has a shape for K columns at these operands (addresses: or of theirs)
+bool hpspmm_layer_grad_covers(int64_t K, uintptr_t addresses);
 // whether the one kernel beats the three it replaces; even: rows of even length (hpspmm_even_rows)
 bool hpspmm_layer_grad_pays(const hpspmm_ctx* ctx, int64_t nnz, bool even);
 int hpspmm_layer_grad_launch(hpspmm_ctx* ctx, const hpspmm_layer_grad_args& a, cudaStream_t s);

@@ -229,7 +229,9 @@ int launch(hpspmm_ctx* ctx, hpspmm_layer_grad_args a, cudaStream_t s) {
 
 // One launch covers up to 256 columns of 16- or 8-byte vectors and 128 of 4-byte ones; a wider row would need the dot
 // products of several slabs added up, and two kernels then.
-static bool covers(int VEC, int64_t K) { return K <= (VEC == 1 ? 128 : 256); }
+bool hpspmm_layer_grad_covers(int64_t K, uintptr_t addresses) {
+  return K <= (hpspmm_vector_width(K, addresses) == 1 ? 128 : 256);
+}
 
 // Whether one pass is faster than the permuted weights, the product and the SDDMM by themselves.  The 4-byte accesses
 // through the permutation are cheap as long as what they reach, 8 bytes per entry, stays in the L2 cache beside the rows of
@@ -249,8 +251,9 @@ bool hpspmm_layer_grad_pays(const hpspmm_ctx* ctx, int64_t nnz, bool even) {
 // R = 2 160 / 206 us, W = 16 134 / 176; K = 128: W = 16, R = 2 227 / 377, W = 32 222 / 352.  K = 96 and 192 stay at three.
 // Blocks per SM: 16 (64 registers) at K = 64 134 us, 18 138, 20 175; at K = 32 18 93, 16 95, 20 113.
 int hpspmm_layer_grad_launch(hpspmm_ctx* ctx, const hpspmm_layer_grad_args& a, cudaStream_t s) {
-  const int VEC = hpspmm_vector_width(a.K, (uintptr_t)a.dC | (uintptr_t)a.H | (uintptr_t)a.dH);
-  if (!covers(VEC, a.K)) return HPSPMM_ERR_UNSUPPORTED;
+  const uintptr_t addresses = (uintptr_t)a.dC | (uintptr_t)a.H | (uintptr_t)a.dH;
+  if (!hpspmm_layer_grad_covers(a.K, addresses)) return HPSPMM_ERR_UNSUPPORTED;
+  const int VEC = hpspmm_vector_width(a.K, addresses);
   const int vecs = (a.K + VEC - 1) / VEC;
 #define GO(V, W, R, U, KS, MINB) return launch<V, W, R, U, KS, MINB>(ctx, a, s)
   if (VEC == 4) {

@@ -148,6 +148,25 @@ def test_both_gradients_in_one_pass(gpu_ctx, pkg, oracle, K):
             b.free()
 
 
+def test_both_gradients_refused_before_anything_is_built(gpu_ctx, pkg):
+    """Weights that fill the L2 cache: no plan can change the answer, so none is built for it."""
+    import torch
+    ctx = gpu_ctx
+    M, per_row = 700_000, 16
+    nnz = M * per_row
+    assert 8 * nnz > ctx.lib.hpspmm_ctx_l2_bytes(ctx.handle) * 5 // 8
+    rp = torch.arange(0, nnz + 1, per_row, dtype=torch.int32, device="cuda")
+    ci = torch.randint(M, (nnz,), dtype=torch.int32, device="cuda")
+    v, x = torch.rand(nnz, device="cuda"), torch.empty((M, 32), device="cuda")
+    torch.cuda.synchronize()
+    layer = pkg.Layer(ctx, M, M, nnz, rp.data_ptr(), ci.data_ptr(), v.data_ptr(), 64)
+    owned = layer.info()["owned_bytes"]
+    st = ctx.lib.hpspmm_layer_backward(ctx.handle, layer.handle, 32, v.data_ptr(), x.data_ptr(), x.data_ptr(), x.data_ptr(),
+                                       v.data_ptr(), None)
+    assert st == pkg.ERR_UNSUPPORTED and layer.info()["owned_bytes"] == owned
+    layer.close()
+
+
 def test_a_layer_is_refused_by_the_context_of_another_device(gpu_ctx, pkg):
     """Every product of the handle, also of a width whose plans are still to be built.  (One GPU is enough: the handle
     begins with its device's ordinal, which is set to another one here.)"""
