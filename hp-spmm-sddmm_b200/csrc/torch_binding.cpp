@@ -115,26 +115,31 @@ Tensor backward_weights(const Tensor& grad, const Tensor& H, int64_t id) {
   return dA;
 }
 
-// Both gradients: one pass over the transpose where the library has a kernel for the width, else the two above.
+// Both gradients: one pass over the transpose where the library has a kernel for the call, else the product and the SDDMM,
+// into the same tensors.
 std::tuple<Tensor, Tensor> backward(const Tensor& grad, const Tensor& H, const Tensor& vals, int64_t id) {
   auto e = entry_of(id);
   const Tensor dC = require_cuda_f32(grad, e->M, "dC"), h = require_cuda_f32(H, e->N, "H");
   const Tensor v = require_weights(vals, *e, grad.device());
   TORCH_CHECK(h.size(1) == dC.size(1) && h.device() == dC.device(), "hpspmm: dC and H differ in width or device");
-  {
-    const c10::cuda::CUDAGuard guard(dC.device());
-    Tensor dH = at::empty({e->N, dC.size(1)}, dC.options()), dA = at::empty({e->nnz}, dC.options());
-    std::lock_guard<std::mutex> lock(e->use);
-    check_open(*e, id);
-    const int st = hpspmm_layer_backward(e->ctx, e->layer, dC.size(1), v.const_data_ptr<float>(), dC.const_data_ptr<float>(),
-                                         h.const_data_ptr<float>(), dH.mutable_data_ptr<float>(),
-                                         dA.mutable_data_ptr<float>(), c10::cuda::getCurrentCUDAStream().stream());
-    if (st != HPSPMM_ERR_UNSUPPORTED) {
-      check(*e, st, "hpspmm_layer_backward");
-      return {dH, dA};
-    }
+  const c10::cuda::CUDAGuard guard(dC.device());
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  Tensor dH = at::empty({e->N, dC.size(1)}, dC.options()), dA = at::empty({e->nnz}, dC.options());
+  const int64_t K = dC.size(1);
+  const float *dc = dC.const_data_ptr<float>(), *hp = h.const_data_ptr<float>();
+  float *dh = dH.mutable_data_ptr<float>(), *da = dA.mutable_data_ptr<float>();
+  Tensor old;
+  std::lock_guard<std::mutex> lock(e->use);
+  check_open(*e, id);
+  const int st = hpspmm_layer_backward(e->ctx, e->layer, K, v.const_data_ptr<float>(), dc, hp, dh, da, stream);
+  if (st != HPSPMM_ERR_UNSUPPORTED) {
+    check(*e, st, "hpspmm_layer_backward");
+    return {dH, dA};
   }
-  return {backward_features(dC, v, id), backward_weights(dC, h, id)};
+  sync_values(*e, v, stream, old);
+  check(*e, hpspmm_layer_backward_features(e->ctx, e->layer, K, dc, dh, stream), "hpspmm_layer_backward_features");
+  check(*e, hpspmm_layer_backward_weights(e->ctx, e->layer, K, dc, hp, da, stream), "hpspmm_layer_backward_weights");
+  return {dH, dA};
 }
 
 // the registered operators, for calls that go through the dispatcher (tracing, fake tensors)

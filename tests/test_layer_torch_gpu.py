@@ -9,13 +9,13 @@ pytestmark = pytest.mark.gpu
 
 
 class _Layer:
-    def __init__(self, pkg, K=16, seed=31):
+    def __init__(self, pkg, K=16, seed=31, max_K=64):
         import torch
         g = pkg.gen_rmat(9, 8, seed=seed)
         self.M, self.N, self.nnz, self.K = g["M"], g["N"], g["nnz"], K
         self.rp, self.ci, self.v = (torch.from_numpy(g[k]).cuda() for k in ("row_ptr", "col_idx", "vals"))
         self.ops = importlib.import_module(pkg.__name__ + ".torch_ops")
-        self.layer = self.ops.TorchLayer(self.rp, self.ci, self.v, self.M, self.N, 64)
+        self.layer = self.ops.TorchLayer(self.rp, self.ci, self.v, self.M, self.N, max_K)
         self.H = torch.from_numpy(pkg.host_fill_uniform(self.N * K, seed, 1, -1.0, 1.0).reshape(self.N, K)).cuda()
         rows = torch.repeat_interleave(torch.arange(self.M, device="cuda"), (self.rp[1:] - self.rp[:-1]).long())
         self.index = torch.stack([rows, self.ci.long()])
@@ -170,3 +170,30 @@ def test_tracers_modes_and_subclasses_see_the_operator(work):
     assert type(work.layer(torch.nn.Parameter(work.H))) is torch.Tensor
     with pytest.raises(RuntimeError):
         work.layer(work.H.cpu().numpy())
+
+
+# widths that one pass does not cover: rows of 4-byte vectors beyond 128 columns, and more than 256 columns
+@pytest.mark.parametrize("K", [129, 260])
+def test_both_gradients_where_one_pass_is_refused(pkg, K):
+    """The product and the SDDMM instead, with the transpose's copy of the weights filled again after an in-place step;
+    nothing is allocated but the two results."""
+    import torch
+    w = _Layer(pkg, K=K, max_K=K)
+    dC = torch.randn((w.M, K), device="cuda")
+    W = w.v.clone().requires_grad_()
+    rows, cols = w.index
+    for scale in (1.0, -0.5, 3.0):
+        with torch.no_grad():
+            W.mul_(scale)
+        H = w.H.clone().requires_grad_()
+        W.grad = None
+        C = w.layer(H, W)
+        C.backward(dC)
+        assert _close(C.detach(), w.product(W.detach(), w.H))
+        assert _close(H.grad, w.dense(W.detach()).T @ dC.double())
+        assert _close(W.grad, (dC.double()[rows] * w.H.double()[cols]).sum(1))
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    out = w.ops.layer_backward(dC, w.H, W.detach(), w.layer.layer_id)
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] - before == 2
+    assert _close(out[0], H.grad.double()) and _close(out[1], W.grad.double())
+    w.layer.close()
