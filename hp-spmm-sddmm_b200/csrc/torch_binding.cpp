@@ -3,6 +3,7 @@
 // A training step on a small graph is three or four launches of a few microseconds each; with the operators and the
 // autograd formula in Python the host took 160 us to issue them.  Arithmetic stays in libhpspmm.so, which this file
 // calls through the C ABI; PyTorch supplies memory, streams and the autograd tape.
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -27,6 +28,7 @@ struct Entry {
   // the weight tensor whose values the layer's transpose holds (kept alive: the layer borrows the device array)
   Tensor vals;
   int64_t vals_version;   // of `vals` when the transpose was filled; -1: unknown, fill it again
+  bool in_graph = false;  // a captured graph fills the transpose: a replay does so without the host knowing
 };
 
 std::mutex g_mutex;   // guards the registry
@@ -61,8 +63,11 @@ Tensor require_weights(const Tensor& t, const Entry& e, const at::Device& device
 
 // Re-gathers the transpose's values when the weight tensor moved or was written in place.  What was held goes to `old`, to
 // be released after the lock.
+// A captured call always records the gather: its graph may be replayed after the weights changed in place, or after a call
+// with others.  From then on nobody knows what the transpose holds, and every call gathers.
 void sync_values(Entry& e, const Tensor& vals, cudaStream_t stream, Tensor& old) {
-  const int64_t version = vals.is_inference() ? -1 : (int64_t)vals._version();
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) e.in_graph = true;
+  const int64_t version = vals.is_inference() || e.in_graph ? -1 : (int64_t)vals._version();
   if (version >= 0 && e.vals.defined() && vals.const_data_ptr() == e.vals.const_data_ptr() && version == e.vals_version)
     return;
   e.vals_version = -1;   // until the update has succeeded

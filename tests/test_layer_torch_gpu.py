@@ -197,3 +197,38 @@ def test_both_gradients_where_one_pass_is_refused(pkg, K):
     assert torch.cuda.memory_stats()["allocation.all.allocated"] - before == 2
     assert _close(out[0], H.grad.double()) and _close(out[1], W.grad.double())
     w.layer.close()
+
+
+def test_weights_of_the_transpose_around_a_capture(work):
+    """Feature gradients alone, captured and eager in turn: a replay uses its weights as they are then, and an eager call
+    never the weights that a recording or a replay has left or not yet left in the transpose."""
+    import torch
+    op, id_ = work.ops.layer_backward_features, work.layer.layer_id
+    dC = torch.randn((work.M, work.K), device="cuda")
+
+    def want(W):
+        return work.dense(W).T @ dC.double()
+
+    W, other, late = work.v.clone(), work.v * -3, work.v * 5
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert _close(op(dC, W, id_), want(W))
+        torch.cuda.synchronize()
+        graph, recorded_only = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = op(dC, W, id_)
+        graph.replay()
+        assert _close(out, want(W))
+        W.mul_(2)
+        graph.replay()
+        assert _close(out, want(W))
+        for _ in range(2):
+            assert _close(op(dC, other, id_), want(other))
+            graph.replay()
+            assert _close(out, want(W))
+        with torch.cuda.graph(recorded_only, stream=side):
+            op(dC, late, id_)
+        assert _close(op(dC, late, id_), want(late))
+        torch.cuda.synchronize()
+        del graph, recorded_only, out
