@@ -204,16 +204,21 @@ int hpspmm_layer_backward(hpspmm_ctx* ctx, hpspmm_layer* g, int64_t K, const flo
   HPSPMM_REQUIRE(ctx, vals && dC && H && dH && dA, "null operand");
   if ((K & 3) == 0) HPSPMM_REQUIRE(ctx, (((uintptr_t)dC | (uintptr_t)H | (uintptr_t)dH) & 15u) == 0,
                                    "dense operands must be 16-byte aligned");
-  // what no plan can change is refused before one is built (rows of uneven length have the higher limit)
-  if (!hpspmm_layer_grad_covers(K, (uintptr_t)dC | (uintptr_t)H | (uintptr_t)dH) ||
-      !hpspmm_layer_grad_pays(ctx, g->nnz, false))
-    return HPSPMM_ERR_UNSUPPORTED;
+  const uintptr_t addresses = (uintptr_t)dC | (uintptr_t)H | (uintptr_t)dH;
+  if (!hpspmm_layer_grad_covers(K, addresses)) return HPSPMM_ERR_UNSUPPORTED;
   hpspmm_device_guard guard(ctx->device);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing((cudaStream_t)stream, &capture) != cudaSuccess) cudaGetLastError();
+  auto pays = [&](bool even) {
+    return hpspmm_layer_grad_pays(ctx, g->M, K, hpspmm_vector_width(K, addresses), g->nnz, even,
+                                  capture != cudaStreamCaptureStatusNone);
+  };
+  if (!pays(true) && !pays(false)) return HPSPMM_ERR_UNSUPPORTED;   // no plan can change that: none is built for it
   int cls;
   const int st = plans_for(ctx, g, K, stream, &cls);
   if (st != HPSPMM_OK) return st;
   const hpspmm_plan* p = g->plan_t[cls];
-  if (!hpspmm_layer_grad_pays(ctx, g->nnz, hpspmm_even_rows(p))) return HPSPMM_ERR_UNSUPPORTED;
+  if (!pays(hpspmm_even_rows(p))) return HPSPMM_ERR_UNSUPPORTED;
   hpspmm_layer_grad_args a;
   memset(&a, 0, sizeof(a));
   a.rows = (int)g->N, a.K = (int)K, a.n_chunks = (int)p->n_chunks, a.S = p->chunk_nnz;

@@ -149,8 +149,9 @@ struct hpspmm_layer_grad_args {
 };
 // whether the kernel has a shape for K columns at these operands (addresses: or of theirs)
 bool hpspmm_layer_grad_covers(int64_t K, uintptr_t addresses);
-// whether the one kernel beats the three it replaces; even: rows of even length (hpspmm_even_rows)
-bool hpspmm_layer_grad_pays(const hpspmm_ctx* ctx, int64_t nnz, bool even);
+// whether the one kernel beats the three it replaces; M: rows of dC, VEC: hpspmm_vector_width of the operands, even: rows of
+// even length (hpspmm_even_rows), captured: the call is recorded in a graph
+bool hpspmm_layer_grad_pays(const hpspmm_ctx* ctx, int64_t M, int64_t K, int VEC, int64_t nnz, bool even, bool captured);
 int hpspmm_layer_grad_launch(hpspmm_ctx* ctx, const hpspmm_layer_grad_args& a, cudaStream_t s);
 
 static inline int hpspmm_set_err(hpspmm_ctx* ctx, int status, const char* what, cudaError_t e) {

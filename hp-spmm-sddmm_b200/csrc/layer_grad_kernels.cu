@@ -233,17 +233,49 @@ bool hpspmm_layer_grad_covers(int64_t K, uintptr_t addresses) {
   return K <= (hpspmm_vector_width(K, addresses) == 1 ? 128 : 256);
 }
 
-// Whether one pass is faster than the permuted weights, the product and the SDDMM by themselves.  The 4-byte accesses
-// through the permutation are cheap as long as what they reach, 8 bytes per entry, stays in the L2 cache beside the rows of
-// dC: three kernels -> one in us, power-law graphs, K = 16 / 32 / 64 / 128:
-//   4 M entries, 250 K rows   118 -> 85 / 131 -> 93 / 180 -> 134 / 280 -> 222     (update of the weights 21, product 79, SDDMM 76 at K = 64)
-//   10 M, 600 K               257 -> 243 / 278 -> 274 / 410 -> 383 / 710 -> 659
-//   14 M, 1 M                 382 -> 471 / 398 -> 480 / 588 -> 624
-// and with uniform columns, where hardly a row of dC is found in the cache, it ends earlier:
-//   6 M, 350 K                170 -> 129 / 212 -> 186 / 335 -> 304 / 722 -> 623
-//   8 M, 500 K                240 -> 234 / 302 -> 308 / 501 -> 511 / 1098 -> 888
-bool hpspmm_layer_grad_pays(const hpspmm_ctx* ctx, int64_t nnz, bool even) {
-  return 8 * nnz <= (even ? ctx->l2_bytes * 7 / 16 : ctx->l2_bytes * 5 / 8);
+// Whether one pass is faster than the permuted weights, the product and the SDDMM by themselves.  All figures are the time
+// of those three divided by the time of one pass, replayed from a graph (no launch overhead), over graphs of 4, 16 and 50
+// entries per row, square.
+//
+// Many entries: the 4-byte accesses through the permutation are cheap as long as what they reach, 8 bytes per entry, stays
+// in the L2 cache beside the rows of dC.
+//   uneven rows: 8 M entries 0.99 to 1.42 at K = 2 to 256; 10 M (5/8 of the cache) in rows of 4: 0.90 to 0.97 at K <= 32,
+//                1.02 to 1.19 from 47 on; in rows of 16 and more 1.00 to 1.35.  14 M in 1 M rows: 0.81, 0.83, 0.94 at K = 16, 32, 64
+//   even rows:   5 M entries 0.97 to 1.54; 6 M 0.99 to 1.50, but in rows of 50 entries K = 96 to 192 0.89 to 0.98.
+//                7.2 M (7/16 of the cache): what loses there has rows of dC that take between a sixth of the cache and the
+//                whole of it: in rows of 4 K = 4 to 20 0.87 to 0.97, of 16 K = 20 to 47 0.91 to 0.99, of 50 K = 96 to 126
+//                0.87 to 0.99; below 1.08 to 1.41, above 1.02 to 1.41.  8 M in 500 K rows: 1.03, 0.98, 0.98, 1.24 at K = 16, 32, 64, 128
+// Few entries: the product and the SDDMM have builds for few chunks, which hide the ends of rows better.
+//   uneven rows, 150 K / 300 K / 500 K / 700 K / 1 M / 1.5 M / 2 M entries, worst of the three graphs:
+//     K = 8   0.82 / 0.84 / 0.72 / 0.81 / 0.84 / 0.94 / 1.03        K = 20  0.84 / 0.90 / 0.77 / 0.92 / 0.95 / 1.16 / 1.19
+//     K = 32  0.96 / 0.98 / 0.89 / 0.98 / 1.07 / 1.23 / 1.45        K = 48  0.92 / 1.04 / 0.93 / 1.09 / 1.10 / 1.27 / 1.31
+//     K = 64  1.06 / 1.17 / 1.11 / 1.06 / 1.18 / 1.50 / 1.31        K = 96  0.66 / 0.63 / 0.82 / 1.00 / 1.10 / 1.23 / 1.12
+//     K = 128 0.86 / 0.89 / 1.06 / 1.33 / 1.27 / 1.24 / 1.22        K = 256 0.67 / 0.77 / 1.14 / 1.10 / 1.31 / 1.31 / 1.16
+//     K = 31, 47, 127 (4-byte vectors) 0.98 to 1.44 at every size
+//   even rows, 100 K / 300 K / 600 K / 700 K / 1 M: K <= 64 1.01 to 1.71 (K = 8 in rows of 4 0.94 once); K = 96 (three vectors
+//     per lane) 0.97 / 0.92 / 0.91 / 1.13 / 1.30; K = 128 1.01 / 0.97 / 1.26 / 1.24 / 1.34; K = 256 0.80 / 0.93 / 1.01 / 1.33 / 1.43
+//     (of these 300 K in rows of 4 and 16 1.24 and 1.18)
+// A call that is not captured pays for three launches instead of one besides, and one of up to 40 M products (even
+// rows, K = 256: 80 M) is over before the host has issued the next: a training step through PyTorch of 11 K to 300 K entries,
+// K = 4 to 128, 88 -> 79 us, even rows, K = 256, 300 K in rows of 50 87 -> 79, and from there on as above (uneven rows, K = 96,
+// 500 K entries 111 -> 120; K = 256, 300 K 116 -> 118).
+bool hpspmm_layer_grad_pays(const hpspmm_ctx* ctx, int64_t M, int64_t K, int VEC, int64_t nnz, bool even, bool captured) {
+  const int64_t reached = 8 * nnz, l2 = ctx->l2_bytes, rows = 4 * K * M;
+  if (even) {
+    if (reached > l2 * 7 / 16 || (reached > l2 * 3 / 8 && rows > l2 / 6 && rows < l2 * 5 / 4)) return false;
+    if (reached > l2 * 5 / 16 && nnz >= 32 * M && VEC > 1 && K > 64 && K <= 192) return false;
+  } else {
+    if (reached > l2 / 2 && (reached > l2 * 5 / 8 || (K < 100 && nnz < 16 * M))) return false;
+  }
+  int chunks_per_sm = 0;   // of 128 entries
+  if (VEC > 1 || K < 31) {
+    if (even)
+      chunks_per_sm = VEC < 4 || K <= 64 ? 0 : (K <= 96 || (K > 128 && K <= 192) ? 36 : (K > 192 && nnz < 32 * M ? 15 : 24));
+    else if (K != 64)
+      chunks_per_sm = K >= 128 ? 24 : (K >= 48 ? 36 : (K >= 32 ? 48 : (K >= 17 ? 72 : 100)));
+  }
+  return nnz > ctx->sm_count * 128ll * chunks_per_sm ||
+         (!captured && nnz * K < (even && K > 192 ? 80000000 : 40000000));
 }
 
 // Shapes: one vector per lane and as wide a group as it takes; two and three vectors per lane, which the SDDMM prefers,

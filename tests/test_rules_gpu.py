@@ -188,3 +188,88 @@ def test_the_signature_names_the_shape_that_is_launched(gpu_ctx, pkg):
             assert below in signature(line * SMS, K) and above in signature(line * SMS + 1, K)
     for K in (64, 96, 98, 132, 192, 260):
         assert "mid" not in signature(17 * SMS, K) and "mid" not in signature(48 * SMS, K)
+
+
+def _layer_graph(nnz, even, M=None):
+    """Square CSR on the GPU with rows of nearly the same length; its columns, the rows of the transpose, likewise, or half
+    of the entries in columns of about 900."""
+    import torch
+    M = M or nnz // (16 if even else 8)
+    rp = torch.arange(M + 1, device="cuda", dtype=torch.int64) * nnz // M
+    ci = torch.randint(M, (nnz,), dtype=torch.int32, device="cuda")
+    if not even:
+        ci[::2] %= nnz // 1800
+    return M, rp.int(), ci
+
+
+def _one_pass(ctx, pkg, nnz, even, Ks, M=None):
+    """For every width whether hpspmm_layer_backward takes the call, captured and not."""
+    import torch
+    M, rp, ci = _layer_graph(nnz, even, M)
+    v, dA = torch.rand(nnz, device="cuda"), torch.empty(nnz, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    taken = {}
+    with torch.cuda.stream(side):
+        s = side.cuda_stream
+        layer = pkg.Layer(ctx, M, M, nnz, rp.data_ptr(), ci.data_ptr(), v.data_ptr(), max(Ks), s)
+        for K in Ks:
+            dC, H, dH = (torch.rand((M, K), device="cuda") for _ in range(3))
+            layer.forward(K, H.data_ptr(), dH.data_ptr(), s)       # builds the plans of the class
+
+            def call():
+                st = ctx.lib.hpspmm_layer_backward(ctx.handle, layer.handle, K, v.data_ptr(), dC.data_ptr(), H.data_ptr(),
+                                                   dH.data_ptr(), dA.data_ptr(), s)
+                assert st in (0, pkg.ERR_UNSUPPORTED)
+                return st == 0
+
+            eager = call()
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=side):
+                dA.zero_()
+                captured = call()
+            del graph
+            taken[K] = (captured, eager)
+        torch.cuda.synchronize()
+        layer.close()
+    return taken
+
+
+@pytest.mark.parametrize("line,even,K", [(100, False, 16), (72, False, 20), (72, False, 30), (48, False, 32), (36, False, 48),
+                                         (36, False, 126), (24, False, 128), (24, False, 256), (36, True, 68), (24, True, 100),
+                                         (36, True, 132), (15, True, 256)])
+def test_one_pass_gradients_of_few_entries(gpu_ctx, pkg, line, even, K):
+    nnz = line * 128 * gpu_ctx.lib.hpspmm_ctx_sm_count(gpu_ctx.handle)
+    small = nnz * K < (80_000_000 if even and K == 256 else 40_000_000)
+    assert _one_pass(gpu_ctx, pkg, nnz, even, [K]) == {K: (False, small)}
+    assert _one_pass(gpu_ctx, pkg, nnz + 1, even, [K]) == {K: (True, True)}
+
+
+def test_one_pass_gradients_of_few_entries_at_other_widths(gpu_ctx, pkg):
+    assert all(c and e for c, e in _one_pass(gpu_ctx, pkg, 20_000, False, [31, 47, 64, 127]).values())
+    assert all(c and e for c, e in _one_pass(gpu_ctx, pkg, 20_000, True, [1, 16, 31, 62, 64, 126, 127]).values())
+    assert all(e and not c for c, e in _one_pass(gpu_ctx, pkg, 20_000, False, [1, 16, 32, 48, 62, 96, 128, 254]).values())
+    for nnz, eager in ((312_499, True), (312_501, False)):
+        assert _one_pass(gpu_ctx, pkg, nnz, False, [128]) == {128: (False, eager)}
+        assert _one_pass(gpu_ctx, pkg, nnz, True, [256], M=8000) == {256: (False, eager)}        # long rows
+    nnz = 24 * 128 * gpu_ctx.lib.hpspmm_ctx_sm_count(gpu_ctx.handle)
+    assert _one_pass(gpu_ctx, pkg, nnz, True, [256], M=8000) == {256: (False, False)}
+    assert _one_pass(gpu_ctx, pkg, nnz + 1, True, [256], M=8000) == {256: (True, True)}
+
+
+def test_one_pass_gradients_of_many_entries(gpu_ctx, pkg):
+    l2 = gpu_ctx.lib.hpspmm_ctx_l2_bytes(gpu_ctx.handle)
+    both, none = (True, True), (False, False)
+    for even, part, M, inside, beyond in (
+            (True, 5 / 16, l2 // 400, {32: both, 100: both}, {32: both, 100: both}),      # 16 entries per row
+            (True, 5 / 16, l2 // 2000, {64: both, 68: both, 192: both}, {64: both, 68: none, 127: both, 192: none, 196: both}),
+            (True, 3 / 8, l2 // 400, {8: both, 32: both}, {8: both, 32: none}),           # rows of dC: 0.08 and 0.32 of the cache
+            (True, 3 / 8, l2 // 50, {8: both, 16: both}, {8: none, 16: both}),            # 0.64 and 1.28
+            (True, 7 / 16, l2 // 400, {8: both}, {8: none}),
+            (False, 1 / 2, l2 // 64, {32: both, 100: both}, {32: none, 100: both}),
+            (False, 1 / 2, l2 // 400, {32: both}, {32: both}),
+            (False, 5 / 8, l2 // 400, {32: both, 100: both}, {32: none, 100: none})):
+        nnz = int(l2 * part) // 8
+        assert _one_pass(gpu_ctx, pkg, nnz, even, list(inside), M) == inside
+        assert _one_pass(gpu_ctx, pkg, nnz + 1, even, list(beyond), M) == beyond
