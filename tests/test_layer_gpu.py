@@ -148,6 +148,40 @@ def test_both_gradients_in_one_pass(gpu_ctx, pkg, oracle, K):
             b.free()
 
 
+@pytest.mark.parametrize("K", [30, 62, 126, 128, 130, 254])
+def test_both_gradients_of_rows_on_4_byte_boundaries(gpu_ctx, pkg, oracle, K):
+    """Even widths whose operands allow only 4-byte vectors: up to 128 columns then."""
+    ctx = gpu_ctx
+    g = pkg.gen_rmat(10, 24, seed=44)
+    M, N, nnz = g["M"], g["N"], g["nnz"]
+    H = pkg.host_fill_uniform(N * K, 44, 1, -1.0, 1.0).reshape(N, K)
+    dC = pkg.host_fill_uniform(M * K, 44, 2, -1.0, 1.0).reshape(M, K)
+    shifted = [np.concatenate([np.zeros(1, np.float32), x.ravel()]) for x in (H, dC)]
+    d_rp, d_ci, d_v, d_H, d_dC = bufs = [ctx.upload(a) for a in (g["row_ptr"], g["col_idx"], g["vals"], *shifted)]
+    layer = pkg.Layer(ctx, M, N, nnz, d_rp, d_ci, d_v, 256)
+    out_H, out_A = ctx.alloc((N * K + 1,), np.float32), ctx.alloc((nnz,), np.float32)
+    rpt, cit, vt, _ = oracle.csr_transpose(M, N, g["row_ptr"], g["col_idx"], g["vals"])
+    for off_C, off_H, off_dH in ((4, 4, 4), (4, 0, 0), (0, 4, 0), (0, 0, 4)):
+        at = [d_dC.ptr + off_C, d_H.ptr + off_H, out_H.ptr + off_dH]
+        st = ctx.lib.hpspmm_layer_backward(ctx.handle, layer.handle, K, d_v.ptr, *at, out_A.ptr, None)
+        if K == 128:
+            assert st == pkg.ERR_INVALID             # a multiple of 4 is refused unless the rows are 16-byte aligned
+        elif K > 128:
+            assert st == pkg.ERR_UNSUPPORTED
+        else:
+            assert st == 0
+            ctx.stream_sync()
+            dC_seen, H_seen = (x[1:] if o else x[:-1] for x, o in ((shifted[1], off_C), (shifted[0], off_H)))
+            ref, abs_sum = oracle.spmm_f64(rpt, cit, vt, dC_seen.reshape(M, K))
+            got = out_H.to_host()
+            check_against_f64((got[1:] if off_dH else got[:-1]).reshape(N, K), ref, abs_sum, "dH")
+            ref, abs_sum = oracle.sddmm_f64(g["row_ptr"], g["col_idx"], dC_seen.reshape(M, K), H_seen.reshape(N, K))
+            check_against_f64(out_A.to_host(), ref, abs_sum, "dA")
+    layer.close()
+    for b in bufs + [out_H, out_A]:
+        b.free()
+
+
 def test_both_gradients_refused_before_anything_is_built(gpu_ctx, pkg):
     """Weights that fill the L2 cache: no plan can change the answer, so none is built for it."""
     import torch
