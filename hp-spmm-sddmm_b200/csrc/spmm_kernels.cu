@@ -660,16 +660,30 @@ int32_t planless_chunk_nnz(int64_t K, int64_t nnz, const hpspmm_opts* opts) {
 
 // Whether a product without a plan lets every warp search row_ptr for its chunk (one launch) instead of building the
 // records and the list of filled rows first (two more).  A search costs a chunk 1 to 2 us of latency and the product its
-// steps along row_ptr, the builders 4 to 8 us a call; with more chunks than fit on the GPU the searches add up, and long
-// rows gain by the records' order (pieces last).  Search -> records in us:
-//   chunks of 128: 700 K entries (37 chunks per SM), power-law K = 32 / 64 / 128 31.2 -> 21.3 / 35.0 -> 25.6 / 45.0 -> 32.6,
-//                  uniform K = 32 16.7 -> 16.6, in 170 K rows 25.6 -> 24.4; 335 K, K = 100 (18 per SM), power-law 31.9 -> 27.7;
-//                  300 K, K = 100 (16 per SM), uniform 16.4 -> 19.4; 150 K, K = 100 (8 per SM), power-law 23.2 -> 22.0, uniform 13.2 -> 16.2
-//   chunks of 64:  335 K (35 per SM), power-law K = 64 20.6 -> 22.1; 300 K (32 per SM), uniform 10.0 -> 13.4
-// (the figures beyond K = 32 with builders that took 1 to 2 us longer).  With very many empty rows between the entries the list
-// pays for itself.
+// steps along row_ptr, the builders 2 to 3 us a call; with more chunks than fit on the GPU (32 warps per SM of the searching
+// builds) the searches add up, and long rows gain by the records' order (pieces last).  Rows of even length gain by records
+// from there on only; a power-law graph would gain below as well, but without a plan the rows are not known, and one kind
+// is not to pay for the other.  Search -> records in us, chunks of 128, square matrices of 4 / 16 / 50 entries per row:
+//   chunks per SM   17                                20                                24
+//     uniform K=100 20.8>22.0 / 15.9>17.7 / 14.4>16.5 23.3>24.3 / 17.6>18.8 / 15.6>17.2 27.8>28.5 / 18.1>19.8 / 16.9>18.7
+//     uniform K=256 43.2>45.9 / 23.5>26.1 / 23.1>25.6 49.9>52.5 / 26.7>29.3 / 25.4>27.6 64.4>65.8 / 29.7>31.9 / 27.9>30.1
+//     skewed  K=100 44.5>26.3 / 27.4>23.3 / 22.2>21.8 43.7>28.1 / 31.9>24.8 / 23.1>23.8 49.5>29.3 / 32.6>26.7 / 24.6>24.6
+//     skewed  K=256 55.9>39.9 / 34.7>31.4 / 27.6>31.1 56.0>41.8 / 38.5>33.4 / 29.5>33.0 65.1>49.5 / 41.3>36.3 / 32.2>34.3
+//   chunks per SM   28                                32                                33
+//     uniform K=32  18.1>20.8 / 11.6>13.6 /  9.3>11.3 19.5>21.2 / 12.6>13.9 /  9.8>11.9 24.2>22.1 / 15.8>14.7 / 12.8>12.2
+//     uniform K=64  21.1>25.3 / 14.2>17.1 / 12.7>14.9 22.4>26.2 / 15.2>17.8 / 13.5>16.1 31.2>27.2 / 20.6>18.1 / 17.8>15.8
+//     uniform K=128 37.9>40.3 / 21.6>23.3 / 20.4>22.1 42.0>44.7 / 23.8>24.9 / 21.8>23.5 62.0>46.3 / 31.6>24.5 / 28.3>23.6
+//     skewed  K=64  47.9>28.9 / 29.0>23.1 / 21.9>21.3 49.2>28.8 / 30.5>23.5 / 22.9>23.3 52.3>28.9 / 35.2>25.1 / 29.3>22.7
+//   chunks per SM   36                                37                                40
+//     uniform K=32  25.2>22.5 / 16.5>14.8 / 13.4>12.1 25.4>24.5 / 16.6>16.4 / 13.5>14.3 26.5>25.4 / 17.0>16.9 / 13.9>14.8
+//     uniform K=64  34.3>27.5 / 21.5>18.5 / 18.7>16.4 35.7>36.5 / 22.1>22.3 / 18.9>20.0 38.5>38.7 / 22.0>23.1 / 19.4>21.0
+//     uniform K=128 65.9>49.1 / 33.1>26.1 / 29.8>25.2 59.2>58.6 / 32.0>31.3 / 28.1>28.5 62.2>61.4 / 32.6>32.0 / 29.3>29.3
+//     skewed  K=64  55.9>30.9 / 36.7>24.2 / 30.2>24.0 62.2>32.4 / 37.5>26.9 / 29.8>24.4 55.6>31.6 / 38.0>25.2 / 30.6>25.3
+// (between 37 and 40 the records' product is in its second wave, and uniform rows of 16 and more entries are up to 8 % behind
+// at K <= 64; everything else is ahead there.)  Chunks of 64: 335 K entries (35 per SM), power-law K = 64 20.6 -> 22.1; 300 K
+// (32 per SM), uniform 10.0 -> 13.4.  With very many empty rows between the entries the list pays for itself.
 bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t n_chunks, int32_t S) {
-  return n_chunks <= ctx->sm_count * (S < 128 ? 40ll : 16ll) && M <= 8 * nnz;
+  return n_chunks <= ctx->sm_count * (S < 128 ? 40ll : 32ll) && M <= 8 * nnz;
 }
 
 // Counters that are set aside at the first product of a width: enough for any later one of up to that width, so that a

@@ -273,3 +273,32 @@ def test_one_pass_gradients_of_many_entries(gpu_ctx, pkg):
         nnz = int(l2 * part) // 8
         assert _one_pass(gpu_ctx, pkg, nnz, even, list(inside), M) == inside
         assert _one_pass(gpu_ctx, pkg, nnz + 1, even, list(beyond), M) == beyond
+
+
+@pytest.mark.parametrize("K", [20, 100, 256])
+def test_planless_products_on_both_sides_of_the_search_line(gpu_ctx, pkg, oracle, K):
+    """One launch that searches row_ptr for its chunks, or three that build records first: up to 40 chunks per SM of fewer
+    than 128 entries, up to 32 of more."""
+    ctx, N = gpu_ctx, 2000
+    sms = ctx.lib.hpspmm_ctx_sm_count(ctx.handle)
+    for S, line in ((32, 40), (96, 40), (128, 32), (160, 32)):
+        for n_chunks in (17 * sms, line * sms, line * sms + 1):
+            rng = np.random.default_rng(S)
+            nnz = n_chunks * S - 5
+            degrees = rng.choice([0, 3, 40, 31, S + 1, 5 * S], size=8 * nnz // S)
+            rp = np.minimum(np.concatenate([[0], np.cumsum(degrees)]), nnz).astype(np.int32)
+            rp[-1] = nnz
+            ci = rng.integers(0, N, nnz).astype(np.int32)
+            v = rng.uniform(-1, 1, nnz).astype(np.float32)
+            M = len(rp) - 1
+            B = pkg.host_fill_uniform(N * K, 9, 1, -1.0, 1.0).reshape(N, K)
+            bufs = [ctx.upload(x) for x in (rp, ci, v, B)]
+            buf, c_ptr, read = guarded_output(ctx, (M, K))
+            before = ctx.launch_count()
+            ctx.spmm_csr(M, N, K, nnz, *bufs, c_ptr, opts=pkg.Opts(chunk_nnz=S))
+            assert ctx.launch_count() - before == (1 if n_chunks <= line * sms else 3), (S, n_chunks)
+            ctx.stream_sync()
+            ref, abs_sum = oracle.spmm_f64(rp, ci, v, B)
+            check_against_f64(read(), ref, abs_sum, "K=%d S=%d chunks=%d" % (K, S, n_chunks))
+            for b in bufs + [buf]:
+                b.free()
