@@ -258,6 +258,25 @@ int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes) {
   return HPSPMM_OK;
 }
 
+int hpspmm_try_scratch(hpspmm_ctx* ctx, size_t bytes) {
+  if (bytes <= ctx->scratch_bytes) return HPSPMM_OK;
+  void* grown = nullptr;
+  const size_t want = bytes + bytes / 4 + 4096;
+  if (hpspmm_device_malloc(&grown, want) != cudaSuccess) {
+    cudaGetLastError();
+    return HPSPMM_ERR_OOM;
+  }
+  const cudaError_t e = cudaDeviceSynchronize();   // the old buffer may still be in use by queued kernels
+  if (e != cudaSuccess) {
+    cudaFree(grown);
+    return hpspmm_set_err(ctx, HPSPMM_ERR_CUDA, "scratch", e);
+  }
+  if (ctx->scratch) cudaFree(ctx->scratch);
+  ctx->scratch = grown;
+  ctx->scratch_bytes = want;
+  return HPSPMM_OK;
+}
+
 int hpspmm_ensure_counters(hpspmm_ctx* ctx, int64_t n, cudaStream_t stream) {
   if (n > ctx->counter_cap) {
     if (ctx->counters) {   // the old ones may still be in use by queued kernels

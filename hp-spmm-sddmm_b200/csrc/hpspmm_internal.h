@@ -213,6 +213,8 @@ struct hpspmm_trace_range {
 #define HPSPMM_TRACE(name) hpspmm_trace_range hpspmm_trace_range__(name)
 
 int hpspmm_ensure_scratch(hpspmm_ctx* ctx, size_t bytes);
+// the same for a caller that can do with less: HPSPMM_ERR_OOM leaves the scratch as it was
+int hpspmm_try_scratch(hpspmm_ctx* ctx, size_t bytes);
 // Two sets of at least `n` counters, zero when work queued on `stream` starts.  hpspmm_take_counters hands out the set for
 // one product, whose kernel clears the first `*n_clear` ints at `*clear`; hpspmm_counters_used tells how many it counts in
 // and how its launch went.  Not for captured calls: a graph may be replayed between any two products, so a captured call

@@ -686,6 +686,12 @@ bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t 
   return n_chunks <= ctx->sm_count * (S < 128 ? 40ll : 32ll) && M <= 8 * nnz;
 }
 
+// Up to here a search costs little enough to do without the records where there is no room for them: a call that is
+// captured cannot allocate, and another may find the device full.
+bool may_search_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t n_chunks) {
+  return n_chunks <= ctx->sm_count * 40ll && M <= 8 * nnz;
+}
+
 // Counters that are set aside at the first product of a width: enough for any later one of up to that width, so that a
 // smaller call never allocates.  Beyond 512 columns as many as the call needs.
 int64_t counters_to_keep(const hpspmm_ctx* ctx, int64_t K, int64_t n_counter, bool search) {
@@ -885,11 +891,16 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
   }
   const int32_t S = planless_chunk_nnz(K, nnz, opts);
   const int64_t n_chunks = (nnz + S - 1) / S;
-  const bool search = searches_for_chunks(ctx, M, nnz, n_chunks, S);
-  const planless_layout lay(M, K, n_chunks, search);
+  bool search = searches_for_chunks(ctx, M, nnz, n_chunks, S);
+  planless_layout lay(M, K, n_chunks, search);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
   const bool eager = capture == cudaStreamCaptureStatusNone;
+  if (!search && lay.bytes > ctx->scratch_bytes && may_search_for_chunks(ctx, M, nnz, n_chunks) &&
+      (!eager || hpspmm_try_scratch(ctx, lay.bytes) != HPSPMM_OK)) {
+    search = true;
+    lay = planless_layout(M, K, n_chunks, true);
+  }
   st = hpspmm_ensure_scratch(ctx, lay.bytes);
   if (st == HPSPMM_OK && eager) st = hpspmm_ensure_counters(ctx, counters_to_keep(ctx, K, lay.n_counter, search), s);
   if (st != HPSPMM_OK) return st;
@@ -959,7 +970,7 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
   if (st != HPSPMM_OK) return st;
   // size the kernel scratch before anything is queued (growing it synchronises the device)
   {
-    size_t need = 0;
+    size_t need = 0, least = 0;   // least: with searches wherever they will do
     int64_t need_counters = 0;
     for (int i = 0; i < n_slabs; ++i) {
       const int64_t w = slabs[i].width;
@@ -968,9 +979,12 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
       const bool search = searches_for_chunks(ctx, M, nnz, n_chunks, S);
       const planless_layout lay(M, w, n_chunks, search);
       need = lay.bytes > need ? lay.bytes : need;
+      const planless_layout small(M, w, n_chunks, search || may_search_for_chunks(ctx, M, nnz, n_chunks));
+      least = small.bytes > least ? small.bytes : least;
       const int64_t keep = counters_to_keep(ctx, w, lay.n_counter, search);
       need_counters = keep > need_counters ? keep : need_counters;
     }
+    if (least < need && hpspmm_try_scratch(ctx, need) != HPSPMM_OK) need = least;
     st = hpspmm_ensure_scratch(ctx, need);
     if (st == HPSPMM_OK) st = hpspmm_ensure_counters(ctx, need_counters, s_run);
     if (st != HPSPMM_OK) return st;

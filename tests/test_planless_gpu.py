@@ -250,3 +250,66 @@ def test_pieces_of_long_rows_come_last(gpu_ctx, pkg, oracle, seed):
     check_against_f64(d_o.to_host(), ref, abs_sum, "SDDMM without a plan")
     for b in bufs + [d_C, d_o]:
         b.free()
+
+
+class _ManyRows(_Work):
+    """36 chunks per SM in three million rows: the records need 24 MB more than a search does."""
+
+    def __init__(self, pkg, oracle, K):
+        import torch
+        rng = np.random.default_rng(130)
+        self.M, self.N, self.K, self.nnz = 3_000_000, 20000, K, 36 * 148 * 128 - 9
+        degrees = np.bincount(rng.integers(0, self.M, self.nnz - 30 * 2000), minlength=self.M)
+        degrees[rng.integers(0, self.M, 30)] += 1
+        degrees[np.arange(30) * 90_000 + 5] += (self.nnz - degrees.sum()) // 30
+        degrees[-1] += self.nnz - degrees.sum()
+        self.rp_h = np.concatenate([[0], np.cumsum(degrees)]).astype(np.int32)
+        self.ci_h = rng.integers(0, self.N, self.nnz).astype(np.int32)
+        self.v_h = rng.uniform(-1, 1, self.nnz).astype(np.float32)
+        self.B_h = pkg.host_fill_uniform(self.N * K, 130, 1, -1.0, 1.0).reshape(self.N, K)
+        self.ref, self.abs_sum = oracle.spmm_f64(self.rp_h, self.ci_h, self.v_h, self.B_h)
+        self.rp, self.ci, self.v, self.B = (torch.from_numpy(x).cuda() for x in (self.rp_h, self.ci_h, self.v_h, self.B_h))
+        self.C = torch.empty((self.M, K), device="cuda")
+
+
+def test_no_room_for_the_records(pkg, oracle):
+    """A product of 33 to 40 chunks per SM searches for them where the scratch has no room for records and cannot grow:
+    under capture, with the device full, and in the host pipeline."""
+    import torch
+    lib = pkg.load_library()
+    before = _Work(pkg, oracle, [300] * 300, 20000, 96, 131)       # sizes the scratch for a search
+    w = _ManyRows(pkg, oracle, 32)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with pkg.Context(0) as ctx, torch.cuda.stream(side):
+        s = side.cuda_stream
+        before.call(ctx, s)
+        before.check("warm-up")
+        opts = pkg.Opts(chunk_nnz=128)
+        before.call(ctx, s, pkg.Opts(chunk_nnz=32))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            w.call(ctx, s, opts)
+        for turn in range(2):
+            graph.replay()
+            w.check("replay %d" % turn)
+        launches = ctx.launch_count()
+        lib.hpspmm_debug_fail_device_alloc(1, 1000)
+        try:
+            w.call(ctx, s, opts)
+            w.check("device full")
+        finally:
+            lib.hpspmm_debug_fail_device_alloc(0, 0)
+        assert ctx.launch_count() - launches == 1
+        del graph
+        w.call(ctx, s, opts)
+        w.check("room again")
+        assert ctx.launch_count() - launches == 1 + 3
+    with pkg.Context(0) as ctx:
+        C = np.full((w.M, w.K), 7.0, np.float32)
+        lib.hpspmm_debug_fail_device_alloc(2, 2)                    # the first one is for the operands
+        try:
+            ctx.spmm_csr_host_multi(w.M, w.N, w.nnz, w.rp_h, w.ci_h, w.v_h, [w.K], [w.B_h], [C], opts=opts)
+        finally:
+            lib.hpspmm_debug_fail_device_alloc(0, 0)
+        check_against_f64(C, w.ref, w.abs_sum, "host pipeline")
