@@ -112,4 +112,18 @@ __device__ __forceinline__ unsigned subwarp_mask() {
 // with ordinary launches, 38.0 like this, 44.7 with the early start; never ahead by more than 2 %.)
 __device__ __forceinline__ void chain_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The first loads after chain_grid(), from which the addresses of all others follow.  A load through the read-only path
+// (__ldg, ld.global.nc) says that its data stays as it is for the whole kernel, which begins before the wait: a compiler may
+// move it in front.  These are ordinary loads and stay behind the wait, and so does everything that depends on them.
+__device__ __forceinline__ int ld_chained(const int* p) {
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int4 ld_chained(const int4* p) {
+  int4 v;
+  asm volatile("ld.global.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 }  // namespace hpspmm

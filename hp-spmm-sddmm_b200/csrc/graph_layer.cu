@@ -40,7 +40,7 @@ __global__ void gather_by_perm_kernel(int64_t n, const int* __restrict__ perm, c
   hpspmm::chain_grid();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride)
-    dst[t] = __ldg(src + perm[t]);
+    dst[t] = __ldg(src + hpspmm::ld_chained(perm + t));
 }
 
 void release(hpspmm_ctx* ctx, hpspmm_layer* g) {

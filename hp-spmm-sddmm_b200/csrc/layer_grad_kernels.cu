@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(BT, MINB) layer_grad_kernel(const __grid_const
   const int slot = (int)((blockIdx.x * (unsigned)BT + threadIdx.x) >> 5);
   if (slot >= a.n_chunks) return;
   int* m = meta[threadIdx.x >> 5];
-  const int4 rec0 = __ldg(a.rec + 2 * (int64_t)slot), rec1 = __ldg(a.rec + 2 * (int64_t)slot + 1);
+  const int4 rec0 = ld_chained(a.rec + 2 * (int64_t)slot), rec1 = ld_chained(a.rec + 2 * (int64_t)slot + 1);
   int base = rec0.x, ri = rec0.y, row = rec0.z, row_end = rec0.w;
   const int n1 = rec1.z;
   if (lane == 0) m[0] = base, m[1] = rec1.x, m[2] = row, m[3] = rec1.y, m[4] = row_end;

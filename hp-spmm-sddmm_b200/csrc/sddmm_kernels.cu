@@ -50,10 +50,10 @@ sddmm_warp_kernel(int n_chunks, int ld, int off0, int cols, int add, int keep_y,
   const uint64_t policy = HINT ? (KS ? policy_evict_last() : policy_for_gathers(keep_y)) : 0ull;
   int(*my)[T] = tiles[threadIdx.x >> 5];
 
-  const int4 p = __ldg(rec + 2 * (int64_t)slot);
+  const int4 p = ld_chained(rec + 2 * (int64_t)slot);
   const int n0 = p.x;
   int ri = p.y, row = p.z, row_end = p.w;
-  const int n1 = __ldg(&rec[2 * (int64_t)slot + 1].z);
+  const int n1 = ld_chained(&rec[2 * (int64_t)slot + 1].z);
 
   auto stage_tile = [&](int stage, int base) {
     const int j = base + lane;

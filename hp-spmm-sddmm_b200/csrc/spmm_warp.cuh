@@ -27,7 +27,11 @@ __device__ __forceinline__ void zero_empty_rows(int M, int K, const int* __restr
   const int64_t stride = (int64_t)n_zero_blocks * warps_per_block * 32;
   int64_t r0 = ((int64_t)zero_block * warps_per_block + (threadIdx.x >> 5)) * 32;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto is_empty = [&](int64_t r) { return r < M && __ldg(row_ptr + r) == __ldg(row_ptr + r + 1); };
+  auto is_empty = [&](int64_t r) {
+    if (r >= M) return false;
+    const int s = ld_chained(row_ptr + r), e = ld_chained(row_ptr + r + 1);
+    return s == e;
+  };
   bool next = is_empty(r0 + lane);
   for (; r0 < M; r0 += stride) {
     unsigned m = __ballot_sync(0xffffffffu, next);
@@ -61,7 +65,7 @@ __device__ __forceinline__ int find_row(const int* __restrict__ row_ptr, int lo,
   while (hi - lo > 1) {
     const int step = (int)(((unsigned)(hi - lo) + 31u) >> 5);
     const int64_t r = lo + (int64_t)lane * step;
-    const unsigned m = __ballot_sync(0xffffffffu, r < hi && __ldg(row_ptr + r) <= t);
+    const unsigned m = __ballot_sync(0xffffffffu, r < hi && ld_chained(row_ptr + r) <= t);
     lo += (__popc(m | 1u) - 1) * step;   // lane 0 probes lo itself
     hi = step < hi - lo ? lo + step : hi;
   }
@@ -233,7 +237,7 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
     if (slot >= a.n_chunks) return;
     int* m = meta[threadIdx.x >> 5];   // what the tail of the kernel needs of the chunk waits in shared memory
     if (LIST) {
-      const int4 p = __ldg(a.rec + 2 * (int64_t)slot), q = __ldg(a.rec + 2 * (int64_t)slot + 1);
+      const int4 p = ld_chained(a.rec + 2 * (int64_t)slot), q = ld_chained(a.rec + 2 * (int64_t)slot + 1);
       base = p.x, ri = p.y, row = p.z, row_end = p.w;
       n1 = q.z;
       if (lane == 0) m[0] = base, m[1] = q.x, m[2] = row, m[3] = q.y, m[4] = row_end;
@@ -254,7 +258,7 @@ __global__ void __launch_bounds__(BT, MINB) spmm_warp_kernel(const __grid_consta
           if (e1 - s1 <= a.S) n1 = s1;
         }
       } else {
-        n1 = __ldg(a.row_ptr + a.M);
+        n1 = ld_chained(a.row_ptr + a.M);
       }
       if (lane == 0) m[0] = base, m[1] = slot, m[2] = row, m[3] = rs, m[4] = row_end;
     }

@@ -654,8 +654,8 @@ row_tile_count_kernel(int M, int tile, const chunk_size cs, const int* __restric
     const int64_t r = r0 + i + threadIdx.x;
     int s = 0, e = 0;
     if (r < M) {
-      s = __ldg(row_ptr + r);
-      e = __ldg(row_ptr + r + 1);
+      s = hpspmm::ld_chained(row_ptr + r);
+      e = hpspmm::ld_chained(row_ptr + r + 1);
     }
     total += __syncthreads_count(e > s);
     if (PIECES) pieces += row_cuts(s, e, cs).pieces();
@@ -713,7 +713,7 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
   hpspmm::chain_grid();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * tile;
-  auto row_start = [&](int64_t r) { return __ldg(row_ptr + (r < M ? r : M)); };
+  auto row_start = [&](int64_t r) { return hpspmm::ld_chained(row_ptr + (r < M ? r : M)); };
   int s = row_start(r0 + threadIdx.x), e = row_start(r0 + threadIdx.x + 1);   // in flight while the counts are added up
   // rows that hold entries and pieces in the tiles above, pieces in all tiles: every load of a thread in flight at once
   constexpr int kPer = kRowTiles / kThreads;   // at most kRowTiles tiles
@@ -721,8 +721,8 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     const int i = q * kThreads + threadIdx.x;
-    rows_of[q] = i < (int)gridDim.x ? __ldg(counts + i) : 0;
-    pieces_of[q] = PIECES && i < (int)gridDim.x ? __ldg(counts + gridDim.x + i) : 0;
+    rows_of[q] = i < (int)gridDim.x ? hpspmm::ld_chained(counts + i) : 0;
+    pieces_of[q] = PIECES && i < (int)gridDim.x ? hpspmm::ld_chained(counts + gridDim.x + i) : 0;
   }
   int before = 0, before_h = 0, all_h = 0;
 #pragma unroll

@@ -313,3 +313,41 @@ def test_no_room_for_the_records(pkg, oracle):
         finally:
             lib.hpspmm_debug_fail_device_alloc(0, 0)
         check_against_f64(C, w.ref, w.abs_sum, "host pipeline")
+
+
+@pytest.mark.parametrize("chunk,per_sm", [(32, 30), (32, 60), (128, 30), (128, 60)])
+def test_operands_written_by_the_kernel_in_front(pkg, oracle, chunk, per_sm):
+    """Two matrices in turn in the same buffers, row_ptr last, each product right behind the copy that brings it and never
+    a synchronisation between: the first loads of a kernel wait for the kernel in front."""
+    import torch
+    rng = np.random.default_rng(chunk)
+    nnz, K, N = per_sm * 148 * chunk - 3, 32, 3000
+    M = nnz // 12
+    works = []
+    for i in range(2):
+        rp = np.sort(rng.integers(0, nnz + 1, M - 1 - 40 * i))
+        rp = np.concatenate([[0], np.zeros(40 * i, np.int64), rp, [nnz]]).astype(np.int32)
+        ci, v = rng.integers(0, N, nnz).astype(np.int32), rng.uniform(-1, 1, nnz).astype(np.float32)
+        B, X = (pkg.host_fill_uniform(n * K, 140 + i, j, -1.0, 1.0).reshape(n, K) for j, n in ((1, N), (2, M)))
+        works.append((oracle.spmm_f64(rp, ci, v, B), oracle.sddmm_f64(rp, ci, X, B),
+                      [torch.from_numpy(a).cuda() for a in (B, X, v, ci, rp)]))
+    now = [torch.empty_like(t) for t in works[0][2]]
+    B, X, v, ci, rp = (t.data_ptr() for t in now)
+    opts = pkg.Opts(chunk_nnz=chunk)
+    with pkg.Context(0) as ctx:
+        s = torch.cuda.current_stream().cuda_stream
+        got = []
+        for turn in range(12):
+            C, out = torch.full((M, K), 7.0, device="cuda"), torch.full((nnz,), 7.0, device="cuda")
+            for dst, src in zip(now, works[turn % 2][2]):
+                dst.copy_(src)
+            ctx.spmm_csr(M, N, K, nnz, rp, ci, v, B, C.data_ptr(), opts=opts, stream=s)
+            now[4].copy_(works[1 - turn % 2][2][4])
+            now[4].copy_(works[turn % 2][2][4])
+            ctx.sddmm_csr(M, N, K, nnz, rp, ci, X, B, out.data_ptr(), opts=opts, stream=s)
+            got.append((C, out))
+        torch.cuda.synchronize()
+        for turn, (C, out) in enumerate(got):
+            (ref_C, sum_C), (ref_out, sum_out), _ = works[turn % 2]
+            check_against_f64(C.cpu().numpy(), ref_C, sum_C, "product, turn %d" % turn)
+            check_against_f64(out.cpu().numpy(), ref_out, sum_out, "SDDMM, turn %d" % turn)
