@@ -351,3 +351,75 @@ def test_operands_written_by_the_kernel_in_front(pkg, oracle, chunk, per_sm):
             (ref_C, sum_C), (ref_out, sum_out), _ = works[turn % 2]
             check_against_f64(C.cpu().numpy(), ref_C, sum_C, "product, turn %d" % turn)
             check_against_f64(out.cpu().numpy(), ref_out, sum_out, "SDDMM, turn %d" % turn)
+
+
+@pytest.mark.parametrize("captured", [True, False])
+def test_products_behind_an_event_join(pkg, oracle, captured):
+    """Products whose launch follows work of two streams: one kernel of their own stream and one, or a copy, of another, with
+    nothing between the join and the launch; also as the first work of a stream that forks."""
+    import torch
+    N = 20000
+    works = [_Work(pkg, oracle, DEGREES, N, K, 150) for K in (32, 100)]
+    plans = []
+    with pkg.Context(0) as ctx:
+        main, other = torch.cuda.Stream(), torch.cuda.Stream()
+        main.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(main):
+            for w in works:
+                plans.append(ctx.plan_create(w.M, w.nnz, w.rp.data_ptr(), w.K, N=N, col_idx=w.ci.data_ptr(),
+                                             stream=main.cuda_stream))
+                w.call(ctx, main.cuda_stream)          # sizes the scratch
+            keep = [(w.rp.clone(), w.v.clone(), w.B.clone()) for w in works]
+            pinned = [w.v.cpu().pin_memory() for w in works]
+            big = torch.rand(1 << 25, device="cuda")
+            main.synchronize()
+
+            def joined(w, i, plan):
+                """row_ptr and B arrive late on the other stream, the weights by a copy there; C is filled on this one."""
+                fork = torch.cuda.Event()
+                fork.record(main)
+                other.wait_event(fork)
+                with torch.cuda.stream(other):
+                    for _ in range(4):
+                        big.mul_(1.0)
+                    w.rp.copy_(keep[i][0])
+                    w.v.copy_(pinned[i], non_blocking=True)
+                    w.B.copy_(keep[i][2])
+                    done = torch.cuda.Event()
+                    done.record(other)
+                w.C.fill_(7.0)
+                main.wait_event(done)
+                ctx.spmm_csr(w.M, w.N, w.K, w.nnz, w.rp.data_ptr(), w.ci.data_ptr(), w.v.data_ptr(), w.B.data_ptr(),
+                             w.C.data_ptr(), plan=plan, stream=main.cuda_stream)
+
+            def steps():
+                for i, w in enumerate(works):
+                    joined(w, i, plans[i])
+                    joined(w, i, None)
+                # the first work of a stream that was forked, its predecessor a product
+                fork = torch.cuda.Event()
+                fork.record(main)
+                other.wait_event(fork)
+                with torch.cuda.stream(other):
+                    ctx.spmm_csr(w.M, w.N, w.K, w.nnz, w.rp.data_ptr(), w.ci.data_ptr(), w.v.data_ptr(), w.B.data_ptr(),
+                                 w.C.data_ptr(), plan=plans[1], stream=other.cuda_stream)
+                    done = torch.cuda.Event()
+                    done.record(other)
+                main.wait_event(done)
+
+            graph = None
+            if captured:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=main):
+                    steps()
+            for turn in range(3):
+                for i, w in enumerate(works):           # what a launch before the join would use
+                    w.B.fill_(float("nan"))
+                    w.v.fill_(3.0)
+                    w.rp.copy_(keep[i][0])
+                graph.replay() if captured else steps()
+                for w in works:
+                    w.check("K=%d, turn %d" % (w.K, turn))
+            del graph
+        for p in plans:
+            ctx.plan_destroy(p)
