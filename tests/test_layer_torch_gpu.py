@@ -81,11 +81,14 @@ def test_weights_that_cannot_be_used_are_refused_every_time(work):
     assert _close(work.layer(work.H, (work.v * 3)[None]), work.product(work.v * 3, work.H))
 
 
-def test_threads_meet_on_one_layer(work):
-    """Three threads on one stream, each with weights of its own that change in every step, beside the engine's."""
+@pytest.mark.parametrize("K", [16, 129])
+def test_threads_meet_on_one_layer(pkg, K):
+    """Three threads on one stream, each with weights of its own that change in every step, beside the engine's; both
+    gradients in one pass, and through the transpose's copy of the weights, which the threads overwrite for each other."""
     import threading
 
     import torch
+    work = _Layer(pkg, K=K, max_K=K)
     want, errors = [work.product(work.v * (t + 1), work.H) for t in range(3)], []
     want_dH = [work.dense(work.v * (t + 1)).T @ torch.ones((work.M, work.K), device="cuda", dtype=torch.float64)
                for t in range(3)]
@@ -109,6 +112,34 @@ def test_threads_meet_on_one_layer(work):
     for t in threads:
         t.join()
     assert not errors, errors[0]
+    work.layer.close()
+
+
+@pytest.mark.parametrize("K", [16, 129])
+def test_feature_gradients_alone_follow_the_weights(pkg, K):
+    """Only H asks for a gradient: the transpose's copy of the weights is filled again when they change in place, when others
+    take their place, and not kept over a step with both gradients."""
+    import torch
+    w = _Layer(pkg, K=K, max_K=K)
+    dC = torch.randn((w.M, K), device="cuda")
+    W, other = w.v.clone(), w.v * 0.25
+
+    def step(vals, learned=False):
+        H = w.H.clone().requires_grad_()
+        vals = vals.clone().requires_grad_() if learned else vals
+        w.layer(H, vals).backward(dC)
+        assert _close(H.grad, w.dense(vals.detach()).T @ dC.double())
+
+    for turn in range(3):
+        step(W)
+        W.mul_(-2)
+        step(W)
+        step(other)
+        step(W, learned=True)
+        step(other)
+        W[:: turn + 2] = 0.5
+        step(W)
+    w.layer.close()
 
 
 def test_closing_under_calls(pkg):
