@@ -21,7 +21,7 @@ Prints one JSON line (rank 0).  `value` is whole-job throughput, device-timed, m
 reference's row loop on the host cores.  `--impl reference` times the reference's own kernels
 (LBSpMM, its flagship, compiled unmodified into oracle/_ref/libref_spmm.so) on one GPU through
 the reference's own entry point, which uploads, runs 200 launches and reports their mean; when that
-library is absent it times the CPU restatement instead and says so.
+library or a GPU is missing it prints a line that says so instead.
 """
 import argparse
 import ctypes
@@ -249,65 +249,56 @@ def time_reference_kernels(lib, g, Bs, coo, which=("lbspmm",)):
 
 
 def run_reference_arm(args, pkg, n_gpus):
+    lib, why = load_ref_lib()
+    if lib is not None:
+        try:
+            import torch
+            if not torch.cuda.is_available():
+                lib, why = None, "no CUDA device for the reference's kernels"
+        except Exception as exc:
+            lib, why = None, "torch unavailable: %s" % exc
+    if lib is None:
+        print(json.dumps({"impl": "reference", "unavailable": why}))
+        return
     g = pkg.gen_rmat(SCALE, EDGE_FACTOR, seed=GRAPH_SEED)
     Bs = {K: pkg.host_fill_uniform(g["N"] * K, GRAPH_SEED, 100 + K, -1.0, 1.0).reshape(g["N"], K) for K in KS}
     info = graph_info(g)
     flops = 2.0 * g["nnz"] * sum(KS)
-    lib, why = load_ref_lib()
-    gpu_ok = False
-    if lib is not None:
-        try:
-            import torch
-            gpu_ok = torch.cuda.is_available()
-            if not gpu_ok:
-                why = "no CUDA device for the reference's kernels"
-        except Exception as exc:
-            why = "torch unavailable: %s" % exc
     cpu = cpu_port_sample(pkg, g, Bs, passes=1)
     line = {"impl": "reference", "metric": METRIC, "unit": "GFLOPS", "n_gpus": n_gpus, "steps": args.steps,
             "warmup": args.warmup, "higher_is_better": True, "scaling": "strong" if n_gpus > 1 else "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic", "cpu_baseline": cpu}
     cfg = {"workload": workload_name(n_gpus)}
     cfg.update(info)
-    if lib is not None and gpu_ok:
-        coo = padded_coo(g)
-        steps = max(1, args.steps)
-        warm = max(1, min(args.warmup, 2))
-        for _ in range(warm):
-            time_reference_kernels(lib, g, Bs, coo)
-        kernel_ms, e2e_ms = [], []
-        launches = 200
-        for _ in range(steps):
-            rec, launches = time_reference_kernels(lib, g, Bs, coo)
-            kernel_ms.append(sum(rec[K]["lbspmm_ms"] for K in KS))
-            # one product end to end = the reference's upload + one launch of its loop + its download
-            e2e_ms.append(sum(rec[K]["lbspmm_upload_ms"] + rec[K]["lbspmm_ms"] + rec[K]["lbspmm_download_ms"]
-                              for K in KS))
-        k_ms, e_ms = statistics.mean(kernel_ms), statistics.mean(e2e_ms)
-        r, c, v = coo
-        h2d = sum(len(r) * 12 + g["N"] * K * 4 for K in KS)
-        d2h = sum(g["M"] * K * 4 for K in KS)
-        cfg["reference_entry"] = ("LBSpMM (HP-SpMM, spmm/mm/spmm_kernel.cu:733-768) on one GPU: per product "
-                                  "Matrix::to(kCUDA) uploads from pageable memory, %d launches timed by its own "
-                                  "GpuTimer, C read back; kernels compiled unmodified for sm_100a" % launches)
-        cfg["per_k_ms"] = {str(K): rec[K]["lbspmm_ms"] for K in KS}
-        cfg["per_k_upload_ms"] = {str(K): rec[K]["lbspmm_upload_ms"] for K in KS}
-        cfg["per_k_download_ms"] = {str(K): rec[K]["lbspmm_download_ms"] for K in KS}
-        line.update({"value": flops / (k_ms * 1e-3) / 1e9, "ms_per_step": k_ms, "kind": "reference",
-                     "e2e": {"value": flops / (e_ms * 1e-3) / 1e9, "unit": "GFLOPS", "h2d_bytes_per_step": int(h2d),
-                             "d2h_bytes_per_step": int(d2h), "ms_per_step": e_ms,
-                             "how": "the reference's own upload (Matrix::to(kCUDA), pageable host memory) + the mean "
-                                    "of its %d timed launches + its own download (Matrix::to(kCPU)), per product" % launches},
-                     "gpu_launches": int(launches * len(KS) * steps), "config": cfg})
-    else:
-        # the reference's kernels cannot run here: time the CPU restatement of its row loop instead
-        steps = max(1, min(args.steps, 10))
-        cpu = cpu_port_sample(pkg, g, Bs, passes=steps)
-        cfg["reference_kernels"] = "unavailable: " + why
-        cfg["reference_entry"] = "CPU restatement of the CSR row loop of spmm/mm/spmm_kernel.cu:324-346, all host threads"
-        line.update({"value": cpu["value"], "ms_per_step": cpu["ms_per_pass"], "kind": "port", "cpu_baseline": cpu,
-                     "e2e": {"value": cpu["value"], "unit": "GFLOPS", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-                     "gpu_launches": 0, "config": cfg})
+    coo = padded_coo(g)
+    steps = max(1, args.steps)
+    warm = max(1, min(args.warmup, 2))
+    for _ in range(warm):
+        time_reference_kernels(lib, g, Bs, coo)
+    kernel_ms, e2e_ms = [], []
+    launches = 200
+    for _ in range(steps):
+        rec, launches = time_reference_kernels(lib, g, Bs, coo)
+        kernel_ms.append(sum(rec[K]["lbspmm_ms"] for K in KS))
+        # one product end to end = the reference's upload + one launch of its loop + its download
+        e2e_ms.append(sum(rec[K]["lbspmm_upload_ms"] + rec[K]["lbspmm_ms"] + rec[K]["lbspmm_download_ms"]
+                          for K in KS))
+    k_ms, e_ms = statistics.mean(kernel_ms), statistics.mean(e2e_ms)
+    r, c, v = coo
+    h2d = sum(len(r) * 12 + g["N"] * K * 4 for K in KS)
+    d2h = sum(g["M"] * K * 4 for K in KS)
+    cfg["reference_entry"] = ("LBSpMM (HP-SpMM, spmm/mm/spmm_kernel.cu:733-768) on one GPU: per product "
+                              "Matrix::to(kCUDA) uploads from pageable memory, %d launches timed by its own "
+                              "GpuTimer, C read back; kernels compiled unmodified for sm_100a" % launches)
+    cfg["per_k_ms"] = {str(K): rec[K]["lbspmm_ms"] for K in KS}
+    cfg["per_k_upload_ms"] = {str(K): rec[K]["lbspmm_upload_ms"] for K in KS}
+    cfg["per_k_download_ms"] = {str(K): rec[K]["lbspmm_download_ms"] for K in KS}
+    line.update({"value": flops / (k_ms * 1e-3) / 1e9, "ms_per_step": k_ms, "kind": "reference",
+                 "e2e": {"value": flops / (e_ms * 1e-3) / 1e9, "unit": "GFLOPS", "h2d_bytes_per_step": int(h2d),
+                         "d2h_bytes_per_step": int(d2h), "ms_per_step": e_ms,
+                         "how": "the reference's own upload (Matrix::to(kCUDA), pageable host memory) + the mean "
+                                "of its %d timed launches + its own download (Matrix::to(kCPU)), per product" % launches},
+                 "gpu_launches": int(launches * len(KS) * steps), "config": cfg})
     print(json.dumps(line))
 
 

@@ -160,6 +160,19 @@ def test_torch_front_end_registers_and_has_no_cpu_path(pkg):
         del ops._layers[-1]
 
 
+def test_reference_arm_without_the_reference(tmp_path):
+    """`bench.py --impl reference` stands for the reference's own kernels or says that they are unavailable: no other
+    program's figure goes out under its name."""
+    import json
+    import subprocess
+    import sys
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="")
+    res = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference"], env=env, cwd=tmp_path,
+                         stdout=subprocess.PIPE, timeout=300, text=True)
+    line = json.loads(res.stdout.strip().splitlines()[-1])
+    assert res.returncode == 0 and line.pop("unavailable") and line == {"impl": "reference"}
+
+
 def test_row_order_reader(pkg, tmp_path):
     """One line of M row ids (the reference's .cugraph_reorder file); anything but a permutation is refused."""
     rng = np.random.default_rng(5)
