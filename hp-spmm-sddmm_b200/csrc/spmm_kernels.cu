@@ -679,11 +679,17 @@ int32_t planless_chunk_nnz(int64_t K, int64_t nnz, const hpspmm_opts* opts) {
 //     uniform K=64  34.3>27.5 / 21.5>18.5 / 18.7>16.4 35.7>36.5 / 22.1>22.3 / 18.9>20.0 38.5>38.7 / 22.0>23.1 / 19.4>21.0
 //     uniform K=128 65.9>49.1 / 33.1>26.1 / 29.8>25.2 59.2>58.6 / 32.0>31.3 / 28.1>28.5 62.2>61.4 / 32.6>32.0 / 29.3>29.3
 //     skewed  K=64  55.9>30.9 / 36.7>24.2 / 30.2>24.0 62.2>32.4 / 37.5>26.9 / 29.8>24.4 55.6>31.6 / 38.0>25.2 / 30.6>25.3
+//   below 32 columns rows of even length gain nothing by records before 41 per SM:
+//   chunks per SM   33                                36                                40
+//     uniform K=1   15.3>16.9 /  9.0>11.1 /  7.4>11.1 16.7>18.0 / 10.4>12.2 /  7.6>11.1 18.2>19.1 / 10.8>12.7 /  8.2>11.1
+//     uniform K=8   21.4>21.4 / 12.2>12.9 / 10.3>11.7 22.3>22.3 / 12.9>13.5 / 10.5>12.1 23.3>23.1 / 13.2>13.6 / 11.2>12.5
+//     uniform K=24  24.2>23.7 / 15.8>16.0 / 13.1>14.4 25.1>24.9 / 16.5>16.5 / 13.5>14.6 26.4>25.8 / 17.1>17.1 / 14.1>15.2
+//     skewed  K=8   48.6>25.1 / 30.4>21.3 / 23.4>18.3 51.7>27.3 / 32.1>21.6 / 23.7>19.6 51.1>28.7 / 33.6>21.4 / 24.7>18.8
 // (between 37 and 40 the records' product is in its second wave, and uniform rows of 16 and more entries are up to 8 % behind
-// at K <= 64; everything else is ahead there.)  Chunks of 64: 335 K entries (35 per SM), power-law K = 64 20.6 -> 22.1; 300 K
+// at K = 32 to 64; everything else is ahead there.)  Chunks of 64: 335 K entries (35 per SM), power-law K = 64 20.6 -> 22.1; 300 K
 // (32 per SM), uniform 10.0 -> 13.4.  With very many empty rows between the entries the list pays for itself.
-bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t nnz, int64_t n_chunks, int32_t S) {
-  return n_chunks <= ctx->sm_count * (S < 128 ? 40ll : 32ll) && M <= 8 * nnz;
+bool searches_for_chunks(const hpspmm_ctx* ctx, int64_t M, int64_t K, int64_t nnz, int64_t n_chunks, int32_t S) {
+  return n_chunks <= ctx->sm_count * (S < 128 || K < 32 ? 40ll : 32ll) && M <= 8 * nnz;
 }
 
 // Up to here a search costs little enough to do without the records where there is no room for them: a call that is
@@ -891,7 +897,7 @@ int hpspmm_spmm_csr_f32(hpspmm_ctx* ctx, const hpspmm_plan* plan, int64_t M, int
   }
   const int32_t S = planless_chunk_nnz(K, nnz, opts);
   const int64_t n_chunks = (nnz + S - 1) / S;
-  bool search = searches_for_chunks(ctx, M, nnz, n_chunks, S);
+  bool search = searches_for_chunks(ctx, M, K, nnz, n_chunks, S);
   planless_layout lay(M, K, n_chunks, search);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
@@ -976,7 +982,7 @@ static int host_products_pipelined(hpspmm_ctx* ctx, int64_t M, int64_t N, int64_
       const int64_t w = slabs[i].width;
       const int32_t S = planless_chunk_nnz(w, nnz, opts);
       const int64_t n_chunks = (nnz + S - 1) / S;
-      const bool search = searches_for_chunks(ctx, M, nnz, n_chunks, S);
+      const bool search = searches_for_chunks(ctx, M, w, nnz, n_chunks, S);
       const planless_layout lay(M, w, n_chunks, search);
       need = lay.bytes > need ? lay.bytes : need;
       const planless_layout small(M, w, n_chunks, search || may_search_for_chunks(ctx, M, nnz, n_chunks));

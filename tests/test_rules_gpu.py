@@ -275,13 +275,14 @@ def test_one_pass_gradients_of_many_entries(gpu_ctx, pkg):
         assert _one_pass(gpu_ctx, pkg, nnz + 1, even, list(beyond), M) == beyond
 
 
-@pytest.mark.parametrize("K", [20, 100, 256])
+@pytest.mark.parametrize("K", [1, 31, 32, 100, 256])
 def test_planless_products_on_both_sides_of_the_search_line(gpu_ctx, pkg, oracle, K):
     """One launch that searches row_ptr for its chunks, or three that build records first: up to 40 chunks per SM of fewer
-    than 128 entries, up to 32 of more."""
+    than 128 entries or below 32 columns, else up to 32."""
     ctx, N = gpu_ctx, 2000
     sms = ctx.lib.hpspmm_ctx_sm_count(ctx.handle)
     for S, line in ((32, 40), (96, 40), (128, 32), (160, 32)):
+        line = 40 if K < 32 else line
         for n_chunks in (17 * sms, line * sms, line * sms + 1):
             rng = np.random.default_rng(S)
             nnz = n_chunks * S - 5
