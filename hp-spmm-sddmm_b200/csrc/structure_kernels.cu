@@ -645,32 +645,26 @@ template <bool PIECES>
 __global__ void __launch_bounds__(kThreads)
 row_tile_count_kernel(int M, int tile, const chunk_size cs, const int* __restrict__ row_ptr, int* __restrict__ counts,
                       int* __restrict__ clear, int64_t n_clear) {
-  __shared__ int part[kThreads / 32];
+  __shared__ int2 part[kThreads / 32];
   hpspmm::chain_grid();
   for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n_clear; i += (int64_t)gridDim.x * kThreads) clear[i] = 0;
   const int64_t r0 = (int64_t)blockIdx.x * tile;
-  int total = 0, pieces = 0;
-  for (int i = 0; i < tile && r0 + i < M; i += kThreads) {
-    const int64_t r = r0 + i + threadIdx.x;
-    int s = 0, e = 0;
-    if (r < M) {
-      s = hpspmm::ld_chained(row_ptr + r);
-      e = hpspmm::ld_chained(row_ptr + r + 1);
-    }
-    total += __syncthreads_count(e > s);
+  const int n = (int)(M - r0 < tile ? M - r0 : tile);
+  int total = 0, pieces = 0;   // of this thread's rows: no barrier between the loads
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += kThreads) {
+    const int s = hpspmm::ld_chained(row_ptr + r0 + i), e = hpspmm::ld_chained(row_ptr + r0 + i + 1);
+    total += e > s ? 1 : 0;
     if (PIECES) pieces += row_cuts(s, e, cs).pieces();
   }
-  if (PIECES) {
-    pieces = __reduce_add_sync(0xffffffffu, pieces);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = pieces;
-    __syncthreads();
-  }
+  total = __reduce_add_sync(0xffffffffu, total);
+  if (PIECES) pieces = __reduce_add_sync(0xffffffffu, pieces);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_int2(total, pieces);
+  __syncthreads();
   if (threadIdx.x == 0) {
+    for (int w = 1; w < kThreads / 32; ++w) total += part[w].x, pieces += part[w].y;
     counts[blockIdx.x] = total;
-    if (PIECES) {
-      for (int w = 1; w < kThreads / 32; ++w) pieces += part[w];
-      counts[gridDim.x + blockIdx.x] = pieces;
-    }
+    if (PIECES) counts[gridDim.x + blockIdx.x] = pieces;
   }
 }
 
@@ -691,9 +685,13 @@ __device__ __forceinline__ void write_chunk_record(int c, int slot, int before, 
   }
 }
 
-// Bound by latency (4 M entries in 250 K rows: 977 blocks, 5.7 us, 4.2 MB): loads are issued before they are needed, chunks
-// are spread over the threads of a block (the longest rows of a power-law graph often stand side by side) and divided by
-// multiplication.  16 M entries in 1 M rows: 16.5 us for matrix order with a warp per long row, 13.7 like this.
+// Bound by latency (4 M entries in 250 K rows: 977 blocks, 5.7 us, 4.2 MB): loads are issued before they are needed, those of
+// the next 256 rows while these are worked on; where rows are longer than two chunks (the longest rows of a power-law graph
+// often stand side by side) the chunks are spread over the threads of a block, elsewhere a row writes its own records and a
+// barrier and the tables in shared memory are saved; chunks are divided by multiplication.
+// Both kernels, matrix order with a warp per long row / a thread a chunk everywhere / this, under ncu, us:
+//   uniform, rows of 4 entries, 1 M rows 17.2 / 21.5 / 16.5, 2.25 M rows 28.9 / 40.3 / 26.8, 8 M rows 82 / 119 / 76;  of 16, 1 M rows 17.7 / 21.7 / 17.0
+//   power-law, of 4, 2.25 M rows 29.0 / 36.5 / 26.7;  of 16, 250 K rows 11.8 / 10.3 / 10.4, 1 M rows 22.7 / 21.2 / 17.1
 //
 // PIECES: the chunks that lie inside one row come after all others, both in matrix order; else all in matrix order.
 // Chunk c = lo + i of a row (row_cuts) with `h` pieces in the rows above it is a piece for i < n - 1, the h + i-th of the
@@ -708,8 +706,9 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
                      const int* __restrict__ counts, int2* __restrict__ nz, int4* __restrict__ rec,
                      const hpspmm_structure_tables t) {
   constexpr int kWarpsHere = kThreads / 32;
-  __shared__ int part[kWarpsHere], part_h[kWarpsHere], part_all[kWarpsHere];
-  __shared__ int bound[kThreads + 1], ranks[kThreads], above[kThreads];   // of the rows at hand: first entries, rank, pieces above
+  // two sets, used in turn: a warp may write the next rows' while another still reads these
+  __shared__ int parts[2][kWarpsHere], parts_h[2][kWarpsHere], part_all[kWarpsHere];
+  __shared__ int bounds[2][kThreads + 1], all_ranks[2][kThreads], all_above[2][kThreads];   // first entries, rank, pieces above
   hpspmm::chain_grid();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * tile;
@@ -737,19 +736,21 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
     before_h = __reduce_add_sync(0xffffffffu, before_h);
     all_h = __reduce_add_sync(0xffffffffu, all_h);
   }
-  if (lane == 0) part[warp] = before, part_h[warp] = before_h, part_all[warp] = all_h;
+  if (lane == 0) parts[1][warp] = before, parts_h[1][warp] = before_h, part_all[warp] = all_h;
   __syncthreads();
   int base = 0, base_h = 0, whole = n_chunks;   // whole: chunks that are no pieces
 #pragma unroll
   for (int w = 0; w < kWarpsHere; ++w) {
-    base += part[w];
-    if (PIECES) base_h += part_h[w], whole -= part_all[w];
+    base += parts[1][w];
+    if (PIECES) base_h += parts_h[1][w], whole -= part_all[w];
   }
-  __syncthreads();
 
-  for (int i0 = 0; i0 < tile && r0 + i0 < M; i0 += kThreads) {
+  int turn = 0;
+  for (int i0 = 0; i0 < tile && r0 + i0 < M; i0 += kThreads, turn ^= 1) {
     const int64_t r = r0 + i0 + threadIdx.x;
-    if (i0 > 0) s = row_start(r), e = row_start(r + 1);
+    int next_s = 0, next_e = 0;   // of the next rows, in flight meanwhile
+    if (i0 + kThreads < tile) next_s = row_start(r + kThreads), next_e = row_start(r + kThreads + 1);
+    int *part = parts[turn], *part_h = parts_h[turn], *bound = bounds[turn], *ranks = all_ranks[turn], *above = all_above[turn];
     const bool has = e > s;
     const row_cuts cuts(s, e, cs);
     const unsigned m = __ballot_sync(0xffffffffu, has);
@@ -769,7 +770,7 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
       h = 0;
     }
     if (lane == 0) part[warp] = __popc(m);
-    __syncthreads();
+    const bool long_rows = __syncthreads_or(cuts.n > 2);
     int rank = base + __popc(m & ((1u << lane) - 1u));
 #pragma unroll
     for (int w = 0; w < kWarpsHere; ++w) {
@@ -780,11 +781,13 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
         base_h += part_h[w];
       }
     }
-    if (threadIdx.x == 0) bound[0] = s;
-    bound[threadIdx.x + 1] = e;
-    ranks[threadIdx.x] = rank;
-    above[threadIdx.x] = h;
-    __syncthreads();
+    if (long_rows) {
+      if (threadIdx.x == 0) bound[0] = s;
+      bound[threadIdx.x + 1] = e;
+      ranks[threadIdx.x] = rank;
+      above[threadIdx.x] = h;
+      __syncthreads();
+    }
     if (has) {
       nz[rank] = make_int2((int)r, e);
       if (t.nz_id) {
@@ -797,9 +800,20 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
         if (t.chunk_start) t.chunk_start[n_chunks] = nnz;
       }
     }
-    // a thread a chunk
-    const int first = bound[0], end = bound[kThreads];
-    const row_cuts all(first, end, cs);
+    // the record of chunk c = own.lo + i of a row
+    auto write = [&](const row_cuts& own, int i, int row_s, int row_e, int64_t row, int rank, int h) {
+      const int c = own.lo + i;
+      int slot = c, prev = c - 1;
+      if (PIECES) {
+        slot = i < own.n - 1 ? whole + h + i : c - h - (own.n - 1);
+        prev = i > 0 ? whole + h + i - 1 : c - 1 - h;
+      }
+      write_chunk_record(c, slot, prev, cs.S, n_chunks, row_s, row_e, (int)row, rank, rec, t);
+    };
+    // a row that holds one cut or two writes their records by itself; with longer rows, a thread a chunk
+    if (!long_rows)
+      for (int i = 0; i < cuts.n; ++i) write(cuts, i, s, e, r, rank, h);
+    const row_cuts all(long_rows ? bound[0] : 0, long_rows ? bound[kThreads] : 0, cs);
 #pragma unroll 4
     for (int k = threadIdx.x; k < all.n; k += kThreads) {
       const int c = all.lo + k;
@@ -808,15 +822,9 @@ row_tile_list_kernel(int M, int nnz, int tile, const chunk_size cs, int n_chunks
       for (int d = kThreads / 2; d >= 1; d >>= 1)
         if (bound[at + d] <= c * cs.S) at += d;
       const row_cuts own(bound[at], bound[at + 1], cs);
-      const int i = c - own.lo, h = above[at];
-      int slot = c, prev = c - 1;
-      if (PIECES) {
-        slot = i < own.n - 1 ? whole + h + i : c - h - (own.n - 1);
-        prev = i > 0 ? whole + h + i - 1 : c - 1 - h;
-      }
-      write_chunk_record(c, slot, prev, cs.S, n_chunks, bound[at], bound[at + 1], (int)(r0 + i0 + at), ranks[at], rec, t);
+      write(own, c - own.lo, bound[at], bound[at + 1], r0 + i0 + at, ranks[at], above[at]);
     }
-    __syncthreads();
+    s = next_s, e = next_e;
   }
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x < kNzPad) {
     // sentinels after the last row: never a row of C, an end no entry reaches; a warp reads 32 rows at once

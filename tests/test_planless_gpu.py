@@ -423,3 +423,38 @@ def test_products_behind_an_event_join(pkg, oracle, captured):
             del graph
         for p in plans:
             ctx.plan_destroy(p)
+
+
+@pytest.mark.parametrize("M", [262_145, 900_001])
+@pytest.mark.parametrize("chunk", [32, 160])
+def test_tiles_of_several_passes(gpu_ctx, pkg, oracle, M, chunk):
+    """Matrices whose tiles of rows the builder walks in several passes: passes with rows longer than two chunks, with
+    shorter ones only, and with none that holds entries, in turn; records with and without a plan."""
+    ctx, K, N = gpu_ctx, 4, 500
+    rng = np.random.default_rng(M + chunk)
+    degrees = rng.integers(0, 4 if chunk == 32 else 12, M)
+    zone = np.arange(M) // 256
+    degrees[zone % 5 == 2] = 0
+    at = np.flatnonzero((zone % 5 == 4) & (np.arange(M) % 64 == 7))[::23]
+    degrees[at] = rng.choice([2 * chunk, 2 * chunk + 1, 3 * chunk, 7 * chunk - 1], size=len(at))
+    at = np.flatnonzero((zone % 5 == 1) & (np.arange(M) % 32 == 3))
+    degrees[at] = rng.integers(1, 2 * chunk + 1, size=len(at))[: len(at)] // 4
+    rp = np.concatenate([[0], np.cumsum(degrees)]).astype(np.int32)
+    nnz = int(rp[-1])
+    assert nnz > 40 * 160 * chunk           # records also without a plan
+    ci, v = rng.integers(0, N, nnz).astype(np.int32), rng.uniform(-1, 1, nnz).astype(np.float32)
+    B, X = (pkg.host_fill_uniform(n * K, M % 1000, j, -1.0, 1.0).reshape(n, K) for j, n in ((1, N), (2, M)))
+    bufs = [ctx.upload(a) for a in (rp, ci, v, B, X)]
+    d_C, d_o = ctx.alloc((M, K), np.float32), ctx.alloc((nnz,), np.float32)
+    opts = pkg.Opts(chunk_nnz=chunk)
+    plan = ctx.plan_create(M, nnz, bufs[0], K, opts, N=N, col_idx=bufs[1])
+    for p in (None, plan):
+        ctx.fill(d_C, M * K, 7.0)
+        ctx.spmm_csr(M, N, K, nnz, *bufs[:4], d_C, plan=p, opts=opts)
+        check_against_f64(d_C.to_host(), *oracle.spmm_f64(rp, ci, v, B), "product, plan=%s" % (p is not None))
+        ctx.fill(d_o, nnz, 7.0)
+        ctx.sddmm_csr(M, N, K, nnz, bufs[0], bufs[1], bufs[4], bufs[3], d_o, plan=p, opts=opts)
+        check_against_f64(d_o.to_host(), *oracle.sddmm_f64(rp, ci, X, B), "SDDMM, plan=%s" % (p is not None))
+    ctx.plan_destroy(plan)
+    for b in bufs + [d_C, d_o]:
+        b.free()
