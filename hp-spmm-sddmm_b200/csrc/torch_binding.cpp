@@ -3,7 +3,6 @@
 // A training step on a small graph is three or four launches of a few microseconds each; with the operators and the
 // autograd formula in Python the host took 160 us to issue them.  Arithmetic stays in libhpspmm.so, which this file
 // calls through the C ABI; PyTorch supplies memory, streams and the autograd tape.
-#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -66,7 +65,8 @@ Tensor require_weights(const Tensor& t, const Entry& e, const at::Device& device
 // A captured call always records the gather: its graph may be replayed after the weights changed in place, or after a call
 // with others.  From then on nobody knows what the transpose holds, and every call gathers.
 void sync_values(Entry& e, const Tensor& vals, cudaStream_t stream, Tensor& old) {
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) e.in_graph = true;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) e.in_graph = true;
   const int64_t version = vals.is_inference() || e.in_graph ? -1 : (int64_t)vals._version();
   if (version >= 0 && e.vals.defined() && vals.const_data_ptr() == e.vals.const_data_ptr() && version == e.vals_version)
     return;
