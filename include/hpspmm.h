@@ -284,7 +284,8 @@ HPSPMM_API int hpspmm_csr_transpose(hpspmm_ctx* ctx, int64_t M, int64_t N, int64
  *   backward           both gradients at once for weights given in A's order, in one pass over the transpose;
  *                      HPSPMM_ERR_UNSUPPORTED, with no gradient computed, where one launch does not cover the rows of
  *                      dC (more than 256 columns, 128 where rows are only 4-byte aligned) or would be slower than two
- *                      (matrices whose weights fill the L2 cache; rows of uneven length with few entries): call the other two then.  The first call of a width
+ *                      (matrices whose weights fill the L2 cache; rows of uneven length with few entries; small calls are
+ *                      refused under capture only): call the other two then.  The first call of a width
  *                      class may have built that class's plans by then, as any product of the class does
  * The best chunk size depends on K, so the handle keeps one pair of plans per width class
  * (K <= 32, K <= 64, wider).  create builds the pair for max_K and synchronises the stream;
